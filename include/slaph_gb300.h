@@ -429,21 +429,17 @@ int slaph_engine_timings(const slaph_engine *eng, double *out, int n);
  * device up front, and latency-critical loops that cannot afford the device
  * synchronisation cudaMalloc/cudaFree may imply.  No counterpart in the
  * reference (it has no GPU code); the result equals slaph_vdaggerv_fetch of
- * slaph_vdaggerv_build(SLAPH_FP64).
+ * slaph_vdaggerv_build(SLAPH_FP64) to rounding (the two may sum the lattice in
+ * different orders).
  *   V_t:  DEVICE pointer, 3*L^3 x nev complex, column-major (one timeslice)
  *   out:  DEVICE pointer, nev x nev complex, column-major
  *   momentum: host array of 3 ints, read during the call and handed to the
  *             device as kernel arguments (the GPU reads no host memory);
  *   stream:   a cudaStream_t (NULL = legacy)
- * Allocates nothing: the phase table lives in a static device array of
- * 4 MiB + 256 B, which every GPU that loads the library holds until the
- * process exits, so L^3 may not exceed 262144 (64^3); larger lattices (and
- * any single extent above that) are rejected with SLAPH_ERR_ARG.  The first call on a device looks up that
- * array's device address (once per device); make that first call before any
- * stream capture.  The work is enqueued on `stream` and not waited for.
- * Every call shares the one array: calls whose work overlaps on the GPU (other
- * streams, or other host threads) race on it and must be serialised by the
- * caller. */
+ * Allocates nothing and shares nothing between calls.  L^3 may not exceed
+ * 262144 (64^3, the static scratch limit of the entry point's first form);
+ * larger lattices (and any single extent above that) are rejected with
+ * SLAPH_ERR_ARG.  The work is enqueued on `stream` and not waited for. */
 int slaph_vdaggerv_noalloc(const slaph_dims *dims, const double *V_t, const int32_t *momentum,
                            double *out, void *stream);
 

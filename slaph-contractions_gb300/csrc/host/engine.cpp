@@ -396,6 +396,12 @@ void Engine::vdaggerv_build(int precision) {
                            U_.as<double2>(), W_.as<double2>(), phase_unit_.as<longlong2>(),
                            unit_op_.as<int32_t>()};
   }
+  std::vector<dev::VdvFamily> families;  // of the FP64 build
+  if (precision == SLAPH_FP64) {
+    std::vector<int32_t> mom;
+    for (int32_t id : computed) mom.insert(mom.end(), ops_[id].momentum, ops_[id].momentum + 3);
+    families = dev::vdv_families(computed, mom, dims_.Lx, dims_.Ly, dims_.Lz, true);
+  }
   int32_t n_gemm = 0;     // GEMM launches of the whole build
   int64_t batch_fit = 1;  // timeslices per GEMM launch that the scratch holds
   if (precision == SLAPH_MIXED) {
@@ -493,8 +499,9 @@ void Engine::vdaggerv_build(int precision) {
     } else {
       for (int32_t t = t0; t < t0 + nt; ++t)
         if (ready[t]) SLAPH_CK(cudaStreamWaitEvent(stream_, ready[t], 0));
-      launch(dev::vdaggerv_fp64(vdv_.as<double2>(), Vb, phase_.as<double2>(), list.as<int32_t>(),
-                                n_comp, t0, nt, geo_, stream_, v_t0),
+      launch(dev::vdaggerv_fp64(vdv_.as<double2>(), Vb, families.data(),
+                                static_cast<int32_t>(families.size()), t0, nt, geo_, stream_,
+                                v_t0),
              "vdaggerv_fp64");
     }
     // Displaced operators of the FP64 build: W = D(V_t) step by step, then

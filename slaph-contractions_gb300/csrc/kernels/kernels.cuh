@@ -8,6 +8,8 @@
 
 #include <cstdint>
 
+#include "vdv_families.hpp"
+
 namespace slaph {
 namespace dev {
 
@@ -80,13 +82,14 @@ cudaError_t vdaggerv_fp64_w(double2 *vdv, double2 const *V, double2 const *W,
 cudaError_t momenta(double2 *phase, int32_t const *mom, int32_t n_ops, Geometry g,
                     cudaStream_t stream);
 
-// VdaggerV[vdv code 2*op][t] = V_t^H diag(phase[op] per site) V_t for every op
-// in ops[0..n) (src/OperatorFactory.cpp:292-300), FP64.  V: consecutive
-// timeslices [t][nev][dim_row] (each column-major), V[0] holding timeslice
-// v_t0 (0: all Lt resident; a ring slot otherwise).  vdv: [2*n_ops][Lt][nev][nev].
-cudaError_t vdaggerv_fp64(double2 *vdv, double2 const *V, double2 const *phase,
-                          int32_t const *ops, int32_t n, int32_t t0, int32_t nt, Geometry g,
-                          cudaStream_t stream, int32_t v_t0 = 0);
+// VdaggerV[vdv code 2*op][t] = V_t^H diag(e^{-ip.x}) V_t for the operators of
+// the families fam[0..n_fam) (host array, vdv_families.hpp;
+// src/OperatorFactory.cpp:292-300), FP64.  V: consecutive timeslices
+// [t][nev][dim_row] (each column-major), V[0] holding timeslice v_t0 (0: all Lt
+// resident; a ring slot otherwise).  vdv: [2*n_ops][Lt][nev][nev].
+cudaError_t vdaggerv_fp64(double2 *vdv, double2 const *V, VdvFamily const *fam, int32_t n_fam,
+                          int32_t t0, int32_t nt, Geometry g, cudaStream_t stream,
+                          int32_t v_t0 = 0);
 // Split-BF16 tensor-core VdaggerV (vdv_tc.cu): same result as vdaggerv_fp64
 // to ~1e-13 relative.  scratch: device buffer of at least
 // vdaggerv_tc_scratch_bytes(g, n, batch) bytes, where batch timeslices are

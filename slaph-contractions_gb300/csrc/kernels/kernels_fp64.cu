@@ -83,80 +83,7 @@ __global__ void momenta_kernel(double2 *phase, int32_t const *mom, int32_t n_ops
 }
 
 // ---------------------------------------------------------------- VdaggerV
-// OperatorFactory::build_vdaggerv, src/OperatorFactory.cpp:292-300:
-// vdv = V^H (diag(mom) V), mom(x) = phase[x / 3].  64 x 64 output tile per
-// CTA, 16 rows of V per step, 4 x 4 outputs per thread.
-constexpr int VT = 64, VK = 16;
-
-// kW: B = W (a displaced copy of V_t, one operator and timeslice per launch:
-// ops[0] is the operator, t0 the timeslice) instead of diag(phase) V_t.
-template <bool kW>
-__global__ void __launch_bounds__(256) vdv_fp64_kernel(double2 *vdv, double2 const *V,
-                                                       double2 const *phase,
-                                                       int32_t const *ops, int32_t t0,
-                                                       Geometry g, double2 const *W,
-                                                       int32_t v_t0) {
-  __shared__ double2 As[VK][VT];
-  __shared__ double2 Bs[VK][VT];
-  int const nev = g.nev;
-  int64_t const dim_row = g.dim_row;
-  int64_t const vol = dim_row / 3;
-  int const tiles = (nev + VT - 1) / VT;
-  int const i0 = (blockIdx.x % tiles) * VT, j0 = (blockIdx.x / tiles) * VT;
-  int const op = ops[blockIdx.y];
-  int const t = t0 + blockIdx.z;
-  int const tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-  double2 const *Vt = V + static_cast<int64_t>(t - v_t0) * nev * dim_row;
-  double2 const *ph = kW ? nullptr : phase + static_cast<int64_t>(op) * vol;
-  double2 acc[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = make_double2(0, 0);
-
-  for (int64_t x0 = 0; x0 < dim_row; x0 += VK) {
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      int const k = tid + 256 * q;
-      int const xx = k % VK, ii = k / VK;
-      int64_t const x = x0 + xx;
-      int const i = i0 + ii, j = j0 + ii;
-      double2 a = make_double2(0, 0), b = make_double2(0, 0);
-      if (x < dim_row) {
-        if (i < nev) a = Vt[static_cast<int64_t>(i) * dim_row + x];
-        if (j < nev)
-          b = kW ? W[static_cast<int64_t>(j) * dim_row + x]
-                 : cmul(ph[x / 3], Vt[static_cast<int64_t>(j) * dim_row + x]);
-      }
-      As[xx][ii] = a;
-      Bs[xx][ii] = b;
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int kk = 0; kk < VK; ++kk) {
-      double2 a[4], b[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        a[q] = As[kk][ty + 16 * q];
-        b[q] = Bs[kk][tx + 16 * q];
-      }
-#pragma unroll
-      for (int p = 0; p < 4; ++p)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) cfmac(acc[p][q], a[p], b[q]);
-    }
-    __syncthreads();
-  }
-  double2 *out = vdv + (static_cast<int64_t>(2 * op) * g.Lt + t) * nev * nev;
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      int const i = i0 + ty + 16 * p, j = j0 + tx + 16 * q;
-      if (i < nev && j < nev) out[i + static_cast<int64_t>(nev) * j] = acc[p][q];
-    }
-}
-
+// (the build itself: vdv_fp64.cu, vdv_tc.cu)
 __global__ void vdv_identity_kernel(double2 *vdv, int32_t op, Geometry g) {
   int64_t const blk = static_cast<int64_t>(g.nev) * g.nev;
   int64_t const k = gidx();
@@ -582,16 +509,6 @@ cudaError_t momenta(double2 *phase, int32_t const *mom, int32_t n_ops, Geometry 
   return cudaGetLastError();
 }
 
-cudaError_t vdaggerv_fp64(double2 *vdv, double2 const *V, double2 const *phase,
-                          int32_t const *ops, int32_t n, int32_t t0, int32_t nt, Geometry g,
-                          cudaStream_t stream, int32_t v_t0) {
-  if (n == 0 || nt == 0) return cudaSuccess;
-  int const tiles = (g.nev + VT - 1) / VT;
-  dim3 grid(tiles * tiles, n, nt);
-  vdv_fp64_kernel<false><<<grid, 256, 0, stream>>>(vdv, V, phase, ops, t0, g, nullptr, v_t0);
-  return cudaGetLastError();
-}
-
 // displace_eigenvectors (src/OperatorFactory.cpp:33-55) for one step on a
 // cubic lattice: W (a copy of V_t) is updated in place line by line, each line
 // of the step's direction in increasing site index as the reference sweeps
@@ -667,15 +584,6 @@ cudaError_t displace(double2 *W, double2 const *U, int32_t dir, int32_t forward,
   if (dir < 0 || dir > 2 || g.Lx != g.Ly || g.Lx != g.Lz) return cudaErrorInvalidValue;
   int64_t const n = static_cast<int64_t>(g.Lx) * g.Lx * g.nev;
   displace_kernel<<<blocks_for(n, 128), 128, 0, stream>>>(W, U, dir, forward, g);
-  return cudaGetLastError();
-}
-
-cudaError_t vdaggerv_fp64_w(double2 *vdv, double2 const *V, double2 const *W,
-                            int32_t const *op, int32_t t, Geometry g, cudaStream_t stream,
-                            int32_t v_t0) {
-  int const tiles = (g.nev + VT - 1) / VT;
-  vdv_fp64_kernel<true><<<dim3(tiles * tiles, 1, 1), 256, 0, stream>>>(vdv, V, nullptr, op, t,
-                                                                       g, W, v_t0);
   return cudaGetLastError();
 }
 

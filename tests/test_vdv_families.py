@@ -1,0 +1,136 @@
+"""Momentum families of VdaggerV (csrc/kernels/vdv_families.hpp): on the CPU,
+that every family reproduces the momenta it stands for; on the GPU, that the
+builds agree with the plain matrix product for momenta, lattices and
+eigenvector counts at the edges of the kernels' tiles and planes."""
+from __future__ import annotations
+
+import ctypes as C
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import PKG
+
+WRAPPER = r"""
+#include "vdv_families.hpp"
+#include <cstring>
+extern "C" int families(int n, const int *ids, const int *mom, int Lx, int Ly, int Lz,
+                        int sheared, int *out, int cap) {
+  std::vector<int32_t> i(ids, ids + n), m(mom, mom + 3 * n);
+  auto f = slaph::dev::vdv_families(i, m, Lx, Ly, Lz, sheared != 0);
+  int const w = sizeof(slaph::dev::VdvFamily) / 4;
+  if (static_cast<int>(f.size()) * w > cap) return -1;
+  std::memcpy(out, f.data(), f.size() * sizeof(slaph::dev::VdvFamily));
+  return static_cast<int>(f.size());
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def planner(tmp_path_factory):
+    d = tmp_path_factory.mktemp("families")
+    (d / "w.cpp").write_text(WRAPPER)
+    so = d / "families.so"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", f"-I{PKG / 'csrc' / 'kernels'}",
+                    str(d / "w.cpp"), str(PKG / "csrc" / "host" / "vdv_families.cpp"), "-o",
+                    str(so)], check=True)
+    return C.CDLL(str(so)).families
+
+
+def momenta(p2):
+    r = range(-3, 4)
+    ps = [(x, y, z) for x in r for y in r for z in r if x * x + y * y + z * z <= p2]
+    return sorted(ps, key=lambda p: (sum(k * k for k in p), p))
+
+
+def unpack(row):
+    f = dict(axis=row[0], n=row[1], sgn=row[2], sh=row[3:5], w=row[5:8], herm=row[8])
+    f["ops"] = [(row[10 + i], row[13 + i], row[16 + i]) for i in range(row[9])]
+    return f
+
+
+def sites(f, h, L):
+    """Sites of plane h, in the kernels' enumeration."""
+    others = [a for a in range(3) if a != f["axis"]]
+    if f["axis"] == 3:
+        return [(x, y, z) for x in range(L[0]) for y in range(L[1]) for z in range(L[2])]
+    out = []
+    for u in range(L[others[0]]):
+        for v in range(L[others[1]]):
+            x = [0, 0, 0]
+            x[others[0]], x[others[1]] = u, v
+            x[f["axis"]] = int(f["sgn"] * (h - f["sh"][0] * u - f["sh"][1] * v)) % f["n"]
+            out.append(tuple(x))
+    return out
+
+
+@pytest.mark.parametrize("sheared", [0, 1])
+@pytest.mark.parametrize("L", [(4, 4, 4), (5, 5, 5), (3, 3, 3), (8, 8, 8), (4, 6, 5), (8, 2, 2),
+                               (1, 9, 7)])
+@pytest.mark.parametrize("p2", [0, 1, 3, 5, 9])
+def test_families_reproduce_their_momenta(planner, L, p2, sheared):
+    moms = momenta(p2)
+    ids = list(range(3, 3 + len(moms)))
+    out = (C.c_int * 20000)()
+    n = planner(len(ids), (C.c_int * len(ids))(*ids),
+                (C.c_int * (3 * len(ids)))(*[k for p in moms for k in p]), *L, sheared, out, 20000)
+    assert n > 0
+    rows = np.array(out[:19 * n]).reshape(n, 19)
+    seen = []
+    for f in map(unpack, rows):
+        assert 1 <= len(f["ops"]) <= 3
+        if f["herm"]:
+            assert not any(f["w"])
+            assert all(dag == 0 for _, _, dag in f["ops"])
+        visited = []
+        for h in range(f["n"]):
+            for x in sites(f, h, L):
+                visited.append(x)
+                inner = sum(w * c / l for w, c, l in zip(f["w"], x, L))
+                for op, k, dag in f["ops"]:
+                    p = moms[op - 3]
+                    want = sum(q * c / l for q, c, l in zip(p, x, L))
+                    have = inner + k * h / f["n"]
+                    d = (want + have if dag else want - have)
+                    assert abs(d - round(d)) < 1e-12
+        assert sorted(visited) == [(x, y, z) for x in range(L[0]) for y in range(L[1])
+                                   for z in range(L[2])]
+        seen += [op for op, _, _ in f["ops"]]
+    assert sorted(seen) == ids
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("L,nev,p2", [
+    ((4, 4, 4), 1, 4), ((4, 4, 4), 33, 9), ((3, 3, 3), 16, 2), ((5, 5, 5), 31, 5),
+    ((7, 7, 7), 65, 3), ((6, 6, 6), 80, 4), ((9, 9, 9), 2, 1), ((4, 6, 5), 34, 3),
+    ((2, 8, 3), 20, 2), ((8, 2, 2), 11, 1), ((1, 9, 7), 17, 3), ((11, 11, 11), 97, 3)])
+def test_build_matches_the_matrix_product(engine_lib, L, nev, p2, precision):
+    from slaph_gb300 import _lib
+    from slaph_gb300.engine import Engine
+    Lt, vol = 3, L[0] * L[1] * L[2]
+    moms = momenta(p2)
+    ops = (_lib.VdvOp * len(moms))()
+    for i, p in enumerate(moms):
+        ops[i].id, ops[i].momentum = i, (C.c_int32 * 3)(*p)
+    eng = Engine(_lib.Dims(Lt, *L, nev, 1, 2, 2))
+    _lib.check(_lib.lib().slaph_engine_set_operators(eng._h, ops, len(moms), -1))
+    rng = np.random.default_rng([nev, p2, *L])
+    V = rng.standard_normal((Lt, nev, 3 * vol, 2)).view(np.complex128)[..., 0]
+    V /= np.linalg.norm(V, axis=2, keepdims=True)
+    for t in range(Lt):
+        eng.set_eigenvectors(t, V[t])
+    eng.vdaggerv_build(precision)
+    x = np.indices(L).reshape(3, -1).repeat(3, axis=1)
+    # Entries of M are sums of 3 vol products of norm at most one in all: FP64
+    # rounds by at most 3 vol units of 2^-53 of that on either side, the split
+    # by 2^-46 of each row's scale per term (at most sqrt(3 vol) scales).
+    tol = 3 * vol * 2.0 ** -52 if precision == 0 else 2 * np.sqrt(3 * vol) * 2.0 ** -44
+    for i, p in enumerate(moms):
+        ph = np.exp(-2j * np.pi * sum(p[a] * x[a] / L[a] for a in range(3)))
+        for t in range(Lt):
+            ref = V[t].conj() @ (ph * V[t]).T
+            err = np.max(np.abs(eng.vdaggerv_fetch(i, t) - ref))
+            assert err < tol, (p, t, err, tol)
+    eng.close()
