@@ -71,14 +71,13 @@ int Engine::read_err_flag() {
 
 namespace {
 
-// Bounds of the split-precision VdaggerV scratch (timeslice batches): at
-// least kTcScratchCap, up to a third of the free device memory and at most
-// kTcScratchMax (larger batches leave less of the last round of tiles idle).
-constexpr size_t kTcScratchCap = 24ULL << 30;
-constexpr size_t kTcScratchMax = 64ULL << 30;
-// Smallest batch capacity of the tensor-core traces (the VdaggerV scratch is
-// reused when it is larger).
-constexpr size_t kTraceScratchMin = 1ULL << 30;
+// Split-precision VdaggerV scratch: as many timeslices as fit, one at least.  A
+// timeslice is n_planes sets of GEMM tiles, so few of them load the chip evenly.
+constexpr size_t kTcScratchCap = 8ULL << 30;
+// Batch capacity of the tensor-core traces and factors (allocated as needed):
+// every batch ends in a partly idle round of tiles, and 1 GiB of operands is
+// only two or three rounds (32^3x64 block pair with |p|^2 <= 2: 42 batches).
+constexpr size_t kTraceScratchMin = 16ULL << 30;
 
 template <typename T>
 void upload(DevBuf &b, std::vector<T> const &v, cudaStream_t s) {
@@ -201,17 +200,59 @@ void Engine::set_operators(slaph_vdv_op const *ops, int32_t n, int32_t index_of_
   if (index_of_unity >= n) throw ArgError("index_of_unity out of range");
   ops_.assign(ops, ops + n);
   index_of_unity_ = index_of_unity;
-  std::vector<int32_t> mom(3 * std::max(n, 1), 0);
-  for (int32_t i = 0; i < n; ++i)
-    for (int c = 0; c < 3; ++c) mom[3 * i + c] = ops[i].momentum[c];
-  upload(mom_dev_, mom, stream_);
-  int64_t const vol = geo_.dim_row / 3;
-  phase_.reserve(sizeof(double2) * vol * std::max(n, 1));
-  launch(dev::momenta(phase_.as<double2>(), mom_dev_.as<int32_t>(), n, geo_, stream_),
-         "momenta");
-  phase_fx_.reserve(sizeof(longlong2) * vol * std::max(n, 1));
-  launch(dev::phase_fixed(phase_fx_.as<longlong2>(), phase_.as<double2>(), vol * n, stream_),
+  // Momentum operators by family and displaced operators (V^H D(V), momentum
+  // not applied) as families of their own.
+  computed_.clear();
+  displaced_.clear();
+  std::vector<int32_t> mom;
+  for (auto const &o : ops_) {
+    if (o.id == index_of_unity_) continue;
+    (o.n_disp > 0 ? displaced_ : computed_).push_back(o.id);
+    if (o.n_disp == 0) mom.insert(mom.end(), o.momentum, o.momentum + 3);
+  }
+  fam_fp64_ = dev::vdv_families(computed_, mom, dims_.Lx, dims_.Ly, dims_.Lz, true,
+                                dev::kVdvFp64Ops);
+  std::vector<dev::VdvFamily> fam = dev::vdv_families(computed_, mom, dims_.Lx, dims_.Ly,
+                                                      dims_.Lz, false, dev::kVdvFamilyOps);
+  bool const planes = dev::vdv_planes_along_x(dims_.Ly, dims_.Lz);
+  dev::VdvTcPlan pl{};
+  pl.n_mom = static_cast<int32_t>(fam.size());
+  pl.n_planes = planes ? dims_.Lx : 1;
+  pl.per = static_cast<int32_t>(geo_.dim_row / pl.n_planes);
+  for (int32_t id : displaced_) {
+    dev::VdvFamily f{};
+    f.axis = planes ? 0 : 3;
+    f.n_planes = pl.n_planes;
+    f.sgn = 1;
+    f.n_ops = 1;
+    f.op[0] = id;
+    fam.push_back(f);
+  }
+  pl.n_fam = static_cast<int32_t>(fam.size());
+  // Phases of the families at the sites of one plane (x = 0).
+  dev::Geometry gp = geo_;
+  if (planes) gp.Lx = 1;
+  std::vector<int32_t> w;
+  for (auto const &f : fam) w.insert(w.end(), f.w, f.w + 3);
+  int64_t const n_ph = static_cast<int64_t>(pl.per / 3) * pl.n_fam;
+  DevBuf w_dev, phase;
+  upload(w_dev, w, stream_);
+  upload(fam_dev_, fam, stream_);
+  phase.reserve(sizeof(double2) * std::max<int64_t>(1, n_ph));
+  phase_fx_.reserve(sizeof(longlong2) * std::max<int64_t>(1, n_ph));
+  roots_.reserve(sizeof(double2) * pl.n_planes);
+  launch(dev::momenta(phase.as<double2>(), w_dev.as<int32_t>(), pl.n_fam, gp, stream_), "momenta");
+  launch(dev::phase_fixed(phase_fx_.as<longlong2>(), phase.as<double2>(), n_ph, stream_),
          "phase_fixed");
+  launch(dev::unit_roots(roots_.as<double2>(), pl.n_planes, stream_), "unit_roots");
+  std::vector<int2> const mn = dev::vdaggerv_tc_tiles(fam, dims_.nev);
+  upload(mn_dev_, mn, stream_);
+  pl.n_mn = static_cast<int32_t>(mn.size());
+  pl.fam = fam_dev_.as<dev::VdvFamily>();
+  pl.phase_fx = phase_fx_.as<longlong2>();
+  pl.roots = roots_.as<double2>();
+  pl.mn = mn_dev_.as<int2>();
+  tc_plan_ = pl;
   vdv_.reserve(sizeof(double2) * 2LL * std::max(n, 1) * dims_.Lt * dims_.nev * dims_.nev);
   SLAPH_CK(cudaStreamSynchronize(stream_));
   ops_set_ = true;
@@ -351,35 +392,20 @@ void Engine::vdaggerv_build(int precision) {
     throw ArgError("unknown precision mode");
   launches_ = 0;
   // Momentum operators (the GEMM paths below) and displaced operators (V^H D(V)).
-  std::vector<int32_t> computed, displaced;
-  for (auto const &o : ops_) {
-    if (o.id == index_of_unity_) continue;
-    (o.n_disp > 0 ? displaced : computed).push_back(o.id);
-  }
+  std::vector<int32_t> const &displaced = displaced_;
+  int32_t const n_all = static_cast<int32_t>(computed_.size() + displaced.size());
   if (!displaced.empty()) {
     bool all = gauge_set_.size() == static_cast<size_t>(dims_.Lt);
     for (char c : gauge_set_) all = all && c;
     if (!all)
       throw StateError("displaced operators need slaph_engine_set_gauge for every timeslice");
   }
-  DevBuf list;
-  int32_t const n_comp = static_cast<int32_t>(computed.size());
   // The split-precision build takes the displaced operators too (after the
   // momentum ones); the FP64 build handles them separately below.
   bool const tc_disp = precision == SLAPH_MIXED && !displaced.empty();
-  std::vector<int32_t> all = computed;
-  if (tc_disp) all.insert(all.end(), displaced.begin(), displaced.end());
-  upload(list, all, stream_);
-  int32_t const n_all = static_cast<int32_t>(all.size());
   dev::VdvDisplaced dd{};
   std::vector<int32_t> d_steps, d_n;
   if (tc_disp) {
-    size_t const sites = static_cast<size_t>(geo_.dim_row / 3);
-    if (phase_unit_.size() < sites * sizeof(longlong2)) {
-      std::vector<longlong2> one(sites, make_longlong2(1LL << 62, 0));
-      upload(phase_unit_, one, stream_);
-      upload(unit_op_, std::vector<int32_t>{0}, stream_);
-    }
     W_.reserve(sizeof(double2) * static_cast<size_t>(geo_.dim_row) * dims_.nev);
     d_steps.assign(2 * dev::kMaxDispSteps * displaced.size(), 0);
     for (size_t k = 0; k < displaced.size(); ++k) {
@@ -393,31 +419,19 @@ void Engine::vdaggerv_build(int precision) {
       }
     }
     dd = dev::VdvDisplaced{static_cast<int32_t>(displaced.size()), d_n.data(), d_steps.data(),
-                           U_.as<double2>(), W_.as<double2>(), phase_unit_.as<longlong2>(),
-                           unit_op_.as<int32_t>()};
-  }
-  std::vector<dev::VdvFamily> families;  // of the FP64 build
-  if (precision == SLAPH_FP64) {
-    std::vector<int32_t> mom;
-    for (int32_t id : computed) mom.insert(mom.end(), ops_[id].momentum, ops_[id].momentum + 3);
-    families = dev::vdv_families(computed, mom, dims_.Lx, dims_.Ly, dims_.Lz, true);
+                           U_.as<double2>(), W_.as<double2>()};
   }
   int32_t n_gemm = 0;     // GEMM launches of the whole build
-  int64_t batch_fit = 1;  // timeslices per GEMM launch that the scratch holds
+  int64_t batch_fit = 1;  // timeslices per GEMM launch
   if (precision == SLAPH_MIXED) {
     int sms = 0;
     SLAPH_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
-    size_t free_b = 0, total_b = 0;
-    SLAPH_CK(cudaMemGetInfo(&free_b, &total_b));
-    size_t const cap = std::max(kTcScratchCap, std::min(kTcScratchMax, free_b / 3));
     int32_t const n_t = ring_slots_ > 0 ? std::max(1, ring_slots_ / 2) : dims_.Lt;
-    int32_t const batch = dev::vdaggerv_tc_batch(geo_, std::max(n_all, 1), sms, cap, n_t);
-    tc_scratch_.reserve(dev::vdaggerv_tc_scratch_bytes(geo_, std::max(n_all, 1), batch));
+    int32_t const batch = dev::vdaggerv_tc_batch(geo_, tc_plan_, sms, kTcScratchCap, n_t);
+    tc_scratch_.reserve(dev::vdaggerv_tc_scratch_bytes(geo_, tc_plan_, batch));
     // The scratch may be larger than this batch needs (kept from an earlier
-    // call): the launch count follows from what it holds.
-    batch_fit = std::max<int64_t>(
-        1, static_cast<int64_t>(tc_scratch_.size() /
-                                dev::vdaggerv_tc_scratch_bytes(geo_, std::max(n_all, 1), 1)));
+    // call): the build takes no more timeslices per launch for it.
+    batch_fit = batch;
     err_.reserve(sizeof(int));
     SLAPH_CK(cudaMemsetAsync(err_.as<void>(), 0, sizeof(int), stream_));
   }
@@ -484,23 +498,23 @@ void Engine::vdaggerv_build(int precision) {
     if (precision == SLAPH_MIXED) {
       int32_t const k =
           n_all > 0 ? dev::vdaggerv_tc_gemm_launches(nt, static_cast<int32_t>(batch_fit)) : 0;
-      launch(dev::vdaggerv_tc(vdv_.as<double2>(), Vb, phase_fx_.as<longlong2>(),
-                              list.as<int32_t>(), n_comp, t0, nt, geo_, tc_scratch_.as<void>(),
-                              tc_scratch_.size(), err_.as<int>(), stream_, ready.data(),
-                              tc_disp ? &dd : nullptr, vdv_ev_.data() + 2 * gemm_done, 2 * k,
-                              v_t0, c == 0),
+      launch(dev::vdaggerv_tc(vdv_.as<double2>(), Vb, tc_plan_, t0, nt, geo_,
+                              tc_scratch_.as<void>(),
+                              dev::vdaggerv_tc_scratch_bytes(geo_, tc_plan_,
+                                                             static_cast<int32_t>(batch_fit)),
+                              err_.as<int>(), stream_, ready.data(), tc_disp ? &dd : nullptr,
+                              vdv_ev_.data() + 2 * gemm_done, 2 * k, v_t0),
              "vdaggerv_tc");
       gemm_done += k;
-      // per timeslice the exponents, A slices and (with momentum operators)
-      // B slices, per displaced operator its steps, exponents and slices; one
-      // GEMM per batch of timeslices
-      if (n_all > 0)
-        launches_ += (2LL + (n_comp > 0 ? 1 : 0) + disp_launches) * nt + k - 1;
+      // per timeslice the exponents and the slices of the momentum families,
+      // per displaced operator its steps, exponents and slices; one GEMM and
+      // one Fourier sum per batch of timeslices
+      if (n_all > 0) launches_ += (2LL + disp_launches) * nt + 2 * k - 1;
     } else {
       for (int32_t t = t0; t < t0 + nt; ++t)
         if (ready[t]) SLAPH_CK(cudaStreamWaitEvent(stream_, ready[t], 0));
-      launch(dev::vdaggerv_fp64(vdv_.as<double2>(), Vb, families.data(),
-                                static_cast<int32_t>(families.size()), t0, nt, geo_, stream_,
+      launch(dev::vdaggerv_fp64(vdv_.as<double2>(), Vb, fam_fp64_.data(),
+                                static_cast<int32_t>(fam_fp64_.size()), t0, nt, geo_, stream_,
                                 v_t0),
              "vdaggerv_fp64");
     }

@@ -161,14 +161,19 @@ class Engine {
   std::vector<cudaEvent_t> tc_ev_;  // three per tensor-core trace batch
   std::vector<cudaEvent_t> vdv_ev_;  // two per split-precision VdaggerV GEMM launch
 
-  DevBuf V_, peram_, noise_, phase_, phase_fx_, vdv_, ops_dev_, mom_dev_, tc_scratch_, err_;
+  DevBuf V_, peram_, noise_, vdv_, tc_scratch_, err_;
   HostBuf host_rb_;  // read-back staging
   DevBuf slot_bits_;  // largest |re|, |im| of every double-float matrix slot (mixed path)
   int read_err_flag();  // the device error flag, through host_rb_ on the engine stream
   std::vector<slaph_vdv_op> ops_;
   DevBuf U_, W_, disp_ops_;  // gauge links, displaced eigenvector scratch, displaced op ids
   DevBuf hyp_dec_;           // decorated links of a chunk of timeslices (HYP smearing)
-  DevBuf phase_unit_, unit_op_;  // phase 1 per site and its operator index (displaced, mixed)
+  // Momentum families of the operator table (set_operators): those of the FP64
+  // build, and the split-precision plan (displaced operators included).
+  std::vector<int32_t> computed_, displaced_;  // operator ids
+  std::vector<dev::VdvFamily> fam_fp64_;
+  dev::VdvTcPlan tc_plan_{};
+  DevBuf fam_dev_, phase_fx_, roots_, mn_dev_;
   std::vector<char> gauge_set_;
   // Eigenvector ring (set_eigenvector_slots): host buffer per timeslice and
   // the compute stream's last use of each half of the ring.

@@ -26,15 +26,11 @@ void add(VdvFamily &f, int32_t op, int32_t k, int32_t dag) {
   ++f.n_ops;
 }
 
-// Planes with fewer entries than this are not worth a Fourier sum of their
-// own (a K step of the kernels holds 16 entries): the lattice is one plane.
-constexpr int64_t kMinPlane = 48;
-
 }  // namespace
 
 std::vector<VdvFamily> vdv_families(std::vector<int32_t> const &ids,
                                     std::vector<int32_t> const &mom, int32_t Lx, int32_t Ly,
-                                    int32_t Lz, bool sheared) {
+                                    int32_t Lz, bool sheared, int32_t max_ops) {
   int32_t const L[3] = {Lx, Ly, Lz};
   bool const cubic = Lx == Ly && Lx == Lz;
   auto plane = [&](int a) { return 3LL * Lx * Ly * Lz / L[a]; };
@@ -54,12 +50,12 @@ std::vector<VdvFamily> vdv_families(std::vector<int32_t> const &ids,
     int axis = -1;
     for (int a = 0; a < 3; ++a) {
       bool const only = p[(a + 1) % 3] == 0 && p[(a + 2) % 3] == 0;
-      if (only && axis < 0 && (a == 0 || sheared) && plane(a) >= kMinPlane) axis = a;
+      if (only && axis < 0 && (a == 0 || sheared) && plane(a) >= kVdvMinPlane) axis = a;
     }
     if (axis >= 0) {
       m.k = p[axis];
       along[axis].push_back(m);
-    } else if (plane(0) < kMinPlane) {
+    } else if (!vdv_planes_along_x(Ly, Lz)) {
       whole.push_back(m);
     } else {
       std::pair<int32_t, int32_t> key{p[1], p[2]};
@@ -72,10 +68,11 @@ std::vector<VdvFamily> vdv_families(std::vector<int32_t> const &ids,
       classes[key].push_back(m);
     }
   }
+  size_t const per_family = static_cast<size_t>(std::clamp(max_ops, 1, kVdvFamilyOps));
   auto emit = [&](VdvFamily const &proto, std::vector<Member> const &ms) {
-    for (size_t b = 0; b < ms.size(); b += kVdvFamilyOps) {
+    for (size_t b = 0; b < ms.size(); b += per_family) {
       VdvFamily f = proto;
-      for (size_t e = b; e < std::min(ms.size(), b + kVdvFamilyOps); ++e)
+      for (size_t e = b; e < std::min(ms.size(), b + per_family); ++e)
         add(f, ms[e].id, ms[e].k, ms[e].dag);
       out.push_back(f);
     }

@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <vector>
 
 #include "vdv_families.hpp"
 
@@ -83,29 +84,46 @@ cudaError_t momenta(double2 *phase, int32_t const *mom, int32_t n_ops, Geometry 
                     cudaStream_t stream);
 
 // VdaggerV[vdv code 2*op][t] = V_t^H diag(e^{-ip.x}) V_t for the operators of
-// the families fam[0..n_fam) (host array, vdv_families.hpp;
+// the families fam[0..n_fam) (host array, vdv_families.hpp, at most kVdvFp64Ops
+// operators each;
 // src/OperatorFactory.cpp:292-300), FP64.  V: consecutive timeslices
 // [t][nev][dim_row] (each column-major), V[0] holding timeslice v_t0 (0: all Lt
 // resident; a ring slot otherwise).  vdv: [2*n_ops][Lt][nev][nev].
+constexpr int kVdvFp64Ops = 3;
 cudaError_t vdaggerv_fp64(double2 *vdv, double2 const *V, VdvFamily const *fam, int32_t n_fam,
                           int32_t t0, int32_t nt, Geometry g, cudaStream_t stream,
                           int32_t v_t0 = 0);
 // Split-BF16 tensor-core VdaggerV (vdv_tc.cu): same result as vdaggerv_fp64
-// to ~1e-13 relative.  scratch: device buffer of at least
-// vdaggerv_tc_scratch_bytes(g, n, batch) bytes, where batch timeslices are
-// processed per launch (vdaggerv_tc_batch picks it from the SM count, the
-// timeslice count and a memory cap); err: device int, set non-zero when a bounded wait gave up.
-size_t vdaggerv_tc_scratch_bytes(Geometry g, int32_t n_ops, int32_t batch);
+// to ~1e-13 relative.  The plan of an operator table: families (planes of
+// constant x, or the whole lattice where those are too small) of the momentum
+// operators, then one family per displaced operator; all pointers are device
+// memory kept by the caller.
+struct VdvTcPlan {
+  int32_t n_fam, n_mom;           // families; those of momentum operators come first
+  int32_t n_planes, per;          // planes, lattice entries (3 x sites) of each
+  VdvFamily const *fam;           // [n_fam]
+  longlong2 const *phase_fx;      // [n_fam][per / 3]: the families' phases x 2^62
+  double2 const *roots;           // [n_planes]: e^{-2 pi i n / n_planes}
+  int2 const *mn;                 // GEMM tiles (m, n) of one plane
+  int32_t n_mn;
+};
+// The (m, n) tiles of one plane: all but those of Hermitian families below the
+// diagonal.
+std::vector<int2> vdaggerv_tc_tiles(std::vector<VdvFamily> const &fam, int32_t nev);
+// Scratch for `batch` timeslices per GEMM launch.
+size_t vdaggerv_tc_scratch_bytes(Geometry g, VdvTcPlan const &pl, int32_t batch);
 // phase_fx[k] = round(phase[k] 2^62) per component, the fixed-point phases the
 // split-precision VdaggerV multiplies with integer arithmetic.
 cudaError_t phase_fixed(longlong2 *phase_fx, double2 const *phase, int64_t n,
                         cudaStream_t stream);
+// roots[n] = e^{-2 pi i n / n_planes}.
+cudaError_t unit_roots(double2 *roots, int32_t n_planes, cudaStream_t stream);
 // Timeslices per GEMM launch for n_t timeslices: at most what max_bytes of
-// scratch holds, chosen for the fewest rounds of one tile per SM over all
-// launches (the last round of each launch is the partly idle one).
-int32_t vdaggerv_tc_batch(Geometry g, int32_t n_ops, int32_t sm_count, size_t max_bytes,
+// scratch holds; the fewest whose rounds of one tile per SM, over all
+// launches, are within 2% of the least.
+int32_t vdaggerv_tc_batch(Geometry g, VdvTcPlan const &pl, int32_t sm_count, size_t max_bytes,
                           int32_t n_t);
-// Displaced operators of the split-precision VdaggerV: ops[n_comp + d] is
+// Displaced operators of the split-precision VdaggerV: family n_mom + d is
 // V_t^H D_d(V_t), D_d the displacement steps of operator d applied in place to
 // a copy W of V_t (displace above), momentum not applied.
 constexpr int kMaxDispSteps = 8;
@@ -115,25 +133,20 @@ struct VdvDisplaced {
   int32_t const *steps;          // host: [n][kMaxDispSteps][2] (dir 0..2, forward 0/1)
   double2 const *U;              // device: links [Lt][site][dir][9]
   double2 *W;                    // device: nev x dim_row scratch
-  longlong2 const *unit_phase;   // device: phase 1 in fixed point (2^62, 0) per site
-  int32_t const *unit_op;        // device: {0}, the operator index into unit_phase
 };
-// ops: device list of n_comp momentum operators followed by disp->n displaced
-// ones; scratch sized by vdaggerv_tc_scratch_bytes for all of them.
-cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, longlong2 const *phase_fx,
-                        int32_t const *ops, int32_t n_comp, int32_t t0, int32_t nt, Geometry g,
-                        void *scratch, size_t scratch_bytes, int *err, cudaStream_t stream,
-                        cudaEvent_t const *t_ready = nullptr,
+cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, VdvTcPlan const &pl, int32_t t0,
+                        int32_t nt, Geometry g, void *scratch, size_t scratch_bytes, int *err,
+                        cudaStream_t stream, cudaEvent_t const *t_ready = nullptr,
                         VdvDisplaced const *disp = nullptr,
                         cudaEvent_t const *gemm_ev = nullptr, int32_t n_gemm_ev = 0,
-                        int32_t v_t0 = 0, bool clear_scratch = true);
-// (V: consecutive timeslices, V[0] holding timeslice v_t0.  clear_scratch:
-// zero the scratch slots first (their padding rows must be zero); a later
-// call on the same scratch in the same build may skip it.  t_ready[t], when
-// given and non-null: event after which timeslice t of V is valid; the
-// slicing of t waits for it on `stream`.  gemm_ev: when given, the
-// events 2k and 2k+1 are recorded on `stream` just before and after the k-th
-// GEMM launch, for k < n_gemm_ev / 2; vdaggerv_tc_gemm_launches gives k's range.)
+                        int32_t v_t0 = 0);
+// (V: consecutive timeslices, V[0] holding timeslice v_t0.  scratch: at least
+// vdaggerv_tc_scratch_bytes of one timeslice; err: device int, set non-zero
+// when a bounded wait gave up.  t_ready[t], when given and non-null: event
+// after which timeslice t of V is valid; the slicing of t waits for it on
+// `stream`.  gemm_ev: when given, the events 2k and 2k+1 are recorded on
+// `stream` just before and after the k-th GEMM launch, for k < n_gemm_ev / 2;
+// vdaggerv_tc_gemm_launches gives k's range.)
 int32_t vdaggerv_tc_gemm_launches(int32_t nt, int32_t batch);
 // One bounded mbarrier wait that nothing completes (selftest.cu): *err = 1
 // once it gives up after `cycles` clock cycles.

@@ -284,15 +284,6 @@ __device__ __forceinline__ void put_b_fx(uint8_t *region, int64_t k_tiles, int c
     *reinterpret_cast<uint32_t *>(blk + p * kBBlk + core_off(r, k)) = bf16x2(dre[p], dim[p]);
 }
 
-__device__ __forceinline__ void put_a(uint8_t *region, int64_t k_tiles, int row, int64_t m,
-                                      double2 x, int e) {
-  put_a_fx(region, k_tiles, row, m, fixed55(x.x, e), fixed55(x.y, e));
-}
-__device__ __forceinline__ void put_b(uint8_t *region, int64_t k_tiles, int col, int64_t m,
-                                      double2 y, int e) {
-  put_b_fx(region, k_tiles, col, m, fixed55(y.x, e), fixed55(y.y, e));
-}
-
 // Exponent e with max |x| < 2^e for a positive maximum (0 for m == 0).
 __device__ __forceinline__ int expo_of_max(double m) {
   int e = 0;

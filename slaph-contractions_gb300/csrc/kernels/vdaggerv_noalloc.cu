@@ -58,7 +58,7 @@ extern "C" int slaph_vdaggerv_noalloc(const slaph_dims *dims, const double *V_t,
     g.dim_row = 3LL * static_cast<int64_t>(vol);
     std::vector<slaph::dev::VdvFamily> const fam =
         slaph::dev::vdv_families({0}, {momentum[0], momentum[1], momentum[2]}, dims->Lx, dims->Ly,
-                                 dims->Lz, true);
+                                 dims->Lz, true, slaph::dev::kVdvFp64Ops);
     check(slaph::dev::vdaggerv_fp64(reinterpret_cast<double2 *>(out),
                                     reinterpret_cast<double2 const *>(V_t), fam.data(),
                                     static_cast<int32_t>(fam.size()), 0, 1, g,

@@ -16,7 +16,7 @@
 namespace slaph {
 namespace dev {
 
-constexpr int kVdvFamilyOps = 3;
+constexpr int kVdvFamilyOps = 8;
 
 struct VdvFamily {
   // Planes of constant h along `axis` (0..2): with u, v the other two
@@ -31,13 +31,20 @@ struct VdvFamily {
   int32_t dag[kVdvFamilyOps];  // the operator is the conjugate transpose of the sum
 };
 
+// Planes with fewer entries than this are not worth a Fourier sum of their own
+// (a K step of the kernels holds 16 entries): the lattice is one plane.
+constexpr int64_t kVdvMinPlane = 48;
+inline bool vdv_planes_along_x(int32_t Ly, int32_t Lz) {
+  return 3LL * Ly * Lz >= kVdvMinPlane;
+}
+
 // Families of the operators `ids` (momenta mom[3 i..] of ids[i]) on an
 // Lx x Ly x Lz lattice.  sheared: the planes may be any {p.x = h}, so that
 // every momentum with a component +-1 has a Hermitian family of its own (half
 // the work of a phase family); otherwise only planes of constant x.
 std::vector<VdvFamily> vdv_families(std::vector<int32_t> const &ids,
                                     std::vector<int32_t> const &mom, int32_t Lx, int32_t Ly,
-                                    int32_t Lz, bool sheared);
+                                    int32_t Lz, bool sheared, int32_t max_ops);
 
 }  // namespace dev
 }  // namespace slaph

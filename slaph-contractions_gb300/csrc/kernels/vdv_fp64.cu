@@ -39,6 +39,7 @@ namespace {
 constexpr int kK = 16;        // lattice entries per step
 constexpr int kThr = 256;     // 16 x 16 threads, kB x kB entries each
 constexpr int kMaxFam = 16;   // families per launch
+static_assert(kVdvFp64Ops == 3, "kernel instances");
 
 struct FamilyArgs {
   VdvFamily f[kMaxFam];
@@ -380,7 +381,7 @@ cudaError_t vdaggerv_fp64(double2 *vdv, double2 const *V, VdvFamily const *fam, 
                           int32_t v_t0) {
   if (n_fam == 0 || nt == 0) return cudaSuccess;
   for (int herm = 0; herm < 2; ++herm)
-    for (int ops = 1; ops <= kVdvFamilyOps; ++ops) {
+    for (int ops = 1; ops <= kVdvFp64Ops; ++ops) {
       FamilyArgs args{};
       int32_t n = 0;
       for (int32_t k = 0; k <= n_fam; ++k) {

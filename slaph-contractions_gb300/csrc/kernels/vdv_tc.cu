@@ -3,15 +3,27 @@
 // VdaggerV = V^H diag(phase) V (src/OperatorFactory.cpp:292-300) with FP64
 // inputs and an FP64-accurate result from BF16 tensor-core products, by the
 // split-BF16 scheme of tc_common.cuh: A' rows are the eigenvectors V_i, B
-// columns W_j = diag(phase) V_j, K' = 2 * 3L^3; rows are scaled by the
+// columns W_j = diag(phase) V_j, K' = 2 * 3L^2 per plane; rows are scaled by the
 // exponent of the eigenvector's largest |entry| (the same for W, |phase| = 1).
 //
-// Data path: slices are written once per timeslice (A) and per timeslice and
-// operator (B) to HBM, already in the tcgen05 core-matrix layout, and streamed
-// into shared memory by the GEMM.  The B columns of all operators of a
-// timeslice form one N dimension (column o nev + j: operator o, eigenvector
-// j), cut into tiles of kTN without padding between operators; the tiles of a
-// batch of timeslices (m tiles x n tiles x timeslices) go to persistent CTAs.
+// Operators come in momentum families (vdv_families.hpp): the GEMM gives the
+// sums over planes of constant x, one set of B columns per family, and
+// vdv_fourier_kernel the operators from them, so that operators that differ in
+// p_x only share their GEMM work, and tiles below the diagonal of a Hermitian
+// family are not computed.  16 operators with |p|^2 <= 4 are 7 families, 13
+// with |p|^2 <= 3 are 5, 3 with |p|^2 <= 1 are 3.  The planes are also what
+// fills the chip: a timeslice gives n_planes times as many tiles as a sum over
+// the whole lattice, so a launch needs few timeslices (and little scratch) for
+// an even load.
+//
+// Data path: V is read once per timeslice to write the A slices and the B
+// slices of all families to HBM, already in the tcgen05 core-matrix layout,
+// from where the GEMM streams them into shared memory.  The B columns of all
+// families form one N dimension (column f nev + j: family f, eigenvector j),
+// cut into tiles of kTN without padding between families.  Padding rows and
+// columns of the last tiles are not written: they only reach output rows and
+// columns that nobody reads.
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -27,102 +39,157 @@ namespace {
 
 using namespace tc;
 
-// Exponent e_i with max_x |V(x, i)| < 2^e_i per eigenvector (one block per i).
-__global__ void colmax_kernel(int32_t *expo, double2 const *Vt, Geometry g) {
-  int const i = blockIdx.x;
+// K tiles (kTK / 2 complex entries) of one plane; planes are padded to whole
+// K tiles.
+__host__ __device__ inline int32_t plane_k_tiles(int32_t per) {
+  return (per + kTK / 2 - 1) / (kTK / 2);
+}
+
+// Exponent e_i with max_x |V(x, i)| < 2^e_i per eigenvector: one cluster of
+// kMaxCtas CTAs per eigenvector (one CTA each leaves most of the memory
+// bandwidth unused: 170 us per timeslice of 220 eigenvectors at 32^3).
+constexpr int kMaxCtas = 8;
+__global__ void __cluster_dims__(kMaxCtas, 1, 1) __launch_bounds__(256)
+    colmax_kernel(int32_t *expo, double2 const *Vt, Geometry g) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  int const i = blockIdx.y, part = blockIdx.x;
   double2 const *col = Vt + static_cast<int64_t>(i) * g.dim_row;
+  int64_t const b = g.dim_row * part / kMaxCtas, e = g.dim_row * (part + 1) / kMaxCtas;
   double m = 0;
-  for (int64_t x = threadIdx.x; x < g.dim_row; x += blockDim.x) {
+#pragma unroll 4
+  for (int64_t x = b + threadIdx.x; x < e; x += 256) {
     double2 const v = col[x];
     m = fmax(m, v.x * v.x + v.y * v.y);
   }
-  __shared__ double red[256];
-  red[threadIdx.x] = m;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] = fmax(red[threadIdx.x], red[threadIdx.x + s]);
-    __syncthreads();
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  __shared__ double red[8];
+  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = m;
+  cluster.sync();
+  if (part == 0 && threadIdx.x == 0) {
+    double mx = 0;
+    for (int q = 0; q < kMaxCtas; ++q) {
+      double const *r = cluster.map_shared_rank(red, q);
+      for (int w = 0; w < 8; ++w) mx = fmax(mx, r[w]);
+    }
+    int ex = 0;
+    mx = sqrt(mx);
+    if (mx > 0) frexp(mx * (1.0 + 1e-15), &ex);
+    expo[i] = ex;
   }
-  if (threadIdx.x == 0) {
-    int e = 0;
-    double const mx = sqrt(red[0]);
-    if (mx > 0) frexp(mx * (1.0 + 1e-15), &e);
-    expo[i] = e;
-  }
+  cluster.sync();  // the other CTAs' shared memory stays until it is read
 }
 
-// A slices of one timeslice: [m_tile][k_tile][slice][kTM x kTK core layout].
-// Thread per (eigenvector i, site-colour x).
-__global__ void slice_a_kernel(uint16_t *out, double2 const *Vt, int32_t const *expo,
-                               int32_t k_tiles, Geometry g) {
-  int64_t const x = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  int const i = blockIdx.y;
-  if (x >= static_cast<int64_t>(k_tiles) * (kTK / 2)) return;
-  double2 v = make_double2(0, 0);
-  if (x < g.dim_row) v = Vt[static_cast<int64_t>(i) * g.dim_row + x];
-  put_a(reinterpret_cast<uint8_t *>(out), k_tiles, i, x, v, expo[i]);
-}
-
-// B slices of W = diag(phase_op) V for the operators ops[0..n_ops) of the
-// call, at global B columns col0 + o nev + j: [n_tile][k_tile][slice][kTN x kTK]
-// over the columns of all operators.  A warp covers one 8-column group of one
-// operator's eigenvectors in one k-tile: lane (r, kg) = (lane % 8, lane / 8)
-// takes eigenvector 8 rg + r and the 4 complex K entries 4 kg .. 4 kg + 3, i.e.
-// one 16-byte row of a core matrix, so that the slice stores of the warp cover
-// one or two 8-row core-matrix columns.  V is read and put in fixed point once
-// for all operators; the phase product is taken in fixed point with integer
-// operations only: with V = F_v 2^(e-55) and phase = P 2^-62 (|P| <= 2^62),
-// W = ((F_v 4) P / 2^64) 2^(e-55), the high word of a 128-bit product.  K
-// entries x >= dim_row are written as zero; columns past the last operator's
-// stay as the per-build clear of the scratch left them (zero).
+// Slices of one timeslice.  kA: the A slices of V, [m_tile][K tile][slice][kTM x
+// kTK]; kB: the B slices of phase_f V for n_fam families at B columns
+// col0 + f nev + j, [n_tile][K tile][slice][kTN x kTK].
+//
+// A warp covers eight eigenvectors in one K tile: lane (r, kg) = (lane % 8,
+// lane / 8) takes eigenvector 8 rg + r and the 4 complex K entries 4 kg .. 4 kg
+// + 3 of the tile, i.e. one 16-byte row of a core matrix.  V is read and put in
+// fixed point once for all of it; the phase product is taken in fixed point
+// with integer operations only: with V = F_v 2^(e-55) and phase = P 2^-62
+// (|P| <= 2^62), W = ((F_v 4) P / 2^64) 2^(e-55), the high word of a 128-bit
+// product.  The A rows of an eigenvector are a row pair (Re v, Im v) and (-Im v,
+// Re v): a lane fetches the packed words of the eigenvector whose row it stores
+// by warp shuffles (the second row is the first with its halves swapped and one
+// sign flipped), so that every slice store of a warp, A or B, fills whole
+// 128-byte core matrices (512 contiguous bytes).  Bound by HBM: 16 bytes read,
+// 48 (A) and 24 per family (B) written per entry.
+template <bool kA, bool kB>
 __global__ void __launch_bounds__(256)
-    slice_b_kernel(uint8_t *out, double2 const *Vt, longlong2 const *phase_fx,
-                   int32_t const *ops, int32_t n_ops, int32_t const *expo, int32_t k_tiles,
-                   int64_t col0, Geometry g) {
+    slice_kernel(uint8_t *a_out, uint8_t *b_out, double2 const *Vt, longlong2 const *phase_fx,
+                 int32_t n_fam, int32_t const *expo, int32_t n_planes, int32_t per, int64_t col0,
+                 Geometry g) {
   int64_t const wid = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / 32;
   int const lane = threadIdx.x % 32;
+  int32_t const ktp = plane_k_tiles(per);
+  int64_t const k_tiles = static_cast<int64_t>(ktp) * n_planes;
   int64_t const groups = (g.nev + 7) / 8;
   if (wid >= groups * k_tiles) return;
   int64_t const kt = wid / groups;
   int const rg = static_cast<int>(wid % groups);
   int const r = lane % 8, kg = lane / 8;
   int const j = rg * 8 + r;
-  if (j >= g.nev) return;
-  int64_t const x0 = kt * (kTK / 2) + 4 * kg;
-  int64_t const sites = g.dim_row / 3;
+  bool const row_ok = j < g.nev;
+  int32_t const plane = static_cast<int32_t>(kt / ktp);
+  int32_t const k0 = static_cast<int32_t>(kt - static_cast<int64_t>(plane) * ktp) * (kTK / 2) +
+                     4 * kg;  // first entry within the plane
   long long vr[4], vi[4];
-  int64_t site[4];
-  int const e = expo[j];
+  int32_t site[4];
+  int const e = row_ok ? expo[j] : 0;
+  double2 const *src = Vt + static_cast<int64_t>(j) * g.dim_row + static_cast<int64_t>(plane) * per;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
-    int64_t const x = x0 + q;
-    bool const in = x < g.dim_row;
-    double2 const v = in ? Vt[static_cast<int64_t>(j) * g.dim_row + x] : make_double2(0, 0);
-    vr[q] = fixed55(v.x, e) * 4;
-    vi[q] = fixed55(v.y, e) * 4;
-    site[q] = in ? x / 3 : 0;
+    int32_t const k = k0 + q;
+    bool const in = row_ok && k < per;
+    double2 const v = in ? src[k] : make_double2(0, 0);
+    vr[q] = fixed55(v.x, e);
+    vi[q] = fixed55(v.y, e);
+    site[q] = in ? k / 3 : 0;
   }
-  for (int o = 0; o < n_ops; ++o) {
-    longlong2 const *ph = phase_fx + static_cast<int64_t>(ops[o]) * sites;
+  if (kA) {
     uint32_t w[kSlices][4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      longlong2 const p = ph[site[q]];
-      long long const wr = __mul64hi(vr[q], p.x) - __mul64hi(vi[q], p.y);
-      long long const wi = __mul64hi(vr[q], p.y) + __mul64hi(vi[q], p.x);
       float dre[kSlices], dim[kSlices];
-      digits6(wr, dre);
-      digits6(wi, dim);
+      digits6(vr[q], dre);
+      digits6(vi[q], dim);
 #pragma unroll
       for (int s = 0; s < kSlices; ++s) w[s][q] = bf16x2(dre[s], dim[s]);
     }
-    int64_t const gc = col0 + static_cast<int64_t>(o) * g.nev + j;
-    int64_t const nt = gc / kTN;
-    int const rr = static_cast<int>(gc % kTN);
-    uint8_t *dst = out + (nt * k_tiles + kt) * kStageB + ((rr >> 3) * 4 + kg) * 128 + (rr & 7) * 16;
 #pragma unroll
-    for (int s = 0; s < kSlices; ++s)
-      *reinterpret_cast<uint4 *>(dst + s * kBBlk) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+    for (int h = 0; h < 2; ++h) {  // the two core-matrix groups of the 16 A rows
+      int const from = 4 * h + r / 2 + 8 * kg;
+      int const i = rg * 8 + 4 * h + r / 2;
+      int const arow = 2 * (i % (kTM / 2)) + (r & 1);
+      uint8_t *dst = a_out + (static_cast<int64_t>(i / (kTM / 2)) * k_tiles + kt) * kStageA +
+                     ((arow >> 3) * 4 + kg) * 128 + (arow & 7) * 16;
+#pragma unroll
+      for (int s = 0; s < kSlices; ++s) {
+        uint32_t x[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          uint32_t const y = __shfl_sync(0xffffffffu, w[s][q], from);
+          x[q] = (r & 1) ? __byte_perm(y, 0, 0x1032) ^ 0x8000u : y;
+        }
+        if (i < g.nev)
+          *reinterpret_cast<uint4 *>(dst + s * kABlk) = make_uint4(x[0], x[1], x[2], x[3]);
+      }
+    }
+  }
+  if (kB && row_ok) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      vr[q] *= 4;
+      vi[q] *= 4;
+    }
+    int32_t const sites = per / 3;
+    for (int f = 0; f < n_fam; ++f) {
+      longlong2 const *ph = phase_fx + static_cast<int64_t>(f) * sites;
+      uint32_t w[kSlices][4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        longlong2 const p = ph[site[q]];
+        long long const wr = __mul64hi(vr[q], p.x) - __mul64hi(vi[q], p.y);
+        long long const wi = __mul64hi(vr[q], p.y) + __mul64hi(vi[q], p.x);
+        float dre[kSlices], dim[kSlices];
+        digits6(wr, dre);
+        digits6(wi, dim);
+#pragma unroll
+        for (int s = 0; s < kSlices; ++s) w[s][q] = bf16x2(dre[s], dim[s]);
+      }
+      int64_t const gc = col0 + static_cast<int64_t>(f) * g.nev + j;
+      int64_t const nt = gc / kTN;
+      int const rr = static_cast<int>(gc % kTN);
+      uint8_t *dst =
+          b_out + (nt * k_tiles + kt) * kStageB + ((rr >> 3) * 4 + kg) * 128 + (rr & 7) * 16;
+#pragma unroll
+      for (int s = 0; s < kSlices; ++s)
+        *reinterpret_cast<uint4 *>(dst + s * kBBlk) =
+            make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
+    }
   }
 }
 
@@ -133,29 +200,41 @@ __global__ void phase_fixed_kernel(longlong2 *dst, double2 const *src, int64_t n
   dst[k] = make_longlong2(__double2ll_rn(ldexp(v.x, 62)), __double2ll_rn(ldexp(v.y, 62)));
 }
 
-// Tile i of a launch: m tile i % m_tiles, n tile (i / m_tiles) % n_tiles,
-// batch slot i / (m_tiles n_tiles) (timeslice t0 + slot).  Slot b has its own A
-// slices, B slices and exponents at stride slot_bytes in the scratch buffer:
-// the eigenvectors' exponents, then per operator o >= n_comp (displaced) the
-// exponents of its B columns at (1 + o) nev.
+__global__ void unit_roots_kernel(double2 *roots, int32_t n) {
+  int32_t const k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  double s, c;
+  sincospi(2.0 * static_cast<double>(k) / static_cast<double>(n), &s, &c);
+  roots[k] = make_double2(c, -s);
+}
+
+// Tile i of a launch: (m, n) tile mn[i % n_mn] of plane (i / n_mn) % n_planes
+// of batch slot i / (n_mn n_planes) (timeslice t0 + slot).  Slot b has its own A
+// slices, B slices, plane sums and exponents at stride slot_bytes in the
+// scratch buffer: the eigenvectors' exponents, then per family f >= n_mom
+// (displaced) the exponents of its B columns at (1 + f) nev.
 struct VdvTiles {
   uint8_t const *scratch;
   size_t slot_bytes, b_off, e_off;
-  int32_t m_tiles, n_tiles, k_tiles;
-  __device__ __forceinline__ void decode(int i, int &mt, int &nt, int &slot) const {
-    mt = i % m_tiles;
-    nt = (i / m_tiles) % n_tiles;
-    slot = i / (m_tiles * n_tiles);
+  int2 const *mn;
+  int32_t n_mn, n_planes, k_tiles;  // k_tiles: of one plane
+  __device__ __forceinline__ void decode(int i, int &mt, int &nt, int &plane, int &slot) const {
+    int2 const t = mn[i % n_mn];
+    mt = t.x;
+    nt = t.y;
+    plane = (i / n_mn) % n_planes;
+    slot = i / (n_mn * n_planes);
   }
   struct Ctx {
     uint8_t const *a, *b;
   };
   __device__ __forceinline__ Ctx context(int i, int lane) const {
-    int mt, nt, slot;
-    decode(i, mt, nt, slot);
+    int mt, nt, plane, slot;
+    decode(i, mt, nt, plane, slot);
     uint8_t const *sbase = scratch + slot * slot_bytes;
-    return Ctx{sbase + static_cast<int64_t>(mt) * k_tiles * kStageA,
-               sbase + b_off + static_cast<int64_t>(nt) * k_tiles * kStageB};
+    int64_t const at = static_cast<int64_t>(plane) * k_tiles;
+    int64_t const all = static_cast<int64_t>(n_planes) * k_tiles;
+    return Ctx{sbase + (mt * all + at) * kStageA, sbase + b_off + (nt * all + at) * kStageB};
   }
   __device__ __forceinline__ void load(Ctx const &c, int kt, uint8_t *dst, uint64_t *bar,
                                        int lane) const {
@@ -163,105 +242,211 @@ struct VdvTiles {
   }
 };
 
-// Epilogue of one VdaggerV tile: D = (hi + lo) 2^(e_i + f_c - 14), rows
-// (2i, 2i+1) = (Re, Im) of VdaggerV_o(i, j) for the tile's B columns c = o nev
-// + j, written to operator o's column-major nev x nev block of timeslice t; e:
-// exponents of the eigenvectors (A rows), f: those of the B columns (the
-// eigenvectors' for momentum operators, |phase| = 1; those of D(V) for the
-// displaced ones, o >= n_comp, at (1 + o) nev).
+// Epilogue of one tile: D = (hi + lo) 2^(e_i + f_c - 14), rows (2i, 2i+1) =
+// (Re, Im) of the plane sum G(i, j) of family f for the tile's B columns c = f
+// nev + j, written to sums[(plane n_cols + c) nev + i] of the slot; e: exponents
+// of the eigenvectors (A rows), f: those of the B columns (the eigenvectors'
+// for momentum families, |phase| = 1; those of D(V) for the displaced ones, f >=
+// n_mom, at (1 + f) nev).  A warp stores 16 consecutive i of a column: 256 bytes.
 struct VdvEpilogue {
   VdvTiles tl;
-  double2 *vdv;
-  int32_t const *ops;
-  int nev, n_comp, n_cols, Lt, t0;
+  size_t s_off;
+  int nev, n_mom, n_cols;
   struct Pre {};
   __device__ __forceinline__ Pre prepare(int, int, int) const { return Pre{}; }
   __device__ __forceinline__ void operator()(Pre const &, int it, int row, int col0,
                                              float const (&hi)[kColsW],
                                              float const (&lo)[kColsW]) const {
-    int mt, nt, slot;
-    tl.decode(it, mt, nt, slot);
+    int mt, nt, plane, slot;
+    tl.decode(it, mt, nt, plane, slot);
     int const i = mt * (kTM / 2) + row / 2;
     if (i >= nev) return;
-    int32_t const *expo =
-        reinterpret_cast<int32_t const *>(tl.scratch + slot * tl.slot_bytes + tl.e_off);
-    int const t = t0 + slot;
+    uint8_t const *sbase = tl.scratch + slot * tl.slot_bytes;
+    int32_t const *expo = reinterpret_cast<int32_t const *>(sbase + tl.e_off);
+    double *sums = reinterpret_cast<double *>(const_cast<uint8_t *>(sbase) + s_off) +
+                   2 * static_cast<int64_t>(plane) * n_cols * nev + 2 * i + (row & 1);
     int const ei = expo[i];
 #pragma unroll
     for (int jj = 0; jj < kColsW; ++jj) {
       int const c = nt * kTN + col0 + jj;
       if (c < n_cols) {
-        int const o = c / nev, j = c - o * nev;
-        int const ec = o < n_comp ? expo[j] : expo[(1 + o) * nev + j];
-        double *outd = reinterpret_cast<double *>(
-            vdv + (static_cast<int64_t>(2 * ops[o]) * Lt + t) * nev * nev);
-        double const val = ldexp(static_cast<double>(hi[jj]) + static_cast<double>(lo[jj]),
-                                 ei + ec - 14);
-        outd[2 * (i + static_cast<int64_t>(nev) * j) + (row & 1)] = val;
+        int const f = c / nev, j = c - f * nev;
+        int const ec = f < n_mom ? expo[j] : expo[(1 + f) * nev + j];
+        sums[2 * static_cast<int64_t>(c) * nev] =
+            ldexp(static_cast<double>(hi[jj]) + static_cast<double>(lo[jj]), ei + ec - 14);
       }
     }
   }
 };
 
-// The GEMM: m_tiles x n_tiles x batch tiles over persistent CTAs, kThreads
+// The GEMM: n_mn x n_planes x batch tiles over persistent CTAs, kThreads
 // threads each.
 __global__ void __launch_bounds__(kThreads, 1)
-    ozaki_gemm_kernel(VdvTiles tl, int32_t n_tiles, double2 *vdv, int32_t const *ops,
-                      int32_t n_ops, int32_t n_comp, int32_t t0, Geometry g, int *err) {
+    ozaki_gemm_kernel(VdvTiles tl, int32_t n_tiles, size_t s_off, int32_t n_cols, int32_t n_mom,
+                      Geometry g, int *err) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  VdvEpilogue epi{tl, vdv, ops, g.nev, n_comp, n_ops * g.nev, g.Lt, t0};
+  VdvEpilogue epi{tl, s_off, g.nev, n_mom, n_cols};
   ozaki_tiles(smem, n_tiles, tl.k_tiles, tl, err, epi);
 }
 
-}  // namespace
+// Operators of family blockIdx.y from its plane sums, timeslice t0 +
+// blockIdx.z: M = sum_h e^{-2 pi i k h / n_planes} G_h for every k of the
+// family.  A thread takes one entry (i, j) and keeps, per distinct |k|, the
+// four real sums G.re cos, G.im sin, G.im cos, G.re sin: they give both signs of
+// k (for a Hermitian family the entry (j, i) is the conjugate of the sum with
+// -k).  Memory-bound: every plane sum is read once, unit stride in i.
+constexpr int kMaxK = 4;  // distinct |k| per pass over the planes
+__global__ void __launch_bounds__(256)
+    vdv_fourier_kernel(double2 *vdv, uint8_t const *scratch, size_t slot_bytes, size_t s_off,
+                       VdvFamily const *fams, double2 const *roots, int32_t n_planes,
+                       int32_t n_cols, int32_t t0, Geometry g) {
+  int const nev = g.nev;
+  int64_t const blk = static_cast<int64_t>(nev) * nev;
+  int64_t const x = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+  if (x >= blk) return;
+  int const i = static_cast<int>(x % nev), j = static_cast<int>(x / nev);
+  VdvFamily const &f = fams[blockIdx.y];
+  if (f.herm && i > j) return;
+  double2 const *G = reinterpret_cast<double2 const *>(scratch + blockIdx.z * slot_bytes + s_off) +
+                     static_cast<int64_t>(blockIdx.y) * blk + x;
+  int64_t const step = static_cast<int64_t>(n_cols) * nev;
+  int const t = t0 + blockIdx.z;
+  for (int o0 = 0; o0 < f.n_ops;) {
+    // the next operators with at most kMaxK distinct |k|
+    int32_t ks[kMaxK];
+    int nk = 0, o1 = o0;
+#pragma unroll
+    for (int q = 0; q < kMaxK; ++q) ks[q] = 0;
+    for (; o1 < f.n_ops; ++o1) {
+      int32_t const k = abs(f.k[o1]);
+      bool known = false;
+#pragma unroll
+      for (int q = 0; q < kMaxK; ++q) known = known || (q < nk && ks[q] == k);
+      if (known) continue;
+      if (nk == kMaxK) break;
+#pragma unroll
+      for (int q = 0; q < kMaxK; ++q)
+        if (q == nk) ks[q] = k;
+      ++nk;
+    }
+    double s[kMaxK][4];
+    int64_t ph[kMaxK];  // |k| h mod n_planes
+#pragma unroll
+    for (int q = 0; q < kMaxK; ++q) {
+      ph[q] = 0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) s[q][u] = 0;
+      ks[q] %= n_planes;
+    }
+    for (int h = 0; h < n_planes; ++h) {
+      double2 const v = G[h * step];
+#pragma unroll
+      for (int q = 0; q < kMaxK; ++q) {
+        if (q >= nk) break;
+        if (ks[q] == 0) {
+          s[q][0] += v.x;
+          s[q][2] += v.y;
+          continue;
+        }
+        double2 const r = roots[ph[q]];  // (cos, -sin)
+        s[q][0] = fma(v.x, r.x, s[q][0]);
+        s[q][1] = fma(v.y, -r.y, s[q][1]);
+        s[q][2] = fma(v.y, r.x, s[q][2]);
+        s[q][3] = fma(v.x, -r.y, s[q][3]);
+        ph[q] += ks[q];
+        if (ph[q] >= n_planes) ph[q] -= n_planes;
+      }
+    }
+    for (int o = o0; o < o1; ++o) {
+      int32_t const k = abs(f.k[o]) % n_planes;
+      double u0 = 0, u1 = 0, u2 = 0, u3 = 0;
+#pragma unroll
+      for (int q = 0; q < kMaxK; ++q)
+        if (q < nk && ks[q] == k) {
+          u0 = s[q][0];
+          u1 = s[q][1];
+          u2 = s[q][2];
+          u3 = s[q][3];
+        }
+      if (f.k[o] < 0) {  // e^{+i phi}
+        u1 = -u1;
+        u3 = -u3;
+      }
+      double2 *out = vdv + (static_cast<int64_t>(2 * f.op[o]) * g.Lt + t) * blk;
+      int64_t const mt = j + static_cast<int64_t>(nev) * i;
+      double2 const plus = make_double2(u0 + u1, u2 - u3);  // the sum with k
+      if (f.dag[o]) {
+        out[mt] = make_double2(plus.x, -plus.y);
+      } else {
+        out[x] = plus;
+        if (f.herm && i != j) out[mt] = make_double2(u0 - u1, -(u2 + u3));
+      }
+    }
+    o0 = o1;
+  }
+}
 
-namespace {
 struct TcLayout {
-  int64_t k_tiles, m_tiles, n_tiles;
-  size_t a_bytes, b_bytes, e_off, slot_bytes;
+  int32_t ktp;
+  int64_t k_tiles, n_cols;
+  size_t a_bytes, s_off, e_off, slot_bytes;
 };
-TcLayout tc_layout(Geometry const &g, int32_t n_ops) {
+TcLayout tc_layout(Geometry const &g, VdvTcPlan const &pl) {
   TcLayout L{};
-  L.k_tiles = (g.dim_row + kTK / 2 - 1) / (kTK / 2);
-  L.m_tiles = (2LL * g.nev + kTM - 1) / kTM;
-  L.n_tiles = (static_cast<int64_t>(n_ops) * g.nev + kTN - 1) / kTN;  // all operators
-  L.a_bytes = static_cast<size_t>(L.m_tiles * L.k_tiles) * kStageA;
-  L.b_bytes = static_cast<size_t>(L.n_tiles * L.k_tiles) * kStageB;
-  L.e_off = L.a_bytes + L.b_bytes;
-  // exponents: the eigenvectors', then room for one set per operator
+  L.ktp = plane_k_tiles(pl.per);
+  L.k_tiles = static_cast<int64_t>(L.ktp) * pl.n_planes;
+  int64_t const m_tiles = (2LL * g.nev + kTM - 1) / kTM;
+  L.n_cols = static_cast<int64_t>(pl.n_fam) * g.nev;
+  int64_t const n_tiles = (L.n_cols + kTN - 1) / kTN;
+  L.a_bytes = static_cast<size_t>(m_tiles * L.k_tiles) * kStageA;
+  L.s_off = L.a_bytes + static_cast<size_t>(n_tiles * L.k_tiles) * kStageB;
+  L.e_off = L.s_off + static_cast<size_t>(pl.n_planes * L.n_cols * g.nev) * sizeof(double2);
+  // exponents: the eigenvectors', then room for one set per family
   L.slot_bytes =
-      (L.e_off + static_cast<size_t>(1 + n_ops) * g.nev * sizeof(int32_t) + 1023) / 1024 * 1024;
+      (L.e_off + static_cast<size_t>(1 + pl.n_fam) * g.nev * sizeof(int32_t) + 1023) / 1024 * 1024;
   return L;
 }
+
 }  // namespace
 
-size_t vdaggerv_tc_scratch_bytes(Geometry g, int32_t n_ops, int32_t batch) {
-  return tc_layout(g, n_ops).slot_bytes * static_cast<size_t>(batch > 0 ? batch : 1);
+std::vector<int2> vdaggerv_tc_tiles(std::vector<VdvFamily> const &fam, int32_t nev) {
+  std::vector<int2> out;
+  int64_t const n_cols = static_cast<int64_t>(fam.size()) * nev;
+  for (int64_t nt = 0; nt * kTN < n_cols; ++nt)
+    for (int32_t mt = 0; mt * (kTM / 2) < nev; ++mt) {
+      // wanted: a column (f, j) of the tile with a full family or j >= the
+      // tile's first row
+      bool want = false;
+      for (int64_t c = nt * kTN; c < std::min<int64_t>(n_cols, (nt + 1) * kTN) && !want; ++c)
+        want = !fam[c / nev].herm || c % nev >= mt * (kTM / 2);
+      if (want) out.push_back(make_int2(mt, static_cast<int32_t>(nt)));
+    }
+  return out;
 }
 
-int32_t vdaggerv_tc_batch(Geometry g, int32_t n_ops, int32_t sm_count, size_t max_bytes,
+size_t vdaggerv_tc_scratch_bytes(Geometry g, VdvTcPlan const &pl, int32_t batch) {
+  return tc_layout(g, pl).slot_bytes * static_cast<size_t>(batch > 0 ? batch : 1);
+}
+
+int32_t vdaggerv_tc_batch(Geometry g, VdvTcPlan const &pl, int32_t sm_count, size_t max_bytes,
                           int32_t n_t) {
-  TcLayout const L = tc_layout(g, n_ops);
-  int64_t const per_t = L.m_tiles * L.n_tiles;  // tiles of one timeslice
+  int64_t const per_t = static_cast<int64_t>(pl.n_mn) * pl.n_planes;  // tiles of one timeslice
   int64_t const sms = sm_count > 0 ? sm_count : 1;
   int64_t const nt = n_t > 0 ? n_t : 1;
-  int64_t fit = static_cast<int64_t>(max_bytes / L.slot_bytes);
+  int64_t fit = static_cast<int64_t>(max_bytes / tc_layout(g, pl).slot_bytes);
   if (fit > nt) fit = nt;
   if (fit < 1) fit = 1;
   // Persistent CTAs take the tiles of a launch in rounds of one tile per SM;
-  // the batch with the fewest rounds over all nt timeslices wastes the least
-  // of the last round of each launch (the smaller batch on a tie).
-  int64_t best = 1, best_rounds = -1;
-  for (int64_t b = 1; b <= fit; ++b) {
+  // the last round of every launch is partly idle.
+  auto rounds = [&](int64_t b) {
     int64_t const launches = (nt + b - 1) / b, last = nt - (launches - 1) * b;
-    int64_t const rounds = (launches - 1) * ((per_t * b + sms - 1) / sms) +
-                           (per_t * last + sms - 1) / sms;
-    if (best_rounds < 0 || rounds < best_rounds) {
-      best = b;
-      best_rounds = rounds;
-    }
-  }
-  return static_cast<int32_t>(best);
+    return (launches - 1) * ((per_t * b + sms - 1) / sms) + (per_t * last + sms - 1) / sms;
+  };
+  int64_t best = rounds(1);
+  for (int64_t b = 2; b <= fit; ++b) best = std::min(best, rounds(b));
+  for (int64_t b = 1; b <= fit; ++b)
+    if (50 * rounds(b) <= 51 * best) return static_cast<int32_t>(b);
+  return static_cast<int32_t>(fit);
 }
 
 cudaError_t phase_fixed(longlong2 *phase_fx, double2 const *phase, int64_t n,
@@ -272,40 +457,38 @@ cudaError_t phase_fixed(longlong2 *phase_fx, double2 const *phase, int64_t n,
   return cudaGetLastError();
 }
 
-cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, longlong2 const *phase_fx,
-                        int32_t const *ops, int32_t n_comp, int32_t t0, int32_t nt, Geometry g,
-                        void *scratch, size_t scratch_bytes, int *err, cudaStream_t stream,
-                        cudaEvent_t const *t_ready, VdvDisplaced const *disp,
-                        cudaEvent_t const *gemm_ev, int32_t n_gemm_ev, int32_t v_t0,
-                        bool clear_scratch) {
+cudaError_t unit_roots(double2 *roots, int32_t n_planes, cudaStream_t stream) {
+  unit_roots_kernel<<<(n_planes + 255) / 256, 256, 0, stream>>>(roots, n_planes);
+  return cudaGetLastError();
+}
+
+cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, VdvTcPlan const &pl, int32_t t0,
+                        int32_t nt, Geometry g, void *scratch, size_t scratch_bytes, int *err,
+                        cudaStream_t stream, cudaEvent_t const *t_ready,
+                        VdvDisplaced const *disp, cudaEvent_t const *gemm_ev,
+                        int32_t n_gemm_ev, int32_t v_t0) {
   int32_t const n_disp = disp ? disp->n : 0;
-  int32_t const n = n_comp + n_disp;
-  if (n == 0 || nt == 0) return cudaSuccess;
-  if (n_disp > 0 && (!disp->n_steps || !disp->steps || !disp->U || !disp->W ||
-                     !disp->unit_phase || !disp->unit_op))
+  if (pl.n_fam == 0 || nt == 0) return cudaSuccess;
+  if (pl.n_mom + n_disp != pl.n_fam ||
+      (n_disp > 0 && (!disp->n_steps || !disp->steps || !disp->U || !disp->W)))
     return cudaErrorInvalidValue;
-  TcLayout const L = tc_layout(g, n);
-  if (L.k_tiles > 0x7fffffffLL / kTK) return cudaErrorInvalidValue;
-  int64_t const batch = static_cast<int64_t>(scratch_bytes / L.slot_bytes);
+  TcLayout const L = tc_layout(g, pl);
+  if (L.k_tiles > 0x7fffffffLL / kTK || L.n_cols > 0x7fffffffLL) return cudaErrorInvalidValue;
+  int64_t batch = static_cast<int64_t>(scratch_bytes / L.slot_bytes);
   if (batch < 1) return cudaErrorInvalidValue;
+  int64_t const per_t = static_cast<int64_t>(pl.n_mn) * pl.n_planes;
+  batch = std::min({batch, std::max<int64_t>(1, 0x7fffffffLL / per_t), int64_t{65535}});
   uint8_t *base = static_cast<uint8_t *>(scratch);
   cudaError_t e = cudaFuncSetAttribute(ozaki_gemm_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(kSmemBytes));
   if (e != cudaSuccess) return e;
-  // Padding rows of the last tiles are never written by the slicing: clear
-  // the slots once per build.
-  if (clear_scratch) {
-    e = cudaMemsetAsync(base, 0,
-                        L.slot_bytes * static_cast<size_t>(std::min<int64_t>(batch, nt)), stream);
-    if (e != cudaSuccess) return e;
-  }
-  int64_t const xs = L.k_tiles * (kTK / 2);
-  unsigned const xb = static_cast<unsigned>((xs + 255) / 256);
-  // slice_b_kernel: one warp per (k-tile, group of 8 eigenvectors)
-  unsigned const bb =
-      static_cast<unsigned>((L.k_tiles * ((g.nev + 7) / 8) * 32 + 255) / 256);
+  // one warp per (K tile, group of 8 eigenvectors)
+  unsigned const sb = static_cast<unsigned>((L.k_tiles * ((g.nev + 7) / 8) * 32 + 255) / 256);
   size_t const links = static_cast<size_t>(g.dim_row / 3) * 27;  // of one timeslice
+  int32_t const sites = pl.per / 3;
+  int64_t const blk = static_cast<int64_t>(g.nev) * g.nev;
+  dim3 const mx(kMaxCtas, static_cast<unsigned>(g.nev));
   int32_t gemm_k = 0;
   for (int32_t tb = t0; tb < t0 + nt; tb += static_cast<int32_t>(batch)) {
     int32_t const nb = static_cast<int32_t>(std::min<int64_t>(batch, t0 + nt - tb));
@@ -318,16 +501,17 @@ cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, longlong2 const *phase_f
       double2 const *Vt = V + static_cast<int64_t>(t - v_t0) * g.nev * g.dim_row;
       uint8_t *slot = base + b * L.slot_bytes;
       int32_t *expo = reinterpret_cast<int32_t *>(slot + L.e_off);
-      colmax_kernel<<<g.nev, 256, 0, stream>>>(expo, Vt, g);
-      slice_a_kernel<<<dim3(xb, g.nev), 256, 0, stream>>>(
-          reinterpret_cast<uint16_t *>(slot), Vt, expo, static_cast<int32_t>(L.k_tiles), g);
-      if (n_comp > 0)
-        slice_b_kernel<<<bb, 256, 0, stream>>>(slot + L.a_bytes, Vt, phase_fx, ops, n_comp, expo,
-                                                static_cast<int32_t>(L.k_tiles), 0, g);
+      colmax_kernel<<<mx, 256, 0, stream>>>(expo, Vt, g);
+      if (pl.n_mom > 0)
+        slice_kernel<true, true><<<sb, 256, 0, stream>>>(slot, slot + L.a_bytes, Vt, pl.phase_fx,
+                                                         pl.n_mom, expo, pl.n_planes, pl.per, 0, g);
+      else
+        slice_kernel<true, false><<<sb, 256, 0, stream>>>(slot, nullptr, Vt, nullptr, 0, expo,
+                                                          pl.n_planes, pl.per, 0, g);
       // Displaced operators: W = D(V_t) in the reference's in-place sweep
       // order, B = W with phase 1 and W's own column exponents.
       for (int32_t d = 0; d < n_disp; ++d) {
-        int32_t const o = n_comp + d;
+        int32_t const f = pl.n_mom + d;
         e = cudaMemcpyAsync(disp->W, Vt, sizeof(double2) * g.nev * g.dim_row,
                             cudaMemcpyDeviceToDevice, stream);
         if (e != cudaSuccess) return e;
@@ -336,25 +520,25 @@ cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, longlong2 const *phase_f
           e = displace(disp->W, disp->U + links * t, st[0], st[1], g, stream);
           if (e != cudaSuccess) return e;
         }
-        int32_t *expo_w = expo + static_cast<int64_t>(1 + o) * g.nev;
-        colmax_kernel<<<g.nev, 256, 0, stream>>>(expo_w, disp->W, g);
-        slice_b_kernel<<<bb, 256, 0, stream>>>(slot + L.a_bytes, disp->W, disp->unit_phase,
-                                                disp->unit_op, 1, expo_w,
-                                                static_cast<int32_t>(L.k_tiles),
-                                                static_cast<int64_t>(o) * g.nev, g);
+        int32_t *expo_w = expo + static_cast<int64_t>(1 + f) * g.nev;
+        colmax_kernel<<<mx, 256, 0, stream>>>(expo_w, disp->W, g);
+        slice_kernel<false, true><<<sb, 256, 0, stream>>>(
+            nullptr, slot + L.a_bytes, disp->W, pl.phase_fx + static_cast<int64_t>(f) * sites, 1,
+            expo_w, pl.n_planes, pl.per, static_cast<int64_t>(f) * g.nev, g);
       }
+      e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
     }
     bool const timed = gemm_ev && 2 * gemm_k + 1 < n_gemm_ev;
     if (timed) {
       e = cudaEventRecord(gemm_ev[2 * gemm_k], stream);
       if (e != cudaSuccess) return e;
     }
-    VdvTiles const tl{base, L.slot_bytes, L.a_bytes, L.e_off, static_cast<int32_t>(L.m_tiles),
-                      static_cast<int32_t>(L.n_tiles), static_cast<int32_t>(L.k_tiles)};
-    int64_t const n_tiles = L.m_tiles * L.n_tiles * nb;
+    VdvTiles const tl{base, L.slot_bytes, L.a_bytes, L.e_off, pl.mn, pl.n_mn, pl.n_planes, L.ktp};
+    int64_t const n_tiles = per_t * nb;
     ozaki_gemm_kernel<<<static_cast<unsigned>(persistent_grid(n_tiles)), kThreads, kSmemBytes,
-                        stream>>>(tl, static_cast<int32_t>(n_tiles), vdv, ops, n, n_comp, tb, g,
-                                  err);
+                        stream>>>(tl, static_cast<int32_t>(n_tiles), L.s_off,
+                                  static_cast<int32_t>(L.n_cols), pl.n_mom, g, err);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (timed) {
@@ -362,6 +546,12 @@ cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, longlong2 const *phase_f
       if (e != cudaSuccess) return e;
     }
     ++gemm_k;
+    vdv_fourier_kernel<<<dim3(static_cast<unsigned>((blk + 255) / 256),
+                              static_cast<unsigned>(pl.n_fam), static_cast<unsigned>(nb)),
+                         256, 0, stream>>>(vdv, base, L.slot_bytes, L.s_off, pl.fam, pl.roots,
+                                           pl.n_planes, static_cast<int32_t>(L.n_cols), tb, g);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }

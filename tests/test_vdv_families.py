@@ -16,9 +16,9 @@ WRAPPER = r"""
 #include "vdv_families.hpp"
 #include <cstring>
 extern "C" int families(int n, const int *ids, const int *mom, int Lx, int Ly, int Lz,
-                        int sheared, int *out, int cap) {
+                        int sheared, int max_ops, int *out, int cap) {
   std::vector<int32_t> i(ids, ids + n), m(mom, mom + 3 * n);
-  auto f = slaph::dev::vdv_families(i, m, Lx, Ly, Lz, sheared != 0);
+  auto f = slaph::dev::vdv_families(i, m, Lx, Ly, Lz, sheared != 0, max_ops);
   int const w = sizeof(slaph::dev::VdvFamily) / 4;
   if (static_cast<int>(f.size()) * w > cap) return -1;
   std::memcpy(out, f.data(), f.size() * sizeof(slaph::dev::VdvFamily));
@@ -46,7 +46,7 @@ def momenta(p2):
 
 def unpack(row):
     f = dict(axis=row[0], n=row[1], sgn=row[2], sh=row[3:5], w=row[5:8], herm=row[8])
-    f["ops"] = [(row[10 + i], row[13 + i], row[16 + i]) for i in range(row[9])]
+    f["ops"] = [(row[10 + i], row[18 + i], row[26 + i]) for i in range(row[9])]
     return f
 
 
@@ -65,21 +65,24 @@ def sites(f, h, L):
     return out
 
 
-@pytest.mark.parametrize("sheared", [0, 1])
+@pytest.mark.parametrize("sheared,max_ops", [(0, 8), (1, 3)])
 @pytest.mark.parametrize("L", [(4, 4, 4), (5, 5, 5), (3, 3, 3), (8, 8, 8), (4, 6, 5), (8, 2, 2),
                                (1, 9, 7)])
 @pytest.mark.parametrize("p2", [0, 1, 3, 5, 9])
-def test_families_reproduce_their_momenta(planner, L, p2, sheared):
+def test_families_reproduce_their_momenta(planner, L, p2, sheared, max_ops):
     moms = momenta(p2)
     ids = list(range(3, 3 + len(moms)))
     out = (C.c_int * 20000)()
     n = planner(len(ids), (C.c_int * len(ids))(*ids),
-                (C.c_int * (3 * len(ids)))(*[k for p in moms for k in p]), *L, sheared, out, 20000)
+                (C.c_int * (3 * len(ids)))(*[k for p in moms for k in p]), *L, sheared,
+                max_ops, out, 20000)
     assert n > 0
-    rows = np.array(out[:19 * n]).reshape(n, 19)
+    rows = np.array(out[:34 * n]).reshape(n, 34)
     seen = []
+    if not sheared:  # one set of planes for all families
+        assert len({(f["axis"], f["n"], f["sgn"], *f["sh"]) for f in map(unpack, rows)}) == 1
     for f in map(unpack, rows):
-        assert 1 <= len(f["ops"]) <= 3
+        assert 1 <= len(f["ops"]) <= max_ops
         if f["herm"]:
             assert not any(f["w"])
             assert all(dag == 0 for _, _, dag in f["ops"])
