@@ -734,10 +734,10 @@ std::unique_ptr<DeviceSchedule> Engine::make_schedule(slaph_plan const *plan, in
   return ds;
 }
 
-// Tensor-core plan of the dense trace groups: per group, one A region per
-// distinct entry row i (the matrices a + i of all A groups) and one B region
-// per distinct entry column j; one GEMM per entry (i, j) over its regions, cut
-// into 64 x 80 tiles.  Groups are packed into batches of at most the scratch
+// Tensor-core plan of the dense trace groups: per group, one A region per block
+// of stacked operand indices (the matrices a + i of all A groups for the
+// indices i of the block, plan_trace_group) and one B region per block of j,
+// cut into 64 x 80 tiles.  Groups are packed into batches of at most the scratch
 // capacity (a group larger than that raises it).
 void Engine::prepare_trace_tc(DeviceSchedule &ds) {
   if (ds.tc_ready) return;
@@ -746,17 +746,29 @@ void Engine::prepare_trace_tc(DeviceSchedule &ds) {
   // Bytes of one 64-row A tile stream and one 80-column B tile stream.
   int64_t const a_tile = static_cast<int64_t>(dev::trace_tc_a_bytes(1, eds));
   int64_t const b_tile = static_cast<int64_t>(dev::trace_tc_b_bytes(1, eds));
+  // Plans by (shape, n_a, n_b), with the offset of their entry tables.
+  struct Planned {
+    TraceGroupPlan p;
+    int64_t tab = 0;
+    size_t bytes = 0;
+  };
+  std::map<std::array<int32_t, 3>, Planned> plans;
+  std::vector<int32_t> entries;
   size_t cap = std::max(tc_scratch_.size(), kTraceScratchMin);
   for (auto const &w : s.waves)
     for (auto const &g : w.groups) {
-      auto const &sh = s.shapes[g.shape];
-      std::vector<int32_t> is(sh.i.begin(), sh.i.end()), js(sh.j.begin(), sh.j.end());
-      std::sort(is.begin(), is.end());
-      std::sort(js.begin(), js.end());
-      size_t const ni = std::unique(is.begin(), is.end()) - is.begin();
-      size_t const nj = std::unique(js.begin(), js.end()) - js.begin();
-      cap = std::max(cap, ni * dev::trace_tc_a_bytes(g.n_a, eds) +
-                              nj * dev::trace_tc_b_bytes(g.n_b, eds));
+      auto const it = plans.emplace(std::array<int32_t, 3>{g.shape, g.n_a, g.n_b}, Planned{});
+      if (!it.second) continue;
+      Planned &pl = it.first->second;
+      pl.p = plan_trace_group(s.shapes[g.shape], g.n_a, g.n_b, dev::kTrTileRows,
+                              dev::kTrTileCols);
+      pl.tab = static_cast<int64_t>(entries.size());
+      entries.insert(entries.end(), pl.p.entry.begin(), pl.p.entry.end());
+      for (auto const &x : pl.p.a)
+        pl.bytes += dev::trace_tc_a_bytes(static_cast<int32_t>(x.size()) * g.n_a, eds);
+      for (auto const &y : pl.p.b)
+        pl.bytes += dev::trace_tc_b_bytes(static_cast<int32_t>(y.size()) * g.n_b, eds);
+      cap = std::max(cap, pl.bytes);
     }
   size_t need = 0;
   int64_t max_expo = 0;
@@ -788,62 +800,59 @@ void Engine::prepare_trace_tc(DeviceSchedule &ds) {
       expo = 0;
     };
     for (auto const &g : w.groups) {
-      auto const &sh = s.shapes[g.shape];
-      std::vector<int32_t> is(sh.i.begin(), sh.i.end()), js(sh.j.begin(), sh.j.end());
-      std::sort(is.begin(), is.end());
-      is.erase(std::unique(is.begin(), is.end()), is.end());
-      std::sort(js.begin(), js.end());
-      js.erase(std::unique(js.begin(), js.end()), js.end());
-      size_t const ab = dev::trace_tc_a_bytes(g.n_a, eds), bb = dev::trace_tc_b_bytes(g.n_b, eds);
-      size_t const gb = is.size() * ab + js.size() * bb;
-      if (used > 0 && used + gb > cap) close();
-      // Regions and exponents of this group, by operand index.
-      size_t const ni = static_cast<size_t>(is.back()) + 1, nj = static_cast<size_t>(js.back()) + 1;
-      std::vector<int64_t> a_reg(ni, -1), b_reg(nj, -1), a_exp(ni, -1), b_exp(nj, -1);
-      for (int32_t i : is) {
-        a_reg[i] = static_cast<int64_t>(used);
-        a_exp[i] = expo;
-        for (int32_t ia = 0; ia < g.n_a; ++ia)
-          av.push_back({static_cast<int64_t>(used), w.group_bases[g.a_off + ia] + i, ia,
-                        static_cast<int32_t>(expo + ia), 0});
-        used += ab;
-        expo += g.n_a;
+      Planned const &pl = plans.at({g.shape, g.n_a, g.n_b});
+      if (used > 0 && used + pl.bytes > cap) close();
+      // Regions and first exponents of this group's blocks.
+      std::vector<int64_t> a_reg, b_reg, a_exp, b_exp;
+      for (auto const &x : pl.p.a) {
+        a_reg.push_back(static_cast<int64_t>(used));
+        a_exp.push_back(expo);
+        int32_t row = 0;
+        for (int32_t i : x)
+          for (int32_t ia = 0; ia < g.n_a; ++ia, ++row)
+            av.push_back({static_cast<int64_t>(used), w.group_bases[g.a_off + ia] + i, row,
+                          static_cast<int32_t>(expo + row), 0});
+        used += dev::trace_tc_a_bytes(row, eds);
+        expo += row;
       }
-      for (int32_t j : js) {
-        b_reg[j] = static_cast<int64_t>(used);
-        b_exp[j] = expo;
-        for (int32_t ib = 0; ib < g.n_b; ++ib)
-          bv.push_back({static_cast<int64_t>(used), w.group_bases[g.b_off + ib] + j, ib,
-                        static_cast<int32_t>(expo + ib), 0});
-        used += bb;
-        expo += g.n_b;
+      for (auto const &y : pl.p.b) {
+        b_reg.push_back(static_cast<int64_t>(used));
+        b_exp.push_back(expo);
+        int32_t col = 0;
+        for (int32_t j : y)
+          for (int32_t ib = 0; ib < g.n_b; ++ib, ++col)
+            bv.push_back({static_cast<int64_t>(used), w.group_bases[g.b_off + ib] + j, col,
+                          static_cast<int32_t>(expo + col), 0});
+        used += dev::trace_tc_b_bytes(col, eds);
+        expo += col;
       }
-      // GEMM tiles, entries in order of their A region (consecutive tiles share
-      // operand streams in L2).
-      int64_t const n_e = static_cast<int64_t>(sh.i.size());
-      std::vector<int64_t> eo(n_e);
-      std::iota(eo.begin(), eo.end(), 0);
-      std::stable_sort(eo.begin(), eo.end(),
-                       [&](int64_t x, int64_t y) { return sh.i[x] < sh.i[y]; });
-      int32_t const mts = (g.n_a + dev::kTrTileRows - 1) / dev::kTrTileRows;
-      int32_t const nts = (g.n_b + dev::kTrTileCols - 1) / dev::kTrTileCols;
       int64_t const plane = static_cast<int64_t>(g.n_a) * g.n_b;
-      for (int64_t e : eo) {
-        int32_t const i = sh.i[e], j = sh.j[e];
-        for (int32_t mt = 0; mt < mts; ++mt)
-          for (int32_t nt = 0; nt < nts; ++nt) {
-            dev::TrTile t{};
-            t.a_src = a_reg[i] + static_cast<int64_t>(mt) * a_tile;
-            t.b_src = b_reg[j] + static_cast<int64_t>(nt) * b_tile;
-            t.out = g.val_base + e * plane + static_cast<int64_t>(nt) * dev::kTrTileCols * g.n_a +
-                    static_cast<int64_t>(mt) * dev::kTrTileRows;
-            t.ea = static_cast<int32_t>(a_exp[i] + mt * dev::kTrTileRows);
-            t.eb = static_cast<int32_t>(b_exp[j] + nt * dev::kTrTileCols);
-            t.rows = std::min(dev::kTrTileRows, g.n_a - mt * dev::kTrTileRows);
-            t.cols = std::min(dev::kTrTileCols, g.n_b - nt * dev::kTrTileCols);
-            t.ld = g.n_a;
-            tiles.push_back(t);
-          }
+      // Tiles in order of their A block (consecutive tiles share operand
+      // streams in L2).
+      for (auto const &pt : pl.p.tiles) {
+        auto const &x = pl.p.a[pt.a];
+        auto const &y = pl.p.b[pt.b];
+        int64_t const off = pl.p.off[pt.a * pl.p.b.size() + pt.b];
+        dev::TrTile t{};
+        t.a_src = a_reg[pt.a] + pt.row / dev::kTrTileRows * a_tile;
+        t.b_src = b_reg[pt.b] + pt.col / dev::kTrTileCols * b_tile;
+        t.ea = static_cast<int32_t>(a_exp[pt.a] + pt.row);
+        t.eb = static_cast<int32_t>(b_exp[pt.b] + pt.col);
+        t.rows = std::min(dev::kTrTileRows, static_cast<int32_t>(x.size()) * g.n_a - pt.row);
+        t.cols = std::min(dev::kTrTileCols, static_cast<int32_t>(y.size()) * g.n_b - pt.col);
+        t.ld = t.n_a = g.n_a;
+        t.n_b = g.n_b;
+        t.row0 = pt.row;
+        t.col0 = pt.col;
+        t.out = g.val_base;
+        if (x.size() == 1 && y.size() == 1) {  // one entry: a plain tile
+          t.tab = -1;
+          t.out += pl.p.entry[off] * plane + static_cast<int64_t>(pt.col) * g.n_a + pt.row;
+        } else {
+          t.tab = pl.tab + off;
+          t.tab_ld = static_cast<int32_t>(y.size());
+        }
+        tiles.push_back(t);
       }
     }
     close();
@@ -852,6 +861,8 @@ void Engine::prepare_trace_tc(DeviceSchedule &ds) {
     upload(wb.tc_tiles, tiles, stream_);
     SLAPH_CK(cudaStreamSynchronize(stream_));
   }
+  upload(ds.tc_entries, entries, stream_);
+  SLAPH_CK(cudaStreamSynchronize(stream_));
   ds.tc_scratch = need;
   ds.tc_expo = max_expo;
   ds.tc_ready = true;
@@ -987,6 +998,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
         t.rows = std::min(dev::kTrTileRows, rows - mt * dev::kTrTileRows);
         t.cols = std::min(dev::kTrTileCols, cols - nt * dev::kTrTileCols);
         t.ld = rows;
+        t.tab = -1;
         tiles.push_back(t);
       }
   };
@@ -1575,7 +1587,8 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
           SLAPH_CK(cudaEventRecord(tc_ev_[3 * bi + 1], stream_));
           launch(dev::trace_tc_gemm(values_.as<double2>(), tc_scratch_.as<uint8_t>(),
                                     tr_expo_.as<int32_t>(), wb.tc_tiles.as<dev::TrTile>() + b.tile_off,
-                                    b.n_tiles, eds, err_.as<int>(), stream_),
+                                    b.n_tiles, ds.tc_entries.as<int32_t>(), eds, err_.as<int>(),
+                                    stream_),
                  "trace_tc_gemm");
           SLAPH_CK(cudaEventRecord(tc_ev_[3 * bi + 2], stream_));
         }

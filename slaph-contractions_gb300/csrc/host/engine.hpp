@@ -102,6 +102,7 @@ struct DeviceSchedule {
   size_t f_scratch = 0;
   int64_t f_out = 0, f_expo = 0;  // doubles2 of dense outputs, exponents per batch
   bool tc_ready = false;
+  DevBuf tc_entries;  // entry tables of the stacked trace tiles (TrTile::tab)
   // Products on the tensor cores: scratch bytes and exponents of the largest level.
   bool p_ready = false;
   size_t p_scratch = 0;

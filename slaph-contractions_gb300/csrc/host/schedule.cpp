@@ -777,6 +777,85 @@ Schedule build_schedule(slaph_dims const &dims, slaph_plan const &plan, int sing
   return b.run(single_block_pair);
 }
 
+TraceGroupPlan plan_trace_group(TraceShape const &shape, int32_t n_a, int32_t n_b,
+                                int32_t tile_rows, int32_t tile_cols) {
+  size_t const n_e = shape.i.size();
+  int32_t ni = 0, nj = 0;
+  for (size_t e = 0; e < n_e; ++e) {
+    ni = std::max(ni, shape.i[e] + 1);
+    nj = std::max(nj, shape.j[e] + 1);
+  }
+  // components over the operand indices of both sides (i, then ni + j)
+  std::vector<int32_t> root(static_cast<size_t>(ni) + nj);
+  for (size_t k = 0; k < root.size(); ++k) root[k] = static_cast<int32_t>(k);
+  auto find = [&](int32_t x) {
+    while (root[x] != x) x = root[x] = root[root[x]];
+    return x;
+  };
+  std::vector<char> has_i(ni, 0), has_j(nj, 0);
+  for (size_t e = 0; e < n_e; ++e) {
+    has_i[shape.i[e]] = has_j[shape.j[e]] = 1;
+    root[find(shape.i[e])] = find(ni + shape.j[e]);
+  }
+  auto blocks = [&](std::vector<char> const &has, int32_t first, bool stack) {
+    std::vector<std::vector<int32_t>> out;
+    std::map<int32_t, size_t> of;
+    for (int32_t k = 0; k < static_cast<int32_t>(has.size()); ++k) {
+      if (!has[k]) continue;
+      auto it = stack ? of.emplace(find(first + k), out.size())
+                      : std::make_pair(of.end(), true);
+      if (it.second) out.emplace_back();
+      (stack ? out[it.first->second] : out.back()).push_back(k);
+    }
+    return out;
+  };
+  TraceGroupPlan best;
+  bool have = false;
+  for (int option = 0; option < 4; ++option) {
+    if ((option & 2) && n_b >= 1 << 15) continue;  // the tile epilogue holds groups in 16 bits
+    TraceGroupPlan p;
+    p.a = blocks(has_i, 0, (option & 1) != 0);
+    p.b = blocks(has_j, ni, (option & 2) != 0);
+    std::vector<std::pair<int32_t, int32_t>> pos_i(ni), pos_j(nj);  // (block, place)
+    for (size_t x = 0; x < p.a.size(); ++x)
+      for (size_t u = 0; u < p.a[x].size(); ++u)
+        pos_i[p.a[x][u]] = {static_cast<int32_t>(x), static_cast<int32_t>(u)};
+    for (size_t y = 0; y < p.b.size(); ++y)
+      for (size_t v = 0; v < p.b[y].size(); ++v)
+        pos_j[p.b[y][v]] = {static_cast<int32_t>(y), static_cast<int32_t>(v)};
+    p.off.assign(p.a.size() * p.b.size(), -1);
+    for (size_t e = 0; e < n_e; ++e) {
+      auto const pi = pos_i[shape.i[e]], pj = pos_j[shape.j[e]];
+      size_t const w = p.b[pj.first].size();
+      int64_t &o = p.off[pi.first * p.b.size() + pj.first];
+      if (o < 0) {
+        o = static_cast<int64_t>(p.entry.size());
+        p.entry.resize(p.entry.size() + p.a[pi.first].size() * w, -1);
+      }
+      p.entry[o + pi.second * w + pj.second] = static_cast<int32_t>(e);
+    }
+    for (size_t x = 0; x < p.a.size(); ++x)
+      for (size_t y = 0; y < p.b.size(); ++y) {
+        int64_t const o = p.off[x * p.b.size() + y];
+        if (o < 0) continue;
+        int32_t const rows = static_cast<int32_t>(p.a[x].size()) * n_a;
+        int32_t const cols = static_cast<int32_t>(p.b[y].size()) * n_b;
+        for (int32_t r = 0; r < rows; r += tile_rows)
+          for (int32_t c = 0; c < cols; c += tile_cols) {
+            bool any = false;
+            for (int32_t u = r / n_a; u <= (std::min(rows, r + tile_rows) - 1) / n_a; ++u)
+              for (int32_t v = c / n_b; v <= (std::min(cols, c + tile_cols) - 1) / n_b; ++v)
+                any = any || p.entry[o + u * static_cast<int64_t>(p.b[y].size()) + v] >= 0;
+            if (any)
+              p.tiles.push_back({static_cast<int32_t>(x), static_cast<int32_t>(y), r, c});
+          }
+      }
+    if (!have || p.tiles.size() < best.tiles.size()) best = std::move(p);
+    have = true;
+  }
+  return best;
+}
+
 ProductPlan plan_products(ProdInst const *prods, int64_t n, int32_t eds) {
   ProductPlan pp;
   int32_t const per_group = eds > 0 && eds <= 64 ? std::max(1, 64 / eds) : 1;

@@ -148,6 +148,30 @@ struct Schedule {
 // and 80 B groups); smaller bipartite sets stay residual.
 constexpr int32_t kMinGroupA = 16, kMinGroupB = 16;
 
+// GEMM plan of a dense trace group of n_a x n_b operand groups.  The entries
+// (i, j) of a shape form connected components of operand indices (the
+// (r1, r2) pair of the matrices); the matrices a + i of all A groups for the
+// indices i of a block are stacked to the rows of one GEMM operand, those of
+// the B groups for a block of j to its columns.  A block is one index, or all
+// the indices of a component on that side: stacking fills tiles of tile_rows x
+// tile_cols that a small group leaves mostly empty, but also computes pairs of a
+// component that are not entries.  Of the four combinations the one with the
+// fewest tiles is taken (tiles without an entry are left out).
+struct TraceGroupPlan {
+  std::vector<std::vector<int32_t>> a, b;  // operand indices of every block
+  struct Tile {
+    int32_t a, b;      // blocks
+    int32_t row, col;  // first row and column of the tile within them
+  };
+  std::vector<Tile> tiles;
+  // Entry of operand indices a[x][u], b[y][v], or -1, at
+  // entry[off[x b.size() + y] + u b[y].size() + v] (off -1: no entry at all).
+  std::vector<int32_t> entry;
+  std::vector<int64_t> off;
+};
+TraceGroupPlan plan_trace_group(TraceShape const &shape, int32_t n_a, int32_t n_b,
+                                int32_t tile_rows, int32_t tile_cols);
+
 // Tensor-core plan of the products of one dependency level (operator*,
 // src/DilutedFactor.cpp:6-51).  Left matrices are taken in order of first
 // appearance; a group starts with the next unused one and adds, up to

@@ -262,14 +262,20 @@ struct TrSliceGroup {
   int32_t slot[8];
   int32_t pad;
 };
-// One output tile of 64 A groups x 80 B groups of one (group, entry) GEMM.
+// One output tile of 64 rows x 80 columns of one GEMM.  tab < 0: value (r, c) at
+// out + c ld + r.  Otherwise the rows are stacked blocks of n_a operand groups
+// and the columns of n_b: row r of the tile is group ia of block u, (row0 + r) =
+// u n_a + ia, column c group ib of block v, (col0 + c) = v n_b + ib, and the
+// value belongs to entry e = entries[tab + u tab_ld + v] (none when negative),
+// at out + e n_a n_b + ib n_a + ia.
 struct TrTile {
   int64_t a_src, b_src;  // byte offsets of the tile's A and B operand streams
-  int64_t out;           // value index of tile row 0, column 0
+  int64_t out;           // value index (see above)
+  int64_t tab;
   int32_t ea, eb;        // exponent indices of tile row 0 and column 0
   int32_t rows, cols;    // valid rows (<= 64) and columns (<= 80)
-  int32_t ld;            // value index distance between columns
-  int32_t pad;
+  int32_t ld;            // tab < 0: value index distance between columns
+  int32_t n_a, n_b, row0, col0, tab_ld;
 };
 constexpr int32_t kTrTileRows = 64, kTrTileCols = 80;
 int64_t trace_tc_k_tiles(int32_t eds);
@@ -290,8 +296,8 @@ cudaError_t trace_tc_slice(uint8_t *scratch, int32_t *expo, TrSliceGroup const *
                            unsigned int const *slot_bits, int32_t eds, cudaStream_t stream);
 // The GEMM tiles of a batch; FP64 trace values into `values`.
 cudaError_t trace_tc_gemm(double2 *values, uint8_t const *scratch, int32_t const *expo,
-                          TrTile const *tiles, int64_t n_tiles, int32_t eds, int *err,
-                          cudaStream_t stream);
+                          TrTile const *tiles, int64_t n_tiles, int32_t const *entries,
+                          int32_t eds, int *err, cudaStream_t stream);
 
 // Generic form of the same GEMM (factor_tc.cu): k_tiles k-tiles of 16
 // complex entries; region sizes for `rows` A rows / `cols` B columns.
@@ -300,7 +306,7 @@ size_t tc_b_bytes(int32_t cols, int32_t k_tiles);
 int32_t gemm_k_tiles(int64_t K);
 cudaError_t tc_gemm(double2 *out, uint8_t const *scratch, int32_t const *expo,
                     TrTile const *tiles, int64_t n_tiles, int32_t k_tiles, int *err,
-                    cudaStream_t stream);
+                    cudaStream_t stream, int32_t const *entries = nullptr);
 
 // One GEMM operand row (A) or column (B) gathered from up to four strided
 // segments of a source array, each with an exact factor (0: +1, 1: +i, 2: -1,

@@ -121,17 +121,20 @@ __global__ void __launch_bounds__(kSliceThreads)
   }
 }
 
-// FP64 trace values of one tile: value (r, c) = (hi + lo) 2^(e_r + e_c - 14)
-// at values[out + c * ld + r], component row & 1 (re, im).
+// FP64 values of one tile (TrTile): value (r, c) = (hi + lo) 2^(e_r + e_c - 14),
+// component row & 1 (re, im).
 struct TraceEpilogue {
   double *values;
   int32_t const *expo;
   TrTile const *tiles;
-  // Lane k holds the exponents of the warp's columns k and 32 + k; the column
-  // loop takes them by warp shuffles.
+  int32_t const *entries;
+  // Lane k holds the exponents, and for stacked tiles the blocks and groups,
+  // of the warp's columns k and 32 + k; the column loop takes them by warp
+  // shuffles.
   struct Pre {
     TrTile t;
     int e0, e1, er;
+    int v0, v1;  // block v << 16 | group ib
   };
   __device__ __forceinline__ Pre prepare(int i, int row, int col0) const {
     Pre p;
@@ -140,6 +143,12 @@ struct TraceEpilogue {
     p.e0 = col0 + lane < p.t.cols ? expo[p.t.eb + col0 + lane] : 0;
     p.e1 = lane < kColsW - 32 && col0 + 32 + lane < p.t.cols ? expo[p.t.eb + col0 + 32 + lane] : 0;
     p.er = row / 2 < p.t.rows ? expo[p.t.ea + row / 2] : 0;
+    p.v0 = p.v1 = 0;
+    if (p.t.tab >= 0) {
+      int const c0 = p.t.col0 + col0 + lane, c1 = c0 + 32;
+      p.v0 = (c0 / p.t.n_b) << 16 | (c0 % p.t.n_b);
+      p.v1 = (c1 / p.t.n_b) << 16 | (c1 % p.t.n_b);
+    }
     return p;
   }
   __device__ __forceinline__ void operator()(Pre const &p, int i, int row, int col0,
@@ -148,13 +157,34 @@ struct TraceEpilogue {
     TrTile const &t = p.t;
     int const r = row / 2;
     bool const row_ok = r < t.rows;
-    double *dst = values + 2 * (t.out + r) + (row & 1);
+    if (t.tab < 0) {
+      double *dst = values + 2 * (t.out + r) + (row & 1);
+#pragma unroll
+      for (int c = 0; c < kColsW; ++c) {
+        int const ec = __shfl_sync(0xffffffffu, c < 32 ? p.e0 : p.e1, c % 32);
+        int const col = col0 + c;
+        if (row_ok && col < t.cols)
+          dst[2 * static_cast<int64_t>(col) * t.ld] =
+              ldexp(static_cast<double>(hi[c]) + static_cast<double>(lo[c]), p.er + ec - 14);
+      }
+      return;
+    }
+    int const u = (t.row0 + r) / t.n_a, ia = (t.row0 + r) % t.n_a;
+    int32_t const *tab = entries + t.tab + static_cast<int64_t>(u) * t.tab_ld;
+    int64_t const plane = static_cast<int64_t>(t.n_a) * t.n_b;
+    double *dst = values + 2 * (t.out + ia) + (row & 1);
+    int v_at = -1, e_at = -1;  // the entry of the current block of columns
 #pragma unroll
     for (int c = 0; c < kColsW; ++c) {
       int const ec = __shfl_sync(0xffffffffu, c < 32 ? p.e0 : p.e1, c % 32);
-      int const col = col0 + c;
-      if (row_ok && col < t.cols)
-        dst[2 * static_cast<int64_t>(col) * t.ld] =
+      int const vb = __shfl_sync(0xffffffffu, c < 32 ? p.v0 : p.v1, c % 32);
+      if (!row_ok || col0 + c >= t.cols) continue;
+      if (vb >> 16 != v_at) {
+        v_at = vb >> 16;
+        e_at = tab[v_at];
+      }
+      if (e_at >= 0)
+        dst[2 * (e_at * plane + static_cast<int64_t>(vb & 0xFFFF) * t.n_a)] =
             ldexp(static_cast<double>(hi[c]) + static_cast<double>(lo[c]), p.er + ec - 14);
     }
   }
@@ -177,9 +207,10 @@ struct TraceSrc {
 
 __global__ void __launch_bounds__(kThreads, 1)
     trace_gemm_kernel(double2 *values, uint8_t const *scratch, int32_t const *expo,
-                      TrTile const *tiles, int32_t n_tiles, int32_t k_tiles, int *err) {
+                      TrTile const *tiles, int32_t n_tiles, int32_t k_tiles,
+                      int32_t const *entries, int *err) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  TraceEpilogue epi{reinterpret_cast<double *>(values), expo, tiles};
+  TraceEpilogue epi{reinterpret_cast<double *>(values), expo, tiles, entries};
   ozaki_tiles(smem, n_tiles, k_tiles, TraceSrc{scratch, tiles}, err, epi);
 }
 
@@ -226,7 +257,7 @@ size_t tc_b_bytes(int32_t cols, int32_t k_tiles) {
 
 cudaError_t tc_gemm(double2 *out, uint8_t const *scratch, int32_t const *expo,
                     TrTile const *tiles, int64_t n_tiles, int32_t k_tiles, int *err,
-                    cudaStream_t stream) {
+                    cudaStream_t stream, int32_t const *entries) {
   if (n_tiles == 0) return cudaSuccess;
   if (k_tiles < 1) return cudaErrorInvalidValue;
   cudaError_t e = cudaFuncSetAttribute(trace_gemm_kernel,
@@ -237,16 +268,16 @@ cudaError_t tc_gemm(double2 *out, uint8_t const *scratch, int32_t const *expo,
     int64_t const n = n_tiles - t0 < 0x7fffffffLL ? n_tiles - t0 : 0x7fffffffLL;
     trace_gemm_kernel<<<static_cast<unsigned>(persistent_grid(n)), kThreads, kSmemBytes,
                         stream>>>(out, scratch, expo, tiles + t0, static_cast<int32_t>(n),
-                                  k_tiles, err);
+                                  k_tiles, entries, err);
   }
   return cudaGetLastError();
 }
 
 cudaError_t trace_tc_gemm(double2 *values, uint8_t const *scratch, int32_t const *expo,
-                          TrTile const *tiles, int64_t n_tiles, int32_t eds, int *err,
-                          cudaStream_t stream) {
+                          TrTile const *tiles, int64_t n_tiles, int32_t const *entries,
+                          int32_t eds, int *err, cudaStream_t stream) {
   return tc_gemm(values, scratch, expo, tiles, n_tiles,
-                 static_cast<int32_t>(trace_tc_k_tiles(eds)), err, stream);
+                 static_cast<int32_t>(trace_tc_k_tiles(eds)), err, stream, entries);
 }
 
 }  // namespace dev
