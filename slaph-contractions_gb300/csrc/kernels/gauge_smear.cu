@@ -12,9 +12,12 @@
 //          replaces U(s,d) by P(U(s,d) (1 - a1) + (a1 / 4) outer).
 // Only a thread's own link is read from U in the outer launch, so it updates U
 // in place.  P is proj_to_su3_imp (:203-210): M (M^H M)^(-1/2) scaled by the
-// principal cube root of 1/det, with (M^H M)^(-1/2) from a cyclic complex
-// Jacobi eigen-decomposition (the principal square root of a Hermitian
-// positive-definite matrix is V diag(sqrt(lambda)) V^H).
+// principal cube root of 1/det (proj_su3 below).
+//
+// Bound by FP64 issue (two multiply-adds per cycle and SM): about 1080
+// operations per decorated link and 1500 per outer link.  24^3x48, three
+// iterations: 134 ms with Jacobi eigen-decompositions of M^H M and FP64
+// transcendentals, 41 ms with the closed form.
 //
 // Sites and neighbours follow GaugeField::init (src/GaugeField.cpp:39-98) on a
 // cubic lattice: s = (x0 L + x1) L + x2, direction d steps x_d periodically.
@@ -42,14 +45,25 @@ __device__ __forceinline__ double2 cadd(double2 a, double2 b) {
 __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 __device__ __forceinline__ double cnorm(double2 a) { return a.x * a.x + a.y * a.y; }
 
-__device__ __forceinline__ double2 csub(double2 a, double2 b) {
-  return make_double2(a.x - b.x, a.y - b.y);
+// acc + a b, acc + conj(a) b, acc + a conj(b)
+__device__ __forceinline__ double2 cmac(double2 acc, double2 a, double2 b) {
+  return make_double2(fma(a.x, b.x, fma(-a.y, b.y, acc.x)), fma(a.x, b.y, fma(a.y, b.x, acc.y)));
+}
+__device__ __forceinline__ double2 cmac_hn(double2 acc, double2 a, double2 b) {
+  return make_double2(fma(a.x, b.x, fma(a.y, b.y, acc.x)), fma(a.x, b.y, fma(-a.y, b.x, acc.y)));
+}
+__device__ __forceinline__ double2 cmac_nh(double2 acc, double2 a, double2 b) {
+  return make_double2(fma(a.x, b.x, fma(a.y, b.y, acc.x)), fma(a.y, b.x, fma(-a.x, b.y, acc.y)));
+}
+// acc - a b
+__device__ __forceinline__ double2 cnmac(double2 acc, double2 a, double2 b) {
+  return make_double2(fma(-a.x, b.x, fma(a.y, b.y, acc.x)), fma(-a.x, b.y, fma(-a.y, b.x, acc.y)));
 }
 __device__ __forceinline__ double2 det3(M3 const &m) {
-  double2 const c0 = csub(cmul(m.e[4], m.e[8]), cmul(m.e[7], m.e[5]));
-  double2 const c1 = csub(cmul(m.e[1], m.e[8]), cmul(m.e[7], m.e[2]));
-  double2 const c2 = csub(cmul(m.e[1], m.e[5]), cmul(m.e[4], m.e[2]));
-  return cadd(csub(cmul(m.e[0], c0), cmul(m.e[3], c1)), cmul(m.e[6], c2));
+  double2 const c0 = cnmac(cmul(m.e[4], m.e[8]), m.e[7], m.e[5]);
+  double2 const c1 = cnmac(cmul(m.e[1], m.e[8]), m.e[7], m.e[2]);
+  double2 const c2 = cnmac(cmul(m.e[1], m.e[5]), m.e[4], m.e[2]);
+  return cmac(cnmac(cmul(m.e[0], c0), m.e[3], c1), m.e[6], c2);
 }
 
 __device__ __forceinline__ M3 load(double2 const *p) {
@@ -69,11 +83,9 @@ __device__ __forceinline__ M3 mul(M3 const &x, M3 const &y) {
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      double2 acc = cmul(x.e[a], y.e[3 * b]);
-      acc = cadd(acc, cmul(x.e[a + 3], y.e[1 + 3 * b]));
-      r.e[a + 3 * b] = cadd(acc, cmul(x.e[a + 6], y.e[2 + 3 * b]));
-    }
+    for (int b = 0; b < 3; ++b)
+      r.e[a + 3 * b] = cmac(cmac(cmul(x.e[a], y.e[3 * b]), x.e[a + 3], y.e[1 + 3 * b]),
+                            x.e[a + 6], y.e[2 + 3 * b]);
   return r;
 }
 __device__ __forceinline__ M3 mul_hn(M3 const &x, M3 const &y) {
@@ -81,11 +93,10 @@ __device__ __forceinline__ M3 mul_hn(M3 const &x, M3 const &y) {
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      double2 acc = cmul(cconj(x.e[3 * a]), y.e[3 * b]);
-      acc = cadd(acc, cmul(cconj(x.e[1 + 3 * a]), y.e[1 + 3 * b]));
-      r.e[a + 3 * b] = cadd(acc, cmul(cconj(x.e[2 + 3 * a]), y.e[2 + 3 * b]));
-    }
+    for (int b = 0; b < 3; ++b)
+      r.e[a + 3 * b] = cmac_hn(cmac_hn(cmul(cconj(x.e[3 * a]), y.e[3 * b]), x.e[1 + 3 * a],
+                                       y.e[1 + 3 * b]),
+                               x.e[2 + 3 * a], y.e[2 + 3 * b]);
   return r;
 }
 __device__ __forceinline__ M3 mul_nh(M3 const &x, M3 const &y) {
@@ -93,79 +104,131 @@ __device__ __forceinline__ M3 mul_nh(M3 const &x, M3 const &y) {
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      double2 acc = cmul(x.e[a], cconj(y.e[b]));
-      acc = cadd(acc, cmul(x.e[a + 3], cconj(y.e[b + 3])));
-      r.e[a + 3 * b] = cadd(acc, cmul(x.e[a + 6], cconj(y.e[b + 6])));
-    }
+    for (int b = 0; b < 3; ++b)
+      r.e[a + 3 * b] = cmac_nh(cmac_nh(cmul(x.e[a], cconj(y.e[b])), x.e[a + 3], y.e[b + 3]),
+                               x.e[a + 6], y.e[b + 6]);
   return r;
 }
 
-// G^H H G and V G for the Jacobi rotation of the pair (p, q): G is the
-// identity but for G(p,p) = c, G(p,q) = s, G(q,p) = -s conj(ph),
-// G(q,q) = c conj(ph), with ph the phase of H(p,q).
-__device__ __forceinline__ void rotate(M3 &h, M3 &v, int p, int q, double c, double s,
-                                       double2 ph) {
-  double2 const phc = cconj(ph);
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {  // columns p, q of H G and V G
-    double2 const hp = h.e[i + 3 * p], hq = cmul(phc, h.e[i + 3 * q]);
-    h.e[i + 3 * p] = make_double2(c * hp.x - s * hq.x, c * hp.y - s * hq.y);
-    h.e[i + 3 * q] = make_double2(s * hp.x + c * hq.x, s * hp.y + c * hq.y);
-    double2 const vp = v.e[i + 3 * p], vq = cmul(phc, v.e[i + 3 * q]);
-    v.e[i + 3 * p] = make_double2(c * vp.x - s * vq.x, c * vp.y - s * vq.y);
-    v.e[i + 3 * q] = make_double2(s * vp.x + c * vq.x, s * vp.y + c * vq.y);
-  }
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {  // rows p, q of G^H (H G)
-    double2 const hp = h.e[p + 3 * j], hq = cmul(ph, h.e[q + 3 * j]);
-    h.e[p + 3 * j] = make_double2(c * hp.x - s * hq.x, c * hp.y - s * hq.y);
-    h.e[q + 3 * j] = make_double2(s * hp.x + c * hq.x, s * hp.y + c * hq.y);
-  }
-  h.e[p + 3 * q] = h.e[q + 3 * p] = make_double2(0, 0);
-}
-
-__device__ __forceinline__ void jacobi_pair(M3 &h, M3 &v, int p, int q) {
-  double2 const apq = h.e[p + 3 * q];
-  double const r = hypot(apq.x, apq.y);
-  if (r == 0) return;
-  double2 const ph = make_double2(apq.x / r, apq.y / r);
-  double const th = (h.e[q + 3 * q].x - h.e[p + 3 * p].x) / (2 * r);
-  double const t = (th >= 0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1));
-  double const c = 1 / sqrt(t * t + 1);
-  rotate(h, v, p, q, c, t * c, ph);
-}
-
-// proj_to_su3_imp (src/GaugeField.cpp:203-210).
+// proj_to_su3_imp (src/GaugeField.cpp:203-210) in closed form.  With A = M^H M
+// and u, v, w the elementary symmetric functions of the singular values of M
+// (the square roots of A's eigenvalues), the Cayley-Hamilton theorem gives
+//   A^(-1/2) = f0 + f1 A + f2 A^2,  d = w (u v - w),
+//   f0 = (u v^2 - w (u^2 + v)) / d, f1 = (2 u v - u^3 - w) / d, f2 = u / d
+// (Hasenfratz, Hoffmann, Schaefer, JHEP 05 (2007) 029); d is a product of sums
+// of singular values, so nothing cancels where they approach one another.
+// w = |det M|; u is the largest root of (u^2 - tr A)^2 - 8 w u - 4 c2 (c2 the
+// sum of A's principal minors), found by Newton's method from above, where the
+// quartic is convex: FP32 steps from sqrt(3 tr A), then FP64 steps until the
+// next correction is negligible; v = (u^2 - tr A) / 2.  The determinant of
+// M A^(-1/2) is det M / w: its principal root y = (det M / w)^(-1/3) comes from
+// FP32 and two FP64 Newton steps y (4 - y^3 z) / 3.  One Newton step of the
+// polar decomposition, X -> (X + X^(-H)) / 2, ends it: whatever error of f0, f1,
+// f2 is left enters squared, and the result is more accurate than one from
+// A's eigenvectors (1.2e-16 rms against 3.7e-16 on blends with singular values
+// 0.7 .. 1; 8.8e-16 without the step).
 __device__ M3 proj_su3(M3 const &m) {
-  M3 h = mul_hn(m, m), v;
+  // A: diagonal a0, a1, a2 and upper entries p = A01, q = A02, r = A12
+  double a[3];
 #pragma unroll
-  for (int i = 0; i < 9; ++i) v.e[i] = make_double2(i % 4 == 0 ? 1.0 : 0.0, 0.0);
-  for (int sweep = 0; sweep < 30; ++sweep) {
-    double const off = cnorm(h.e[3]) + cnorm(h.e[6]) + cnorm(h.e[7]);
-    double const diag = cnorm(h.e[0]) + cnorm(h.e[4]) + cnorm(h.e[8]);
-    if (off <= 1e-32 * diag) break;
-    jacobi_pair(h, v, 0, 1);
-    jacobi_pair(h, v, 0, 2);
-    jacobi_pair(h, v, 1, 2);
+  for (int i = 0; i < 3; ++i) {
+    a[i] = cnorm(m.e[3 * i]);
+#pragma unroll
+    for (int k = 1; k < 3; ++k)
+      a[i] = fma(m.e[k + 3 * i].x, m.e[k + 3 * i].x,
+                 fma(m.e[k + 3 * i].y, m.e[k + 3 * i].y, a[i]));
   }
-  // X = V diag(lambda^-1/2) V^H, out = M X
-  double d[3];
+  auto dot = [&](int i, int j) {
+    return cmac_hn(cmac_hn(cmul(cconj(m.e[3 * i]), m.e[3 * j]), m.e[1 + 3 * i], m.e[1 + 3 * j]),
+                   m.e[2 + 3 * i], m.e[2 + 3 * j]);
+  };
+  double2 const p = dot(0, 1), q = dot(0, 2), r = dot(1, 2);
+  double const np = cnorm(p), nq = cnorm(q), nr = cnorm(r);
+  double const c1 = a[0] + a[1] + a[2];
+  double const c2 = (fma(a[0], a[1], -np) + fma(a[0], a[2], -nq)) + fma(a[1], a[2], -nr);
+  double2 const det = det3(m);
+  double const d2 = cnorm(det);
+  double const iw = rsqrt(d2);
+  double const w = d2 * iw;
+  // in units of sqrt(tr A) while in FP32
+  double const is = rsqrt(c1), is2 = is * is;
+  float const t2 = static_cast<float>(4 * c2 * is2 * is2),
+              tw = static_cast<float>(8 * w * is2 * is);
+  float x0 = 1.7320508f;
 #pragma unroll
-  for (int i = 0; i < 3; ++i) d[i] = 1 / sqrt(h.e[4 * i].x);
-  M3 vd;
+  for (int k = 0; k < 6; ++k) {
+    float const g = x0 * x0 - 1.f, dp = 4.f * x0 * g - tw;
+    float const step = (g * g - tw * x0 - t2) / dp;
+    if (step > 0.f) x0 -= step;  // from above; rounding ends the descent
+  }
+  double u = static_cast<double>(x0) * (c1 * is);
+  for (int k = 0; k < 30; ++k) {
+    double const g = fma(u, u, -c1);
+    double const pu = fma(g, g, -fma(8 * w, u, 4 * c2));
+    double const step = pu / fma(4 * u, g, -8 * w);
+    u -= step;
+    if (!(fabs(step) > 1e-5 * u)) break;  // quadratic: the next step is about 1e-10
+  }
+  double const v = 0.5 * fma(u, u, -c1);
+  double const uv = u * v;
+  double const id = iw / (uv - w);
+  double const f2 = u * id;
+  double const f1 = (fma(2.0, uv, -w) - u * u * u) * id;
+  double const f0 = fma(uv, v, -w * fma(u, u, v)) * id;
+  // B = f0 + f1 A + f2 A^2 (Hermitian, same storage as A)
+  double const b0 = fma(f2, fma(a[0], a[0], np + nq), fma(f1, a[0], f0));
+  double const b1 = fma(f2, fma(a[1], a[1], np + nr), fma(f1, a[1], f0));
+  double const b2 = fma(f2, fma(a[2], a[2], nq + nr), fma(f1, a[2], f0));
+  // (A^2)01 = A01 (a0 + a1) + A02 conj(A12) and so on
+  auto off = [&](double2 z, double s, double2 zz) {
+    double const c = fma(f2, s, f1);
+    return make_double2(fma(c, z.x, f2 * zz.x), fma(c, z.y, f2 * zz.y));
+  };
+  double2 const zero = make_double2(0, 0);
+  double2 const bp = off(p, a[0] + a[1], cmac_nh(zero, q, r));
+  double2 const bq = off(q, a[0] + a[2], cmul(p, r));
+  double2 const br = off(r, a[1] + a[2], cmac_hn(zero, p, q));
+  // y = (det / w)^(-1/3)
+  double2 const z = make_double2(det.x * iw, det.y * iw);
+  float sf, cf;
+  sincosf(-atan2f(static_cast<float>(z.y), static_cast<float>(z.x)) / 3.f, &sf, &cf);
+  double2 y = make_double2(static_cast<double>(cf), static_cast<double>(sf));
 #pragma unroll
-  for (int i = 0; i < 9; ++i) vd.e[i] = make_double2(v.e[i].x * d[i / 3], v.e[i].y * d[i / 3]);
-  M3 out = mul(m, mul_nh(vd, v));
-  // det^(-1/3) on the principal branch
-  double2 const det = det3(out);
-  double const mag = pow(hypot(det.x, det.y), -1.0 / 3.0);
-  double sn, cs;
-  sincos(-atan2(det.y, det.x) / 3.0, &sn, &cs);
-  double2 const f = make_double2(mag * cs, mag * sn);
+  for (int k = 0; k < 2; ++k) {
+    double2 const y3z = cmul(cmul(cmul(y, y), y), z);
+    y = cmul(y, make_double2((4.0 - y3z.x) * (1.0 / 3.0), -y3z.y * (1.0 / 3.0)));
+  }
+  M3 x;
 #pragma unroll
-  for (int i = 0; i < 9; ++i) out.e[i] = cmul(out.e[i], f);
-  return out;
+  for (int i = 0; i < 3; ++i) {
+    double2 const m0 = cmul(m.e[i], y), m1 = cmul(m.e[i + 3], y), m2 = cmul(m.e[i + 6], y);
+    auto real = [](double2 acc, double2 t, double s) {
+      return make_double2(fma(t.x, s, acc.x), fma(t.y, s, acc.y));
+    };
+    // columns of B: (b0, conj p, conj q), (p, b1, conj r), (q, r, b2)
+    x.e[i] = cmac_nh(cmac_nh(make_double2(m0.x * b0, m0.y * b0), m1, bp), m2, bq);
+    x.e[i + 3] = cmac_nh(real(cmul(m0, bp), m1, b1), m2, br);
+    x.e[i + 6] = real(cmac(cmul(m0, bq), m1, br), m2, b2);
+  }
+  // (X + conj(cof X) / conj(det X)) / 2
+  M3 cf3;
+#pragma unroll
+  for (int b = 0; b < 3; ++b)
+#pragma unroll
+    for (int a1 = 0; a1 < 3; ++a1) {
+      int const r1 = (a1 + 1) % 3, r2 = (a1 + 2) % 3, s1 = 3 * ((b + 1) % 3), s2 = 3 * ((b + 2) % 3);
+      cf3.e[a1 + 3 * b] = cnmac(cmul(x.e[r1 + s1], x.e[r2 + s2]), x.e[r1 + s2], x.e[r2 + s1]);
+    }
+  double2 const dx =
+      cmac(cmac(cmul(x.e[0], cf3.e[0]), x.e[1], cf3.e[1]), x.e[2], cf3.e[2]);
+  double const h = 0.5 / cnorm(dx);
+  double2 const hd = make_double2(dx.x * h, dx.y * h);  // 1 / (2 conj(det X))
+#pragma unroll
+  for (int i = 0; i < 9; ++i) {
+    double2 const t = cmul(hd, cconj(cf3.e[i]));
+    x.e[i] = make_double2(fma(0.5, x.e[i].x, t.x), fma(0.5, x.e[i].y, t.y));
+  }
+  return x;
 }
 
 __device__ __forceinline__ int64_t step(int64_t s, int dir, int L, int delta) {
@@ -223,7 +286,7 @@ __global__ void hyp_outer_kernel(double2 *U, double2 const *dec, int32_t L, int6
   M3 outer;
 #pragma unroll
   for (int i = 0; i < 9; ++i) outer.e[i] = make_double2(0, 0);
-#pragma unroll
+#pragma unroll 1  // (unrolled: 244 registers, half the warps per SM)
   for (int nd = 0; nd < 3; ++nd) {
     if (nd == dir) continue;
     int const plane = 3 - dir - nd;
