@@ -405,21 +405,27 @@ void Engine::vdaggerv_build(int precision) {
   bool const tc_disp = precision == SLAPH_MIXED && !displaced.empty();
   dev::VdvDisplaced dd{};
   std::vector<int32_t> d_steps, d_n;
-  if (tc_disp) {
-    W_.reserve(sizeof(double2) * static_cast<size_t>(geo_.dim_row) * dims_.nev);
+  if (!displaced.empty()) {
+    bool several = false, backward = false;
     d_steps.assign(2 * dev::kMaxDispSteps * displaced.size(), 0);
     for (size_t k = 0; k < displaced.size(); ++k) {
       slaph_vdv_op const &op = ops_[displaced[k]];
       if (op.n_disp > dev::kMaxDispSteps) throw UnsupportedError("too many displacement steps");
       d_n.push_back(op.n_disp);
+      several = several || op.n_disp > 1;
       for (int32_t s = 0; s < op.n_disp; ++s) {
         char const ax = op.disp[2 * s + 1];
         d_steps[2 * (k * dev::kMaxDispSteps + s)] = ax == 'x' ? 0 : ax == 'y' ? 1 : 2;
         d_steps[2 * (k * dev::kMaxDispSteps + s) + 1] = op.disp[2 * s] == '>' ? 1 : 0;
+        backward = backward || op.disp[2 * s] != '>';
       }
     }
+    W_.reserve(sizeof(double2) * static_cast<size_t>(geo_.dim_row) * dims_.nev *
+               (several ? 2 : 1));
+    if (backward) line_p_.reserve(U_.size());
     dd = dev::VdvDisplaced{static_cast<int32_t>(displaced.size()), d_n.data(), d_steps.data(),
-                           U_.as<double2>(), W_.as<double2>()};
+                           U_.as<double2>(), backward ? line_p_.as<double2>() : nullptr,
+                           W_.as<double2>()};
   }
   int32_t n_gemm = 0;     // GEMM launches of the whole build
   int64_t batch_fit = 1;  // timeslices per GEMM launch
@@ -469,12 +475,12 @@ void Engine::vdaggerv_build(int precision) {
   size_t const n_v = static_cast<size_t>(geo_.dim_row) * dims_.nev;  // per timeslice
   size_t const links = static_cast<size_t>(geo_.dim_row / 3) * 27;
   bool const fp64_disp = !displaced.empty() && !tc_disp;
-  if (fp64_disp) {
-    W_.reserve(sizeof(double2) * n_v);
-    upload(disp_ops_, displaced, stream_);
-  }
+  if (fp64_disp) upload(disp_ops_, displaced, stream_);
   int64_t disp_launches = 0;  // per timeslice, split-precision displaced operators
   for (int32_t n : d_n) disp_launches += n + 2;
+  if (dd.P)
+    launch(dev::line_products(line_p_.as<double2>(), U_.as<double2>(), geo_, stream_),
+           "line_products");
   int32_t gemm_done = 0;
   for (size_t c = 0; c < ranges.size(); ++c) {
     int32_t const t0 = ranges[c].first, nt = ranges[c].second;
@@ -522,22 +528,21 @@ void Engine::vdaggerv_build(int precision) {
     // V_t^H W in FP64 (src/OperatorFactory.cpp:289-290, 300); the momentum is
     // not applied.
     if (fp64_disp) {
-      for (int32_t t = t0; t < t0 + nt; ++t)
+      for (int32_t t = t0; t < t0 + nt; ++t) {
+        double2 const *Ut = U_.as<double2>() + links * t;
+        double2 const *Pt = dd.P ? dd.P + links * t : nullptr;
         for (size_t k = 0; k < displaced.size(); ++k) {
-          slaph_vdv_op const &op = ops_[displaced[k]];
-          SLAPH_CK(cudaMemcpyAsync(W_.as<double2>(), Vb + n_v * (t - v_t0),
-                                   n_v * sizeof(double2), cudaMemcpyDeviceToDevice, stream_));
-          for (int32_t st = 0; st < op.n_disp; ++st) {
-            char const ax = op.disp[2 * st + 1];
-            launch(dev::displace(W_.as<double2>(), U_.as<double2>() + links * t,
-                                 ax == 'x' ? 0 : ax == 'y' ? 1 : 2,
-                                 op.disp[2 * st] == '>' ? 1 : 0, geo_, stream_),
-                   "displace");
-          }
-          launch(dev::vdaggerv_fp64_w(vdv_.as<double2>(), Vb, W_.as<double2>(),
-                                      disp_ops_.as<int32_t>() + k, t, geo_, stream_, v_t0),
+          double2 const *Wt = nullptr;
+          launch(dev::displaced_vectors(&Wt, dd.W, Vb + n_v * (t - v_t0), Ut, Pt,
+                                        d_steps.data() + 2 * dev::kMaxDispSteps * k, d_n[k], geo_,
+                                        stream_),
+                 "displaced_vectors");
+          launches_ += d_n[k] - 1;
+          launch(dev::vdaggerv_fp64_w(vdv_.as<double2>(), Vb, Wt, disp_ops_.as<int32_t>() + k, t,
+                                      geo_, stream_, v_t0),
                  "vdaggerv_fp64_w");
         }
+      }
     }
     if (ring_slots_ > 0) SLAPH_CK(cudaEventRecord(ev_half_[c % 2], stream_));
   }

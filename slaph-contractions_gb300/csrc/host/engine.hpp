@@ -167,7 +167,9 @@ class Engine {
   DevBuf slot_bits_;  // largest |re|, |im| of every double-float matrix slot (mixed path)
   int read_err_flag();  // the device error flag, through host_rb_ on the engine stream
   std::vector<slaph_vdv_op> ops_;
-  DevBuf U_, W_, disp_ops_;  // gauge links, displaced eigenvector scratch, displaced op ids
+  // gauge links, displaced eigenvector scratch, displaced op ids, line products
+  // of the links
+  DevBuf U_, W_, disp_ops_, line_p_;
   DevBuf hyp_dec_;           // decorated links of a chunk of timeslices (HYP smearing)
   // Momentum families of the operator table (set_operators): those of the FP64
   // build, and the split-precision plan (displaced operators included).

@@ -62,9 +62,6 @@ int32_t gamma_row_host(int32_t m, int32_t c);
 int32_t gamma_phase_host(int32_t m, int32_t c);
 cudaError_t upload_gamma(cudaStream_t stream);
 
-// One displacement step of W (a copy of V_t) in place on a cubic lattice, in
-// the reference's sweep order (displace_eigenvectors,
-// src/OperatorFactory.cpp:33-55); U: the timeslice's links [site][dir][a + 3 b].
 // One HYP smearing iteration (GaugeField::smearing_hyp, src/GaugeField.cpp:
 // 322-427) of n_t consecutive timeslices of links U ([t][site][dir][9]) of a
 // cubic L^3 lattice, in place; dec: scratch of n_t
@@ -72,8 +69,16 @@ cudaError_t upload_gamma(cudaStream_t stream);
 int64_t hyp_scratch_doubles_per_timeslice(int32_t L);
 cudaError_t hyp_smear(double2 *U, double2 *dec, int32_t L, int32_t n_t, double alpha1,
                       double alpha2, cudaStream_t stream);
-cudaError_t displace(double2 *W, double2 const *U, int32_t dir, int32_t forward, Geometry g,
-                     cudaStream_t stream);
+// Displaced eigenvectors D(V_t) on a cubic lattice: n steps ((dir 0..2, forward
+// 0/1) pairs, host array) with the result of the reference's in-place sweeps
+// (displace_eigenvectors, src/OperatorFactory.cpp:33-55).  U: the timeslice's
+// links [site][dir][a + 3 b]; P: the timeslice's line_products (read by backward
+// steps only); W: scratch of nev x dim_row, twice that for n > 1.  *out: the
+// result, in W.  line_products: of all g.Lt timeslices, in the layout of U.
+cudaError_t line_products(double2 *P, double2 const *U, Geometry g, cudaStream_t stream);
+cudaError_t displaced_vectors(double2 const **out, double2 *W, double2 const *V, double2 const *U,
+                              double2 const *P, int32_t const *steps, int32_t n, Geometry g,
+                              cudaStream_t stream);
 // VdaggerV[2 op][t] = V_t^H W in FP64 (*op: device pointer to the operator id).
 cudaError_t vdaggerv_fp64_w(double2 *vdv, double2 const *V, double2 const *W,
                             int32_t const *op, int32_t t, Geometry g, cudaStream_t stream,
@@ -124,15 +129,16 @@ cudaError_t unit_roots(double2 *roots, int32_t n_planes, cudaStream_t stream);
 int32_t vdaggerv_tc_batch(Geometry g, VdvTcPlan const &pl, int32_t sm_count, size_t max_bytes,
                           int32_t n_t);
 // Displaced operators of the split-precision VdaggerV: family n_mom + d is
-// V_t^H D_d(V_t), D_d the displacement steps of operator d applied in place to
-// a copy W of V_t (displace above), momentum not applied.
+// V_t^H D_d(V_t), D_d the displacement steps of operator d (displaced_vectors
+// above), momentum not applied.
 constexpr int kMaxDispSteps = 8;
 struct VdvDisplaced {
   int32_t n;                     // number of displaced operators
   int32_t const *n_steps;        // host: steps per operator
   int32_t const *steps;          // host: [n][kMaxDispSteps][2] (dir 0..2, forward 0/1)
   double2 const *U;              // device: links [Lt][site][dir][9]
-  double2 *W;                    // device: nev x dim_row scratch
+  double2 const *P;              // device: line_products of U, null without backward steps
+  double2 *W;                    // device scratch of displaced_vectors
 };
 cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, VdvTcPlan const &pl, int32_t t0,
                         int32_t nt, Geometry g, void *scratch, size_t scratch_bytes, int *err,

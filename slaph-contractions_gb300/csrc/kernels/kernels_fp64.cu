@@ -510,81 +510,147 @@ cudaError_t momenta(double2 *phase, int32_t const *mom, int32_t n_ops, Geometry 
 }
 
 // displace_eigenvectors (src/OperatorFactory.cpp:33-55) for one step on a
-// cubic lattice: W (a copy of V_t) is updated in place line by line, each line
-// of the step's direction in increasing site index as the reference sweeps
-// it, so a site reads the already-displaced value of a preceding neighbour.
-// Forward: W(s) = U(s, d) W(s + d); backward: W(s) = U(s - d, d)^H W(s - d)
-// (forward_uv / backward_uv, src/GaugeField.cpp:543-560).  U: links of the
-// timeslice, [site][dir][a + 3 b].  One thread per (eigenvector, line).
-__global__ void displace_kernel(double2 *W, double2 const *U, int32_t dir, int32_t forward,
-                                Geometry g) {
-  int const L = g.Lx;
+// cubic lattice.  The reference updates its copy in place, each line of the
+// step's direction in increasing site index, so a site reads the
+// already-displaced value of a preceding neighbour.  Forward, W(c) = U(c) V(c +
+// 1) for the sites c of a line, only the last site wraps to one: W(L - 1) =
+// U(L - 1) W(0).  Backward, W(c) = U(c - 1)^H W(c - 1) with W(0) = U(L - 1)^H
+// V(L - 1), every site is a product of links applied to V(L - 1): W(c) = P(c)
+// V(L - 1), P(0) = U(L - 1)^H, P(c) = U(c - 1)^H P(c - 1) (forward_uv /
+// backward_uv, src/GaugeField.cpp:543-560).  Out of place, all sites are
+// independent; P does not depend on the eigenvector and is formed once per
+// timeslice (line_products, all timeslices in one launch: a line is a serial
+// chain of L products: 105 us for one timeslice at 24^3, 440 us for 48).
+
+namespace {
+
+struct Line {
+  int64_t base, stride;
+  int c;
+};
+__device__ __forceinline__ Line line_of(int64_t s, int dir, int L) {
+  int64_t const stride = dir == 0 ? static_cast<int64_t>(L) * L : dir == 1 ? L : 1;
+  int const c = static_cast<int>(s / stride % L);
+  return {s - c * stride, stride, c};
+}
+
+// P(c) of every line of direction blockIdx.y and timeslice blockIdx.z, one
+// thread per line: [t][site][dir][a + 3 b].
+__global__ void line_product_kernel(double2 *P, double2 const *U, int32_t L) {
   int64_t const lines = static_cast<int64_t>(L) * L;
-  int64_t const k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (k >= lines * g.nev) return;
-  int64_t const ev = k / lines, l = k % lines;
-  int64_t stride, base;
-  if (dir == 0) {
-    stride = lines;
-    base = l;
-  } else if (dir == 1) {
-    stride = L;
-    base = (l / L) * lines + (l % L);
-  } else {
-    stride = 1;
-    base = l * L;
-  }
-  double2 *col = W + ev * g.dim_row;
-  double2 carry[3];  // forward: updated first site; backward: updated previous site
+  int64_t const l = gidx();
+  int const dir = blockIdx.y;
+  if (l >= lines) return;
+  P += blockIdx.z * lines * L * 27;
+  U += blockIdx.z * lines * L * 27;
+  int64_t const stride = dir == 0 ? lines : dir == 1 ? L : 1;
+  int64_t const base = dir == 0 ? l : dir == 1 ? (l / L) * lines + l % L : l * L;
+  double2 p[9], u[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) p[k] = make_double2(k % 4 == 0 ? 1.0 : 0.0, 0.0);
   for (int c = 0; c < L; ++c) {
-    int64_t const s = base + c * stride;
-    double2 v[3], out[3];
-    double2 const *u;
-    if (forward) {
-      int64_t const up = base + ((c + 1) % L) * stride;
-      bool const updated = c + 1 == L && c > 0;  // the wrap reads the updated first site
+    double2 const *src = U + ((base + (c + L - 1) % L * stride) * 3 + dir) * 9;
 #pragma unroll
-      for (int b = 0; b < 3; ++b) v[b] = updated ? carry[b] : col[3 * up + b];
-      u = U + (s * 3 + dir) * 9;
+    for (int k = 0; k < 9; ++k) u[k] = src[k];
+    double2 *dst = P + ((base + c * stride) * 3 + dir) * 9;
+    double2 r[9];
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
         double2 acc = make_double2(0, 0);
 #pragma unroll
-        for (int b = 0; b < 3; ++b) cfma(acc, u[a + 3 * b], v[b]);
-        out[a] = acc;
-      }
-      if (c == 0)
-#pragma unroll
-        for (int a = 0; a < 3; ++a) carry[a] = out[a];
-    } else {
-      int64_t const dn = base + ((c + L - 1) % L) * stride;
-#pragma unroll
-      for (int b = 0; b < 3; ++b) v[b] = c == 0 ? col[3 * dn + b] : carry[b];
-      u = U + (dn * 3 + dir) * 9;
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        double2 acc = make_double2(0, 0);
-#pragma unroll
-        for (int b = 0; b < 3; ++b) {
-          double2 const ub = u[b + 3 * a];
-          cfma(acc, make_double2(ub.x, -ub.y), v[b]);
-        }
-        out[a] = acc;
+        for (int k = 0; k < 3; ++k) cfmac(acc, u[k + 3 * a], p[k + 3 * b]);
+        r[a + 3 * b] = acc;
+        dst[a + 3 * b] = acc;
       }
 #pragma unroll
-      for (int a = 0; a < 3; ++a) carry[a] = out[a];
-    }
-#pragma unroll
-    for (int a = 0; a < 3; ++a) col[3 * s + a] = out[a];
+    for (int k = 0; k < 9; ++k) p[k] = r[k];
   }
 }
 
-cudaError_t displace(double2 *W, double2 const *U, int32_t dir, int32_t forward, Geometry g,
-                     cudaStream_t stream) {
-  if (dir < 0 || dir > 2 || g.Lx != g.Ly || g.Lx != g.Lz) return cudaErrorInvalidValue;
-  int64_t const n = static_cast<int64_t>(g.Lx) * g.Lx * g.nev;
-  displace_kernel<<<blocks_for(n, 128), 128, 0, stream>>>(W, U, dir, forward, g);
+// One thread per site, kDispEv eigenvectors with the site's matrix in
+// registers.  Bound by FP64 issue (36 multiply-adds per site and eigenvector).
+constexpr int kDispEv = 8;
+__global__ void __launch_bounds__(128)
+    displace_kernel(double2 *W, double2 const *V, double2 const *M, int32_t dir, int32_t forward,
+                    Geometry g) {
+  int const L = g.Lx;
+  int64_t const s = gidx();
+  if (s >= g.dim_row / 3) return;
+  Line const ln = line_of(s, dir, L);
+  double2 m[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) m[k] = M[(s * 3 + dir) * 9 + k];
+  bool const wrap = forward && ln.c + 1 == L && L > 1;
+  int64_t const from = forward ? ln.base + (wrap ? 1 : (ln.c + 1) % L) * ln.stride
+                               : ln.base + (L - 1) * ln.stride;
+  if (wrap) {  // U(L - 1) U(0), applied to V(1)
+    double2 const *u0 = M + (ln.base * 3 + dir) * 9;
+    double2 r[9];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        double2 acc = make_double2(0, 0);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) cfma(acc, m[a + 3 * k], u0[k + 3 * b]);
+        r[a + 3 * b] = acc;
+      }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) m[k] = r[k];
+  }
+  int const e0 = blockIdx.y * kDispEv, e1 = min(g.nev, e0 + kDispEv);
+  for (int ev = e0; ev < e1; ++ev) {
+    double2 const *src = V + ev * g.dim_row + 3 * from;
+    double2 v[3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b) v[b] = src[b];
+    double2 *dst = W + ev * g.dim_row + 3 * s;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      double2 acc = make_double2(0, 0);
+#pragma unroll
+      for (int b = 0; b < 3; ++b) cfma(acc, m[a + 3 * b], v[b]);
+      dst[a] = acc;
+    }
+  }
+}
+
+}  // namespace
+
+cudaError_t line_products(double2 *P, double2 const *U, Geometry g, cudaStream_t stream) {
+  if (g.Lx != g.Ly || g.Lx != g.Lz) return cudaErrorInvalidValue;
+  int64_t const lines = static_cast<int64_t>(g.Lx) * g.Lx;
+  for (int32_t t = 0; t < g.Lt; t += 65535) {
+    int64_t const at = t * lines * g.Lx * 27;
+    line_product_kernel<<<dim3(blocks_for(lines, 32), 3, g.Lt - t < 65535 ? g.Lt - t : 65535), 32,
+                          0, stream>>>(P + at, U + at, g.Lx);
+  }
   return cudaGetLastError();
+}
+
+cudaError_t displace(double2 *W, double2 const *V, double2 const *U, double2 const *P,
+                     int32_t dir, int32_t forward, Geometry g, cudaStream_t stream) {
+  if (dir < 0 || dir > 2 || g.Lx != g.Ly || g.Lx != g.Lz) return cudaErrorInvalidValue;
+  displace_kernel<<<dim3(blocks_for(g.dim_row / 3, 128), blocks_for(g.nev, kDispEv)), 128, 0,
+                    stream>>>(W, V, forward ? U : P, dir, forward, g);
+  return cudaGetLastError();
+}
+
+cudaError_t displaced_vectors(double2 const **out, double2 *W, double2 const *V, double2 const *U,
+                              double2 const *P, int32_t const *steps, int32_t n, Geometry g,
+                              cudaStream_t stream) {
+  int64_t const n_v = static_cast<int64_t>(g.nev) * g.dim_row;
+  double2 const *src = V;
+  for (int32_t k = 0; k < n; ++k) {
+    double2 *dst = W + (k % 2) * n_v;
+    cudaError_t const e = displace(dst, src, U, P, steps[2 * k], steps[2 * k + 1], g, stream);
+    if (e != cudaSuccess) return e;
+    src = dst;
+  }
+  *out = src;
+  return cudaSuccess;
 }
 
 cudaError_t vdaggerv_identity(double2 *vdv, int32_t op, Geometry g, cudaStream_t stream) {

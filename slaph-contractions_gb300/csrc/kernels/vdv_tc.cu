@@ -45,9 +45,30 @@ __host__ __device__ inline int32_t plane_k_tiles(int32_t per) {
   return (per + kTK / 2 - 1) / (kTK / 2);
 }
 
-// Exponent e_i with max_x |V(x, i)| < 2^e_i per eigenvector: one cluster of
-// kMaxCtas CTAs per eigenvector (one CTA each leaves most of the memory
-// bandwidth unused: 170 us per timeslice of 220 eigenvectors at 32^3).
+// |v| as a float, the mantissa cut to 23 bits: integer operations on the two
+// words, for 2^-126 <= |v| < 2^128 (smaller gives zero).
+__device__ __forceinline__ float abs_cut(double v, unsigned int &hi) {
+  hi = static_cast<unsigned int>(__double2hiint(v)) & 0x7FFFFFFFu;
+  int const t = static_cast<int>(hi) - (896 << 20);
+  return t < (1 << 20) ? 0.f
+                       : __uint_as_float(__funnelshift_l(static_cast<unsigned int>(__double2loint(v)),
+                                                         static_cast<unsigned int>(t), 3));
+}
+// Exponent e with sqrt(n2) (1 + 1e-15) < 2^e, 0 for n2 = 0.
+__device__ __forceinline__ int expo_of_norm2(double n2) {
+  int e = 0;
+  double const m = sqrt(n2);
+  if (m > 0) frexp(m * (1.0 + 1e-15), &e);
+  return e;
+}
+
+// Exponent e_i with max_x |V(x, i)| < 2^e_i per eigenvector, by one cluster of
+// kMaxCtas CTAs.  |v|^2 in FP64 would be bound by the FP64 units (three
+// operations per entry: 140 us per timeslice of 220 eigenvectors at 32^3, 2.5
+// TB/s), so the norms are taken in FP32 from cut mantissas, which puts the
+// largest |v|^2 between n (1 - 2^-20) and n (1 + 2^-20); only where those two
+// have different exponents, or the entries leave the FP32 range, is the column
+// read again in FP64.
 constexpr int kMaxCtas = 8;
 __global__ void __cluster_dims__(kMaxCtas, 1, 1) __launch_bounds__(256)
     colmax_kernel(int32_t *expo, double2 const *Vt, Geometry g) {
@@ -56,29 +77,63 @@ __global__ void __cluster_dims__(kMaxCtas, 1, 1) __launch_bounds__(256)
   int const i = blockIdx.y, part = blockIdx.x;
   double2 const *col = Vt + static_cast<int64_t>(i) * g.dim_row;
   int64_t const b = g.dim_row * part / kMaxCtas, e = g.dim_row * (part + 1) / kMaxCtas;
-  double m = 0;
+  __shared__ unsigned int red[2][8];
+  __shared__ double red64[8];
+  __shared__ int again;
+  unsigned int top = 0;  // largest high word
+  float n2 = 0;
 #pragma unroll 4
   for (int64_t x = b + threadIdx.x; x < e; x += 256) {
     double2 const v = col[x];
-    m = fmax(m, v.x * v.x + v.y * v.y);
+    unsigned int h0, h1;
+    float const p = abs_cut(v.x, h0), q = abs_cut(v.y, h1);
+    top = max(top, max(h0, h1));
+    n2 = fmaxf(n2, fmaf(p, p, q * q));
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  __shared__ double red[8];
-  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = m;
+  top = __reduce_max_sync(0xffffffffu, top);
+  unsigned int const nb = __reduce_max_sync(0xffffffffu, __float_as_uint(n2));
+  if (threadIdx.x % 32 == 0) {
+    red[0][threadIdx.x / 32] = top;
+    red[1][threadIdx.x / 32] = nb;
+  }
   cluster.sync();
   if (part == 0 && threadIdx.x == 0) {
-    double mx = 0;
+    unsigned int t = 0, m = 0;
     for (int q = 0; q < kMaxCtas; ++q) {
-      double const *r = cluster.map_shared_rank(red, q);
-      for (int w = 0; w < 8; ++w) mx = fmax(mx, r[w]);
+      unsigned int const *r = cluster.map_shared_rank(&red[0][0], q);
+      for (int w = 0; w < 8; ++w) {
+        t = max(t, r[w]);
+        m = max(m, r[8 + w]);
+      }
     }
-    int ex = 0;
-    mx = sqrt(mx);
-    if (mx > 0) frexp(mx * (1.0 + 1e-15), &ex);
-    expo[i] = ex;
+    double const n = static_cast<double>(__uint_as_float(m));
+    int const lo = expo_of_norm2(n * (1.0 - 0x1p-20)), up = expo_of_norm2(n * (1.0 + 0x1p-20));
+    // within 2^-50 .. 2^50 the squares stay in the FP32 range
+    bool const fits = t >= (973u << 20) && t < (1073u << 20);
+    again = !(fits && lo == up);
+    if (!again) expo[i] = lo;
   }
-  cluster.sync();  // the other CTAs' shared memory stays until it is read
+  cluster.sync();
+  if (*cluster.map_shared_rank(&again, 0) != 0) {
+    double m = 0;
+    for (int64_t x = b + threadIdx.x; x < e; x += 256) {
+      double2 const v = col[x];
+      m = fmax(m, v.x * v.x + v.y * v.y);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (threadIdx.x % 32 == 0) red64[threadIdx.x / 32] = m;
+    cluster.sync();
+    if (part == 0 && threadIdx.x == 0) {
+      double mx = 0;
+      for (int q = 0; q < kMaxCtas; ++q) {
+        double const *r = cluster.map_shared_rank(red64, q);
+        for (int w = 0; w < 8; ++w) mx = fmax(mx, r[w]);
+      }
+      expo[i] = expo_of_norm2(mx);
+    }
+  }
+  cluster.sync();  // a CTA's shared memory stays until the others have read it
 }
 
 // Slices of one timeslice.  kA: the A slices of V, [m_tile][K tile][slice][kTM x
@@ -508,22 +563,21 @@ cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, VdvTcPlan const &pl, int
       else
         slice_kernel<true, false><<<sb, 256, 0, stream>>>(slot, nullptr, Vt, nullptr, 0, expo,
                                                           pl.n_planes, pl.per, 0, g);
-      // Displaced operators: W = D(V_t) in the reference's in-place sweep
-      // order, B = W with phase 1 and W's own column exponents.
+      // Displaced operators: B = D(V_t) with phase 1 and its own column
+      // exponents.
+      double2 const *Ut = disp ? disp->U + links * t : nullptr;
+      double2 const *Pt = disp && disp->P ? disp->P + links * t : nullptr;
       for (int32_t d = 0; d < n_disp; ++d) {
         int32_t const f = pl.n_mom + d;
-        e = cudaMemcpyAsync(disp->W, Vt, sizeof(double2) * g.nev * g.dim_row,
-                            cudaMemcpyDeviceToDevice, stream);
+        double2 const *Wt = nullptr;
+        e = displaced_vectors(&Wt, disp->W, Vt, Ut, Pt,
+                              disp->steps + 2 * static_cast<int64_t>(d) * kMaxDispSteps,
+                              disp->n_steps[d], g, stream);
         if (e != cudaSuccess) return e;
-        for (int32_t k = 0; k < disp->n_steps[d]; ++k) {
-          int32_t const *st = disp->steps + 2 * (static_cast<int64_t>(d) * kMaxDispSteps + k);
-          e = displace(disp->W, disp->U + links * t, st[0], st[1], g, stream);
-          if (e != cudaSuccess) return e;
-        }
         int32_t *expo_w = expo + static_cast<int64_t>(1 + f) * g.nev;
-        colmax_kernel<<<mx, 256, 0, stream>>>(expo_w, disp->W, g);
+        colmax_kernel<<<mx, 256, 0, stream>>>(expo_w, Wt, g);
         slice_kernel<false, true><<<sb, 256, 0, stream>>>(
-            nullptr, slot + L.a_bytes, disp->W, pl.phase_fx + static_cast<int64_t>(f) * sites, 1,
+            nullptr, slot + L.a_bytes, Wt, pl.phase_fx + static_cast<int64_t>(f) * sites, 1,
             expo_w, pl.n_planes, pl.per, static_cast<int64_t>(f) * g.nev, g);
       }
       e = cudaGetLastError();

@@ -137,3 +137,37 @@ def test_build_matches_the_matrix_product(engine_lib, L, nev, p2, precision):
             err = np.max(np.abs(eng.vdaggerv_fetch(i, t) - ref))
             assert err < tol, (p, t, err, tol)
     eng.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shift", [-300, -130, -60, -40, 0, 40, 60, 130, 300])
+def test_split_precision_build_scales_exactly(engine_lib, shift):
+    """Eigenvectors times 2^shift: the split works on scaled integers, so the
+    blocks are those of the unscaled eigenvectors times 2^(2 shift), bit for
+    bit, whichever way the columns' exponents are found.  Some columns have
+    their largest entry on a power of two, where a bound of the norm does not
+    settle the exponent."""
+    from slaph_gb300 import _lib
+    from slaph_gb300.engine import Engine
+    L, nev = 4, 19
+    rng = np.random.default_rng(3)
+    V = rng.uniform(-0.4, 0.4, (nev, 3 * L ** 3, 2)).view(np.complex128)[..., 0]
+    V[3, 7], V[5, 11], V[8, 100] = 1.0, 0.5j, -1.0 + 2.0 ** -40
+    V[9] = 0.0
+    ops = (_lib.VdvOp * 2)()
+    for i, p in enumerate([(1, 0, 0), (1, -1, 2)]):
+        ops[i].id, ops[i].momentum = i, (C.c_int32 * 3)(*p)
+    x = np.indices((L, L, L)).reshape(3, -1).repeat(3, axis=1)
+    blocks = []
+    for s in (0, shift):
+        eng = Engine(_lib.Dims(1, L, L, L, nev, 1, 2, 2))
+        _lib.check(_lib.lib().slaph_engine_set_operators(eng._h, ops, 2, -1))
+        eng.set_eigenvectors(0, V * 2.0 ** s)
+        eng.vdaggerv_build(1)
+        blocks.append([eng.vdaggerv_fetch(i, 0) for i in range(2)])
+        eng.close()
+    for i, p in enumerate([(1, 0, 0), (1, -1, 2)]):
+        assert np.array_equal(blocks[0][i] * 2.0 ** (2 * shift), blocks[1][i])
+        ref = V.conj() @ (np.exp(-2j * np.pi * (np.array(p) @ x) / L) * V).T
+        # 47 bits of each row's scale per term, 192 terms
+        assert np.max(np.abs(blocks[0][i] - ref)) < 2 * 192 * 2.0 ** -46
