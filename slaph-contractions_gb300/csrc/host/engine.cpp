@@ -512,10 +512,10 @@ void Engine::vdaggerv_build(int precision) {
                               vdv_ev_.data() + 2 * gemm_done, 2 * k, v_t0),
              "vdaggerv_tc");
       gemm_done += k;
-      // per timeslice the exponents and the slices of the momentum families,
-      // per displaced operator its steps, exponents and slices; one GEMM and
-      // one Fourier sum per batch of timeslices
-      if (n_all > 0) launches_ += (2LL + disp_launches) * nt + 2 * k - 1;
+      // per batch of timeslices the norms, exponents and slices of the momentum
+      // families, one GEMM and one Fourier sum; per timeslice and displaced
+      // operator its steps, exponents and slices
+      if (n_all > 0) launches_ += disp_launches * nt + 5LL * k - 1;
     } else {
       for (int32_t t = t0; t < t0 + nt; ++t)
         if (ready[t]) SLAPH_CK(cudaStreamWaitEvent(stream_, ready[t], 0));

@@ -69,16 +69,22 @@ cudaError_t upload_gamma(cudaStream_t stream);
 int64_t hyp_scratch_doubles_per_timeslice(int32_t L);
 cudaError_t hyp_smear(double2 *U, double2 *dec, int32_t L, int32_t n_t, double alpha1,
                       double alpha2, cudaStream_t stream);
+// Largest entry of a column, as it is found in pieces (norm_max.cuh): high word
+// of the largest |re|, |im|, and the largest |v|^2 as the bits of a float.
+struct NormMax {
+  unsigned int top, n2;
+};
 // Displaced eigenvectors D(V_t) on a cubic lattice: n steps ((dir 0..2, forward
 // 0/1) pairs, host array) with the result of the reference's in-place sweeps
 // (displace_eigenvectors, src/OperatorFactory.cpp:33-55).  U: the timeslice's
 // links [site][dir][a + 3 b]; P: the timeslice's line_products (read by backward
 // steps only); W: scratch of nev x dim_row, twice that for n > 1.  *out: the
-// result, in W.  line_products: of all g.Lt timeslices, in the layout of U.
+// result, in W, whose columns' largest entries are added to norms[nev].
+// line_products: of all g.Lt timeslices, in the layout of U.
 cudaError_t line_products(double2 *P, double2 const *U, Geometry g, cudaStream_t stream);
 cudaError_t displaced_vectors(double2 const **out, double2 *W, double2 const *V, double2 const *U,
                               double2 const *P, int32_t const *steps, int32_t n, Geometry g,
-                              cudaStream_t stream);
+                              cudaStream_t stream, NormMax *norms = nullptr);
 // VdaggerV[2 op][t] = V_t^H W in FP64 (*op: device pointer to the operator id).
 cudaError_t vdaggerv_fp64_w(double2 *vdv, double2 const *V, double2 const *W,
                             int32_t const *op, int32_t t, Geometry g, cudaStream_t stream,

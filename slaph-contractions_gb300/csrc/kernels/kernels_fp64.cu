@@ -8,6 +8,7 @@
 #include <cstdint>
 
 #include "kernels.cuh"
+#include "norm_max.cuh"
 
 namespace slaph {
 namespace dev {
@@ -570,14 +571,16 @@ __global__ void line_product_kernel(double2 *P, double2 const *U, int32_t L) {
 }
 
 // One thread per site, kDispEv eigenvectors with the site's matrix in
-// registers.  Bound by FP64 issue (36 multiply-adds per site and eigenvector).
+// registers.  Bound by FP64 issue (36 multiply-adds per site and eigenvector);
+// the largest norms of the columns (norms, when given: see NormMax) are integer
+// and FP32 work beside it.
 constexpr int kDispEv = 8;
 __global__ void __launch_bounds__(128)
     displace_kernel(double2 *W, double2 const *V, double2 const *M, int32_t dir, int32_t forward,
-                    Geometry g) {
+                    NormMax *norms, Geometry g) {
   int const L = g.Lx;
-  int64_t const s = gidx();
-  if (s >= g.dim_row / 3) return;
+  bool const on = gidx() < g.dim_row / 3;  // (no early return: warp reductions below)
+  int64_t const s = on ? gidx() : 0;
   Line const ln = line_of(s, dir, L);
   double2 m[9];
 #pragma unroll
@@ -607,13 +610,16 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
     for (int b = 0; b < 3; ++b) v[b] = src[b];
     double2 *dst = W + ev * g.dim_row + 3 * s;
+    NormMax nm{0, 0};
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
       double2 acc = make_double2(0, 0);
 #pragma unroll
       for (int b = 0; b < 3; ++b) cfma(acc, m[a + 3 * b], v[b]);
-      dst[a] = acc;
+      if (on) dst[a] = acc;
+      norm_max(nm, acc);
     }
+    if (norms) norm_max_add(norms + ev, nm);
   }
 }
 
@@ -630,22 +636,26 @@ cudaError_t line_products(double2 *P, double2 const *U, Geometry g, cudaStream_t
   return cudaGetLastError();
 }
 
+namespace {
 cudaError_t displace(double2 *W, double2 const *V, double2 const *U, double2 const *P,
-                     int32_t dir, int32_t forward, Geometry g, cudaStream_t stream) {
+                     int32_t dir, int32_t forward, NormMax *norms, Geometry g,
+                     cudaStream_t stream) {
   if (dir < 0 || dir > 2 || g.Lx != g.Ly || g.Lx != g.Lz) return cudaErrorInvalidValue;
   displace_kernel<<<dim3(blocks_for(g.dim_row / 3, 128), blocks_for(g.nev, kDispEv)), 128, 0,
-                    stream>>>(W, V, forward ? U : P, dir, forward, g);
+                    stream>>>(W, V, forward ? U : P, dir, forward, norms, g);
   return cudaGetLastError();
 }
+}  // namespace
 
 cudaError_t displaced_vectors(double2 const **out, double2 *W, double2 const *V, double2 const *U,
                               double2 const *P, int32_t const *steps, int32_t n, Geometry g,
-                              cudaStream_t stream) {
+                              cudaStream_t stream, NormMax *norms) {
   int64_t const n_v = static_cast<int64_t>(g.nev) * g.dim_row;
   double2 const *src = V;
   for (int32_t k = 0; k < n; ++k) {
     double2 *dst = W + (k % 2) * n_v;
-    cudaError_t const e = displace(dst, src, U, P, steps[2 * k], steps[2 * k + 1], g, stream);
+    cudaError_t const e = displace(dst, src, U, P, steps[2 * k], steps[2 * k + 1],
+                                   k + 1 == n ? norms : nullptr, g, stream);
     if (e != cudaSuccess) return e;
     src = dst;
   }

@@ -14,7 +14,9 @@
 // with |p|^2 <= 3 are 5, 3 with |p|^2 <= 1 are 3.  The planes are also what
 // fills the chip: a timeslice gives n_planes times as many tiles as a sum over
 // the whole lattice, so a launch needs few timeslices (and little scratch) for
-// an even load.
+// an even load.  (Slicing the next timeslices on a second stream during a GEMM
+// gains nothing but the last round: the GEMM's ten warps of 168 registers leave
+// no room for another CTA on an SM.)
 //
 // Data path: V is read once per timeslice to write the A slices and the B
 // slices of all families to HBM, already in the tcgen05 core-matrix layout,
@@ -23,13 +25,13 @@
 // cut into tiles of kTN without padding between families.  Padding rows and
 // columns of the last tiles are not written: they only reach output rows and
 // columns that nobody reads.
-#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdint>
 
 #include "kernels.cuh"
+#include "norm_max.cuh"
 #include "tc_common.cuh"
 
 namespace slaph {
@@ -45,15 +47,6 @@ __host__ __device__ inline int32_t plane_k_tiles(int32_t per) {
   return (per + kTK / 2 - 1) / (kTK / 2);
 }
 
-// |v| as a float, the mantissa cut to 23 bits: integer operations on the two
-// words, for 2^-126 <= |v| < 2^128 (smaller gives zero).
-__device__ __forceinline__ float abs_cut(double v, unsigned int &hi) {
-  hi = static_cast<unsigned int>(__double2hiint(v)) & 0x7FFFFFFFu;
-  int const t = static_cast<int>(hi) - (896 << 20);
-  return t < (1 << 20) ? 0.f
-                       : __uint_as_float(__funnelshift_l(static_cast<unsigned int>(__double2loint(v)),
-                                                         static_cast<unsigned int>(t), 3));
-}
 // Exponent e with sqrt(n2) (1 + 1e-15) < 2^e, 0 for n2 = 0.
 __device__ __forceinline__ int expo_of_norm2(double n2) {
   int e = 0;
@@ -62,81 +55,53 @@ __device__ __forceinline__ int expo_of_norm2(double n2) {
   return e;
 }
 
-// Exponent e_i with max_x |V(x, i)| < 2^e_i per eigenvector, by one cluster of
-// kMaxCtas CTAs.  |v|^2 in FP64 would be bound by the FP64 units (three
-// operations per entry: 140 us per timeslice of 220 eigenvectors at 32^3, 2.5
-// TB/s), so the norms are taken in FP32 from cut mantissas, which puts the
-// largest |v|^2 between n (1 - 2^-20) and n (1 + 2^-20); only where those two
-// have different exponents, or the entries leave the FP32 range, is the column
-// read again in FP64.
-constexpr int kMaxCtas = 8;
-__global__ void __cluster_dims__(kMaxCtas, 1, 1) __launch_bounds__(256)
-    colmax_kernel(int32_t *expo, double2 const *Vt, Geometry g) {
-  namespace cg = cooperative_groups;
-  cg::cluster_group cluster = cg::this_cluster();
-  int const i = blockIdx.y, part = blockIdx.x;
-  double2 const *col = Vt + static_cast<int64_t>(i) * g.dim_row;
-  int64_t const b = g.dim_row * part / kMaxCtas, e = g.dim_row * (part + 1) / kMaxCtas;
-  __shared__ unsigned int red[2][8];
-  __shared__ double red64[8];
-  __shared__ int again;
-  unsigned int top = 0;  // largest high word
-  float n2 = 0;
-#pragma unroll 4
-  for (int64_t x = b + threadIdx.x; x < e; x += 256) {
-    double2 const v = col[x];
-    unsigned int h0, h1;
-    float const p = abs_cut(v.x, h0), q = abs_cut(v.y, h1);
-    top = max(top, max(h0, h1));
-    n2 = fmaxf(n2, fmaf(p, p, q * q));
-  }
-  top = __reduce_max_sync(0xffffffffu, top);
-  unsigned int const nb = __reduce_max_sync(0xffffffffu, __float_as_uint(n2));
-  if (threadIdx.x % 32 == 0) {
-    red[0][threadIdx.x / 32] = top;
-    red[1][threadIdx.x / 32] = nb;
-  }
-  cluster.sync();
-  if (part == 0 && threadIdx.x == 0) {
-    unsigned int t = 0, m = 0;
-    for (int q = 0; q < kMaxCtas; ++q) {
-      unsigned int const *r = cluster.map_shared_rank(&red[0][0], q);
-      for (int w = 0; w < 8; ++w) {
-        t = max(t, r[w]);
-        m = max(m, r[8 + w]);
-      }
-    }
-    double const n = static_cast<double>(__uint_as_float(m));
-    int const lo = expo_of_norm2(n * (1.0 - 0x1p-20)), up = expo_of_norm2(n * (1.0 + 0x1p-20));
-    // within 2^-50 .. 2^50 the squares stay in the FP32 range
-    bool const fits = t >= (973u << 20) && t < (1073u << 20);
-    again = !(fits && lo == up);
-    if (!again) expo[i] = lo;
-  }
-  cluster.sync();
-  if (*cluster.map_shared_rank(&again, 0) != 0) {
-    double m = 0;
-    for (int64_t x = b + threadIdx.x; x < e; x += 256) {
-      double2 const v = col[x];
-      m = fmax(m, v.x * v.x + v.y * v.y);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (threadIdx.x % 32 == 0) red64[threadIdx.x / 32] = m;
-    cluster.sync();
-    if (part == 0 && threadIdx.x == 0) {
-      double mx = 0;
-      for (int q = 0; q < kMaxCtas; ++q) {
-        double const *r = cluster.map_shared_rank(red64, q);
-        for (int w = 0; w < 8; ++w) mx = fmax(mx, r[w]);
-      }
-      expo[i] = expo_of_norm2(mx);
-    }
-  }
-  cluster.sync();  // a CTA's shared memory stays until the others have read it
+// norms[slot][i] of columns i of V, timeslice blockIdx.z (slots at slot_bytes),
+// one warp per kNormChunk entries: 5.5 TB/s, against 2.5 TB/s for FP64 norms.
+constexpr int kNormChunk = 2048;  // entries per warp
+__global__ void __launch_bounds__(32)
+    norm_kernel(uint8_t *norms, size_t slot_bytes, double2 const *V, Geometry g) {
+  int const i = blockIdx.y;
+  double2 const *col = V + (static_cast<int64_t>(blockIdx.z) * g.nev + i) * g.dim_row;
+  int64_t const b = static_cast<int64_t>(blockIdx.x) * kNormChunk;
+  int64_t const e = min(g.dim_row, b + kNormChunk);
+  NormMax m{0, 0};
+#pragma unroll 8
+  for (int64_t x = b + threadIdx.x; x < e; x += 32) norm_max(m, col[x]);
+  norm_max_add(reinterpret_cast<NormMax *>(norms + blockIdx.z * slot_bytes) + i, m);
 }
 
-// Slices of one timeslice.  kA: the A slices of V, [m_tile][K tile][slice][kTM x
+// Exponents e_i with max_x |V(x, i)| < 2^e_i from the columns' norms, one warp
+// per column; where the norm does not settle the exponent the column is read
+// again in FP64.  The norms are zeroed for their next use.
+__global__ void __launch_bounds__(32)
+    expo_kernel(uint8_t *norms, uint8_t *expo, size_t slot_bytes, double2 const *V, Geometry g) {
+  int const i = blockIdx.x, lane = threadIdx.x;
+  NormMax *m = reinterpret_cast<NormMax *>(norms + blockIdx.y * slot_bytes) + i;
+  NormMax const x = *m;
+  double const n = static_cast<double>(__uint_as_float(x.n2));
+  int ex = expo_of_norm2(n * (1.0 - 0x1p-20));
+  // within 2^-50 .. 2^50 the squares stay in the FP32 range
+  bool const fits = x.top >= (973u << 20) && x.top < (1073u << 20);
+  if (!fits || ex != expo_of_norm2(n * (1.0 + 0x1p-20))) {
+    double2 const *col = V + (static_cast<int64_t>(blockIdx.y) * g.nev + i) * g.dim_row;
+    double mx = 0;
+#pragma unroll 4
+    for (int64_t k = lane; k < g.dim_row; k += 32) {
+      double2 const v = col[k];
+      mx = fmax(mx, v.x * v.x + v.y * v.y);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    ex = expo_of_norm2(mx);
+  }
+  __syncwarp();
+  if (lane == 0) {
+    reinterpret_cast<int32_t *>(expo + blockIdx.y * slot_bytes)[i] = ex;
+    *m = NormMax{0, 0};
+  }
+}
+
+// Slices of timeslice blockIdx.y (slots at slot_bytes).  kA: the A slices of V, [m_tile][K tile][slice][kTM x
 // kTK]; kB: the B slices of phase_f V for n_fam families at B columns
 // col0 + f nev + j, [n_tile][K tile][slice][kTN x kTK].
 //
@@ -154,9 +119,13 @@ __global__ void __cluster_dims__(kMaxCtas, 1, 1) __launch_bounds__(256)
 // 48 (A) and 24 per family (B) written per entry.
 template <bool kA, bool kB>
 __global__ void __launch_bounds__(256)
-    slice_kernel(uint8_t *a_out, uint8_t *b_out, double2 const *Vt, longlong2 const *phase_fx,
-                 int32_t n_fam, int32_t const *expo, int32_t n_planes, int32_t per, int64_t col0,
-                 Geometry g) {
+    slice_kernel(uint8_t *a_out, uint8_t *b_out, size_t slot_bytes, double2 const *V,
+                 longlong2 const *phase_fx, int32_t n_fam, uint8_t const *expos, int32_t n_planes,
+                 int32_t per, int64_t col0, Geometry g) {
+  a_out += blockIdx.y * slot_bytes;
+  b_out += blockIdx.y * slot_bytes;
+  int32_t const *expo = reinterpret_cast<int32_t const *>(expos + blockIdx.y * slot_bytes);
+  double2 const *Vt = V + static_cast<int64_t>(blockIdx.y) * g.nev * g.dim_row;
   int64_t const wid = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) / 32;
   int const lane = threadIdx.x % 32;
   int32_t const ktp = plane_k_tiles(per);
@@ -444,7 +413,7 @@ __global__ void __launch_bounds__(256)
 struct TcLayout {
   int32_t ktp;
   int64_t k_tiles, n_cols;
-  size_t a_bytes, s_off, e_off, slot_bytes;
+  size_t a_bytes, s_off, e_off, n_off, slot_bytes;
 };
 TcLayout tc_layout(Geometry const &g, VdvTcPlan const &pl) {
   TcLayout L{};
@@ -456,9 +425,10 @@ TcLayout tc_layout(Geometry const &g, VdvTcPlan const &pl) {
   L.a_bytes = static_cast<size_t>(m_tiles * L.k_tiles) * kStageA;
   L.s_off = L.a_bytes + static_cast<size_t>(n_tiles * L.k_tiles) * kStageB;
   L.e_off = L.s_off + static_cast<size_t>(pl.n_planes * L.n_cols * g.nev) * sizeof(double2);
-  // exponents: the eigenvectors', then room for one set per family
+  // exponents: the eigenvectors', then room for one set per family; norms
+  L.n_off = (L.e_off + static_cast<size_t>(1 + pl.n_fam) * g.nev * sizeof(int32_t) + 15) / 16 * 16;
   L.slot_bytes =
-      (L.e_off + static_cast<size_t>(1 + pl.n_fam) * g.nev * sizeof(int32_t) + 1023) / 1024 * 1024;
+      (L.n_off + static_cast<size_t>(g.nev) * sizeof(NormMax) + 1023) / 1024 * 1024;
   return L;
 }
 
@@ -540,48 +510,63 @@ cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, VdvTcPlan const &pl, int
   if (e != cudaSuccess) return e;
   // one warp per (K tile, group of 8 eigenvectors)
   unsigned const sb = static_cast<unsigned>((L.k_tiles * ((g.nev + 7) / 8) * 32 + 255) / 256);
+  unsigned const nc = static_cast<unsigned>((g.dim_row + kNormChunk - 1) / kNormChunk);
   size_t const links = static_cast<size_t>(g.dim_row / 3) * 27;  // of one timeslice
   int32_t const sites = pl.per / 3;
   int64_t const blk = static_cast<int64_t>(g.nev) * g.nev;
-  dim3 const mx(kMaxCtas, static_cast<unsigned>(g.nev));
   int32_t gemm_k = 0;
   for (int32_t tb = t0; tb < t0 + nt; tb += static_cast<int32_t>(batch)) {
     int32_t const nb = static_cast<int32_t>(std::min<int64_t>(batch, t0 + nt - tb));
-    for (int32_t b = 0; b < nb; ++b) {
+    if (t_ready)
+      for (int32_t t = tb; t < tb + nb; ++t)
+        if (t_ready[t]) {
+          e = cudaStreamWaitEvent(stream, t_ready[t], 0);
+          if (e != cudaSuccess) return e;
+        }
+    unsigned const unb = static_cast<unsigned>(nb);
+    double2 const *Vb = V + static_cast<int64_t>(tb - v_t0) * g.nev * g.dim_row;
+    if (gemm_k == 0) {  // norms start at zero; expo_kernel leaves them so
+      e = cudaMemset2DAsync(base + L.n_off, L.slot_bytes, 0,
+                            static_cast<size_t>(g.nev) * sizeof(NormMax), unb, stream);
+      if (e != cudaSuccess) return e;
+    }
+    norm_kernel<<<dim3(nc, static_cast<unsigned>(g.nev), unb), 32, 0, stream>>>(base + L.n_off,
+                                                                            L.slot_bytes, Vb, g);
+    expo_kernel<<<dim3(static_cast<unsigned>(g.nev), unb), 32, 0, stream>>>(
+        base + L.n_off, base + L.e_off, L.slot_bytes, Vb, g);
+    if (pl.n_mom > 0)
+      slice_kernel<true, true><<<dim3(sb, unb), 256, 0, stream>>>(
+          base, base + L.a_bytes, L.slot_bytes, Vb, pl.phase_fx, pl.n_mom, base + L.e_off,
+          pl.n_planes, pl.per, 0, g);
+    else
+      slice_kernel<true, false><<<dim3(sb, unb), 256, 0, stream>>>(
+          base, base + L.a_bytes, L.slot_bytes, Vb, nullptr, 0, base + L.e_off, pl.n_planes,
+          pl.per, 0, g);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    // Displaced operators: B = D(V_t) with phase 1 and its own column exponents.
+    for (int32_t b = 0; b < nb && n_disp > 0; ++b) {
       int32_t const t = tb + b;
-      if (t_ready && t_ready[t]) {
-        e = cudaStreamWaitEvent(stream, t_ready[t], 0);
-        if (e != cudaSuccess) return e;
-      }
-      double2 const *Vt = V + static_cast<int64_t>(t - v_t0) * g.nev * g.dim_row;
+      double2 const *Vt = Vb + static_cast<int64_t>(b) * g.nev * g.dim_row;
       uint8_t *slot = base + b * L.slot_bytes;
-      int32_t *expo = reinterpret_cast<int32_t *>(slot + L.e_off);
-      colmax_kernel<<<mx, 256, 0, stream>>>(expo, Vt, g);
-      if (pl.n_mom > 0)
-        slice_kernel<true, true><<<sb, 256, 0, stream>>>(slot, slot + L.a_bytes, Vt, pl.phase_fx,
-                                                         pl.n_mom, expo, pl.n_planes, pl.per, 0, g);
-      else
-        slice_kernel<true, false><<<sb, 256, 0, stream>>>(slot, nullptr, Vt, nullptr, 0, expo,
-                                                          pl.n_planes, pl.per, 0, g);
-      // Displaced operators: B = D(V_t) with phase 1 and its own column
-      // exponents.
-      double2 const *Ut = disp ? disp->U + links * t : nullptr;
-      double2 const *Pt = disp && disp->P ? disp->P + links * t : nullptr;
       for (int32_t d = 0; d < n_disp; ++d) {
         int32_t const f = pl.n_mom + d;
         double2 const *Wt = nullptr;
-        e = displaced_vectors(&Wt, disp->W, Vt, Ut, Pt,
+        e = displaced_vectors(&Wt, disp->W, Vt, disp->U + links * t,
+                              disp->P ? disp->P + links * t : nullptr,
                               disp->steps + 2 * static_cast<int64_t>(d) * kMaxDispSteps,
-                              disp->n_steps[d], g, stream);
+                              disp->n_steps[d], g, stream,
+                              reinterpret_cast<NormMax *>(slot + L.n_off));
         if (e != cudaSuccess) return e;
-        int32_t *expo_w = expo + static_cast<int64_t>(1 + f) * g.nev;
-        colmax_kernel<<<mx, 256, 0, stream>>>(expo_w, Wt, g);
-        slice_kernel<false, true><<<sb, 256, 0, stream>>>(
-            nullptr, slot + L.a_bytes, Wt, pl.phase_fx + static_cast<int64_t>(f) * sites, 1,
+        uint8_t *expo_w = slot + L.e_off + static_cast<size_t>(1 + f) * g.nev * sizeof(int32_t);
+        expo_kernel<<<dim3(static_cast<unsigned>(g.nev), 1), 32, 0, stream>>>(slot + L.n_off, expo_w,
+                                                                          0, Wt, g);
+        slice_kernel<false, true><<<dim3(sb, 1), 256, 0, stream>>>(
+            nullptr, slot + L.a_bytes, 0, Wt, pl.phase_fx + static_cast<int64_t>(f) * sites, 1,
             expo_w, pl.n_planes, pl.per, static_cast<int64_t>(f) * g.nev, g);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
       }
-      e = cudaGetLastError();
-      if (e != cudaSuccess) return e;
     }
     bool const timed = gemm_ev && 2 * gemm_k + 1 < n_gemm_ev;
     if (timed) {
