@@ -944,10 +944,13 @@ void Engine::prepare_product_tc(DeviceSchedule &ds) {
 //          rows (m, a), columns (gamma, r2, b2, c), K = (bd, v):
 //          A = conj(s(bd, a) Q2M_m(a, bd nev + v)),
 //          B = Gval[gamma][bd] P_r2((4t+Grow[gamma][bd]) nev + v, b2 eds + c)
-// Dense FP64 outputs go to f_out_; gathers write the factor slots.
+// Dense double-float outputs go to f_out_; gathers write the factor slots, in the
+// layouts in which they are read.
 void Engine::prepare_factor_tc(DeviceSchedule &ds) {
   if (ds.f_ready) return;
   Schedule const &s = ds.s;
+  std::vector<uint8_t> const need =
+      factor_layouts(s, dev::prod_tc_supported(s.eds));
   int32_t const eds = s.eds, nev = dims_.nev, dilE = dims_.dilE, nb = geo_.nb;
   int32_t const n_rnd = dims_.n_rnd, Lt = dims_.Lt;
   int64_t const prow = 4LL * nev * Lt;            // perambulator rows
@@ -971,7 +974,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
   std::vector<dev::Q1Gather> g1;
   std::vector<dev::Q2Gather> g2;
   ds.f_batches.clear();
-  size_t need = 0;
+  size_t need_scr = 0;
   int64_t need_out = 0, need_expo = 0;
 
   auto add_vec = [&](int64_t dst, int32_t row, int32_t expo, int64_t stride, int32_t seg_len,
@@ -1176,7 +1179,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
                   static_cast<int32_t>(o.codes.size()) * nev, o.q2m, eA_q2m[k], eB_q2m[k]);
     }
     b.t1[1] = static_cast<int64_t>(tiles.size()) - b.t1[0];
-    need = std::max(need, off1);
+    need_scr = std::max(need_scr, off1);
     // -- phase 2: Q2 bicliques (A from the Q2M outputs, B from the perambulators)
     std::vector<std::vector<int64_t>> regA2(batch_ts.size()), regB2(batch_ts.size()),
         out2(batch_ts.size());
@@ -1257,7 +1260,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
       }
     }
     b.t2[1] = static_cast<int64_t>(tiles.size()) - b.t2[0];
-    need = std::max(need, off2);
+    need_scr = std::max(need_scr, off2);
     // -- gathers
     b.g1[0] = static_cast<int64_t>(g1.size());
     for (size_t k = 0; k < batch_ts.size(); ++k) {
@@ -1271,6 +1274,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
         g.col0 = (q.r2 * nb + q.b) * 4 * eds;
         g.gamma = q.gamma;
         g.slot = q.slot;
+        g.need = need[q.slot];
         g1.push_back(g);
       }
     }
@@ -1293,6 +1297,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
                 static_cast<int64_t>(rows) * (static_cast<int64_t>(ci) * eds);
         g.ld = rows;
         g.slot = q.slot;
+        g.need = need[q.slot];
         g2.push_back(g);
       }
     }
@@ -1323,7 +1328,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
   upload(ds.fg1, g1, stream_);
   upload(ds.fg2, g2, stream_);
   SLAPH_CK(cudaStreamSynchronize(stream_));
-  ds.f_scratch = need;
+  ds.f_scratch = need_scr;
   ds.f_out = need_out;
   ds.f_expo = need_expo;
   ds.f_ready = true;
@@ -1431,6 +1436,10 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
       df_slots_t_.reserve(df_bytes);
       slot_bits_.reserve(sizeof(unsigned int) *
                          std::max<int64_t>(1, s.n_factor_slots + s.max_prod_slots));
+      // (Q0 factors add their largest entries by atomicMax)
+      SLAPH_CK(cudaMemsetAsync(slot_bits_.as<void>(), 0,
+                               sizeof(unsigned int) * std::max<int64_t>(1, s.n_factor_slots),
+                               stream_));
       int64_t const n_vdv = 2LL * static_cast<int64_t>(ops_.size()) * dims_.Lt * nev * nev;
       int64_t const n_noise = 4LL * nev * dims_.Lt * dims_.n_rnd;
       DevBuf vdv_df, noise_df, q0m, q1r;
@@ -1446,19 +1455,20 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
                              q1r.as<float4>(), nullptr, ds.q0m.as<dev::Q0MInst>(),
                              s.q0m.size(), ds.q1r.as<dev::Q1RInst>(), s.q1r.size(), nullptr, 0,
                              ds.q0.as<dev::Q0Inst>(), s.q0.size(), nullptr, 0, nullptr, 0,
-                             vdv_df.as<float4>(), noise_df.as<float4>(), nullptr, geo_, stream_),
+                             vdv_df.as<float4>(), noise_df.as<float4>(), nullptr,
+                             slot_bits_.as<unsigned int>(), geo_, stream_),
              "factors_df");
       launches_ += 2;
       prepare_factor_tc(ds);
       tc_scratch_.reserve(std::max<size_t>(1, ds.f_scratch));
-      f_out_.reserve(sizeof(double2) * std::max<int64_t>(1, ds.f_out));
+      f_out_.reserve(sizeof(float4) * std::max<int64_t>(1, ds.f_out));
       tr_expo_.reserve(sizeof(int32_t) * std::max<int64_t>(1, ds.f_expo));
       err_.reserve(sizeof(int));
       SLAPH_CK(cudaMemsetAsync(err_.as<void>(), 0, sizeof(int), stream_));
       int32_t const kt1 = dev::gemm_k_tiles(nev), kt2 = dev::gemm_k_tiles(4 * nev);
       uint8_t *scr = tc_scratch_.as<uint8_t>();
       int32_t *ex = tr_expo_.as<int32_t>();
-      double2 *fo = f_out_.as<double2>();
+      float4 *fo = f_out_.as<float4>();
       auto const *fv = ds.fvec.as<dev::GVec>();
       auto const *ft = ds.ftiles.as<dev::TrTile>();
       auto count = [&](int64_t n) { launches_ += n > 0 ? 1 : 0; };
@@ -1476,32 +1486,30 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
                                        vdv_.as<double2>(), kt1, stream_),
                    "slice Q2M B");
         count(b.a_x1[1]); count(b.a_q2m[1]); count(b.b_x1[1]); count(b.b_q2m[1]);
-        cuda_check(dev::tc_gemm(fo, scr, ex, ft + b.t1[0], b.t1[1], kt1, err_.as<int>(), stream_),
+        cuda_check(dev::tc_gemm_df(fo, scr, ex, ft + b.t1[0], b.t1[1], kt1, err_.as<int>(), stream_),
                    "factor GEMM (X1, Q2M)");
         count(b.t1[1]);
-        cuda_check(dev::gvec_slice_f64(scr, ex, fv + b.a_q2[0], b.a_q2[1], true, true, fo, kt2,
-                                       stream_),
+        cuda_check(dev::gvec_slice_df(scr, ex, fv + b.a_q2[0], b.a_q2[1], true, true, fo, kt2,
+                                      stream_),
                    "slice Q2 A");
         cuda_check(dev::gvec_slice_f64(scr, ex, fv + b.b_q2[0], b.b_q2[1], false, false,
                                        peram_.as<double2>(), kt2, stream_),
                    "slice Q2 B");
         count(b.a_q2[1]); count(b.b_q2[1]);
-        cuda_check(dev::tc_gemm(fo, scr, ex, ft + b.t2[0], b.t2[1], kt2, err_.as<int>(), stream_),
+        cuda_check(dev::tc_gemm_df(fo, scr, ex, ft + b.t2[0], b.t2[1], kt2, err_.as<int>(), stream_),
                    "factor GEMM (Q2)");
         count(b.t2[1]);
         cuda_check(dev::q1_gather(df_slots_.as<float4>(), df_slots_t_.as<float4>(),
+                                  slot_bits_.as<unsigned int>(),
                                   ds.fg1.as<dev::Q1Gather>() + b.g1[0], b.g1[1], fo, dims_.dilE,
                                   stream_),
                    "q1_gather");
         cuda_check(dev::q2_gather(df_slots_.as<float4>(), df_slots_t_.as<float4>(),
+                                  slot_bits_.as<unsigned int>(),
                                   ds.fg2.as<dev::Q2Gather>() + b.g2[0], b.g2[1], fo, eds, stream_),
                    "q2_gather");
         count(b.g1[1]); count(b.g2[1]);
       }
-      // largest entries of the factor slots for the trace-operand slicing
-      launch(dev::slot_maxbits(slot_bits_.as<unsigned int>(), df_slots_.as<float4>(), 0,
-                               s.n_factor_slots, eds, stream_),
-             "slot_maxbits");
       SLAPH_CK(cudaEventRecord(ev_[1], stream_));
       SLAPH_CK(cudaEventSynchronize(ev_[1]));  // intermediates are freed here
     }

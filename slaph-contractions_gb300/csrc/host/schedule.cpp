@@ -543,6 +543,7 @@ class Builder {
     auto const &o = op(type, ql);
     int32_t const vdv = vdv_code(o);
     int32_t const base = n_factor_slots_;
+    s_.factor_lists.push_back(base);
     std::vector<SymE> entries;
     for (int k = 0; k < o.n_rnd_pairs; ++k) {
       int const r1 = o.rnd_pairs[2 * k], r2 = o.rnd_pairs[2 * k + 1];
@@ -775,6 +776,29 @@ Schedule build_schedule(slaph_dims const &dims, slaph_plan const &plan, int sing
   if (dims.n_rnd > 16) throw UnsupportedError("at most 16 random vectors (16-bit used masks)");
   Builder b(dims, plan);
   return b.run(single_block_pair);
+}
+
+std::vector<uint8_t> factor_layouts(Schedule const &s, bool tc_products) {
+  int64_t const n = s.n_factor_slots;
+  std::vector<uint8_t> need(n, 0), base(n, 0);
+  for (auto const &w : s.waves) {
+    for (auto const &p : w.prods) {
+      if (p.a < n) need[p.a] |= tc_products ? kNeedTransposed : kNeedStored;
+      if (p.b < n) need[p.b] |= kNeedStored;
+    }
+    // trace lists name the first slot of an operand list: all of it is marked
+    for (int32_t k : w.unique_lists) {
+      auto const &l = w.lists[k];
+      if (l.a_base < n) base[l.a_base] |= kNeedStored;
+      if (l.b_base >= 0 && l.b_base < n) base[l.b_base] |= kNeedTransposed;
+    }
+  }
+  for (size_t q = 0; q < s.factor_lists.size(); ++q) {
+    int64_t const b = s.factor_lists[q];
+    int64_t const e = q + 1 < s.factor_lists.size() ? s.factor_lists[q + 1] : n;
+    for (int64_t x = b; x < e; ++x) need[x] |= base[b];
+  }
+  return need;
 }
 
 TraceGroupPlan plan_trace_group(TraceShape const &shape, int32_t n_a, int32_t n_b,

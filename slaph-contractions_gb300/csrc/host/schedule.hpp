@@ -132,6 +132,7 @@ struct Schedule {
   std::vector<Q1Inst> q1;
   std::vector<Q2Inst> q2;
   int64_t n_factor_slots = 0;
+  std::vector<int32_t> factor_lists;  // first slot of every factor list, increasing
 
   std::vector<TraceShape> shapes;
   std::vector<Wave> waves;
@@ -190,6 +191,13 @@ struct ProductPlan {
   int64_t n_tiles = 0;
 };
 ProductPlan plan_products(ProdInst const *prods, int64_t n, int32_t eds);
+
+// Layouts in which the factor slots are read, over all waves: as stored (kNeedStored) by the A side of
+// the traces and the right side of the products, transposed (kNeedTransposed)
+// by the B side of the traces and the left side of the tensor-core products
+// (both sides of other products read the stored one).
+constexpr uint8_t kNeedStored = 1, kNeedTransposed = 2;
+std::vector<uint8_t> factor_layouts(Schedule const &s, bool tc_products);
 
 // Builds the schedule; throws EmptyError with the reference's messages when a
 // random-vector combination is empty.  single_block_pair >= 0 restricts the

@@ -11,7 +11,7 @@
 //     (:221-243 with K = (bd, v), the gamma_5 signs s folded into the rows and
 //      the gamma phases into the columns)
 // They run on the split-BF16 tile pipeline of tc_common.cuh (the GEMM kernel
-// of trace_tc.cu, whose epilogue writes dense FP64 complex outputs).  Operand
+// of trace_tc.cu, whose epilogue writes dense double-float outputs).  Operand
 // rows and columns are gathered from up to four strided segments of a source
 // array, each with an exact factor +-1, +-i, and cut into slices here; K is
 // padded with zeros to whole k-tiles.
@@ -112,62 +112,71 @@ __global__ void __launch_bounds__(kGThreads)
   }
 }
 
-__device__ __forceinline__ float4 df_of(double2 v) {
-  float const rh = static_cast<float>(v.x), ih = static_cast<float>(v.y);
-  return make_float4(rh, static_cast<float>(v.x - static_cast<double>(rh)), ih,
-                     static_cast<float>(v.y - static_cast<double>(ih)));
-}
-__device__ __forceinline__ double2 phase_mul(int code, double2 v) {
+__device__ __forceinline__ float4 phase_mul(int code, float4 v) {
   switch (code & 3) {
-    case 1: return make_double2(-v.y, v.x);
-    case 2: return make_double2(-v.x, -v.y);
-    case 3: return make_double2(v.y, -v.x);
+    case 1: return make_float4(-v.z, -v.w, v.x, v.y);
+    case 2: return make_float4(-v.x, -v.y, -v.z, -v.w);
+    case 3: return make_float4(v.z, v.w, -v.x, -v.y);
     default: return v;
   }
 }
 
-// Q1 (src/DilutedFactorFactory.cpp:146-164) from X1: entry (a, c) of the
-// factor is gamma_phase[row] X1[row0 + a, col0 + Grow[row] eds + c] with
-// row = a / dilE; written double-float in both layouts.
-__global__ void q1_gather_kernel(float4 *sn, float4 *st, Q1Gather const *g, double2 const *x,
-                                 int32_t dilE) {
-  Q1Gather const q = g[blockIdx.y];
-  int const eds = 4 * dilE;
-  int const k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= eds * eds) return;
-  int const a = k % eds, c = k / eds;
-  int const row = a / dilE;
-  double2 const v = x[q.x_off + (q.row0 + a) +
-                      static_cast<int64_t>(q.ld) *
-                          (q.col0 + c_gamma_row_tc[q.gamma][row] * eds + c)];
-  float4 const f = df_of(phase_mul(c_gamma_phase_tc[q.gamma][row], v));
-  int64_t const ms = static_cast<int64_t>(eds) * eds;
-  sn[q.slot * ms + k] = f;
-  st[q.slot * ms + c + static_cast<int64_t>(eds) * a] = f;
+// Entry (a, c) of a factor: Q1 (src/DilutedFactorFactory.cpp:146-164) from X1 is
+// gamma_phase[row] X1[row0 + a, col0 + Grow[row] eds + c] with row = a / dilE; Q2
+// from its GEMM output y[off + a + ld c].
+__device__ __forceinline__ float4 entry(Q1Gather const &q, float4 const *x, int a, int c, int eds) {
+  int const row = a / (eds / 4);
+  float4 const v = x[q.x_off + (q.row0 + a) +
+                     static_cast<int64_t>(q.ld) *
+                         (q.col0 + c_gamma_row_tc[q.gamma][row] * eds + c)];
+  return phase_mul(c_gamma_phase_tc[q.gamma][row], v);
+}
+__device__ __forceinline__ float4 entry(Q2Gather const &q, float4 const *y, int a, int c, int) {
+  return y[q.off + a + static_cast<int64_t>(q.ld) * c];
 }
 
-// Q2 from its GEMM output: entry (a, c) at y[off + a + ld c].
-__global__ void q2_gather_kernel(float4 *sn, float4 *st, Q2Gather const *g, double2 const *y,
-                                 int32_t eds) {
-  Q2Gather const q = g[blockIdx.y];
-  int const k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= eds * eds) return;
-  int const a = k % eds, c = k / eds;
-  float4 const f = df_of(y[q.off + a + static_cast<int64_t>(q.ld) * c]);
-  int64_t const ms = static_cast<int64_t>(eds) * eds;
-  sn[q.slot * ms + k] = f;
-  st[q.slot * ms + c + static_cast<int64_t>(eds) * a] = f;
-}
-
-template <typename I, typename F>
-cudaError_t in_chunks(I const *p, int64_t n, F &&launch) {
-  for (int64_t s = 0; s < n; s += 65535) {
-    int const c = static_cast<int>(n - s < 65535 ? n - s : 65535);
-    launch(p + s, c);
-    cudaError_t const e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+// One CTA per factor slot, in chunks of up to 32 rows: entries are read along
+// a, where the source is contiguous, and pass through shared memory for the
+// transposed layout, so that the stores of both layouts fill whole lines.
+// Memory-bound: 16 bytes read and 16 written per entry and layout (with the
+// transposed stores straight from registers, 32 lanes a line each, 24^3x48
+// Nev 120 took 7.1 ms against 2.1).
+constexpr int kGatherRows = 32;
+template <typename G>
+__global__ void __launch_bounds__(256)
+    gather_kernel(float4 *sn, float4 *st, unsigned int *slot_bits, G const *g, float4 const *src,
+                  int32_t eds) {
+  __shared__ float4 tile[64 * (kGatherRows + 1)];
+  __shared__ unsigned int red[8];
+  G const q = g[blockIdx.x];
+  int64_t const at = static_cast<int64_t>(q.slot) * eds * eds;
+  unsigned int mx = 0;
+  for (int a0 = 0; a0 < eds; a0 += kGatherRows) {
+    int const ra = min(kGatherRows, eds - a0), n = ra * eds;
+    for (int k = threadIdx.x; k < n; k += 256) {
+      int const a = k % ra, c = k / ra;
+      float4 const v = entry(q, src, a0 + a, c, eds);
+      mx = max(mx, max(__float_as_uint(v.x) & 0x7FFFFFFFu, __float_as_uint(v.z) & 0x7FFFFFFFu));
+      if (q.need & 1) sn[at + a0 + a + eds * c] = v;
+      if (q.need & 2) tile[c * (kGatherRows + 1) + a] = v;
+    }
+    if (q.need & 2) {
+      __syncthreads();
+      for (int k = threadIdx.x; k < n; k += 256) {
+        int const c = k % eds, a = k / eds;
+        st[at + c + eds * (a0 + a)] = tile[c * (kGatherRows + 1) + a];
+      }
+      __syncthreads();
+    }
   }
-  return cudaSuccess;
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = mx;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int w = 1; w < 8; ++w) mx = max(mx, red[w]);
+    slot_bits[q.slot] = mx;
+  }
 }
 
 }  // namespace
@@ -212,21 +221,20 @@ cudaError_t gvec_slice_df(uint8_t *scratch, int32_t *expo, GVec const *items, in
   return cudaGetLastError();
 }
 
-cudaError_t q1_gather(float4 *sn, float4 *st, Q1Gather const *g, int64_t n, double2 const *x,
-                      int32_t dilE, cudaStream_t stream) {
-  int const eds = 4 * dilE;
-  unsigned const bx = static_cast<unsigned>((eds * eds + 255) / 256);
-  return in_chunks(g, n, [&](Q1Gather const *p, int c) {
-    q1_gather_kernel<<<dim3(bx, c), 256, 0, stream>>>(sn, st, p, x, dilE);
-  });
+cudaError_t q1_gather(float4 *sn, float4 *st, unsigned int *slot_bits, Q1Gather const *g,
+                      int64_t n, float4 const *x, int32_t dilE, cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  if (n > 0x7fffffffLL || dilE > 16) return cudaErrorInvalidValue;
+  gather_kernel<<<static_cast<unsigned>(n), 256, 0, stream>>>(sn, st, slot_bits, g, x, 4 * dilE);
+  return cudaGetLastError();
 }
 
-cudaError_t q2_gather(float4 *sn, float4 *st, Q2Gather const *g, int64_t n, double2 const *y,
-                      int32_t eds, cudaStream_t stream) {
-  unsigned const bx = static_cast<unsigned>((eds * eds + 255) / 256);
-  return in_chunks(g, n, [&](Q2Gather const *p, int c) {
-    q2_gather_kernel<<<dim3(bx, c), 256, 0, stream>>>(sn, st, p, y, eds);
-  });
+cudaError_t q2_gather(float4 *sn, float4 *st, unsigned int *slot_bits, Q2Gather const *g,
+                      int64_t n, float4 const *y, int32_t eds, cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  if (n > 0x7fffffffLL || eds > 64) return cudaErrorInvalidValue;
+  gather_kernel<<<static_cast<unsigned>(n), 256, 0, stream>>>(sn, st, slot_bits, g, y, eds);
+  return cudaGetLastError();
 }
 
 int32_t gemm_k_tiles(int64_t K) { return static_cast<int32_t>((K + kTK / 2 - 1) / (kTK / 2)); }

@@ -203,14 +203,16 @@ cudaError_t split_df(float4 *dst_n, float4 *dst_t, double2 const *src, int64_t n
 // Mixed path: FP64 -> double-float (float4) copy.
 cudaError_t to_df(float4 *dst, double2 const *src, int64_t n, cudaStream_t stream);
 // Mixed path: all factor intermediates and factors in double-float; factors
-// written into the slot buffers in both layouts (sn stored, st transposed).
+// written into the slot buffers in both layouts (sn stored, st transposed), Q0
+// factors with the largest |re|, |im| of their slots (slot_maxbits), added to
+// slot_bits.
 cudaError_t factors_df(float4 *sn, float4 *st, float4 *q0m_buf, float4 *q1r_buf,
                        float4 *q2m_buf, Q0MInst const *q0m_i, int64_t n_q0m,
                        Q1RInst const *q1r_i, int64_t n_q1r, Q2MInst const *q2m_i, int64_t n_q2m,
                        Q0Inst const *q0_i, int64_t n_q0, Q1Inst const *q1_i, int64_t n_q1,
                        Q2Inst const *q2_i, int64_t n_q2, float4 const *vdv,
-                       float4 const *noise, float4 const *peram, Geometry g,
-                       cudaStream_t stream);
+                       float4 const *noise, float4 const *peram, unsigned int *slot_bits,
+                       Geometry g, cudaStream_t stream);
 // slots[c] = slots[a] * slots[b] in double-float, both layouts written.
 cudaError_t products_df(float4 *slots_n, float4 *slots_t, ProdInst const *p, int64_t n,
                         int32_t eds, cudaStream_t stream);
@@ -319,6 +321,11 @@ int32_t gemm_k_tiles(int64_t K);
 cudaError_t tc_gemm(double2 *out, uint8_t const *scratch, int32_t const *expo,
                     TrTile const *tiles, int64_t n_tiles, int32_t k_tiles, int *err,
                     cudaStream_t stream, int32_t const *entries = nullptr);
+// The same with double-float results (re_hi, re_lo, im_hi, im_lo), for plain
+// tiles: the short K of the factor GEMMs leaves no time for FP64 conversions.
+cudaError_t tc_gemm_df(float4 *out, uint8_t const *scratch, int32_t const *expo,
+                       TrTile const *tiles, int64_t n_tiles, int32_t k_tiles, int *err,
+                       cudaStream_t stream);
 
 // One GEMM operand row (A) or column (B) gathered from up to four strided
 // segments of a source array, each with an exact factor (0: +1, 1: +i, 2: -1,
@@ -346,20 +353,22 @@ cudaError_t gvec_slice_df(uint8_t *scratch, int32_t *expo, GVec const *items, in
                           bool is_a, bool conj, float4 const *src, int32_t k_tiles,
                           cudaStream_t stream);
 // Q1 factor slots from the dense product X1 (factor_tc.cu); Q2 slots from the
-// dense Q2 GEMM output.
+// dense Q2 GEMM output; both double-float, as tc_gemm_df writes them.  need: the
+// layouts to write (1 stored, 2 transposed); slot_bits: largest |re|, |im| of
+// the slot (slot_maxbits).
 struct Q1Gather {
   int64_t x_off;  // element offset of X1 of the factor's timeslice
-  int32_t ld, row0, col0, gamma, slot, pad;
+  int32_t ld, row0, col0, gamma, slot, need;
 };
 struct Q2Gather {
   int64_t off;  // element offset of the factor's (0, 0) entry
-  int32_t ld, slot;
+  int32_t ld, slot, need, pad;
 };
 cudaError_t upload_gamma_tc(cudaStream_t stream);
-cudaError_t q1_gather(float4 *sn, float4 *st, Q1Gather const *g, int64_t n, double2 const *x,
-                      int32_t dilE, cudaStream_t stream);
-cudaError_t q2_gather(float4 *sn, float4 *st, Q2Gather const *g, int64_t n, double2 const *y,
-                      int32_t eds, cudaStream_t stream);
+cudaError_t q1_gather(float4 *sn, float4 *st, unsigned int *slot_bits, Q1Gather const *g,
+                      int64_t n, float4 const *x, int32_t dilE, cudaStream_t stream);
+cudaError_t q2_gather(float4 *sn, float4 *st, unsigned int *slot_bits, Q2Gather const *g,
+                      int64_t n, float4 const *y, int32_t eds, cudaStream_t stream);
 
 // values[i] = hi + lo of values_df[i] for i < n_values, the FP64 trace values
 // the terms read.

@@ -1176,25 +1176,31 @@ __device__ __forceinline__ void store_factor_df(float4 *sn, float4 *st, int slot
 }
 
 __global__ void q0_df_kernel(float4 *sn, float4 *st, Q0Inst const *inst, float4 const *q0m,
-                             float4 const *noise, Geometry g) {
+                             float4 const *noise, unsigned int *slot_bits, Geometry g) {
   Q0Inst const in = inst[blockIdx.y];
   int const nev = g.nev, dilE = g.dilE, eds = 4 * dilE;
   int const k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= eds * eds) return;
-  int const a = k % eds, b = k / eds;
-  int const d = b / dilE;
-  int const gr = c_gamma_row[in.gamma][d];
-  CDf acc = cdf_zero();
-  if (a / dilE == gr) {
-    int const e1 = a % dilE;
-    float4 const *M = q0m + static_cast<int64_t>(in.m) * nev * eds;
-    float4 const *rho = noise + static_cast<int64_t>(in.r1) * g.Lt * 4 * nev;
-    double2 const val = c_gamma_val[in.gamma][d];
-    for (int v = e1; v < nev; v += dilE)
-      cdf_mac(acc, gamma_mul(val, M[v + static_cast<int64_t>(nev) * b]),
-              conj_df(rho[gr + 4 * (v + static_cast<int64_t>(nev) * in.t)]));
+  unsigned int mx = 0;
+  if (k < eds * eds) {
+    int const a = k % eds, b = k / eds;
+    int const d = b / dilE;
+    int const gr = c_gamma_row[in.gamma][d];
+    CDf acc = cdf_zero();
+    if (a / dilE == gr) {
+      int const e1 = a % dilE;
+      float4 const *M = q0m + static_cast<int64_t>(in.m) * nev * eds;
+      float4 const *rho = noise + static_cast<int64_t>(in.r1) * g.Lt * 4 * nev;
+      double2 const val = c_gamma_val[in.gamma][d];
+      for (int v = e1; v < nev; v += dilE)
+        cdf_mac(acc, gamma_mul(val, M[v + static_cast<int64_t>(nev) * b]),
+                conj_df(rho[gr + 4 * (v + static_cast<int64_t>(nev) * in.t)]));
+    }
+    float4 const f = cdf_value(acc);
+    mx = max(__float_as_uint(f.x) & 0x7FFFFFFFu, __float_as_uint(f.z) & 0x7FFFFFFFu);
+    store_factor_df(sn, st, in.slot, k, eds, f);
   }
-  store_factor_df(sn, st, in.slot, k, eds, cdf_value(acc));
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if (threadIdx.x % 32 == 0 && mx != 0) atomicMax(slot_bits + in.slot, mx);
 }
 
 __global__ void q1_df_kernel(float4 *sn, float4 *st, Q1Inst const *inst, float4 const *q1r,
@@ -1255,8 +1261,8 @@ cudaError_t factors_df(float4 *sn, float4 *st, float4 *q0m_buf, float4 *q1r_buf,
                        Q1RInst const *q1r_i, int64_t n_q1r, Q2MInst const *q2m_i, int64_t n_q2m,
                        Q0Inst const *q0_i, int64_t n_q0, Q1Inst const *q1_i, int64_t n_q1,
                        Q2Inst const *q2_i, int64_t n_q2, float4 const *vdv,
-                       float4 const *noise, float4 const *peram, Geometry g,
-                       cudaStream_t stream) {
+                       float4 const *noise, float4 const *peram, unsigned int *slot_bits,
+                       Geometry g, cudaStream_t stream) {
   int const eds = 4 * g.dilE;
   int64_t const per_m = static_cast<int64_t>(g.nev) * eds;
   int64_t const per_f = static_cast<int64_t>(eds) * eds;
@@ -1279,7 +1285,7 @@ cudaError_t factors_df(float4 *sn, float4 *st, float4 *q0m_buf, float4 *q1r_buf,
   });
   if (e != cudaSuccess) return e;
   e = chunked(q0_i, n_q0, [&](Q0Inst const *p, int c, int64_t) {
-    q0_df_kernel<<<dim3(blocks256(per_f), c), 256, 0, stream>>>(sn, st, p, q0m_buf, noise, g);
+    q0_df_kernel<<<dim3(blocks256(per_f), c), 256, 0, stream>>>(sn, st, p, q0m_buf, noise, slot_bits, g);
   });
   if (e != cudaSuccess) return e;
   e = chunked(q1_i, n_q1, [&](Q1Inst const *p, int c, int64_t) {

@@ -217,13 +217,6 @@ struct ProdTiles {
   }
 };
 
-// x 2^sh for |sh| <= 252, as two multiplications by powers of two (each exact
-// for a normal result).
-__device__ __forceinline__ float scale2(float x, int sh) {
-  int const s1 = sh / 2, s2 = sh - s1;
-  return (x * __int_as_float((s1 + 127) << 23)) * __int_as_float((s2 + 127) << 23);
-}
-
 // Epilogue: A' row 2 cr + (re | im), cr = l eds + i; column c = u eds + j.
 // A warp's 32 rows lie in one left matrix l.  Before the tile is promoted,
 // lane k fetches the product slot and the column exponent of the warp's

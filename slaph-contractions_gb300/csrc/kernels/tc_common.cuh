@@ -207,6 +207,13 @@ __device__ __forceinline__ void digits6(long long F, float (&d)[kSlices]) {
   d[5] = __int_as_float(__byte_perm(lo, 0x4B000000u, 0x7441)) - bias;
 }
 
+// x 2^sh for |sh| <= 252, as two multiplications by powers of two (each exact
+// for a normal result).
+__device__ __forceinline__ float scale2(float x, int sh) {
+  int const s1 = sh / 2, s2 = sh - s1;
+  return (x * __int_as_float((s1 + 127) << 23)) * __int_as_float((s2 + 127) << 23);
+}
+
 // Two small integers held exactly in floats to a BF16 pair (a in the low half).
 __device__ __forceinline__ uint32_t bf16x2(float a, float b) {
   uint32_t r;

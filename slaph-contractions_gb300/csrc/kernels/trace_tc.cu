@@ -122,7 +122,9 @@ __global__ void __launch_bounds__(kSliceThreads)
 }
 
 // FP64 values of one tile (TrTile): value (r, c) = (hi + lo) 2^(e_r + e_c - 14),
-// component row & 1 (re, im).
+// component row & 1 (re, im).  kDf: plain tiles, the values as (hi, lo) floats
+// in the place of a double.
+template <bool kDf>
 struct TraceEpilogue {
   double *values;
   int32_t const *expo;
@@ -157,6 +159,18 @@ struct TraceEpilogue {
     TrTile const &t = p.t;
     int const r = row / 2;
     bool const row_ok = r < t.rows;
+    if (kDf) {
+      float2 *dst = reinterpret_cast<float2 *>(values) + 2 * (t.out + r) + (row & 1);
+#pragma unroll
+      for (int c = 0; c < kColsW; ++c) {
+        int const ec = __shfl_sync(0xffffffffu, c < 32 ? p.e0 : p.e1, c % 32);
+        int const sh = min(max(p.er + ec - 14, -252), 254);  // above: infinity
+        if (row_ok && col0 + c < t.cols)
+          dst[2 * static_cast<int64_t>(col0 + c) * t.ld] =
+              make_float2(scale2(hi[c], sh), scale2(lo[c], sh));
+      }
+      return;
+    }
     if (t.tab < 0) {
       double *dst = values + 2 * (t.out + r) + (row & 1);
 #pragma unroll
@@ -205,12 +219,13 @@ struct TraceSrc {
   }
 };
 
+template <bool kDf>
 __global__ void __launch_bounds__(kThreads, 1)
     trace_gemm_kernel(double2 *values, uint8_t const *scratch, int32_t const *expo,
                       TrTile const *tiles, int32_t n_tiles, int32_t k_tiles,
                       int32_t const *entries, int *err) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  TraceEpilogue epi{reinterpret_cast<double *>(values), expo, tiles, entries};
+  TraceEpilogue<kDf> epi{reinterpret_cast<double *>(values), expo, tiles, entries};
   ozaki_tiles(smem, n_tiles, k_tiles, TraceSrc{scratch, tiles}, err, epi);
 }
 
@@ -255,22 +270,37 @@ size_t tc_b_bytes(int32_t cols, int32_t k_tiles) {
   return static_cast<size_t>((cols + kTN - 1) / kTN) * k_tiles * kStageB;
 }
 
-cudaError_t tc_gemm(double2 *out, uint8_t const *scratch, int32_t const *expo,
-                    TrTile const *tiles, int64_t n_tiles, int32_t k_tiles, int *err,
-                    cudaStream_t stream, int32_t const *entries) {
+namespace {
+template <bool kDf>
+cudaError_t gemm(void *out, uint8_t const *scratch, int32_t const *expo, TrTile const *tiles,
+                 int64_t n_tiles, int32_t k_tiles, int *err, cudaStream_t stream,
+                 int32_t const *entries) {
   if (n_tiles == 0) return cudaSuccess;
   if (k_tiles < 1) return cudaErrorInvalidValue;
-  cudaError_t e = cudaFuncSetAttribute(trace_gemm_kernel,
+  cudaError_t e = cudaFuncSetAttribute(trace_gemm_kernel<kDf>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(kSmemBytes));
   if (e != cudaSuccess) return e;
   for (int64_t t0 = 0; t0 < n_tiles; t0 += 0x7fffffffLL) {
     int64_t const n = n_tiles - t0 < 0x7fffffffLL ? n_tiles - t0 : 0x7fffffffLL;
-    trace_gemm_kernel<<<static_cast<unsigned>(persistent_grid(n)), kThreads, kSmemBytes,
-                        stream>>>(out, scratch, expo, tiles + t0, static_cast<int32_t>(n),
-                                  k_tiles, entries, err);
+    trace_gemm_kernel<kDf><<<static_cast<unsigned>(persistent_grid(n)), kThreads, kSmemBytes,
+                             stream>>>(static_cast<double2 *>(out), scratch, expo, tiles + t0,
+                                       static_cast<int32_t>(n), k_tiles, entries, err);
   }
   return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t tc_gemm(double2 *out, uint8_t const *scratch, int32_t const *expo,
+                    TrTile const *tiles, int64_t n_tiles, int32_t k_tiles, int *err,
+                    cudaStream_t stream, int32_t const *entries) {
+  return gemm<false>(out, scratch, expo, tiles, n_tiles, k_tiles, err, stream, entries);
+}
+
+cudaError_t tc_gemm_df(float4 *out, uint8_t const *scratch, int32_t const *expo,
+                       TrTile const *tiles, int64_t n_tiles, int32_t k_tiles, int *err,
+                       cudaStream_t stream) {
+  return gemm<true>(out, scratch, expo, tiles, n_tiles, k_tiles, err, stream, nullptr);
 }
 
 cudaError_t trace_tc_gemm(double2 *values, uint8_t const *scratch, int32_t const *expo,
