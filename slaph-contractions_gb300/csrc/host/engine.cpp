@@ -970,6 +970,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
   for (size_t i = 0; i < s.q2.size(); ++i) q2_t[s.q2[i].t].push_back(static_cast<int32_t>(i));
 
   std::vector<dev::GVec> vec;
+  std::vector<dev::GVecGroup> vgroups;
   std::vector<dev::TrTile> tiles;
   std::vector<dev::Q1Gather> g1;
   std::vector<dev::Q2Gather> g2;
@@ -1080,7 +1081,22 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
     std::vector<TOut> tos(batch_ts.size());
     // -- phase 1 vectors: X1 A (df source), Q2M A (f64), X1 B (f64), Q2M B (f64)
     auto begin = [&](int64_t (&r)[2]) { r[0] = static_cast<int64_t>(vec.size()); };
-    auto end = [&](int64_t (&r)[2]) { r[1] = static_cast<int64_t>(vec.size()) - r[0]; };
+    // the vectors since begin as groups: (offset, count) in vgroups
+    auto end = [&](int64_t (&r)[2]) {
+      int64_t const first = static_cast<int64_t>(vgroups.size());
+      int64_t const n = static_cast<int64_t>(vec.size());
+      for (int64_t k = r[0]; k < n;) {
+        dev::GVecGroup g{k, 0, 0};
+        do {
+          ++g.n;
+          ++k;
+        } while (k < n && vec[k].dst == vec[g.first].dst && vec[k].row % 8 != 0 &&
+                 vec[k].row == vec[k - 1].row + 1);
+        vgroups.push_back(g);
+      }
+      r[0] = first;
+      r[1] = static_cast<int64_t>(vgroups.size()) - first;
+    };
     std::vector<int64_t> regA_x1(batch_ts.size()), regB_x1(batch_ts.size()),
         regA_q2m(batch_ts.size()), regB_q2m(batch_ts.size());
     std::vector<int32_t> eA_x1(batch_ts.size()), eB_x1(batch_ts.size()),
@@ -1324,6 +1340,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
   }
   flush();
   upload(ds.fvec, vec, stream_);
+  upload(ds.fvgroups, vgroups, stream_);
   upload(ds.ftiles, tiles, stream_);
   upload(ds.fg1, g1, stream_);
   upload(ds.fg2, g2, stream_);
@@ -1469,30 +1486,31 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
       uint8_t *scr = tc_scratch_.as<uint8_t>();
       int32_t *ex = tr_expo_.as<int32_t>();
       float4 *fo = f_out_.as<float4>();
-      auto const *fv = ds.fvec.as<dev::GVec>();
+      auto const *fi = ds.fvec.as<dev::GVec>();
+      auto const *fv = ds.fvgroups.as<dev::GVecGroup>();
       auto const *ft = ds.ftiles.as<dev::TrTile>();
       auto count = [&](int64_t n) { launches_ += n > 0 ? 1 : 0; };
       for (auto const &b : ds.f_batches) {
-        cuda_check(dev::gvec_slice_df(scr, ex, fv + b.a_x1[0], b.a_x1[1], true, true,
+        cuda_check(dev::gvec_slice_df(scr, ex, fv + b.a_x1[0], b.a_x1[1], fi, true, true,
                                       q1r.as<float4>(), kt1, stream_),
                    "slice X1 A");
-        cuda_check(dev::gvec_slice_f64(scr, ex, fv + b.a_q2m[0], b.a_q2m[1], true, false,
+        cuda_check(dev::gvec_slice_f64(scr, ex, fv + b.a_q2m[0], b.a_q2m[1], fi, true, false,
                                        peram_.as<double2>(), kt1, stream_),
                    "slice Q2M A");
-        cuda_check(dev::gvec_slice_f64(scr, ex, fv + b.b_x1[0], b.b_x1[1], false, false,
+        cuda_check(dev::gvec_slice_f64(scr, ex, fv + b.b_x1[0], b.b_x1[1], fi, false, false,
                                        peram_.as<double2>(), kt1, stream_),
                    "slice X1 B");
-        cuda_check(dev::gvec_slice_f64(scr, ex, fv + b.b_q2m[0], b.b_q2m[1], false, false,
+        cuda_check(dev::gvec_slice_f64(scr, ex, fv + b.b_q2m[0], b.b_q2m[1], fi, false, false,
                                        vdv_.as<double2>(), kt1, stream_),
                    "slice Q2M B");
         count(b.a_x1[1]); count(b.a_q2m[1]); count(b.b_x1[1]); count(b.b_q2m[1]);
         cuda_check(dev::tc_gemm_df(fo, scr, ex, ft + b.t1[0], b.t1[1], kt1, err_.as<int>(), stream_),
                    "factor GEMM (X1, Q2M)");
         count(b.t1[1]);
-        cuda_check(dev::gvec_slice_df(scr, ex, fv + b.a_q2[0], b.a_q2[1], true, true, fo, kt2,
+        cuda_check(dev::gvec_slice_df(scr, ex, fv + b.a_q2[0], b.a_q2[1], fi, true, true, fo, kt2,
                                       stream_),
                    "slice Q2 A");
-        cuda_check(dev::gvec_slice_f64(scr, ex, fv + b.b_q2[0], b.b_q2[1], false, false,
+        cuda_check(dev::gvec_slice_f64(scr, ex, fv + b.b_q2[0], b.b_q2[1], fi, false, false,
                                        peram_.as<double2>(), kt2, stream_),
                    "slice Q2 B");
         count(b.a_q2[1]); count(b.b_q2[1]);

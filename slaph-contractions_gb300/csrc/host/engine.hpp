@@ -92,13 +92,13 @@ struct DeviceSchedule {
   // timeslices.  Phase 1: X1 = Q1R x perambulator blocks and the Q2M
   // intermediates (K = nev); phase 2: Q2 (K = 4 nev); then gathers into slots.
   struct FBatch {
-    int64_t a_x1[2], a_q2m[2], b_x1[2], b_q2m[2], a_q2[2], b_q2[2];  // (offset, count) in fvec
+    int64_t a_x1[2], a_q2m[2], b_x1[2], b_q2m[2], a_q2[2], b_q2[2];  // (offset, count) in fvgroups
     int64_t t1[2], t2[2];  // in ftiles
     int64_t g1[2], g2[2];  // in fg1 / fg2
   };
   bool f_ready = false;
   std::vector<FBatch> f_batches;
-  DevBuf fvec, ftiles, fg1, fg2;
+  DevBuf fvec, fvgroups, ftiles, fg1, fg2;
   size_t f_scratch = 0;
   int64_t f_out = 0, f_expo = 0;  // doubles2 of dense outputs, exponents per batch
   bool tc_ready = false;

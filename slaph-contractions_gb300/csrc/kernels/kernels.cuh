@@ -344,13 +344,19 @@ struct GVec {
   int32_t n_seg, seg_len;
   GSeg seg[kGMaxSeg];
 };
-// Slices operand vectors (A rows with put conj(v) when conj, or B columns)
-// from an FP64 or a double-float source.
-cudaError_t gvec_slice_f64(uint8_t *scratch, int32_t *expo, GVec const *items, int64_t n,
-                           bool is_a, bool conj, double2 const *src, int32_t k_tiles,
+// Up to eight consecutive operand vectors of one region, items[first .. first +
+// n), the first one's row a multiple of 8.
+struct GVecGroup {
+  int64_t first;
+  int32_t n, pad;
+};
+// Slices the operand vectors of n groups (A rows with put conj(v) when conj, or B
+// columns) from an FP64 or a double-float source.
+cudaError_t gvec_slice_f64(uint8_t *scratch, int32_t *expo, GVecGroup const *groups, int64_t n,
+                           GVec const *items, bool is_a, bool conj, double2 const *src, int32_t k_tiles,
                            cudaStream_t stream);
-cudaError_t gvec_slice_df(uint8_t *scratch, int32_t *expo, GVec const *items, int64_t n,
-                          bool is_a, bool conj, float4 const *src, int32_t k_tiles,
+cudaError_t gvec_slice_df(uint8_t *scratch, int32_t *expo, GVecGroup const *groups, int64_t n,
+                          GVec const *items, bool is_a, bool conj, float4 const *src, int32_t k_tiles,
                           cudaStream_t stream);
 // Q1 factor slots from the dense product X1 (factor_tc.cu); Q2 slots from the
 // dense Q2 GEMM output; both double-float, as tc_gemm_df writes them.  need: the

@@ -254,50 +254,6 @@ __device__ __forceinline__ int expo_of_absbits64(unsigned long long b) {
   return ex == 0 ? -1021 : ex - 1022;
 }
 
-// Writes the slices of complex element x = (fr, fi) 2^(e-55) (K index m,
-// K' = 2m, 2m+1) of A row `row` of a tile stream laid out
-// [m_tile][k_tile][slice][kTM x kTK]: row 2r gets (Re x, Im x), row 2r+1 gets
-// (-Im x, Re x) (the negated digits of Im x).
-__device__ __forceinline__ void put_a_fx(uint8_t *region, int64_t k_tiles, int row, int64_t m,
-                                         long long fr, long long fi) {
-  float dre[kSlices], dim[kSlices];
-  digits6(fr, dre);
-  digits6(fi, dim);
-  int const mt = row / (kTM / 2), r0 = 2 * (row % (kTM / 2));
-  int64_t const kt = m / (kTK / 2);
-  int const k = 2 * static_cast<int>(m % (kTK / 2));
-  uint8_t *blk = region + (static_cast<int64_t>(mt) * k_tiles + kt) * kStageA;
-#pragma unroll
-  for (int p = 0; p < kSlices; ++p) {
-    uint8_t *b = blk + p * kABlk;
-    *reinterpret_cast<uint32_t *>(b + core_off(r0, k)) = bf16x2(dre[p], dim[p]);
-    *reinterpret_cast<uint32_t *>(b + core_off(r0 + 1, k)) = bf16x2(-dim[p], dre[p]);
-  }
-}
-
-// The same for B column `col` of a stream laid out [n_tile][k_tile][slice][kTN x kTK]:
-// (Re y, Im y).
-__device__ __forceinline__ void put_b_fx(uint8_t *region, int64_t k_tiles, int col, int64_t m,
-                                         long long fr, long long fi) {
-  float dre[kSlices], dim[kSlices];
-  digits6(fr, dre);
-  digits6(fi, dim);
-  int const nt = col / kTN, r = col % kTN;
-  int64_t const kt = m / (kTK / 2);
-  int const k = 2 * static_cast<int>(m % (kTK / 2));
-  uint8_t *blk = region + (static_cast<int64_t>(nt) * k_tiles + kt) * kStageB;
-#pragma unroll
-  for (int p = 0; p < kSlices; ++p)
-    *reinterpret_cast<uint32_t *>(blk + p * kBBlk + core_off(r, k)) = bf16x2(dre[p], dim[p]);
-}
-
-// Exponent e with max |x| < 2^e for a positive maximum (0 for m == 0).
-__device__ __forceinline__ int expo_of_max(double m) {
-  int e = 0;
-  if (m > 0) frexp(m * (1.0 + 1e-15), &e);
-  return e;
-}
-
 // The tiles of one launch, each a 128 x 80 output tile of D = A' B^T over
 // k_tiles k-tiles, computed by a persistent CTA: CTA b takes tiles b, b + G,
 // b + 2G, ... (G = gridDim.x, at most one CTA per SM).  The operands:
