@@ -672,6 +672,54 @@ void Engine::set_factor_lifetime(int mode) {
   factor_lifetime_ = mode;
 }
 
+namespace {
+
+// Q1 factors that differ in gamma only pick Dirac blocks of the same products
+// R P, whose four blocks cost as much as four factors: shared when a (Q1R, r2, b)
+// has more than five factors on average (the pion-rho set: nine).
+constexpr double kQ1Share = 5.0;
+// Instances per batch: 256 MiB of products at dilE = 8.
+constexpr int64_t kX1Batch = 4096;
+
+void plan_shared_q1(DeviceSchedule &ds, Schedule const &s, cudaStream_t stream) {
+  if (ds.x1_ready) return;
+  ds.x1_ready = true;
+  auto key = [&](int32_t k) {
+    auto const &q = s.q1[k];
+    return std::make_tuple(q.t, q.b, q.r, q.r2);
+  };
+  std::vector<int32_t> ord(s.q1.size());
+  std::iota(ord.begin(), ord.end(), 0);
+  std::stable_sort(ord.begin(), ord.end(), [&](int32_t x, int32_t y) { return key(x) < key(y); });
+  size_t distinct = 0;
+  for (size_t k = 0; k < ord.size(); ++k)
+    if (k == 0 || key(ord[k]) != key(ord[k - 1])) ++distinct;
+  if (distinct == 0 ||
+      static_cast<double>(ord.size()) < kQ1Share * static_cast<double>(distinct))
+    return;
+  std::vector<dev::X1Inst> xs;
+  std::vector<dev::Q1Pick> picks;
+  for (size_t k = 0; k < ord.size(); ++k) {
+    auto const &q = s.q1[ord[k]];
+    if (k == 0 || key(ord[k]) != key(ord[k - 1])) {
+      if (xs.size() % kX1Batch == 0)
+        ds.x1_batches.push_back({static_cast<int64_t>(xs.size()), 0,
+                                 static_cast<int64_t>(picks.size()), 0});
+      xs.push_back({q.t, q.b, q.r, q.r2});
+      ++ds.x1_batches.back().n_x;
+      ds.x1_max = std::max(ds.x1_max, ds.x1_batches.back().n_x);
+    }
+    auto &b = ds.x1_batches.back();
+    picks.push_back({static_cast<int32_t>(b.n_x - 1), q.gamma, q.slot});
+    ++b.n_p;
+  }
+  upload(ds.x1, xs, stream);
+  upload(ds.q1_picks, picks, stream);
+  SLAPH_CK(cudaStreamSynchronize(stream));
+}
+
+}  // namespace
+
 std::unique_ptr<DeviceSchedule> Engine::make_schedule(slaph_plan const *plan, int bp) {
   auto const t0 = std::chrono::steady_clock::now();
   auto ds = std::make_unique<DeviceSchedule>();
@@ -1437,9 +1485,21 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
       launch(dev::q0(slots_.as<double2>(), ds.q0.as<dev::Q0Inst>(), s.q0.size(),
                      q0m.as<double2>(), noise_.as<double2>(), geo_, stream_),
              "q0");
-      launch(dev::q1(slots_.as<double2>(), ds.q1.as<dev::Q1Inst>(), s.q1.size(),
-                     q1r.as<double2>(), peram_.as<double2>(), geo_, stream_),
-             "q1");
+      plan_shared_q1(ds, s, stream_);
+      if (ds.x1_batches.empty())
+        launch(dev::q1(slots_.as<double2>(), ds.q1.as<dev::Q1Inst>(), s.q1.size(),
+                       q1r.as<double2>(), peram_.as<double2>(), geo_, stream_),
+               "q1");
+      // (f_out_, scratch of the split-precision factors, holds the products)
+      f_out_.reserve(sizeof(double2) * static_cast<size_t>(ds.x1_max) * 4 * ms);
+      for (auto const &b : ds.x1_batches) {
+        launch(dev::q1_shared(slots_.as<double2>(), f_out_.as<double2>(),
+                              ds.x1.as<dev::X1Inst>() + b.x_off, b.n_x,
+                              ds.q1_picks.as<dev::Q1Pick>() + b.p_off, b.n_p, q1r.as<double2>(),
+                              peram_.as<double2>(), geo_, stream_),
+               "q1_shared");
+        ++launches_;
+      }
       launch(dev::q2(slots_.as<double2>(), ds.q2.as<dev::Q2Inst>(), s.q2.size(),
                      q2m.as<double2>(), peram_.as<double2>(), geo_, stream_),
              "q2");

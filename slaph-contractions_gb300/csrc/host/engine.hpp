@@ -87,6 +87,15 @@ struct DeviceSchedule {
     std::vector<PLevel> p_levels;
   };
   std::vector<std::unique_ptr<WaveBufs>> waves;
+  // Q1 factors of the FP64 path that share their products (x1 instances, picks)
+  // in batches of (offset, count) pairs; empty when there are too few to share.
+  struct X1Batch {
+    int64_t x_off, n_x, p_off, n_p;
+  };
+  bool x1_ready = false;
+  std::vector<X1Batch> x1_batches;
+  DevBuf x1, q1_picks;
+  int64_t x1_max = 0;  // instances of the largest batch
   double plan_seconds = 0;
   // Q1/Q2 factors on the tensor cores (mixed precision), in batches of
   // timeslices.  Phase 1: X1 = Q1R x perambulator blocks and the Q2M

@@ -32,6 +32,13 @@ struct Q1Inst {
 struct Q2Inst {
   int32_t t, b2, m, r2, gamma, slot;
 };
+// Q1 factors of one (Q1R, r2, b): the product that they share, and each of them.
+struct X1Inst {
+  int32_t t, b, r, r2;
+};
+struct Q1Pick {
+  int32_t x, gamma, slot;  // x: instance of the batch
+};
 struct ProdInst {
   int32_t a, b, c;
 };
@@ -181,6 +188,10 @@ cudaError_t q1(double2 *slots, Q1Inst const *inst, int64_t n, double2 const *q1r
                double2 const *peram, Geometry g, cudaStream_t stream);
 cudaError_t q2(double2 *slots, Q2Inst const *inst, int64_t n, double2 const *q2m,
                double2 const *peram, Geometry g, cudaStream_t stream);
+// Q1 factors that share their products: x is scratch of n_x 64 dilE^2 entries.
+cudaError_t q1_shared(double2 *slots, double2 *x, X1Inst const *xi, int64_t n_x,
+                      Q1Pick const *picks, int64_t n, double2 const *q1r, double2 const *peram,
+                      Geometry g, cudaStream_t stream);
 
 // slots[c] = slots[a] * slots[b] (operator*, src/DilutedFactor.cpp:6-51).
 cudaError_t products(double2 *slots, ProdInst const *p, int64_t n, int32_t eds,

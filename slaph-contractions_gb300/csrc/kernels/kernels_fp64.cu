@@ -33,6 +33,16 @@ __device__ __forceinline__ void cfmac(double2 &acc, double2 a, double2 b) {
   acc.y = fma(a.x, b.y, fma(-a.y, b.x, acc.y));
 }
 
+// |a| >= |b| as hypot would decide it: the squares settle it unless they are
+// within rounding of one another or near the ends of the range (hypot is some
+// 50 FP64 operations, five times the rest of a compensated addition).
+__device__ __forceinline__ bool not_smaller(double2 a, double2 b) {
+  double const p = fma(a.x, a.x, a.y * a.y), q = fma(b.x, b.x, b.y * b.y);
+  double const hi = fmax(p, q);
+  if (hi > 1e-270 && hi < 1e270 && fabs(p - q) > 1e-14 * hi) return p > q;
+  return hypot(a.x, a.y) >= hypot(b.x, b.y);
+}
+
 // Neumaier accumulator on complex values, include/KahanAccumulator.hpp:14-48;
 // with kahan == 0 it is NativeAccumulator (:50-72).
 struct Acc {
@@ -46,7 +56,7 @@ struct Acc {
       return;
     }
     double2 const t = make_double2(s.x + x.x, s.y + x.y);
-    if (hypot(s.x, s.y) >= hypot(x.x, x.y)) {
+    if (not_smaller(s, x)) {
       c.x += (s.x - t.x) + x.x;
       c.y += (s.y - t.y) + x.y;
     } else {
@@ -166,39 +176,44 @@ __global__ void q1r_kernel(double2 *out, Q1RInst const *inst, double2 const *vdv
 // signs, applied in q2_kernel):
 // M[col dilE + e, row nev + v] = sum_w conj(P_r1[(4t + row) nev + w,
 //                                               (4 b1 + col) dilE + e]) vdv[w, v].
-// Per CTA a 32 x 64 tile of one dirac row; 16 w per step.
+// Per CTA a 32 x 64 tile of the rows (dirac row, a) of all four Dirac blocks, so
+// that only the last of 4 eds / 32 tiles has padding; 16 w per step.
 constexpr int MT = 32, NT = 64, KT = 16;
 __global__ void __launch_bounds__(256) q2m_kernel(double2 *out, Q2MInst const *inst,
                                                   double2 const *vdv, double2 const *peram,
                                                   Geometry g) {
   __shared__ double2 As[KT][MT + 1];
   __shared__ double2 Bs[KT][NT];
-  Q2MInst const in = inst[blockIdx.z];
+  Q2MInst const in = inst[blockIdx.y];
   int const nev = g.nev, eds = 4 * g.dilE;
-  int const ntile = (nev + NT - 1) / NT, mtile = (eds + MT - 1) / MT;
-  int const row = blockIdx.y;  // dirac row of the perambulator block
+  int const ntile = (nev + NT - 1) / NT;
   int const v0 = (blockIdx.x % ntile) * NT;
-  int const a0 = (blockIdx.x / ntile) * MT;
-  if (a0 >= mtile * MT) return;
+  int const m0 = (blockIdx.x / ntile) * MT;
   int const tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
   int64_t const rows = peram_rows(g);
-  double2 const *P = peram_of(peram, in.r1, g) +
-                     (static_cast<int64_t>(4 * in.t + row) * nev) +
+  double2 const *P = peram_of(peram, in.r1, g) + static_cast<int64_t>(4 * in.t) * nev +
                      rows * (static_cast<int64_t>(in.b1) * eds);
   double2 const *m = vdv_block(vdv, in.vdv, in.t, g);
+  // Rows that this thread stages, and whether its outputs are wanted at all
+  // (warps without any skip the arithmetic).
+  double2 const *row_p[2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    int const mm = m0 + tid / KT + 16 * q;
+    row_p[q] = mm < 4 * eds ? P + static_cast<int64_t>(mm / eds) * nev + rows * (mm % eds) : nullptr;
+  }
+  bool const warp_on = m0 + (ty & ~1) < 4 * eds;
   double2 acc[2][4];
 #pragma unroll
   for (int p = 0; p < 2; ++p)
 #pragma unroll
     for (int q = 0; q < 4; ++q) acc[p][q] = make_double2(0, 0);
   for (int w0 = 0; w0 < nev; w0 += KT) {
+    int const wk = w0 + tid % KT;
 #pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      int const k = tid + 256 * q;
-      int const ww = k % KT, aa = k / KT;
-      int const w = w0 + ww, a = a0 + aa;
-      As[ww][aa] = (w < nev && a < eds) ? P[w + rows * a] : make_double2(0, 0);
-    }
+    for (int q = 0; q < 2; ++q)
+      As[tid % KT][tid / KT + 16 * q] =
+          wk < nev && row_p[q] ? row_p[q][wk] : make_double2(0, 0);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       int const k = tid + 256 * q;
@@ -208,27 +223,29 @@ __global__ void __launch_bounds__(256) q2m_kernel(double2 *out, Q2MInst const *i
                                         : make_double2(0, 0);
     }
     __syncthreads();
+    if (warp_on)
 #pragma unroll 4
-    for (int kk = 0; kk < KT; ++kk) {
-      double2 a[2], b[4];
+      for (int kk = 0; kk < KT; ++kk) {
+        double2 a[2], b[4];
 #pragma unroll
-      for (int p = 0; p < 2; ++p) a[p] = As[kk][ty + 16 * p];
+        for (int p = 0; p < 2; ++p) a[p] = As[kk][ty + 16 * p];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) b[q] = Bs[kk][tx + 16 * q];
+        for (int q = 0; q < 4; ++q) b[q] = Bs[kk][tx + 16 * q];
 #pragma unroll
-      for (int p = 0; p < 2; ++p)
+        for (int p = 0; p < 2; ++p)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) cfmac(acc[p][q], a[p], b[q]);
-    }
+          for (int q = 0; q < 4; ++q) cfmac(acc[p][q], a[p], b[q]);
+      }
     __syncthreads();
   }
-  double2 *o = out + static_cast<int64_t>(blockIdx.z) * eds * 4 * nev;
+  double2 *o = out + static_cast<int64_t>(blockIdx.y) * eds * 4 * nev;
 #pragma unroll
   for (int p = 0; p < 2; ++p)
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      int const a = a0 + ty + 16 * p, v = v0 + tx + 16 * q;
-      if (a < eds && v < nev) o[a + static_cast<int64_t>(eds) * (row * nev + v)] = acc[p][q];
+      int const mm = m0 + ty + 16 * p, v = v0 + tx + 16 * q;
+      if (mm < 4 * eds && v < nev)
+        o[mm % eds + static_cast<int64_t>(eds) * (mm / eds * nev + v)] = acc[p][q];
     }
 }
 
@@ -278,6 +295,37 @@ __global__ void q1_kernel(double2 *slots, Q1Inst const *inst, double2 const *q1r
   double2 acc = make_double2(0, 0);
   for (int v = 0; v < nev; ++v) cfma(acc, R[a + static_cast<int64_t>(eds) * v], P[v]);
   slots[static_cast<int64_t>(in.slot) * eds * eds + k] = cmul(c_gamma_val[in.gamma][row], acc);
+}
+
+// The products R P_r2 of all four Dirac blocks d of the perambulator, shared by
+// the Q1 factors that differ in gamma only: X[a, d eds + c] = sum_v R[a, v]
+// P_r2[(4t + d) nev + v, b eds + c], summed as in q1_kernel.  One CTA per
+// instance and Dirac block.
+__global__ void x1_kernel(double2 *out, X1Inst const *inst, double2 const *q1r,
+                          double2 const *peram, Geometry g) {
+  X1Inst const in = inst[blockIdx.y];
+  int const nev = g.nev, eds = 4 * g.dilE;
+  int const k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= 4 * eds * eds) return;
+  int const a = k % eds, c = k / eds % eds, d = k / (eds * eds);
+  int64_t const rows = peram_rows(g);
+  double2 const *R = q1r + static_cast<int64_t>(in.r) * nev * eds + a;
+  double2 const *P = peram_of(peram, in.r2, g) + static_cast<int64_t>(4 * in.t + d) * nev +
+                     rows * (static_cast<int64_t>(in.b) * eds + c);
+  double2 acc = make_double2(0, 0);
+  for (int v = 0; v < nev; ++v) cfma(acc, R[static_cast<int64_t>(eds) * v], P[v]);
+  out[static_cast<int64_t>(blockIdx.y) * 4 * eds * eds + k] = acc;
+}
+
+// Q1 factors from those products: val[row] X[a, Grow[row] eds + c].
+__global__ void q1_pick_kernel(double2 *slots, Q1Pick const *inst, double2 const *x, int32_t dilE) {
+  Q1Pick const in = inst[blockIdx.y];
+  int const eds = 4 * dilE;
+  int const k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= eds * eds) return;
+  int const row = k % eds / dilE;
+  double2 const v = x[(4LL * in.x + c_gamma_row[in.gamma][row]) * eds * eds + k];
+  slots[static_cast<int64_t>(in.slot) * eds * eds + k] = cmul(c_gamma_val[in.gamma][row], v);
 }
 
 // Q2 factor, src/DilutedFactorFactory.cpp:214-243:
@@ -338,7 +386,9 @@ __global__ void __launch_bounds__(256) product_kernel(double2 *slots, ProdInst c
 
 // ---------------------------------------------------------------- traces
 // factor_to_trace, src/DilutedTrace.cpp:84-165: tr(L R) per entry (or tr(F)).
-// One CTA per list, one warp per entry, one lane per row.
+// One CTA per list, one lane per row; a warp takes 32 / eds entries at once when
+// the matrices have 16 rows or fewer (16 rows left half of its lanes idle:
+// 4^3x8 pipi set at eds 16, 5.2 -> 2.6 ms).
 __global__ void __launch_bounds__(256) trace_kernel(double2 *values, TraceList const *lists,
                                                     int32_t const *which,
                                                     int32_t const *shape_i,
@@ -349,31 +399,41 @@ __global__ void __launch_bounds__(256) trace_kernel(double2 *values, TraceList c
   int64_t const off = shape_off[L.shape];
   int const n = static_cast<int>(shape_off[L.shape + 1] - off);
   int const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  int const per = eds <= 16 ? 32 / eds : 1;  // entries per warp
+  int const sub = per > 1 ? lane / eds : 0, i0 = per > 1 ? lane % eds : lane;
   int64_t const ms = static_cast<int64_t>(eds) * eds;
-  for (int e = warp; e < n; e += blockDim.x / 32) {
-    int const ia = shape_i[off + e], jb = shape_j[off + e];
+  for (int e0 = warp * per; e0 < n; e0 += blockDim.x / 32 * per) {
+    int const e = e0 + sub;
+    bool const on = sub < per && e < n;
+    int const ia = on ? shape_i[off + e] : 0, jb = on ? shape_j[off + e] : -1;
     double2 const *A = slots + (static_cast<int64_t>(L.a_base) + ia) * ms;
     double2 acc = make_double2(0, 0);
-    if (jb >= 0) {
+    if (on && jb >= 0) {
       double2 const *B = slots + (static_cast<int64_t>(L.b_base) + jb) * ms;
-      for (int i = lane; i < eds; i += 32) {
+      for (int i = i0; i < eds; i += 32) {
         double2 row = make_double2(0, 0);
         for (int j = 0; j < eds; ++j) cfma(row, A[i + eds * j], B[j + eds * i]);
         acc.x += row.x;
         acc.y += row.y;
       }
-    } else {
-      for (int i = lane; i < eds; i += 32) {
+    } else if (on) {
+      for (int i = i0; i < eds; i += 32) {
         acc.x += A[i + eds * i].x;
         acc.y += A[i + eds * i].y;
       }
     }
+    // sum over the lanes of an entry (rows i0 + s beyond its last add nothing)
+    int const width = per > 1 ? eds : 32;
 #pragma unroll
     for (int s = 16; s > 0; s >>= 1) {
-      acc.x += __shfl_down_sync(0xffffffffu, acc.x, s);
-      acc.y += __shfl_down_sync(0xffffffffu, acc.y, s);
+      double const x = __shfl_down_sync(0xffffffffu, acc.x, s);
+      double const y = __shfl_down_sync(0xffffffffu, acc.y, s);
+      if (i0 + s < width) {
+        acc.x += x;
+        acc.y += y;
+      }
     }
-    if (lane == 0) values[L.val_off + static_cast<int64_t>(e) * L.stride] = acc;
+    if (on && i0 == 0) values[L.val_off + static_cast<int64_t>(e) * L.stride] = acc;
   }
 }
 
@@ -708,9 +768,9 @@ cudaError_t q2m(double2 *out, Q2MInst const *inst, int64_t n, double2 const *vdv
                 double2 const *peram, Geometry g, cudaStream_t stream) {
   int const eds = 4 * g.dilE;
   int64_t const per = static_cast<int64_t>(eds) * 4 * g.nev;
-  int const ntile = (g.nev + NT - 1) / NT, mtile = (eds + MT - 1) / MT;
+  int const ntile = (g.nev + NT - 1) / NT, mtile = (4 * eds + MT - 1) / MT;
   return chunked(inst, n, [&](Q2MInst const *p, int c, int64_t s) {
-    q2m_kernel<<<dim3(ntile * mtile, 4, c), 256, 0, stream>>>(out + s * per, p, vdv, peram, g);
+    q2m_kernel<<<dim3(ntile * mtile, c), 256, 0, stream>>>(out + s * per, p, vdv, peram, g);
   });
 }
 
@@ -727,6 +787,20 @@ cudaError_t q1(double2 *slots, Q1Inst const *inst, int64_t n, double2 const *q1r
   int64_t const per = 16LL * g.dilE * g.dilE;
   return chunked(inst, n, [&](Q1Inst const *p, int c, int64_t) {
     q1_kernel<<<dim3(blocks_for(per, 256), c), 256, 0, stream>>>(slots, p, q1r_, peram, g);
+  });
+}
+
+cudaError_t q1_shared(double2 *slots, double2 *x, X1Inst const *xi, int64_t n_x,
+                      Q1Pick const *picks, int64_t n, double2 const *q1r_, double2 const *peram,
+                      Geometry g, cudaStream_t stream) {
+  int64_t const per = 16LL * g.dilE * g.dilE;
+  cudaError_t const e = chunked(xi, n_x, [&](X1Inst const *p, int c, int64_t s) {
+    x1_kernel<<<dim3(blocks_for(4 * per, 256), c), 256, 0, stream>>>(x + s * 4 * per, p, q1r_,
+                                                                     peram, g);
+  });
+  if (e != cudaSuccess) return e;
+  return chunked(picks, n, [&](Q1Pick const *p, int c, int64_t) {
+    q1_pick_kernel<<<dim3(blocks_for(per, 256), c), 256, 0, stream>>>(slots, p, x, g.dilE);
   });
 }
 
