@@ -929,6 +929,8 @@ void Engine::prepare_product_tc(DeviceSchedule &ds) {
   Schedule const &s = ds.s;
   int32_t const eds = s.eds;
   int64_t const a_bytes = dev::prod_tc_a_bytes(eds), r_bytes = dev::prod_tc_r_bytes(eds);
+  int sms = 0;
+  SLAPH_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
   size_t need = 0;
   int64_t max_expo = 0;
   for (size_t wi = 0; wi < s.waves.size(); ++wi) {
@@ -949,6 +951,12 @@ void Engine::prepare_product_tc(DeviceSchedule &ds) {
       int32_t const u_base = static_cast<int32_t>(u_list.size());
       u_list.insert(u_list.end(), pp.u_list.begin(), pp.u_list.end());
       out_tab.insert(out_tab.end(), pp.out_tab.begin(), pp.out_tab.end());
+      // Right matrices per unit of work: six units per SM, so that the last ones
+      // end together; at least four, for which the A operand is copied once.
+      int64_t steps = 0;
+      for (auto const &pg : pp.groups) steps += pg.n_u;
+      int32_t const unit = static_cast<int32_t>(
+          std::clamp<int64_t>(steps / (6 * std::max(sms, 1)), 4, dev::kProdSteps));
       for (auto const &pg : pp.groups) {
         dev::ProdGroup g{};
         for (int x = 0; x < 4; ++x) g.l[x] = pg.l[x];
@@ -957,8 +965,13 @@ void Engine::prepare_product_tc(DeviceSchedule &ds) {
         g.u_off = u_base + pg.u_off;
         int32_t const gi = static_cast<int32_t>(groups.size() - pl.g_off);
         g.ea = 64 * gi;
-        int32_t const n_t = (eds * g.n_u + dev::kTrTileCols - 1) / dev::kTrTileCols;
-        for (int32_t nt = 0; nt < n_t; ++nt) tiles.push_back({gi, nt});
+        if (dev::prod_tc_steps(eds)) {
+          for (int32_t u = 0; u < g.n_u; u += unit)
+            tiles.push_back({gi, 0, g.u_off + u, std::min(unit, g.n_u - u), g.n_l, g.ea});
+        } else {
+          int32_t const n_t = (eds * g.n_u + dev::kTrTileCols - 1) / dev::kTrTileCols;
+          for (int32_t nt = 0; nt < n_t; ++nt) tiles.push_back({gi, nt, 0, 0, 0, 0});
+        }
         groups.push_back(g);
       }
       pl.n_g = static_cast<int64_t>(groups.size()) - pl.g_off;

@@ -245,9 +245,15 @@ struct ProdGroup {
   int32_t u_off;  // first column block in u_list / out_tab
   int32_t ea;     // exponent index of the group's row 0 (64 g)
 };
+// One unit of GEMM work.  eds = 64: the 80-column tile nt of the group.  eds = 16,
+// 32: the n (at most kProdSteps) right matrices u_list[u .. u + n) of the group,
+// one GEMM step each; n_l and ea repeat the group's.
+constexpr int32_t kProdSteps = 32;
 struct ProdTile {
   int32_t group, nt;
+  int32_t u, n, n_l, ea;
 };
+inline bool prod_tc_steps(int32_t eds) { return eds == 16 || eds == 32; }
 __host__ __device__ inline int64_t prod_tc_r_bytes(int32_t eds) {
   return 24LL * eds * eds;  // (eds / 16) k-tiles x 6 slices x eds columns x 32 bytes
 }

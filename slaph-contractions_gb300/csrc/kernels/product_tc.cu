@@ -17,9 +17,20 @@
 // the left matrices (conjugated, so that the conjugating form gives the plain
 // product), one exponent per row; each distinct right matrix of the level is
 // sliced once into a stream of its own, [k-tile][slice][8-column group][512
-// bytes] with one exponent per column, and the producer of the GEMM gathers a
-// tile's B stage from those streams with one bulk copy per (slice, right
-// matrix).
+// bytes] with one exponent per column.
+//
+// product_step_kernel (eds = 16, 32) takes one right matrix per step against the
+// group's A operand, which stays in shared memory: a step is K = eds, one or
+// two k-tiles, so promotion and epilogue, not the MMAs, bound it.  With the
+// general tile (tc_common.cuh: 80 columns, eight promotion warps that hold 40
+// columns of running sums and hand them to an unrolled epilogue) a tile's MMAs
+// took 2.7 us of 14: the code did not fit the instruction cache and nothing
+// overlapped.  Here sixteen promotion warps take eight columns each in one
+// straight pass (there is one chunk, so no running sums), two accumulator sets
+// let the next step's MMAs run meanwhile, a right matrix is one bulk copy, and
+// pairs that the level does not ask for are skipped.  24^3x48 Nev 120: 9.8 ->
+// 3.8 ms.  eds = 64 does not fit (A alone is 192 KB) and keeps the general
+// tile, whose producer gathers the B stage with one copy per (slice, matrix).
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -305,6 +316,252 @@ __global__ void __launch_bounds__(kThreads, 1)
   ozaki_tiles(smem, n_tiles, tl.k_tiles, tl, err, epi);
 }
 
+// ---------------------------------------------------------------- steps
+constexpr int kStepWarps = 16;  // promotion warps: quadrant w % 4, column block w / 4
+constexpr int kStepThreads = 32 * (kStepWarps + 2);
+constexpr int kStepStages = 4;  // right matrices in flight
+constexpr uint32_t kStepTmem = 256;  // columns per accumulator set (6 eds used)
+
+__host__ __device__ inline uint32_t step_a_bytes(int eds) { return eds / 16 * kStageA; }
+__host__ __device__ inline uint32_t step_smem(int eds) {
+  return step_a_bytes(eds) + kStepStages * 24u * eds * eds;
+}
+
+struct StepArgs {
+  uint8_t const *scratch;  // A regions from 0, right-matrix streams from r_off
+  int64_t a_bytes, r_off;
+  ProdTile const *units;
+  int32_t n_units;
+  int32_t const *u_list;
+  int32_t const *expo;  // A rows from 0 (64 per group), right columns from r_expo
+  int64_t r_expo;
+  int32_t const *out_tab;
+  float4 *slots_n, *slots_t;
+  unsigned int *slot_bits;
+  int *err;
+};
+
+template <int kEds>
+__global__ void __launch_bounds__(kStepThreads, 1) product_step_kernel(StepArgs const g) {
+  constexpr int kKT = kEds / 16;                      // k-tiles
+  constexpr uint32_t kRB = 24u * kEds * kEds;         // bytes of a right matrix
+  constexpr int kColBlocks = kEds / 8;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ __align__(8) uint64_t a_full, a_empty, b_full[kStepStages], b_empty[kStepStages];
+  __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], done_bar;
+  __shared__ uint32_t tmem_slot;
+  int const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  uint8_t *const b_smem = smem + step_a_bytes(kEds);
+  if (threadIdx.x == 0) {
+    mbar_init(&a_full, 1);
+    mbar_init(&a_empty, 1);
+    for (int s = 0; s < kStepStages; ++s) {
+      mbar_init(&b_full[s], 1);
+      mbar_init(&b_empty[s], 1);
+    }
+    for (int s = 0; s < 2; ++s) {
+      mbar_init(&acc_full[s], 1);
+      mbar_init(&acc_empty[s], kStepWarps);
+    }
+    mbar_init(&done_bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&tmem_slot)),
+                 "r"(kTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  uint32_t const tmem = tmem_slot;
+
+  if (warp == kStepWarps) {  // producer
+    bool ok = true;
+    uint32_t n_a = 0, n_b = 0;  // A operands, right matrices issued
+    for (int i = blockIdx.x; i < g.n_units && ok; i += gridDim.x) {
+      ProdTile const t = g.units[i];
+      int const idx = lane < t.n ? g.u_list[t.u + lane] : 0;
+      if (lane == 0) {
+        if (n_a > 0) ok = mbar_wait(&a_empty, (n_a - 1) & 1, g.err, 1);
+        if (ok) {
+          mbar_expect_tx(&a_full, step_a_bytes(kEds));
+          bulk_g2s(smem, g.scratch + t.group * g.a_bytes, step_a_bytes(kEds), &a_full);
+        }
+      }
+      ok = __shfl_sync(0xffffffffu, ok, 0);
+      if (!ok) break;
+      ++n_a;
+      for (int s = 0; s < t.n && ok; ++s) {
+        int const r = __shfl_sync(0xffffffffu, idx, s);
+        uint32_t const st = n_b % kStepStages, use = n_b / kStepStages;
+        if (lane == 0) {
+          if (use > 0) ok = mbar_wait(&b_empty[st], (use - 1) & 1, g.err, 1);
+          if (ok) {
+            mbar_expect_tx(&b_full[st], kRB);
+            bulk_g2s(b_smem + st * kRB, g.scratch + g.r_off + static_cast<int64_t>(r) * kRB, kRB,
+                     &b_full[st]);
+          }
+        }
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        if (ok) ++n_b;
+      }
+    }
+    // All copies have landed before shared memory is released (immediate when
+    // the MMA warp consumed them).
+    if (lane == 0) {
+      if (n_a > 0) mbar_wait(&a_full, (n_a - 1) & 1, g.err, 6);
+      for (uint32_t q = n_b > kStepStages ? n_b - kStepStages : 0; q < n_b; ++q)
+        mbar_wait(&b_full[q % kStepStages], (q / kStepStages) & 1, g.err, 6);
+    }
+  } else if (warp == kStepWarps + 1) {
+    if (lane == 0) {  // MMA issuer
+      bool ok = true;
+      uint32_t n_a = 0, n_s = 0;
+      uint32_t const a_base = smem_u32(smem);
+      for (int i = blockIdx.x; i < g.n_units && ok; i += gridDim.x, ++n_a) {
+        int const n = g.units[i].n;
+        ok = mbar_wait(&a_full, n_a & 1, g.err, 3);
+        for (int s = 0; s < n && ok; ++s, ++n_s) {
+          uint32_t const st = n_s % kStepStages, set = n_s % 2;
+          ok = mbar_wait(&b_full[st], (n_s / kStepStages) & 1, g.err, 3) &&
+               (n_s < 2 || mbar_wait(&acc_empty[set], (n_s / 2 - 1) & 1, g.err, 2));
+          if (!ok) break;
+          tc_fence_after();
+          uint32_t const b_base = smem_u32(b_smem + st * kRB);
+          uint32_t const d = tmem + set * kStepTmem;
+          // the 21 slice pairs as 9 MMAs per k-step (tc_common.cuh)
+#pragma unroll
+          for (int ks = 0; ks < 2 * kKT; ++ks) {
+#pragma unroll
+            for (int p = 0; p < kSlices; ++p) {
+#pragma unroll
+              for (int q0 = 0; q0 < kSlices - p; q0 += kLevelGroup) {
+                int const nb = min(kLevelGroup, kSlices - p - q0);
+                uint64_t const ad =
+                    smem_desc(a_base + (ks / 2) * kStageA + p * kABlk + (ks % 2) * 256, 128, 512);
+                uint64_t const bd = smem_desc(
+                    b_base + (ks / 2) * (kSlices * kEds * 64) + q0 * (kEds * 64) + (ks % 2) * 256,
+                    128, 512);
+                mma_bf16(d + static_cast<uint32_t>((p + q0) * kEds), ad, bd,
+                         ks == 0 && p == 0 ? 0u : 1u, idesc_n(nb * kEds));
+              }
+            }
+          }
+          mma_commit(&b_empty[st]);
+          mma_commit(&acc_full[set]);
+        }
+        if (ok) mma_commit(&a_empty);
+      }
+      mma_commit(&done_bar);
+      mbar_wait(&done_bar, 0, g.err, 4);
+    }
+  } else {
+    // Promotion: A' row 2 cr + (re | im), cr = l kEds + i; columns 8 blk .. of the
+    // step's right matrix.  A warp's rows lie in one left matrix, its columns in
+    // one right matrix: one product slot per warp and step.
+    int const quad = warp % 4, blk = warp / 4;
+    int const row = 32 * quad + lane, cr = row / 2, l = cr / kEds, ri = cr % kEds;
+    bool const blk_on = blk < kColBlocks;
+    uint32_t const lane_addr =
+        tmem + (static_cast<uint32_t>(32 * quad) << 16) + static_cast<uint32_t>(8 * blk);
+    int64_t const ms = kEds * kEds;
+    uint32_t n_s = 0;
+    bool ok = true;
+    for (int i = blockIdx.x; i < g.n_units && ok; i += gridDim.x) {
+      ProdTile const t = g.units[i];
+      bool const on = blk_on && l < t.n_l;  // warp-uniform
+      // lane s holds the right matrix and the product slot of step s
+      int const idx = lane < t.n ? g.u_list[t.u + lane] : 0;
+      int const slots = on && lane < t.n ? g.out_tab[4 * (t.u + lane) + l] : -1;
+      int const er = on ? g.expo[t.ea + cr] : 0;
+      auto column_expo = [&](int s) {  // lane c: exponent of column 8 blk + c of step s
+        int const r = __shfl_sync(0xffffffffu, idx, s);
+        return blk_on && lane < 8
+                   ? g.expo[g.r_expo + static_cast<int64_t>(r) * kEds + 8 * blk + lane]
+                   : 0;
+      };
+      int ec_next = column_expo(0);
+      for (int s = 0; s < t.n; ++s, ++n_s) {
+        uint32_t const set = n_s % 2;
+        int const slot = __shfl_sync(0xffffffffu, slots, s);
+        int const ec_lane = ec_next;
+        if (s + 1 < t.n) ec_next = column_expo(s + 1);
+        if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[set], (n_s / 2) & 1, g.err, 5))) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        uint32_t r0[3][8], r1[3][8];
+        if (slot >= 0) {  // warp-uniform
+          uint32_t const ca = lane_addr + set * kStepTmem;
+#pragma unroll
+          for (int v = 0; v < 3; ++v) tmem_ld8_issue(ca + static_cast<uint32_t>(v * kEds), r0[v]);
+#pragma unroll
+          for (int v = 0; v < 3; ++v)
+            tmem_ld8_issue(ca + static_cast<uint32_t>((3 + v) * kEds), r1[v]);
+          tmem_ld_wait(r0);
+          tmem_ld_wait(r1);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[set]);
+        if (slot < 0) continue;
+        unsigned int mx = 0;
+        float4 *const dst = (row & 1) ? g.slots_t + slot * ms + static_cast<int64_t>(kEds) * ri
+                                      : g.slots_n + slot * ms + ri;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          // the chunk's value in (hi, lo), as in tc_common.cuh
+          float s1, x1, s2, x2, s3, x3;
+          two_sum(__uint_as_float(r0[0][u]), __uint_as_float(r0[1][u]) * 0x1p-8f, s1, x1);
+          two_sum(s1, __uint_as_float(r0[2][u]) * 0x1p-16f, s2, x2);
+          float const low = fmaf(__uint_as_float(r1[2][u]), 0x1p-16f,
+                                 fmaf(__uint_as_float(r1[1][u]), 0x1p-8f,
+                                      __uint_as_float(r1[0][u]))) *
+                            0x1p-24f;
+          two_sum(s2, low, s3, x3);
+          float const e = (x1 + x2) + x3;
+          float const hi = s3 + e, lo = e - (hi - s3);
+          int const sh = max(er + __shfl_sync(0xffffffffu, ec_lane, u) - 14, -252);
+          float const h = scale2(hi, sh), lw = scale2(lo, sh);
+          float const oh = __shfl_xor_sync(0xffffffffu, h, 1);
+          float const ol = __shfl_xor_sync(0xffffffffu, lw, 1);
+          mx = max(mx, __float_as_uint(h) & 0x7FFFFFFFu);
+          int const j = 8 * blk + u;
+          // the even lane of a row pair (Re) stores the natural layout, the odd
+          // one (Im) the transposed
+          dst[(row & 1) ? j : kEds * j] = (row & 1) ? make_float4(oh, ol, h, lw)
+                                                    : make_float4(h, lw, oh, ol);
+        }
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        if (lane == 0) atomicMax(g.slot_bits + slot, mx);
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+                 "r"(kTmemCols)
+                 : "memory");
+  }
+}
+
+template <int kEds>
+cudaError_t launch_steps(StepArgs const &args, cudaStream_t stream) {
+  cudaError_t const e = cudaFuncSetAttribute(product_step_kernel<kEds>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(step_smem(kEds)));
+  if (e != cudaSuccess) return e;
+  product_step_kernel<kEds><<<static_cast<unsigned>(persistent_grid(args.n_units)), kStepThreads,
+                              step_smem(kEds), stream>>>(args);
+  return cudaGetLastError();
+}
+
 }  // namespace
 
 bool prod_tc_supported(int32_t eds) { return eds == 16 || eds == 32 || eds == 64; }
@@ -327,6 +584,13 @@ cudaError_t products_tc(float4 *slots_n, float4 *slots_t, uint8_t *scratch, int6
   if (n_r > 0)
     prod_slice_r_kernel<<<static_cast<unsigned>(n_r), kPSliceThreads, 0, stream>>>(
         scratch + r_off, expo + r_expo, r_slots, slots_n, eds);
+  if (prod_tc_steps(eds)) {
+    cudaError_t const se = cudaGetLastError();
+    if (se != cudaSuccess) return se;
+    StepArgs const args{scratch, a_bytes, r_off, tiles, static_cast<int32_t>(n_tiles), u_list,
+                        expo, r_expo, out_tab, slots_n, slots_t, slot_bits, err};
+    return eds == 32 ? launch_steps<32>(args, stream) : launch_steps<16>(args, stream);
+  }
   cudaError_t e = cudaFuncSetAttribute(product_gemm_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(kSmemBytes));
