@@ -391,94 +391,107 @@ class Builder {
         uniq.push_back(ord[p]);
       }
     }
-    // Runs of equal (shape, a_base) among the two-matrix lists: the B set of
-    // each A group, in increasing b_base.  A groups with equal (shape, B set)
-    // form a complete bipartite set.
+    // Runs of equal (shape, a_base) among the two-matrix lists `u` (in key order):
+    // the B set of each A group, in increasing b_base.  A groups with equal
+    // (shape, B set) form a complete bipartite set.
     struct Run {
       int32_t shape, a;
-      int64_t begin, end;  // into uniq
+      int64_t begin, end;  // into u
       uint64_t hash;
     };
-    std::vector<Run> runs;
-    for (int64_t p = 0; p < static_cast<int64_t>(uniq.size());) {
-      auto const &l = w.lists[uniq[p]];
-      int64_t q = p;
-      uint64_t h = 1469598103934665603ULL;
-      while (q < static_cast<int64_t>(uniq.size()) && w.lists[uniq[q]].shape == l.shape &&
-             w.lists[uniq[q]].a_base == l.a_base) {
-        h = (h ^ static_cast<uint32_t>(w.lists[uniq[q]].b_base)) * 1099511628211ULL;
-        ++q;
-      }
-      if (l.b_base >= 0) runs.push_back({l.shape, l.a_base, p, q, h});
-      p = q;
-    }
-    auto same_set = [&](Run const &x, Run const &y) {
-      if (x.shape != y.shape || x.end - x.begin != y.end - y.begin || x.hash != y.hash)
-        return false;
-      for (int64_t u = 0; u < x.end - x.begin; ++u)
-        if (w.lists[uniq[x.begin + u]].b_base != w.lists[uniq[y.begin + u]].b_base)
-          return false;
-      return true;
-    };
-    // Runs in order of (shape, B-set hash, B-set size), ties in run order.
-    struct RunKey {
-      int32_t shape, k;
-      uint64_t hash;
-      int64_t size;
-      bool operator<(RunKey const &o) const {
-        return std::tie(shape, hash, size, k) < std::tie(o.shape, o.hash, o.size, o.k);
-      }
-    };
-    std::vector<int32_t> run_ord(runs.size());
-    {
-      std::vector<RunKey> keys(runs.size());
-      for (size_t k = 0; k < runs.size(); ++k)
-        keys[k] = {runs[k].shape, static_cast<int32_t>(k), runs[k].hash,
-                   runs[k].end - runs[k].begin};
-      std::sort(keys.begin(), keys.end());
-      for (size_t p = 0; p < keys.size(); ++p) run_ord[p] = keys[p].k;
-    }
     std::vector<char> in_group(n, 0);
     w.groups.clear();
     w.group_bases.clear();
     int64_t val = 0;
-    for (size_t p = 0; p < run_ord.size();) {
-      size_t q = p + 1;
-      while (q < run_ord.size() && same_set(runs[run_ord[p]], runs[run_ord[q]])) ++q;
-      Run const &r0 = runs[run_ord[p]];
-      int32_t const n_a = static_cast<int32_t>(q - p);
-      int32_t const n_b = static_cast<int32_t>(r0.end - r0.begin);
-      if (n_a >= kMinGroupA && n_b >= kMinGroupB) {
-        TraceGroup g{};
-        g.shape = r0.shape;
-        g.n_a = n_a;
-        g.n_b = n_b;
-        g.a_off = static_cast<int64_t>(w.group_bases.size());
-        std::vector<int32_t> members(run_ord.begin() + p, run_ord.begin() + q);
-        std::sort(members.begin(), members.end(),
-                  [&](int32_t x, int32_t y) { return runs[x].a < runs[y].a; });
-        for (int32_t m : members) w.group_bases.push_back(runs[m].a);
-        g.b_off = static_cast<int64_t>(w.group_bases.size());
-        for (int64_t u = r0.begin; u < r0.end; ++u)
-          w.group_bases.push_back(w.lists[uniq[u]].b_base);
-        g.val_base = val;
-        int64_t const n_e = static_cast<int64_t>(s_.shapes[g.shape].i.size());
-        int64_t const plane = static_cast<int64_t>(n_a) * n_b;
-        for (int32_t ia = 0; ia < n_a; ++ia) {
-          Run const &r = runs[members[ia]];
-          for (int64_t u = r.begin; u < r.end; ++u) {
-            auto &l = w.lists[uniq[u]];
-            l.val_off = val + (u - r.begin) * n_a + ia;
-            l.stride = static_cast<int32_t>(plane);
-            in_group[uniq[u]] = 1;
-          }
+    auto group_pass = [&](std::vector<int32_t> const &u, int32_t min_a, int32_t min_b) {
+      std::vector<Run> runs;
+      for (int64_t p = 0; p < static_cast<int64_t>(u.size());) {
+        auto const &l = w.lists[u[p]];
+        int64_t q = p;
+        uint64_t h = 1469598103934665603ULL;
+        while (q < static_cast<int64_t>(u.size()) && w.lists[u[q]].shape == l.shape &&
+               w.lists[u[q]].a_base == l.a_base) {
+          h = (h ^ static_cast<uint32_t>(w.lists[u[q]].b_base)) * 1099511628211ULL;
+          ++q;
         }
-        val += n_e * plane;
-        w.n_group_entries += n_e * plane;
-        w.groups.push_back(g);
+        if (l.b_base >= 0) runs.push_back({l.shape, l.a_base, p, q, h});
+        p = q;
       }
-      p = q;
-    }
+      auto same_set = [&](Run const &x, Run const &y) {
+        if (x.shape != y.shape || x.end - x.begin != y.end - y.begin || x.hash != y.hash)
+          return false;
+        for (int64_t k = 0; k < x.end - x.begin; ++k)
+          if (w.lists[u[x.begin + k]].b_base != w.lists[u[y.begin + k]].b_base) return false;
+        return true;
+      };
+      // Runs in order of (shape, B-set hash, B-set size), ties in run order.
+      struct RunKey {
+        int32_t shape, k;
+        uint64_t hash;
+        int64_t size;
+        bool operator<(RunKey const &o) const {
+          return std::tie(shape, hash, size, k) < std::tie(o.shape, o.hash, o.size, o.k);
+        }
+      };
+      std::vector<int32_t> run_ord(runs.size());
+      {
+        std::vector<RunKey> keys(runs.size());
+        for (size_t k = 0; k < runs.size(); ++k)
+          keys[k] = {runs[k].shape, static_cast<int32_t>(k), runs[k].hash,
+                     runs[k].end - runs[k].begin};
+        std::sort(keys.begin(), keys.end());
+        for (size_t p = 0; p < keys.size(); ++p) run_ord[p] = keys[p].k;
+      }
+      for (size_t p = 0; p < run_ord.size();) {
+        size_t q = p + 1;
+        while (q < run_ord.size() && same_set(runs[run_ord[p]], runs[run_ord[q]])) ++q;
+        Run const &r0 = runs[run_ord[p]];
+        int32_t const n_a = static_cast<int32_t>(q - p);
+        int32_t const n_b = static_cast<int32_t>(r0.end - r0.begin);
+        if (n_a >= min_a && n_b >= min_b) {
+          TraceGroup g{};
+          g.shape = r0.shape;
+          g.n_a = n_a;
+          g.n_b = n_b;
+          g.a_off = static_cast<int64_t>(w.group_bases.size());
+          std::vector<int32_t> members(run_ord.begin() + p, run_ord.begin() + q);
+          std::sort(members.begin(), members.end(),
+                    [&](int32_t x, int32_t y) { return runs[x].a < runs[y].a; });
+          for (int32_t m : members) w.group_bases.push_back(runs[m].a);
+          g.b_off = static_cast<int64_t>(w.group_bases.size());
+          for (int64_t k = r0.begin; k < r0.end; ++k)
+            w.group_bases.push_back(w.lists[u[k]].b_base);
+          g.val_base = val;
+          int64_t const n_e = static_cast<int64_t>(s_.shapes[g.shape].i.size());
+          int64_t const plane = static_cast<int64_t>(n_a) * n_b;
+          for (int32_t ia = 0; ia < n_a; ++ia) {
+            Run const &r = runs[members[ia]];
+            for (int64_t k = r.begin; k < r.end; ++k) {
+              auto &l = w.lists[u[k]];
+              l.val_off = val + (k - r.begin) * n_a + ia;
+              l.stride = static_cast<int32_t>(plane);
+              in_group[u[k]] = 1;
+            }
+          }
+          val += n_e * plane;
+          w.n_group_entries += n_e * plane;
+          w.groups.push_back(g);
+        }
+        p = q;
+      }
+    };
+    group_pass(uniq, kMinGroupA, kMinGroupB);
+    // In an off-diagonal block pair every A group meets all B groups of the
+    // other block and, for the diagrams with traces at one timeslice, a few of
+    // its own timeslice: no two sets are equal.  Without those few the rest is
+    // complete (32^3x64 block pair with |p|^2 <= 2: 608 sets of 312-323 B groups
+    // that share 304; one by one their 3.8M entries took 8.0 ms, as groups
+    // 0.7 with the 5.4K lists left over).
+    std::vector<int32_t> left;
+    for (int32_t k : uniq)
+      if (!in_group[k] && w.lists[k].b_base >= 0 && !w.same_time[k]) left.push_back(k);
+    group_pass(left, kMinSplitA, kMinSplitB);
+    std::vector<uint8_t>().swap(w.same_time);
     w.n_group_values = val;
     w.unique_lists.clear();
     w.residual_lists.clear();
@@ -665,6 +678,7 @@ class Builder {
     tl.val_off = w_.n_values;
     w_.n_values += static_cast<int64_t>(s_.shapes[shape].i.size());
     w_.lists.push_back(tl);
+    w_.same_time.push_back(b && a.t == b->t ? 1 : 0);
     list_shape_.push_back(shape);
     return static_cast<int32_t>(w_.lists.size()) - 1;
   }

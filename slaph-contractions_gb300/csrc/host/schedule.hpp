@@ -104,6 +104,9 @@ struct Wave {
   std::vector<ProdInst> prods;        // ordered by dependency level
   std::vector<int64_t> prod_level_off;  // prods of level k: [off[k], off[k+1])
   std::vector<TraceList> lists;
+  // Whether both operands of a list start at the same timeslice (dropped once
+  // the lists are grouped).
+  std::vector<uint8_t> same_time;
   int64_t n_values = 0;
   // Lists that repeat the operands of an earlier list share its values.  Of
   // the distinct lists, those in groups are dense GEMMs; the rest, residual,
@@ -148,6 +151,9 @@ struct Schedule {
 // Smallest operand-group counts for a dense trace group (GEMM tiles hold 64 A
 // and 80 B groups); smaller bipartite sets stay residual.
 constexpr int32_t kMinGroupA = 16, kMinGroupB = 16;
+// The same for the groups found after the lists with both operands at one
+// timeslice are set aside (group_lists).
+constexpr int32_t kMinSplitA = 32, kMinSplitB = 32;
 
 // GEMM plan of a dense trace group of n_a x n_b operand groups.  The entries
 // (i, j) of a shape form connected components of operand indices (the
