@@ -835,7 +835,12 @@ void Engine::prepare_trace_tc(DeviceSchedule &ds) {
     DeviceSchedule::TcBatch cur{0, 0, 0, 0, 0, 0};
     size_t used = 0;
     int64_t expo = 0;
+    // A regions of the batch by their first slot and size: (region, first
+    // exponent, first item in av).  Groups of different shapes often have the
+    // same A operands (the C3c and C4cB traces of one product list): sliced once.
+    std::map<std::pair<int32_t, int32_t>, std::vector<std::array<int64_t, 3>>> seen;
     auto close = [&] {
+      seen.clear();
       // the batch's slicing items as row groups: offsets into ag / bg
       int64_t const ga = static_cast<int64_t>(ag.size()), gb = static_cast<int64_t>(bg.size());
       slice_groups(av, static_cast<size_t>(cur.a_off), av.size(), dev::kTrSliceRowsA, ag);
@@ -852,21 +857,45 @@ void Engine::prepare_trace_tc(DeviceSchedule &ds) {
       used = 0;
       expo = 0;
     };
-    for (auto const &g : w.groups) {
+    // groups with the same first A operand next to one another (in one batch)
+    std::vector<int32_t> g_ord(w.groups.size());
+    std::iota(g_ord.begin(), g_ord.end(), 0);
+    std::stable_sort(g_ord.begin(), g_ord.end(), [&](int32_t x, int32_t y) {
+      auto const &gx = w.groups[x], &gy = w.groups[y];
+      return std::make_pair(w.group_bases[gx.a_off], gx.n_a) <
+             std::make_pair(w.group_bases[gy.a_off], gy.n_a);
+    });
+    for (int32_t gi : g_ord) {
+      TraceGroup const &g = w.groups[gi];
       Planned const &pl = plans.at({g.shape, g.n_a, g.n_b});
       if (used > 0 && used + pl.bytes > cap) close();
       // Regions and first exponents of this group's blocks.
       std::vector<int64_t> a_reg, b_reg, a_exp, b_exp;
       for (auto const &x : pl.p.a) {
+        int32_t const rows = static_cast<int32_t>(x.size()) * g.n_a;
+        auto slot = [&](int32_t row) {
+          return w.group_bases[g.a_off + row % g.n_a] + x[row / g.n_a];
+        };
+        auto &same = seen[{slot(0), rows}];
+        std::array<int64_t, 3> const *hit = nullptr;
+        for (auto const &c : same) {
+          int32_t row = 0;
+          while (row < rows && av[c[2] + row].slot == slot(row)) ++row;
+          if (row == rows) hit = &c;
+        }
+        if (hit) {
+          a_reg.push_back((*hit)[0]);
+          a_exp.push_back((*hit)[1]);
+          continue;
+        }
+        same.push_back({static_cast<int64_t>(used), expo, static_cast<int64_t>(av.size())});
         a_reg.push_back(static_cast<int64_t>(used));
         a_exp.push_back(expo);
-        int32_t row = 0;
-        for (int32_t i : x)
-          for (int32_t ia = 0; ia < g.n_a; ++ia, ++row)
-            av.push_back({static_cast<int64_t>(used), w.group_bases[g.a_off + ia] + i, row,
-                          static_cast<int32_t>(expo + row), 0});
-        used += dev::trace_tc_a_bytes(row, eds);
-        expo += row;
+        for (int32_t row = 0; row < rows; ++row)
+          av.push_back({static_cast<int64_t>(used), slot(row), row,
+                        static_cast<int32_t>(expo + row), 0});
+        used += dev::trace_tc_a_bytes(rows, eds);
+        expo += rows;
       }
       for (auto const &y : pl.p.b) {
         b_reg.push_back(static_cast<int64_t>(used));
