@@ -30,6 +30,8 @@ void cuda_check(cudaError_t e, char const *what) {
 
 void DevBuf::reserve(size_t bytes) {
   if (bytes <= n_) return;
+  // work that still uses the smaller allocation may be in flight
+  if (p_) SLAPH_CK(cudaDeviceSynchronize());
   release();
   if (bytes == 0) return;
   cudaError_t const e = cudaMalloc(&p_, bytes);
@@ -78,6 +80,24 @@ constexpr size_t kTcScratchCap = 8ULL << 30;
 // every batch ends in a partly idle round of tiles, and 1 GiB of operands is
 // only two or three rounds (32^3x64 block pair with |p|^2 <= 2: 42 batches).
 constexpr size_t kTraceScratchMin = 16ULL << 30;
+// Factor intermediates up to this size stay allocated between contractions (a
+// cudaMalloc and cudaFree of each took 0.2-1.4 ms per contraction); larger ones
+// are given back once the factors are built.
+constexpr size_t kFactorWorkKept = 4ULL << 30;
+
+// Consecutive 256-byte aligned pieces of one allocation.
+class Pieces {
+ public:
+  size_t add(size_t bytes) {
+    size_t const at = size_;
+    size_ += (bytes + 255) / 256 * 256;
+    return at;
+  }
+  size_t size() const { return size_; }
+
+ private:
+  size_t size_ = 0;
+};
 
 template <typename T>
 void upload(DevBuf &b, std::vector<T> const &v, cudaStream_t s) {
@@ -173,7 +193,7 @@ Engine::~Engine() {
     if (e) cudaEventDestroy(e);
   if (ev_pn_used_) cudaEventDestroy(ev_pn_used_);
   if (up_stream_) cudaStreamDestroy(up_stream_);
-  for (auto *v : {&tc_ev_, &vdv_ev_})
+  for (auto *v : {&ev_pool_, &vdv_ev_})
     for (auto &e : *v)
       if (e) cudaEventDestroy(e);
   if (stream_) cudaStreamDestroy(stream_);
@@ -556,19 +576,18 @@ void Engine::vdaggerv_build(int precision) {
                                stream_),
          "vdaggerv_daggers");
   SLAPH_CK(cudaEventRecord(ev_[1], stream_));
-  SLAPH_CK(cudaEventSynchronize(ev_[1]));
+  // one wait for the build, its error flag behind it
+  int const code = precision == SLAPH_MIXED ? read_err_flag() : 0;
+  if (precision != SLAPH_MIXED) SLAPH_CK(cudaEventSynchronize(ev_[1]));
   timings[0] = elapsed_ms(ev_[0], ev_[1]);
   timings[5] = static_cast<double>(launches_);
   double t_gemm = 0;
   for (int32_t k = 0; k < n_gemm; ++k) t_gemm += elapsed_ms(vdv_ev_[2 * k], vdv_ev_[2 * k + 1]);
   timings[11] = t_gemm;
   timings[12] = static_cast<double>(n_gemm);
-  if (precision == SLAPH_MIXED) {
-    int const code = read_err_flag();
-    if (code != 0)
-      throw TimeoutError("split-precision VdaggerV: a bounded device wait gave up (stage " +
-                         std::to_string(code) + ")");
-  }
+  if (code != 0)
+    throw TimeoutError("split-precision VdaggerV: a bounded device wait gave up (stage " +
+                       std::to_string(code) + ")");
   vdv_built_ = true;
 }
 
@@ -1495,6 +1514,27 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
   running_.reserve(sizeof(double2) * n_run);
   SLAPH_CK(cudaMemsetAsync(running_.as<void>(), 0, sizeof(double2) * n_run, stream_));
   double t_f = 0, t_pt = 0, t_as = 0, t_tr = 0, t_sl = 0, t_gm = 0, t_pr = 0;
+  // Timing marks on the stream, read after the one wait at the end: the host
+  // runs ahead of the device through all stages and waves.
+  size_t marks = 0;
+  auto mark = [&] {
+    if (marks == ev_pool_.size()) {
+      cudaEvent_t e = nullptr;
+      SLAPH_CK(cudaEventCreate(&e));
+      ev_pool_.push_back(e);
+    }
+    SLAPH_CK(cudaEventRecord(ev_pool_[marks], stream_));
+    return ev_pool_[marks++];
+  };
+  struct Span {
+    cudaEvent_t from, to;
+    double *sum;
+  };
+  std::vector<Span> spans;
+  if (mixed) {
+    err_.reserve(sizeof(int));
+    SLAPH_CK(cudaMemsetAsync(err_.as<void>(), 0, sizeof(int), stream_));
+  }
   int64_t n_pr = 0;
   int64_t n_tr = 0, n_gm = 0;
   double st[8] = {};
@@ -1506,47 +1546,49 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
     int64_t const nev = dims_.nev;
 
     // ---- factors
-    SLAPH_CK(cudaEventRecord(ev_[0], stream_));
+    cudaEvent_t const f_begin = mark();
+    Pieces pc;
     if (!mixed) {
       slots_.reserve(sizeof(double2) * ms *
                      std::max<int64_t>(1, s.n_factor_slots + s.max_prod_slots));
-      DevBuf q0m, q1r, q2m;
-      q0m.reserve(sizeof(double2) * std::max<int64_t>(1, s.q0m.size()) * nev * eds);
-      q1r.reserve(sizeof(double2) * std::max<int64_t>(1, s.q1r.size()) * nev * eds);
-      q2m.reserve(sizeof(double2) * std::max<int64_t>(1, s.q2m.size()) * eds * 4 * nev);
+      size_t const o_q0m = pc.add(sizeof(double2) * s.q0m.size() * nev * eds);
+      size_t const o_q1r = pc.add(sizeof(double2) * s.q1r.size() * nev * eds);
+      size_t const o_q2m = pc.add(sizeof(double2) * s.q2m.size() * eds * 4 * nev);
+      f_work_.reserve(std::max<size_t>(1, pc.size()));
+      auto *q0m = reinterpret_cast<double2 *>(f_work_.as<char>() + o_q0m);
+      auto *q1r = reinterpret_cast<double2 *>(f_work_.as<char>() + o_q1r);
+      auto *q2m = reinterpret_cast<double2 *>(f_work_.as<char>() + o_q2m);
       double2 const *vdv = vdv_.as<double2>();
-      launch(dev::q0m(q0m.as<double2>(), ds.q0m.as<dev::Q0MInst>(), s.q0m.size(), vdv,
+      launch(dev::q0m(q0m, ds.q0m.as<dev::Q0MInst>(), s.q0m.size(), vdv,
                       noise_.as<double2>(), geo_, stream_),
              "q0m");
-      launch(dev::q1r(q1r.as<double2>(), ds.q1r.as<dev::Q1RInst>(), s.q1r.size(), vdv,
+      launch(dev::q1r(q1r, ds.q1r.as<dev::Q1RInst>(), s.q1r.size(), vdv,
                       noise_.as<double2>(), geo_, stream_),
              "q1r");
-      launch(dev::q2m(q2m.as<double2>(), ds.q2m.as<dev::Q2MInst>(), s.q2m.size(), vdv,
+      launch(dev::q2m(q2m, ds.q2m.as<dev::Q2MInst>(), s.q2m.size(), vdv,
                       peram_.as<double2>(), geo_, stream_),
              "q2m");
       launch(dev::q0(slots_.as<double2>(), ds.q0.as<dev::Q0Inst>(), s.q0.size(),
-                     q0m.as<double2>(), noise_.as<double2>(), geo_, stream_),
+                     q0m, noise_.as<double2>(), geo_, stream_),
              "q0");
       plan_shared_q1(ds, s, stream_);
       if (ds.x1_batches.empty())
         launch(dev::q1(slots_.as<double2>(), ds.q1.as<dev::Q1Inst>(), s.q1.size(),
-                       q1r.as<double2>(), peram_.as<double2>(), geo_, stream_),
+                       q1r, peram_.as<double2>(), geo_, stream_),
                "q1");
       // (f_out_, scratch of the split-precision factors, holds the products)
       f_out_.reserve(sizeof(double2) * static_cast<size_t>(ds.x1_max) * 4 * ms);
       for (auto const &b : ds.x1_batches) {
         launch(dev::q1_shared(slots_.as<double2>(), f_out_.as<double2>(),
                               ds.x1.as<dev::X1Inst>() + b.x_off, b.n_x,
-                              ds.q1_picks.as<dev::Q1Pick>() + b.p_off, b.n_p, q1r.as<double2>(),
+                              ds.q1_picks.as<dev::Q1Pick>() + b.p_off, b.n_p, q1r,
                               peram_.as<double2>(), geo_, stream_),
                "q1_shared");
         ++launches_;
       }
       launch(dev::q2(slots_.as<double2>(), ds.q2.as<dev::Q2Inst>(), s.q2.size(),
-                     q2m.as<double2>(), peram_.as<double2>(), geo_, stream_),
+                     q2m, peram_.as<double2>(), geo_, stream_),
              "q2");
-      SLAPH_CK(cudaEventRecord(ev_[1], stream_));
-      SLAPH_CK(cudaEventSynchronize(ev_[1]));  // intermediates are freed here
     } else {
       // Double-float matrices in both layouts: factors now, products per wave.
       size_t const df_bytes =
@@ -1561,20 +1603,24 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
                                stream_));
       int64_t const n_vdv = 2LL * static_cast<int64_t>(ops_.size()) * dims_.Lt * nev * nev;
       int64_t const n_noise = 4LL * nev * dims_.Lt * dims_.n_rnd;
-      DevBuf vdv_df, noise_df, q0m, q1r;
-      vdv_df.reserve(sizeof(float4) * std::max<int64_t>(1, n_vdv));
-      noise_df.reserve(sizeof(float4) * n_noise);
-      launch(dev::to_df(vdv_df.as<float4>(), vdv_.as<double2>(), n_vdv, stream_), "to_df");
-      launch(dev::to_df(noise_df.as<float4>(), noise_.as<double2>(), n_noise, stream_), "to_df");
-      q0m.reserve(sizeof(float4) * std::max<int64_t>(1, s.q0m.size()) * nev * eds);
-      q1r.reserve(sizeof(float4) * std::max<int64_t>(1, s.q1r.size()) * nev * eds);
+      size_t const o_vdv = pc.add(sizeof(float4) * n_vdv);
+      size_t const o_noise = pc.add(sizeof(float4) * n_noise);
+      size_t const o_q0m = pc.add(sizeof(float4) * s.q0m.size() * nev * eds);
+      size_t const o_q1r = pc.add(sizeof(float4) * s.q1r.size() * nev * eds);
+      f_work_.reserve(std::max<size_t>(1, pc.size()));
+      auto *vdv_df = reinterpret_cast<float4 *>(f_work_.as<char>() + o_vdv);
+      auto *noise_df = reinterpret_cast<float4 *>(f_work_.as<char>() + o_noise);
+      auto *q0m = reinterpret_cast<float4 *>(f_work_.as<char>() + o_q0m);
+      auto *q1r = reinterpret_cast<float4 *>(f_work_.as<char>() + o_q1r);
+      launch(dev::to_df(vdv_df, vdv_.as<double2>(), n_vdv, stream_), "to_df");
+      launch(dev::to_df(noise_df, noise_.as<double2>(), n_noise, stream_), "to_df");
       // Q0 and the Q1R intermediates in double-float; Q2M, Q1 and Q2 on the
       // tensor cores below.
-      launch(dev::factors_df(df_slots_.as<float4>(), df_slots_t_.as<float4>(), q0m.as<float4>(),
-                             q1r.as<float4>(), nullptr, ds.q0m.as<dev::Q0MInst>(),
+      launch(dev::factors_df(df_slots_.as<float4>(), df_slots_t_.as<float4>(), q0m,
+                             q1r, nullptr, ds.q0m.as<dev::Q0MInst>(),
                              s.q0m.size(), ds.q1r.as<dev::Q1RInst>(), s.q1r.size(), nullptr, 0,
                              ds.q0.as<dev::Q0Inst>(), s.q0.size(), nullptr, 0, nullptr, 0,
-                             vdv_df.as<float4>(), noise_df.as<float4>(), nullptr,
+                             vdv_df, noise_df, nullptr,
                              slot_bits_.as<unsigned int>(), geo_, stream_),
              "factors_df");
       launches_ += 2;
@@ -1582,8 +1628,6 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
       tc_scratch_.reserve(std::max<size_t>(1, ds.f_scratch));
       f_out_.reserve(sizeof(float4) * std::max<int64_t>(1, ds.f_out));
       tr_expo_.reserve(sizeof(int32_t) * std::max<int64_t>(1, ds.f_expo));
-      err_.reserve(sizeof(int));
-      SLAPH_CK(cudaMemsetAsync(err_.as<void>(), 0, sizeof(int), stream_));
       int32_t const kt1 = dev::gemm_k_tiles(nev), kt2 = dev::gemm_k_tiles(4 * nev);
       uint8_t *scr = tc_scratch_.as<uint8_t>();
       int32_t *ex = tr_expo_.as<int32_t>();
@@ -1594,7 +1638,7 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
       auto count = [&](int64_t n) { launches_ += n > 0 ? 1 : 0; };
       for (auto const &b : ds.f_batches) {
         cuda_check(dev::gvec_slice_df(scr, ex, fv + b.a_x1[0], b.a_x1[1], fi, true, true,
-                                      q1r.as<float4>(), kt1, stream_),
+                                      q1r, kt1, stream_),
                    "slice X1 A");
         cuda_check(dev::gvec_slice_f64(scr, ex, fv + b.a_q2m[0], b.a_q2m[1], fi, true, false,
                                        peram_.as<double2>(), kt1, stream_),
@@ -1630,10 +1674,12 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
                    "q2_gather");
         count(b.g1[1]); count(b.g2[1]);
       }
-      SLAPH_CK(cudaEventRecord(ev_[1], stream_));
-      SLAPH_CK(cudaEventSynchronize(ev_[1]));  // intermediates are freed here
     }
-    t_f += elapsed_ms(ev_[0], ev_[1]);
+    spans.push_back({f_begin, mark(), &t_f});
+    if (f_work_.size() > kFactorWorkKept) {
+      SLAPH_CK(cudaStreamSynchronize(stream_));
+      f_work_.release();
+    }
 
     // ---- waves: products, traces, terms, accumulation
     values_.reserve(sizeof(double2) * std::max<int64_t>(1, s.max_values));
@@ -1644,13 +1690,11 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
       if (p_tc) prepare_product_tc(ds);
       tc_scratch_.reserve(std::max<size_t>(1, std::max(ds.tc_scratch, ds.p_scratch)));
       tr_expo_.reserve(sizeof(int32_t) * std::max<int64_t>(1, std::max(ds.tc_expo, ds.p_expo)));
-      err_.reserve(sizeof(int));
-      SLAPH_CK(cudaMemsetAsync(err_.as<void>(), 0, sizeof(int), stream_));
     }
     for (size_t wi = 0; wi < s.waves.size(); ++wi) {
       Wave const &w = s.waves[wi];
       auto &wb = *ds.waves[wi];
-      SLAPH_CK(cudaEventRecord(ev_[2], stream_));
+      cudaEvent_t const w_begin = mark();
       auto const *prods = wb.prods.as<dev::ProdInst>();
       // the tensor-core products take the largest entries of their slots by
       // atomicMax from zero
@@ -1686,7 +1730,7 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
                "slot_maxbits");
       int64_t const n_res = static_cast<int64_t>(w.residual_lists.size());
       int64_t const n_uni = static_cast<int64_t>(w.unique_lists.size());
-      SLAPH_CK(cudaEventRecord(ev_[5], stream_));
+      cudaEvent_t const w_prod = mark();
       if (mixed) {
         values_df_.reserve(sizeof(float4) * std::max<int64_t>(1, s.max_values));
         if (n_res > 0)
@@ -1695,21 +1739,16 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
                                 ds.shape_j.as<int32_t>(), ds.shape_off.as<int64_t>(),
                                 df_slots_.as<float4>(), df_slots_t_.as<float4>(), eds, stream_),
                  "traces_df");
-        SLAPH_CK(cudaEventRecord(ev_[6], stream_));
+        if (n_res > 0) spans.push_back({w_prod, mark(), &t_tr});
         int64_t const gv = w.n_group_values;
         if (w.n_values > gv)
           launch(dev::df_values_to_fp64(values_.as<double2>() + gv, values_df_.as<float4>() + gv,
                                         w.n_values - gv, stream_),
                  "df_values_to_fp64");
         // Dense groups on the tensor cores: slice, then GEMM, per batch.
-        while (tc_ev_.size() < 3 * wb.tc_batches.size()) {
-          cudaEvent_t e = nullptr;
-          SLAPH_CK(cudaEventCreate(&e));
-          tc_ev_.push_back(e);
-        }
         for (size_t bi = 0; bi < wb.tc_batches.size(); ++bi) {
           auto const &b = wb.tc_batches[bi];
-          SLAPH_CK(cudaEventRecord(tc_ev_[3 * bi], stream_));
+          cudaEvent_t const b_begin = mark();
           cuda_check(dev::trace_tc_slice(tc_scratch_.as<uint8_t>(), tr_expo_.as<int32_t>(),
                                          wb.tc_a.as<dev::TrSliceGroup>() + b.a_off, b.n_a,
                                          wb.tc_b.as<dev::TrSliceGroup>() + b.b_off, b.n_b,
@@ -1717,13 +1756,15 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
                                          slot_bits_.as<unsigned int>(), eds, stream_),
                      "trace_tc_slice");
           launches_ += (b.n_a > 0 ? 1 : 0) + (b.n_b > 0 ? 1 : 0);
-          SLAPH_CK(cudaEventRecord(tc_ev_[3 * bi + 1], stream_));
+          cudaEvent_t const b_sliced = mark();
+          spans.push_back({b_begin, b_sliced, &t_sl});
           launch(dev::trace_tc_gemm(values_.as<double2>(), tc_scratch_.as<uint8_t>(),
                                     tr_expo_.as<int32_t>(), wb.tc_tiles.as<dev::TrTile>() + b.tile_off,
                                     b.n_tiles, ds.tc_entries.as<int32_t>(), eds, err_.as<int>(),
                                     stream_),
                  "trace_tc_gemm");
-          SLAPH_CK(cudaEventRecord(tc_ev_[3 * bi + 2], stream_));
+          spans.push_back({b_sliced, mark(), &t_gm});
+          ++n_gm;
         }
       } else {
         if (n_uni > 0)
@@ -1732,10 +1773,10 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
                              ds.shape_j.as<int32_t>(), ds.shape_off.as<int64_t>(),
                              slots_.as<double2>(), eds, stream_),
                  "traces");
-        SLAPH_CK(cudaEventRecord(ev_[6], stream_));
+        if (n_uni > 0) spans.push_back({w_prod, mark(), &t_tr});
       }
       bool const traced = mixed ? n_res > 0 : n_uni > 0;
-      SLAPH_CK(cudaEventRecord(ev_[3], stream_));
+      cudaEvent_t const w_traced = mark();
       launch(dev::terms(term_val_.as<double2>(), wb.terms.as<dev::Term>(),
                         static_cast<int64_t>(w.terms.size()), wb.lists.as<dev::TraceList>(),
                         values_.as<double2>(), ds.shape_mask.as<uint16_t>(),
@@ -1746,28 +1787,11 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
                              wb.seg_off.as<int64_t>(), wb.n_seg, wb.idx.as<int32_t>(),
                              term_val_.as<double2>(), stream_),
              "accumulate");
-      SLAPH_CK(cudaEventRecord(ev_[4], stream_));
-      SLAPH_CK(cudaEventSynchronize(ev_[4]));
-      t_pt += elapsed_ms(ev_[2], ev_[3]);
-      t_as += elapsed_ms(ev_[3], ev_[4]);
-      t_pr += elapsed_ms(ev_[2], ev_[5]);
+      spans.push_back({w_begin, w_traced, &t_pt});
+      spans.push_back({w_traced, mark(), &t_as});
+      spans.push_back({w_begin, w_prod, &t_pr});
       n_pr += static_cast<int64_t>(w.prod_level_off.size() > 0 ? w.prod_level_off.size() - 1 : 0);
-      if (traced) {
-        t_tr += elapsed_ms(ev_[5], ev_[6]);
-        ++n_tr;
-      }
-      if (mixed)
-        for (size_t bi = 0; bi < wb.tc_batches.size(); ++bi) {
-          t_sl += elapsed_ms(tc_ev_[3 * bi], tc_ev_[3 * bi + 1]);
-          t_gm += elapsed_ms(tc_ev_[3 * bi + 1], tc_ev_[3 * bi + 2]);
-          ++n_gm;
-        }
-    }
-    if (mixed) {
-      int const code = read_err_flag();
-      if (code != 0)
-        throw TimeoutError("tensor-core factors or traces: a bounded device wait gave up "
-                           "(stage " + std::to_string(code) + ")");
+      if (traced) ++n_tr;
     }
     st[6] += static_cast<double>(s.n_unique_entries);
     st[7] += static_cast<double>(s.n_group_entries);
@@ -1780,6 +1804,24 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
   }
   // Perambulators and noise are not read after the factor stages.
   SLAPH_CK(cudaEventRecord(ev_pn_used_, stream_));
+  // ---- output: C[t] = correlator[t][i] / Lt (src/Diagram.cpp:141-143), with the
+  // error flag behind it
+  size_t const n_host = static_cast<size_t>(n_outputs * dims_.Lt);
+  host_rb_.reserve((n_host + 1) * sizeof(double2));
+  double2 *host = host_rb_.as<double2>();
+  int *const flag = reinterpret_cast<int *>(host + n_host);
+  *flag = 0;
+  if (n_host > 0) {
+    launch(dev::divide(running_.as<double2>(), static_cast<int64_t>(n_host),
+                       static_cast<double>(dims_.Lt), stream_),
+           "divide");
+    SLAPH_CK(cudaMemcpyAsync(host, running_.as<double2>(), n_host * sizeof(double2),
+                             cudaMemcpyDeviceToHost, stream_));
+  }
+  if (mixed)
+    SLAPH_CK(cudaMemcpyAsync(flag, err_.as<void>(), sizeof(int), cudaMemcpyDeviceToHost, stream_));
+  SLAPH_CK(cudaStreamSynchronize(stream_));
+  for (auto const &sp : spans) *sp.sum += elapsed_ms(sp.from, sp.to);
   timings[1] = t_f;
   timings[2] = t_pt;
   timings[3] = t_as;
@@ -1792,20 +1834,10 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
   timings[10] = t_sl;
   timings[14] = t_pr;
   timings[15] = static_cast<double>(n_pr);
-
-  // ---- output: C[t] = correlator[t][i] / Lt (src/Diagram.cpp:141-143)
-  size_t const n_host = static_cast<size_t>(n_outputs * dims_.Lt);
-  host_rb_.reserve(std::max<size_t>(1, n_host) * sizeof(double2));
-  double2 const *host = host_rb_.as<double2>();
-  if (n_host > 0)
-    SLAPH_CK(cudaMemcpyAsync(host_rb_.as<double2>(), running_.as<double2>(),
-                             n_host * sizeof(double2), cudaMemcpyDeviceToHost, stream_));
-  SLAPH_CK(cudaStreamSynchronize(stream_));
-  double const inv = static_cast<double>(dims_.Lt);
-  for (size_t i = 0; i < n_host; ++i) {
-    corr_out[2 * i] = host[i].x / inv;
-    corr_out[2 * i + 1] = host[i].y / inv;
-  }
+  if (*flag != 0)
+    throw TimeoutError("tensor-core factors or traces: a bounded device wait gave up (stage " +
+                       std::to_string(*flag) + ")");
+  if (n_host > 0) std::memcpy(corr_out, host, n_host * sizeof(double2));
   for (int k = 0; k < 8; ++k) stats[k] = st[k];
 }
 

@@ -168,7 +168,7 @@ class Engine {
   std::vector<cudaEvent_t> ev_v_, ev_p_, ev_n_;
   std::vector<char> pend_v_, pend_p_, pend_n_;
   cudaEvent_t ev_v_used_ = nullptr, ev_pn_used_ = nullptr;
-  std::vector<cudaEvent_t> tc_ev_;  // three per tensor-core trace batch
+  std::vector<cudaEvent_t> ev_pool_;  // timing events of a contraction
   std::vector<cudaEvent_t> vdv_ev_;  // two per split-precision VdaggerV GEMM launch
 
   DevBuf V_, peram_, noise_, vdv_, tc_scratch_, err_;
@@ -198,7 +198,7 @@ class Engine {
 
   // Working buffers of the contraction.
   DevBuf slots_, df_slots_, df_slots_t_, values_, values_df_, term_val_, running_, tr_expo_,
-      f_out_;
+      f_out_, f_work_;
 
   std::unique_ptr<DeviceSchedule> sched_;
   slaph_plan const *sched_plan_ = nullptr;

@@ -409,6 +409,8 @@ cudaError_t terms(double2 *term_val, Term const *t, int64_t n, TraceList const *
 cudaError_t accumulate(double2 *running, int32_t const *seg_out, int64_t const *seg_off,
                        int64_t n_seg, int32_t const *idx, double2 const *term_val,
                        cudaStream_t stream);
+// x[k] /= d for k < n (both components).
+cudaError_t divide(double2 *x, int64_t n, double d, cudaStream_t stream);
 
 }  // namespace dev
 }  // namespace slaph

@@ -520,6 +520,11 @@ __global__ void accumulate_kernel(double2 *running, int32_t const *seg_out,
   running[seg_out[s]] = acc;
 }
 
+__global__ void divide_kernel(double2 *x, int64_t n, double d) {
+  int64_t const k = gidx();
+  if (k < n) x[k] = make_double2(x[k].x / d, x[k].y / d);
+}
+
 int blocks_for(int64_t n, int threads) {
   return static_cast<int>((n + threads - 1) / threads);
 }
@@ -845,6 +850,12 @@ cudaError_t terms(double2 *term_val, Term const *t, int64_t n, TraceList const *
   if (n == 0) return cudaSuccess;
   term_kernel<<<blocks_for(n, 128), 128, 0, stream>>>(term_val, t, n, lists, values,
                                                       shape_mask, shape_off, kahan);
+  return cudaGetLastError();
+}
+
+cudaError_t divide(double2 *x, int64_t n, double d, cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  divide_kernel<<<blocks_for(n, 256), 256, 0, stream>>>(x, n, d);
   return cudaGetLastError();
 }
 
