@@ -1044,7 +1044,7 @@ void Engine::prepare_product_tc(DeviceSchedule &ds) {
 }
 
 // Tensor-core plan of the Q1/Q2 factors (factor_tc.cu).  Per timeslice t:
-//   X1[t]  rows (Q1R r at t, a), columns (r2, b, d, c), K = v:
+//   X1[t]  rows (Q1R r at t, a), columns (r2, b, d, c) of the (r2, b) in use, K = v:
 //          A = conj(Q1R_r(a, v)), B = P_r2((4t+d) nev + v, b eds + c)
 //   Q2M[t] rows (pair (b1, r1), a, bd), columns (VdaggerV code, v), K = w:
 //          A = P_r1((4t+bd) nev + w, b1 eds + a) (conjugated by the GEMM form),
@@ -1061,7 +1061,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
   std::vector<uint8_t> const need =
       factor_layouts(s, dev::prod_tc_supported(s.eds));
   int32_t const eds = s.eds, nev = dims_.nev, dilE = dims_.dilE, nb = geo_.nb;
-  int32_t const n_rnd = dims_.n_rnd, Lt = dims_.Lt;
+  int32_t const Lt = dims_.Lt;
   int64_t const prow = 4LL * nev * Lt;            // perambulator rows
   int64_t const prs = prow * nb * eds;            // perambulator elements per random vector
   int64_t const blk = static_cast<int64_t>(nev) * nev;
@@ -1077,6 +1077,16 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
   for (size_t i = 0; i < s.q2m.size(); ++i) q2m_t[s.q2m[i].t].push_back(static_cast<int32_t>(i));
   for (size_t i = 0; i < s.q1.size(); ++i) q1_t[s.q1[i].t].push_back(static_cast<int32_t>(i));
   for (size_t i = 0; i < s.q2.size(); ++i) q2_t[s.q2[i].t].push_back(static_cast<int32_t>(i));
+  // (r2, b) of the perambulator columns that the Q1 factors of a timeslice use:
+  // the columns of X1 (all of them for a whole configuration, one or two of the
+  // blocks b for a single block pair).
+  std::vector<std::vector<std::pair<int32_t, int32_t>>> x1_cb(Lt);
+  for (auto const &q : s.q1) x1_cb[q.t].push_back({q.r2, q.b});
+  for (auto &v : x1_cb) {
+    std::sort(v.begin(), v.end());
+    v.erase(std::unique(v.begin(), v.end()), v.end());
+  }
+  auto x1_columns = [&](int t) { return static_cast<int32_t>(x1_cb[t].size()) * 4 * eds; };
 
   std::vector<dev::GVec> vec;
   std::vector<dev::GVecGroup> vgroups;
@@ -1130,7 +1140,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
                      std::vector<std::vector<std::array<int32_t, 3>>> &bic_cols) {
     TPlan p;
     int32_t const nr = static_cast<int32_t>(q1r_t[t].size());
-    int32_t const x1_rows = nr * eds, x1_cols = n_rnd * nb * 4 * eds;
+    int32_t const x1_rows = nr * eds, x1_cols = x1_columns(t);
     std::map<std::pair<int32_t, int32_t>, int32_t> pairs;
     std::map<int32_t, int32_t> codes;
     for (int32_t m : q2m_t[t]) {
@@ -1140,7 +1150,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
     int32_t const q2m_rows = static_cast<int32_t>(pairs.size()) * eds * 4;
     int32_t const q2m_cols = static_cast<int32_t>(codes.size()) * nev;
     if (nr > 0)
-      p.s1 += dev::tc_a_bytes(x1_rows, kt1) + dev::tc_b_bytes(x1_cols, kt1);
+      p.s1 += dev::tc_a_bytes(x1_rows, kt1) + dev::tc_b_bytes(std::max(x1_cols, 1), kt1);
     if (!q2m_t[t].empty())
       p.s1 += dev::tc_a_bytes(q2m_rows, kt1) + dev::tc_b_bytes(q2m_cols, kt1);
     p.out += static_cast<int64_t>(x1_rows) * x1_cols + static_cast<int64_t>(q2m_rows) * q2m_cols;
@@ -1225,7 +1235,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
       o.x1_rows = static_cast<int32_t>(o.rloc.size()) * eds;
       o.q2m_rows = static_cast<int32_t>(o.pairs.size()) * eds * 4;
       o.x1 = out;
-      out += static_cast<int64_t>(o.x1_rows) * n_rnd * nb * 4 * eds;
+      out += static_cast<int64_t>(o.x1_rows) * x1_columns(t);
       o.q2m = out;
       out += static_cast<int64_t>(o.q2m_rows) * static_cast<int64_t>(o.codes.size()) * nev;
     }
@@ -1265,16 +1275,16 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
       int const t = batch_ts[k];
       regB_x1[k] = static_cast<int64_t>(off1);
       eB_x1[k] = expo;
-      int32_t const cols = n_rnd * nb * 4 * eds;
       if (tos[k].x1_rows > 0) {
-        for (int32_t r2 = 0; r2 < n_rnd; ++r2)
-          for (int32_t b2 = 0; b2 < nb; ++b2)
-            for (int32_t d = 0; d < 4; ++d)
-              for (int32_t c = 0; c < eds; ++c)
-                add_vec(regB_x1[k], ((r2 * nb + b2) * 4 + d) * eds + c, expo++, 1, nev,
-                        {{r2 * prs + (4LL * t + d) * nev + prow * (static_cast<int64_t>(b2) * eds + c),
-                          0, 0}});
-        off1 += dev::tc_b_bytes(cols, kt1);
+        int32_t col = 0;
+        for (auto const &cb : x1_cb[t])
+          for (int32_t d = 0; d < 4; ++d)
+            for (int32_t c = 0; c < eds; ++c)
+              add_vec(regB_x1[k], col++, expo++, 1, nev,
+                      {{cb.first * prs + (4LL * t + d) * nev +
+                            prow * (static_cast<int64_t>(cb.second) * eds + c),
+                        0, 0}});
+        off1 += dev::tc_b_bytes(std::max(col, 1), kt1);
       }
     }
     end(b.b_x1);
@@ -1297,7 +1307,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
     for (size_t k = 0; k < batch_ts.size(); ++k) {
       TOut &o = tos[k];
       if (o.x1_rows > 0)
-        add_tiles(regA_x1[k], regB_x1[k], a_tile1, b_tile1, o.x1_rows, n_rnd * nb * 4 * eds, o.x1,
+        add_tiles(regA_x1[k], regB_x1[k], a_tile1, b_tile1, o.x1_rows, x1_columns(batch_ts[k]), o.x1,
                   eA_x1[k], eB_x1[k]);
       if (o.q2m_rows > 0)
         add_tiles(regA_q2m[k], regB_q2m[k], a_tile1, b_tile1, o.q2m_rows,
@@ -1396,7 +1406,11 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
         g.x_off = o.x1;
         g.ld = o.x1_rows;
         g.row0 = o.rloc.at(q.r) * eds;
-        g.col0 = (q.r2 * nb + q.b) * 4 * eds;
+        auto const &cb = x1_cb[q.t];
+        g.col0 = static_cast<int32_t>(
+                     std::lower_bound(cb.begin(), cb.end(), std::make_pair(q.r2, q.b)) -
+                     cb.begin()) *
+                 4 * eds;
         g.gamma = q.gamma;
         g.slot = q.slot;
         g.need = need[q.slot];
@@ -1616,11 +1630,9 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
       launch(dev::to_df(noise_df, noise_.as<double2>(), n_noise, stream_), "to_df");
       // Q0 and the Q1R intermediates in double-float; Q2M, Q1 and Q2 on the
       // tensor cores below.
-      launch(dev::factors_df(df_slots_.as<float4>(), df_slots_t_.as<float4>(), q0m,
-                             q1r, nullptr, ds.q0m.as<dev::Q0MInst>(),
-                             s.q0m.size(), ds.q1r.as<dev::Q1RInst>(), s.q1r.size(), nullptr, 0,
-                             ds.q0.as<dev::Q0Inst>(), s.q0.size(), nullptr, 0, nullptr, 0,
-                             vdv_df, noise_df, nullptr,
+      launch(dev::factors_df(df_slots_.as<float4>(), df_slots_t_.as<float4>(), q0m, q1r,
+                             ds.q0m.as<dev::Q0MInst>(), s.q0m.size(), ds.q1r.as<dev::Q1RInst>(),
+                             s.q1r.size(), ds.q0.as<dev::Q0Inst>(), s.q0.size(), vdv_df, noise_df,
                              slot_bits_.as<unsigned int>(), geo_, stream_),
              "factors_df");
       launches_ += 2;
@@ -1732,19 +1744,13 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
       int64_t const n_uni = static_cast<int64_t>(w.unique_lists.size());
       cudaEvent_t const w_prod = mark();
       if (mixed) {
-        values_df_.reserve(sizeof(float4) * std::max<int64_t>(1, s.max_values));
         if (n_res > 0)
-          launch(dev::traces_df(values_df_.as<float4>(), wb.lists.as<dev::TraceList>(),
+          launch(dev::traces_df(values_.as<double2>(), wb.lists.as<dev::TraceList>(),
                                 wb.residual.as<int32_t>(), n_res, ds.shape_i.as<int32_t>(),
                                 ds.shape_j.as<int32_t>(), ds.shape_off.as<int64_t>(),
                                 df_slots_.as<float4>(), df_slots_t_.as<float4>(), eds, stream_),
                  "traces_df");
         if (n_res > 0) spans.push_back({w_prod, mark(), &t_tr});
-        int64_t const gv = w.n_group_values;
-        if (w.n_values > gv)
-          launch(dev::df_values_to_fp64(values_.as<double2>() + gv, values_df_.as<float4>() + gv,
-                                        w.n_values - gv, stream_),
-                 "df_values_to_fp64");
         // Dense groups on the tensor cores: slice, then GEMM, per batch.
         for (size_t bi = 0; bi < wb.tc_batches.size(); ++bi) {
           auto const &b = wb.tc_batches[bi];

@@ -197,7 +197,7 @@ class Engine {
   int64_t launches_ = 0;
 
   // Working buffers of the contraction.
-  DevBuf slots_, df_slots_, df_slots_t_, values_, values_df_, term_val_, running_, tr_expo_,
+  DevBuf slots_, df_slots_, df_slots_t_, values_, term_val_, running_, tr_expo_,
       f_out_, f_work_;
 
   std::unique_ptr<DeviceSchedule> sched_;

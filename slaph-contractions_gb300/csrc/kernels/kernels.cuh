@@ -206,24 +206,18 @@ cudaError_t traces(double2 *values, TraceList const *lists, int32_t const *which
                    int64_t const *shape_off, double2 const *slots, int32_t eds,
                    cudaStream_t stream);
 
-// Mixed path: matrices in double-float form (float4 = re hi, re lo, im hi,
-// im lo per complex), written as stored (dst_n) and transposed (dst_t); traces
-// as compensated FP32 dot products over unit-stride operands.
-cudaError_t split_df(float4 *dst_n, float4 *dst_t, double2 const *src, int64_t n, int32_t eds,
-                     cudaStream_t stream);
+// Mixed path: matrices in double-float form (float4 = re hi, re lo, im hi, im lo
+// per complex), as stored and transposed; traces as compensated FP32 dot products
+// over unit-stride operands.
 // Mixed path: FP64 -> double-float (float4) copy.
 cudaError_t to_df(float4 *dst, double2 const *src, int64_t n, cudaStream_t stream);
-// Mixed path: all factor intermediates and factors in double-float; factors
-// written into the slot buffers in both layouts (sn stored, st transposed), Q0
-// factors with the largest |re|, |im| of their slots (slot_maxbits), added to
-// slot_bits.
+// Mixed path: the Q0M and Q1R intermediates and the Q0 factors in double-float;
+// Q0 written into the slot buffers in both layouts (sn stored, st transposed),
+// the largest |re|, |im| of their slots (slot_maxbits) added to slot_bits.
 cudaError_t factors_df(float4 *sn, float4 *st, float4 *q0m_buf, float4 *q1r_buf,
-                       float4 *q2m_buf, Q0MInst const *q0m_i, int64_t n_q0m,
-                       Q1RInst const *q1r_i, int64_t n_q1r, Q2MInst const *q2m_i, int64_t n_q2m,
-                       Q0Inst const *q0_i, int64_t n_q0, Q1Inst const *q1_i, int64_t n_q1,
-                       Q2Inst const *q2_i, int64_t n_q2, float4 const *vdv,
-                       float4 const *noise, float4 const *peram, unsigned int *slot_bits,
-                       Geometry g, cudaStream_t stream);
+                       Q0MInst const *q0m_i, int64_t n_q0m, Q1RInst const *q1r_i, int64_t n_q1r,
+                       Q0Inst const *q0_i, int64_t n_q0, float4 const *vdv, float4 const *noise,
+                       unsigned int *slot_bits, Geometry g, cudaStream_t stream);
 // slots[c] = slots[a] * slots[b] in double-float, both layouts written.
 cudaError_t products_df(float4 *slots_n, float4 *slots_t, ProdInst const *p, int64_t n,
                         int32_t eds, cudaStream_t stream);
@@ -264,9 +258,8 @@ cudaError_t products_tc(float4 *slots_n, float4 *slots_t, uint8_t *scratch, int6
                         int32_t const *r_slots, int64_t n_r, int32_t const *u_list,
                         int32_t const *out_tab, ProdTile const *tiles, int64_t n_tiles,
                         int32_t eds, unsigned int *slot_bits, int *err, cudaStream_t stream);
-// Trace values as double-float pairs (re_hi, re_lo, im_hi, im_lo) into
-// values_df, laid out as for traces().
-cudaError_t traces_df(float4 *values_df, TraceList const *lists, int32_t const *which,
+// Trace values (FP64 sums of the double-float results), laid out as for traces().
+cudaError_t traces_df(double2 *values, TraceList const *lists, int32_t const *which,
                       int64_t n_which, int32_t const *shape_i, int32_t const *shape_j,
                       int64_t const *shape_off, float4 const *slots_n, float4 const *slots_t,
                       int32_t eds, cudaStream_t stream);
@@ -392,11 +385,6 @@ cudaError_t q1_gather(float4 *sn, float4 *st, unsigned int *slot_bits, Q1Gather 
                       int64_t n, float4 const *x, int32_t dilE, cudaStream_t stream);
 cudaError_t q2_gather(float4 *sn, float4 *st, unsigned int *slot_bits, Q2Gather const *g,
                       int64_t n, float4 const *y, int32_t eds, cudaStream_t stream);
-
-// values[i] = hi + lo of values_df[i] for i < n_values, the FP64 trace values
-// the terms read.
-cudaError_t df_values_to_fp64(double2 *values, float4 const *values_df, int64_t n_values,
-                              cudaStream_t stream);
 
 // Term values (resolve_request / inner_product, src/Diagram.cpp:9-94,
 // src/DilutedTrace.cpp:5-82) with the native (0) or Kahan (1) accumulator.

@@ -882,26 +882,6 @@ namespace slaph {
 namespace dev {
 namespace {
 
-// Each matrix in both layouts: dst_n[k] as stored (column-major), dst_t the
-// transpose, so that tr(L R) = sum_k L[k] R^T[k] reads both operands with
-// unit stride.
-__global__ void split_df_kernel(float4 *dst_n, float4 *dst_t, double2 const *src, int64_t n,
-                                int32_t eds) {
-  int64_t const k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (k >= n) return;
-  double2 const v = src[k];
-  float const rh = static_cast<float>(v.x), ih = static_cast<float>(v.y);
-  float const rl = static_cast<float>(v.x - static_cast<double>(rh));
-  float const il = static_cast<float>(v.y - static_cast<double>(ih));
-  float4 const f = make_float4(rh, rl, ih, il);
-  int64_t const ms = static_cast<int64_t>(eds) * eds;
-  int64_t const slot = k / ms;
-  int const e = static_cast<int>(k % ms);
-  int const i = e % eds, j = e / eds;
-  dst_n[k] = f;
-  dst_t[slot * ms + j + static_cast<int64_t>(eds) * i] = f;
-}
-
 struct DfAcc {
   float s, c;
 };
@@ -931,7 +911,7 @@ __device__ __forceinline__ void df_warp_sum(DfAcc &a) {
   }
 }
 
-__global__ void __launch_bounds__(256) trace_df_kernel(float4 *values, TraceList const *lists,
+__global__ void __launch_bounds__(256) trace_df_kernel(double2 *values, TraceList const *lists,
                                                        int32_t const *which,
                                                        int32_t const *shape_i,
                                                        int32_t const *shape_j,
@@ -983,17 +963,9 @@ __global__ void __launch_bounds__(256) trace_df_kernel(float4 *values, TraceList
     df_warp_sum(ai);
     if (lane == 0)
       values[L.val_off + static_cast<int64_t>(e) * L.stride] =
-          make_float4(ar.s, ar.c, ai.s, ai.c);
+          make_double2(static_cast<double>(ar.s) + static_cast<double>(ar.c),
+                       static_cast<double>(ai.s) + static_cast<double>(ai.c));
   }
-}
-
-// Double-float (s, c) pairs to FP64: values[k] = (s_re + c_re, s_im + c_im).
-__global__ void df_to_fp64_kernel(double2 *dst, float4 const *src, int64_t n) {
-  int64_t const k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-  if (k >= n) return;
-  float4 const v = src[k];
-  dst[k] = make_double2(static_cast<double>(v.x) + static_cast<double>(v.y),
-                        static_cast<double>(v.z) + static_cast<double>(v.w));
 }
 
 // Mixed path: C = A B in double-float arithmetic (operator*,
@@ -1054,14 +1026,6 @@ __global__ void __launch_bounds__(256) product_df_kernel(float4 *slots_n, float4
 
 }  // namespace
 
-cudaError_t split_df(float4 *dst_n, float4 *dst_t, double2 const *src, int64_t n, int32_t eds,
-                     cudaStream_t stream) {
-  if (n <= 0) return cudaSuccess;
-  split_df_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(dst_n, dst_t, src,
-                                                                              n, eds);
-  return cudaGetLastError();
-}
-
 cudaError_t products_df(float4 *slots_n, float4 *slots_t, ProdInst const *p, int64_t n,
                         int32_t eds, cudaStream_t stream) {
   if (n == 0) return cudaSuccess;
@@ -1081,21 +1045,13 @@ cudaError_t products_df(float4 *slots_n, float4 *slots_t, ProdInst const *p, int
   return cudaGetLastError();
 }
 
-cudaError_t traces_df(float4 *values_df, TraceList const *lists, int32_t const *which,
+cudaError_t traces_df(double2 *values, TraceList const *lists, int32_t const *which,
                       int64_t n_which, int32_t const *shape_i, int32_t const *shape_j,
                       int64_t const *shape_off, float4 const *slots_n, float4 const *slots_t,
                       int32_t eds, cudaStream_t stream) {
   if (n_which == 0) return cudaSuccess;
   trace_df_kernel<<<static_cast<unsigned>(n_which), 256, 0, stream>>>(
-      values_df, lists, which, shape_i, shape_j, shape_off, slots_n, slots_t, eds);
-  return cudaGetLastError();
-}
-
-cudaError_t df_values_to_fp64(double2 *values, float4 const *values_df, int64_t n_values,
-                              cudaStream_t stream) {
-  if (n_values <= 0) return cudaSuccess;
-  df_to_fp64_kernel<<<static_cast<unsigned>((n_values + 255) / 256), 256, 0, stream>>>(
-      values, values_df, n_values);
+      values, lists, which, shape_i, shape_j, shape_off, slots_n, slots_t, eds);
   return cudaGetLastError();
 }
 
@@ -1154,21 +1110,27 @@ __device__ __forceinline__ float4 const *vdv_block_df(float4 const *vdv, int cod
   return vdv + (static_cast<int64_t>(code) * g.Lt + t) * g.nev * static_cast<int64_t>(g.nev);
 }
 
+// A thread takes the four Dirac indices d of one (v, e): they share the entries
+// of VdaggerV (32^3x64 block pair: 1.5 -> 1.1 ms each for q0m and q1r).
 __global__ void q0m_df_kernel(float4 *out, Q0MInst const *inst, float4 const *vdv,
                               float4 const *noise, Geometry g) {
   Q0MInst const in = inst[blockIdx.y];
   int const nev = g.nev, eds = 4 * g.dilE;
   int const k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nev * eds) return;
-  int const v = k % nev, c = k / nev;
-  int const e = c % g.dilE, d = c / g.dilE;
+  if (k >= nev * g.dilE) return;
+  int const v = k % nev, e = k / nev;
   float4 const *m = vdv_block_df(vdv, in.vdv, in.t, g);
   float4 const *rho = noise + static_cast<int64_t>(in.r2) * g.Lt * 4 * nev;
-  CDf acc = cdf_zero();
-  for (int w = e; w < nev; w += g.dilE)
-    cdf_mac(acc, rho[d + 4 * (w + static_cast<int64_t>(nev) * in.t)],
-            m[v + static_cast<int64_t>(nev) * w]);
-  out[static_cast<int64_t>(blockIdx.y) * nev * eds + k] = cdf_value(acc);
+  CDf acc[4] = {cdf_zero(), cdf_zero(), cdf_zero(), cdf_zero()};
+  for (int w = e; w < nev; w += g.dilE) {
+    float4 const x = m[v + static_cast<int64_t>(nev) * w];
+    float4 const *rw = rho + 4 * (w + static_cast<int64_t>(nev) * in.t);
+#pragma unroll
+    for (int d = 0; d < 4; ++d) cdf_mac(acc[d], rw[d], x);
+  }
+  float4 *o = out + static_cast<int64_t>(blockIdx.y) * nev * eds + v;
+#pragma unroll
+  for (int d = 0; d < 4; ++d) o[static_cast<int64_t>(nev) * (e + g.dilE * d)] = cdf_value(acc[d]);
 }
 
 __global__ void q1r_df_kernel(float4 *out, Q1RInst const *inst, float4 const *vdv,
@@ -1176,80 +1138,20 @@ __global__ void q1r_df_kernel(float4 *out, Q1RInst const *inst, float4 const *vd
   Q1RInst const in = inst[blockIdx.y];
   int const nev = g.nev, eds = 4 * g.dilE;
   int const k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nev * eds) return;
-  int const a = k % eds, j = k / eds;
-  int const e = a % g.dilE, d = a / g.dilE;
+  if (k >= nev * g.dilE) return;
+  int const e = k % g.dilE, j = k / g.dilE;
   float4 const *m = vdv_block_df(vdv, in.vdv, in.t, g);
   float4 const *rho = noise + static_cast<int64_t>(in.r1) * g.Lt * 4 * nev;
-  CDf acc = cdf_zero();
-  for (int v = e; v < nev; v += g.dilE)
-    cdf_macc(acc, rho[d + 4 * (v + static_cast<int64_t>(nev) * in.t)],
-             m[v + static_cast<int64_t>(nev) * j]);
-  out[static_cast<int64_t>(blockIdx.y) * nev * eds + k] = cdf_value(acc);
-}
-
-__global__ void __launch_bounds__(256) q2m_df_kernel(float4 *out, Q2MInst const *inst,
-                                                     float4 const *vdv, float4 const *peram,
-                                                     Geometry g) {
-  __shared__ float4 As[KT][MT + 1];
-  __shared__ float4 Bs[KT][NT];
-  Q2MInst const in = inst[blockIdx.z];
-  int const nev = g.nev, eds = 4 * g.dilE;
-  int const ntile = (nev + NT - 1) / NT, mtile = (eds + MT - 1) / MT;
-  int const row = blockIdx.y;
-  int const v0 = (blockIdx.x % ntile) * NT;
-  int const a0 = (blockIdx.x / ntile) * MT;
-  if (a0 >= mtile * MT) return;
-  int const tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-  int64_t const rows = peram_rows(g);
-  float4 const *P = peram + static_cast<int64_t>(in.r1) * rows * g.nb * 4 * g.dilE +
-                    (static_cast<int64_t>(4 * in.t + row) * nev) +
-                    rows * (static_cast<int64_t>(in.b1) * eds);
-  float4 const *m = vdv_block_df(vdv, in.vdv, in.t, g);
-  CDf acc[2][4];
+  CDf acc[4] = {cdf_zero(), cdf_zero(), cdf_zero(), cdf_zero()};
+  for (int v = e; v < nev; v += g.dilE) {
+    float4 const x = m[v + static_cast<int64_t>(nev) * j];
+    float4 const *rv = rho + 4 * (v + static_cast<int64_t>(nev) * in.t);
 #pragma unroll
-  for (int p = 0; p < 2; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) acc[p][q] = cdf_zero();
-  float4 const z = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int w0 = 0; w0 < nev; w0 += KT) {
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      int const k = tid + 256 * q;
-      int const ww = k % KT, aa = k / KT;
-      int const w = w0 + ww, a = a0 + aa;
-      As[ww][aa] = (w < nev && a < eds) ? P[w + rows * a] : z;
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      int const k = tid + 256 * q;
-      int const ww = k % KT, vv = k / KT;
-      int const w = w0 + ww, v = v0 + vv;
-      Bs[ww][vv] = (w < nev && v < nev) ? m[w + static_cast<int64_t>(nev) * v] : z;
-    }
-    __syncthreads();
-    for (int kk = 0; kk < KT; ++kk) {
-      float4 a[2], b[4];
-#pragma unroll
-      for (int p = 0; p < 2; ++p) a[p] = As[kk][ty + 16 * p];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) b[q] = Bs[kk][tx + 16 * q];
-#pragma unroll
-      for (int p = 0; p < 2; ++p)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) cdf_macc(acc[p][q], a[p], b[q]);
-    }
-    __syncthreads();
+    for (int d = 0; d < 4; ++d) cdf_macc(acc[d], rv[d], x);
   }
-  float4 *o = out + static_cast<int64_t>(blockIdx.z) * eds * 4 * nev;
+  float4 *o = out + static_cast<int64_t>(blockIdx.y) * nev * eds + e + static_cast<int64_t>(eds) * j;
 #pragma unroll
-  for (int p = 0; p < 2; ++p)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      int const a = a0 + ty + 16 * p, v = v0 + tx + 16 * q;
-      if (a < eds && v < nev)
-        o[a + static_cast<int64_t>(eds) * (row * nev + v)] = cdf_value(acc[p][q]);
-    }
+  for (int d = 0; d < 4; ++d) o[g.dilE * d] = cdf_value(acc[d]);
 }
 
 __device__ __forceinline__ void store_factor_df(float4 *sn, float4 *st, int slot, int k, int eds,
@@ -1288,49 +1190,6 @@ __global__ void q0_df_kernel(float4 *sn, float4 *st, Q0Inst const *inst, float4 
   if (threadIdx.x % 32 == 0 && mx != 0) atomicMax(slot_bits + in.slot, mx);
 }
 
-__global__ void q1_df_kernel(float4 *sn, float4 *st, Q1Inst const *inst, float4 const *q1r,
-                             float4 const *peram, Geometry g) {
-  Q1Inst const in = inst[blockIdx.y];
-  int const nev = g.nev, dilE = g.dilE, eds = 4 * dilE;
-  int const k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= eds * eds) return;
-  int const a = k % eds, c = k / eds;
-  int const row = a / dilE;
-  int64_t const rows = peram_rows(g);
-  float4 const *R = q1r + static_cast<int64_t>(in.r) * nev * eds;
-  float4 const *P = peram + static_cast<int64_t>(in.r2) * rows * g.nb * 4 * g.dilE +
-                    static_cast<int64_t>(4 * in.t + c_gamma_row[in.gamma][row]) * nev +
-                    rows * (static_cast<int64_t>(in.b) * eds + c);
-  CDf acc = cdf_zero();
-  for (int v = 0; v < nev; ++v) cdf_mac(acc, R[a + static_cast<int64_t>(eds) * v], P[v]);
-  store_factor_df(sn, st, in.slot, k, eds, gamma_mul(c_gamma_val[in.gamma][row], cdf_value(acc)));
-}
-
-__global__ void q2_df_kernel(float4 *sn, float4 *st, Q2Inst const *inst, float4 const *q2m,
-                             float4 const *peram, Geometry g) {
-  Q2Inst const in = inst[blockIdx.y];
-  int const nev = g.nev, dilE = g.dilE, eds = 4 * dilE;
-  int const k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= eds * eds) return;
-  int const a = k % eds, c = k / eds;
-  int const r = a / dilE;
-  int64_t const rows = peram_rows(g);
-  float4 const *M = q2m + static_cast<int64_t>(in.m) * eds * 4 * nev;
-  float4 const *Pr = peram + static_cast<int64_t>(in.r2) * rows * g.nb * 4 * g.dilE +
-                     rows * (static_cast<int64_t>(in.b2) * eds + c);
-  CDf total = cdf_zero();
-  for (int bd = 0; bd < 4; ++bd) {
-    float4 const *P = Pr + static_cast<int64_t>(4 * in.t + c_gamma_row[in.gamma][bd]) * nev;
-    float4 const *Mb = M + a + static_cast<int64_t>(eds) * bd * nev;
-    bool const flip = (bd + r == 3) || (bd - r > 1) || (r - bd > 1);
-    double2 const val = c_gamma_val[in.gamma][bd];
-    double2 const s = flip ? make_double2(-val.x, -val.y) : val;
-    for (int v = 0; v < nev; ++v)
-      cdf_mac(total, gamma_mul(s, Mb[static_cast<int64_t>(eds) * v]), P[v]);
-  }
-  store_factor_df(sn, st, in.slot, k, eds, cdf_value(total));
-}
-
 int blocks256(int64_t n) { return static_cast<int>((n + 255) / 256); }
 
 }  // namespace
@@ -1342,43 +1201,25 @@ cudaError_t to_df(float4 *dst, double2 const *src, int64_t n, cudaStream_t strea
 }
 
 cudaError_t factors_df(float4 *sn, float4 *st, float4 *q0m_buf, float4 *q1r_buf,
-                       float4 *q2m_buf, Q0MInst const *q0m_i, int64_t n_q0m,
-                       Q1RInst const *q1r_i, int64_t n_q1r, Q2MInst const *q2m_i, int64_t n_q2m,
-                       Q0Inst const *q0_i, int64_t n_q0, Q1Inst const *q1_i, int64_t n_q1,
-                       Q2Inst const *q2_i, int64_t n_q2, float4 const *vdv,
-                       float4 const *noise, float4 const *peram, unsigned int *slot_bits,
-                       Geometry g, cudaStream_t stream) {
+                       Q0MInst const *q0m_i, int64_t n_q0m, Q1RInst const *q1r_i, int64_t n_q1r,
+                       Q0Inst const *q0_i, int64_t n_q0, float4 const *vdv, float4 const *noise,
+                       unsigned int *slot_bits, Geometry g, cudaStream_t stream) {
   int const eds = 4 * g.dilE;
   int64_t const per_m = static_cast<int64_t>(g.nev) * eds;
   int64_t const per_f = static_cast<int64_t>(eds) * eds;
   cudaError_t e;
   e = chunked(q0m_i, n_q0m, [&](Q0MInst const *p, int c, int64_t s) {
-    q0m_df_kernel<<<dim3(blocks256(per_m), c), 256, 0, stream>>>(q0m_buf + s * per_m, p, vdv,
+    q0m_df_kernel<<<dim3(blocks256(per_m / 4), c), 256, 0, stream>>>(q0m_buf + s * per_m, p, vdv,
                                                                  noise, g);
   });
   if (e != cudaSuccess) return e;
   e = chunked(q1r_i, n_q1r, [&](Q1RInst const *p, int c, int64_t s) {
-    q1r_df_kernel<<<dim3(blocks256(per_m), c), 256, 0, stream>>>(q1r_buf + s * per_m, p, vdv,
+    q1r_df_kernel<<<dim3(blocks256(per_m / 4), c), 256, 0, stream>>>(q1r_buf + s * per_m, p, vdv,
                                                                  noise, g);
   });
   if (e != cudaSuccess) return e;
-  int const ntile = (g.nev + NT - 1) / NT, mtile = (eds + MT - 1) / MT;
-  int64_t const per_q2m = static_cast<int64_t>(eds) * 4 * g.nev;
-  e = chunked(q2m_i, n_q2m, [&](Q2MInst const *p, int c, int64_t s) {
-    q2m_df_kernel<<<dim3(ntile * mtile, 4, c), 256, 0, stream>>>(q2m_buf + s * per_q2m, p, vdv,
-                                                                 peram, g);
-  });
-  if (e != cudaSuccess) return e;
-  e = chunked(q0_i, n_q0, [&](Q0Inst const *p, int c, int64_t) {
+  return chunked(q0_i, n_q0, [&](Q0Inst const *p, int c, int64_t) {
     q0_df_kernel<<<dim3(blocks256(per_f), c), 256, 0, stream>>>(sn, st, p, q0m_buf, noise, slot_bits, g);
-  });
-  if (e != cudaSuccess) return e;
-  e = chunked(q1_i, n_q1, [&](Q1Inst const *p, int c, int64_t) {
-    q1_df_kernel<<<dim3(blocks256(per_f), c), 256, 0, stream>>>(sn, st, p, q1r_buf, peram, g);
-  });
-  if (e != cudaSuccess) return e;
-  return chunked(q2_i, n_q2, [&](Q2Inst const *p, int c, int64_t) {
-    q2_df_kernel<<<dim3(blocks256(per_f), c), 256, 0, stream>>>(sn, st, p, q2m_buf, peram, g);
   });
 }
 
