@@ -166,6 +166,14 @@ __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
   e = (a - (s - bb)) + (b - bb);
 }
 
+// Error-free x + b 2^-k into (s, e), w = 2^-k, for an x that is a multiple of the
+// ulp of b w: s - x is then exact (Dekker's fast two-sum, which needs no order of
+// magnitudes for such an x), and b w is exact inside the FMAs.
+__device__ __forceinline__ void scaled_sum(float x, float b, float w, float &s, float &e) {
+  s = fmaf(b, w, x);
+  e = fmaf(b, w, -(s - x));
+}
+
 // ---------------------------------------------------------------- slicing
 // 64-bit fixed point of v relative to 2^e: F = round(v 2^(55-e)), |F| <= 2^55.
 __device__ __forceinline__ long long fixed55(double v, int e) {
@@ -212,6 +220,23 @@ __device__ __forceinline__ void digits6(long long F, float (&d)[kSlices]) {
 __device__ __forceinline__ float scale2(float x, int sh) {
   int const s1 = sh / 2, s2 = sh - s1;
   return (x * __int_as_float((s1 + 127) << 23)) * __int_as_float((s2 + 127) << 23);
+}
+
+// v 2^sh as a double, by integer operations: v = 0 or normal, |sh| <= kShMax.
+constexpr int kShMax = 640;
+__device__ __forceinline__ double widen_scaled(float v, int sh) {
+  unsigned int const b = __float_as_uint(v), m = b & 0x7FFFFFFFu;
+  unsigned int const hi =
+      (m >> 3) + (static_cast<unsigned int>(896 + sh) << 20) | (b & 0x80000000u);
+  return m < 0x800000u ? 0.0 : __hiloint2double(static_cast<int>(hi), static_cast<int>(m << 29));
+}
+// (hi + lo) 2^sh rounded to a double, (hi, lo) a promoted tile entry (finite;
+// zero or far above the subnormals).  FP64 units run at 1/64 of the FP32 rate:
+// two conversions, the addition and ldexp of a 128 x 80 tile took longer than the
+// MMAs of the next tile's first chunk, which hide them; one addition does not.
+__device__ __forceinline__ double df_scaled(float hi, float lo, int sh) {
+  if (abs(sh) > kShMax) return ldexp(static_cast<double>(hi) + static_cast<double>(lo), sh);
+  return widen_scaled(hi, sh) + widen_scaled(lo, sh);
 }
 
 // Two small integers held exactly in floats to a BF16 pair (a in the low half).
@@ -279,7 +304,14 @@ __device__ __forceinline__ int expo_of_absbits64(unsigned long long b) {
 // Chunk value of one column, sum_l E_l 2^-8l: levels 0 and 1 are exact
 // integers in FP32; levels 3..5 (at most 2^-24 of the row scale) are summed in
 // FP32 first, rounding by at most 2^-24 of their own magnitude, then levels 1,
-// 2 and that sum enter through error-free two-sums.
+// 2 and that sum enter through error-free sums (scaled_sum: the partial sums are
+// multiples of 1, 2^-8 and 2^-16, the addends below 2^17, 2^9.6 and 2^3).  With
+// general two-sums and one wait per three loads a promotion cost 3.4 us of a
+// chunk's 20 (the MMAs wait for it: the six accumulators leave no room for a
+// second set); with these sums, the next loads in flight and the accumulators
+// released at the last load 2.8 us.  Sixteen warps of 20 columns measured the same
+// (traces of 24^3x48 Nev 120 9.8 ms against 10.0, of 64 timeslices Nev 220 one
+// block pair 19.1 against 18.7).
 constexpr int kPromoWarps = 8;
 constexpr int kProducerWarp = kPromoWarps, kMmaWarp = kPromoWarps + 1;
 constexpr int kThreads = 32 * (kPromoWarps + 2);
@@ -337,7 +369,7 @@ __device__ __forceinline__ void ozaki_tiles(uint8_t *smem, int n_tiles, int k_ti
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(&acc_full, 1);
-    mbar_init(&acc_empty, kPromoWarps * 32);
+    mbar_init(&acc_empty, kPromoWarps);
     mbar_init(&done_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -455,35 +487,44 @@ __device__ __forceinline__ void ozaki_tiles(uint8_t *smem, int n_tiles, int k_ti
           break;
         }
         tc_fence_after();
+        // Levels 0..2 (r0), then 3..5 (r1), eight columns at a time; the next
+        // three loads are in flight while the last three are added up.
+        uint32_t r0[3][8], r1[3][8];
+#pragma unroll
+        for (int l = 0; l < 3; ++l)
+          tmem_ld8_issue(lane_addr + static_cast<uint32_t>(l * kTN), r0[l]);
 #pragma unroll
         for (int cb = 0; cb < kColsW / 8; ++cb) {
-          // Levels 0..2, then 3..5, eight columns at a time (the registers of
-          // three warps on one SM sub-partition share its 16K).
           uint32_t const ca = lane_addr + static_cast<uint32_t>(cb * 8);
-          uint32_t r[3][8];
+          tmem_ld_wait(r0);
 #pragma unroll
-          for (int l = 0; l < 3; ++l) tmem_ld8_issue(ca + static_cast<uint32_t>(l * kTN), r[l]);
-          tmem_ld_wait(r);
+          for (int l = 0; l < 3; ++l)
+            tmem_ld8_issue(ca + static_cast<uint32_t>((3 + l) * kTN), r1[l]);
           float s2[8], xs[8];
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
             float s1, x1, x2;
-            two_sum(__uint_as_float(r[0][u]), __uint_as_float(r[1][u]) * 0x1p-8f, s1, x1);
-            two_sum(s1, __uint_as_float(r[2][u]) * 0x1p-16f, s2[u], x2);
+            scaled_sum(__uint_as_float(r0[0][u]), __uint_as_float(r0[1][u]), 0x1p-8f, s1, x1);
+            scaled_sum(s1, __uint_as_float(r0[2][u]), 0x1p-16f, s2[u], x2);
             xs[u] = x1 + x2;
           }
+          tmem_ld_wait(r1);
+          if (cb + 1 < kColsW / 8) {
 #pragma unroll
-          for (int l = 0; l < 3; ++l)
-            tmem_ld8_issue(ca + static_cast<uint32_t>((3 + l) * kTN), r[l]);
-          tmem_ld_wait(r);
+            for (int l = 0; l < 3; ++l)
+              tmem_ld8_issue(ca + static_cast<uint32_t>(8 + l * kTN), r0[l]);
+          } else {
+            tc_fence_before();  // all read: the next chunk's MMAs may start
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty);
+          }
 #pragma unroll
           for (int u = 0; u < 8; ++u) {
-            float const low =
-                fmaf(__uint_as_float(r[2][u]), 0x1p-16f,
-                     fmaf(__uint_as_float(r[1][u]), 0x1p-8f, __uint_as_float(r[0][u]))) *
-                0x1p-24f;
+            float const low = fmaf(__uint_as_float(r1[2][u]), 0x1p-16f,
+                                   fmaf(__uint_as_float(r1[1][u]), 0x1p-8f,
+                                        __uint_as_float(r1[0][u])));
             float s3, x3;
-            two_sum(s2[u], low, s3, x3);
+            scaled_sum(s2[u], low, 0x1p-24f, s3, x3);
             // Running (hi, lo) += (s3, xs + x3), renormalised so that
             // |lo| <= ulp(hi)/2.
             int const j = cb * 8 + u;
@@ -495,8 +536,6 @@ __device__ __forceinline__ void ozaki_tiles(uint8_t *smem, int n_tiles, int k_ti
             hi[j] = h;
           }
         }
-        tc_fence_before();
-        mbar_arrive(&acc_empty);
       }
       // After a timeout the values are incomplete; *err makes the host discard them.
       if (ok) epi(pre, i, row, col0, hi, lo);

@@ -178,8 +178,7 @@ struct TraceEpilogue {
         int const ec = __shfl_sync(0xffffffffu, c < 32 ? p.e0 : p.e1, c % 32);
         int const col = col0 + c;
         if (row_ok && col < t.cols)
-          dst[2 * static_cast<int64_t>(col) * t.ld] =
-              ldexp(static_cast<double>(hi[c]) + static_cast<double>(lo[c]), p.er + ec - 14);
+          dst[2 * static_cast<int64_t>(col) * t.ld] = df_scaled(hi[c], lo[c], p.er + ec - 14);
       }
       return;
     }
@@ -199,7 +198,7 @@ struct TraceEpilogue {
       }
       if (e_at >= 0)
         dst[2 * (e_at * plane + static_cast<int64_t>(vb & 0xFFFF) * t.n_a)] =
-            ldexp(static_cast<double>(hi[c]) + static_cast<double>(lo[c]), p.er + ec - 14);
+            df_scaled(hi[c], lo[c], p.er + ec - 14);
     }
   }
 };

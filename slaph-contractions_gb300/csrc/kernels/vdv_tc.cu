@@ -290,14 +290,19 @@ struct VdvEpilogue {
     double *sums = reinterpret_cast<double *>(const_cast<uint8_t *>(sbase) + s_off) +
                    2 * static_cast<int64_t>(plane) * n_cols * nev + 2 * i + (row & 1);
     int const ei = expo[i];
+    int const c0 = nt * kTN + col0;
+    int f = c0 / nev, j = c0 - f * nev - 1;
 #pragma unroll
     for (int jj = 0; jj < kColsW; ++jj) {
-      int const c = nt * kTN + col0 + jj;
+      int const c = c0 + jj;
+      if (++j == nev) {
+        j = 0;
+        ++f;
+      }
       if (c < n_cols) {
-        int const f = c / nev, j = c - f * nev;
         int const ec = f < n_mom ? expo[j] : expo[(1 + f) * nev + j];
         sums[2 * static_cast<int64_t>(c) * nev] =
-            ldexp(static_cast<double>(hi[jj]) + static_cast<double>(lo[jj]), ei + ec - 14);
+            df_scaled(hi[jj], lo[jj], ei + ec - 14);
       }
     }
   }
