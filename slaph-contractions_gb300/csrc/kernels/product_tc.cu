@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kPSliceThreads)
       mx = row_max(v, mx, 1 | 2 | 4);
     }
     // |hi + lo| < 2^e whenever |hi| < 2^e (|lo| <= ulp(hi) / 2).
-    int const e = expo_of_absbits(mx);
+    int const e = wide_expo(mx);  // K' = 2 eds <= 128
     if (lane % 8 == 0) expo[gr.ea + cr] = e;
     int const arow = 2 * cr + (r & 1);
     uint8_t *base = region + ((arow >> 3) * 4 + kc) * 128 + (arow & 7) * 16;
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kPSliceThreads)
       for (int q = 0; q < 4; ++q) v[q] = src[kt * (kTK / 2) + 4 * kc + q];
       mx = row_max(v, mx, 1 | 2);
     }
-    int const e = expo_of_absbits(mx);
+    int const e = wide_expo(mx);  // K' = 2 eds <= 128
     if (kc == 0) expo[static_cast<int64_t>(blockIdx.x) * eds + j] = e;
     for (int kt = 0; kt < k_tiles; ++kt) {
       float4 v[4];

@@ -197,7 +197,7 @@ __device__ __forceinline__ long long fixed55(double v, int e) {
 // The 6 balanced base-256 digits of a 64-bit fixed-point value F (|F| <= 2^55)
 // at 2^48, 2^40, ..., 2^8, as floats: F = sum_p d_p 2^(48-8p) + r with
 // |r| <= 2^7, d_0 in [-128, 128] and d_1..d_5 in [-128, 127] (all exact in
-// BF16).  With G = F + C, C = 0x808080808080 (2^7 in every byte below the
+// BF16; for |F| <= 2^56, d_0 in [-256, 256], exact too).  With G = F + C, C = 0x808080808080 (2^7 in every byte below the
 // top), the lower digits are the bytes 5..1 of G minus 128 and the top digit is
 // G >> 48: the sum of the digits is G - C + 2^7 - (G mod 2^8).  Each lower
 // digit is one byte permutation into the mantissa of 2^23 and one FP32
@@ -247,7 +247,7 @@ __device__ __forceinline__ uint32_t bf16x2(float a, float b) {
 }
 
 // The same for a float, with integer operations only: round(v 2^(55-e)) for
-// |v| < 2^e (then the shift below is at most 31 and |F| < 2^55).
+// |v| < 2^(e+1) (then the shift below is at most 32 and |F| <= 2^56).
 __device__ __forceinline__ long long fixed55f(float v, int e) {
   int const bits = __float_as_int(v);
   int const ex = (bits >> 23) & 0xFF;
@@ -256,7 +256,7 @@ __device__ __forceinline__ long long fixed55f(float v, int e) {
   int const sh = ex - 150 + 55 - e;
   long long F;
   if (sh >= 0) {
-    F = m << (sh < 31 ? sh : 31);
+    F = m << (sh < 32 ? sh : 32);
   } else if (sh > -40) {
     F = (m + (1LL << (-sh - 1))) >> (-sh);
   } else {
@@ -272,7 +272,15 @@ __device__ __forceinline__ int expo_of_absbits(unsigned int b) {
   int const ex = static_cast<int>(b >> 23);
   return ex == 0 ? -125 : ex - 126;
 }
-// The same for a double bit pattern.
+// One less, max |x| < 2^(e+1): the top digit takes the ninth bit that BF16 holds
+// (|d_0| <= 256), the slices keep one bit more and the dropped slice pairs weigh
+// half as much, or a quarter when both operands do so.  Level 0 and 1 sums over K'
+// values are then at most 2^15 K' and 2^15 K' + 2^14 K' with one wide operand
+// (exact up to K' = 341: chunks of 10 k-tiles instead of 16), 2^16 K' with two
+// (K' = 256).
+constexpr int kWideChunkKT = 10;
+__device__ __forceinline__ int wide_expo(unsigned int b) { return expo_of_absbits(b) - 1; }
+// The exponent e of max |x| < 2^e from a double bit pattern.
 __device__ __forceinline__ int expo_of_absbits64(unsigned long long b) {
   if (b == 0) return 0;
   int const ex = static_cast<int>(b >> 52);
@@ -310,8 +318,8 @@ __device__ __forceinline__ int expo_of_absbits64(unsigned long long b) {
 // chunk's 20 (the MMAs wait for it: the six accumulators leave no room for a
 // second set); with these sums, the next loads in flight and the accumulators
 // released at the last load 2.8 us.  Sixteen warps of 20 columns measured the same
-// (traces of 24^3x48 Nev 120 9.8 ms against 10.0, of 64 timeslices Nev 220 one
-// block pair 19.1 against 18.7).
+// (traces of 24^3x48 Nev 120 9.8 ms against 10.0, of one block pair of 64
+// timeslices 19.1 against 18.7).
 constexpr int kPromoWarps = 8;
 constexpr int kProducerWarp = kPromoWarps, kMmaWarp = kPromoWarps + 1;
 constexpr int kThreads = 32 * (kPromoWarps + 2);
@@ -352,7 +360,7 @@ __device__ __forceinline__ void load_contiguous(uint8_t const *a, uint8_t const 
   bulk_g2s(dst + kStageA, b + static_cast<int64_t>(kt) * kStageB, kStageB, bar);
 }
 
-template <typename Src, typename Epilogue>
+template <int kChunk = kChunkKT, typename Src, typename Epilogue>
 __device__ __forceinline__ void ozaki_tiles(uint8_t *smem, int n_tiles, int k_tiles,
                                             Src const &src, int *err, Epilogue const &epi) {
   __shared__ __align__(8) uint64_t full_bar[kStages], empty_bar[kStages];
@@ -360,7 +368,7 @@ __device__ __forceinline__ void ozaki_tiles(uint8_t *smem, int n_tiles, int k_ti
   __shared__ uint32_t tmem_slot;
 
   int const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  int const n_chunks = (k_tiles + kChunkKT - 1) / kChunkKT;
+  int const n_chunks = (k_tiles + kChunk - 1) / kChunk;
   int const first_tile = blockIdx.x, tile_step = gridDim.x;
 
   if (threadIdx.x == 0) {
@@ -424,8 +432,8 @@ __device__ __forceinline__ void ozaki_tiles(uint8_t *smem, int n_tiles, int k_ti
           }
           tc_fence_after();
           bool first = true;  // the chunk's first k-step starts every accumulator
-          int const kt_end = min(k_tiles, (c + 1) * kChunkKT);
-          for (int kt = c * kChunkKT; kt < kt_end; ++kt, ++g) {
+          int const kt_end = min(k_tiles, (c + 1) * kChunk);
+          for (int kt = c * kChunk; kt < kt_end; ++kt, ++g) {
             int const s = static_cast<int>(g % kStages);
             uint32_t const use = static_cast<uint32_t>(g / kStages);
             if (!mbar_wait(&full_bar[s], use & 1, err, 3)) {

@@ -53,6 +53,16 @@ __global__ void __launch_bounds__(256)
   if (lane == 0) bits[first + w] = mx;
 }
 
+// Exponents of the operands: A's are wide (tc_common.cuh).  The rms error of mixed
+// contractions against FP64 ones (24 timeslices, Nev 50, dilE 8) is 1.5e-13 with no
+// wide operand in traces and products, 1.1e-13 as it is and 1.0e-13 with B wide too;
+// the trace GEMM of one block pair (64 timeslices, dilE 8), promoted every 10 k-tiles
+// instead of 16, takes 18.7 ms instead of 17.9.
+template <bool kIsA>
+__device__ __forceinline__ int group_expo(unsigned int bits) {
+  return kIsA ? wide_expo(bits) : expo_of_absbits(bits);
+}
+
 // One row group per CTA (TrSliceGroup), one pass over its matrices with the
 // largest entries of their slots (slot_maxbits): the warps take k-tiles in
 // turn.  In a k-tile, lane (r, kc) = (lane / 4, lane % 4) converts the four
@@ -72,12 +82,12 @@ __global__ void __launch_bounds__(kSliceThreads)
   int const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   if (threadIdx.x < gr.n)
     expo[gr.expo0 + threadIdx.x] =
-        expo_of_absbits(slot_bits[groups[blockIdx.x].slot[threadIdx.x]]);
+        group_expo<kIsA>(slot_bits[groups[blockIdx.x].slot[threadIdx.x]]);
   int const r = lane / 4, kc = lane % 4;
   int const mi = kIsA ? r / 2 : r;  // matrix of this lane
   if (mi >= gr.n) return;
   int const slot = groups[blockIdx.x].slot[mi];
-  int const e = expo_of_absbits(slot_bits[slot]);
+  int const e = group_expo<kIsA>(slot_bits[slot]);
   float4 const *src = slots + static_cast<int64_t>(slot) * ms + 4 * kc;
   uint8_t *region = scratch + gr.dst;
   uint8_t *base;
@@ -225,7 +235,9 @@ __global__ void __launch_bounds__(kThreads, 1)
                       int32_t const *entries, int *err) {
   extern __shared__ __align__(1024) uint8_t smem[];
   TraceEpilogue<kDf> epi{reinterpret_cast<double *>(values), expo, tiles, entries};
-  ozaki_tiles(smem, n_tiles, k_tiles, TraceSrc{scratch, tiles}, err, epi);
+  // the factor stage's operands (kDf) have plain exponents, the traces' A wide ones
+  ozaki_tiles<kDf ? kChunkKT : kWideChunkKT>(smem, n_tiles, k_tiles, TraceSrc{scratch, tiles},
+                                             err, epi);
 }
 
 }  // namespace
