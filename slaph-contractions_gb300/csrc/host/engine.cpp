@@ -969,6 +969,23 @@ void Engine::prepare_trace_tc(DeviceSchedule &ds) {
   ds.tc_ready = true;
 }
 
+namespace {
+// Whether a mixed-precision schedule takes its products to the tensor cores.  A
+// matrix that fills its padding always does; a padded one from 16384 / (4 dilE)
+// products per wave on, below which the three launches per level cost more than
+// the double-float kernel's one.  18 timeslices, three random vectors, products
+// of all waves in the double-float kernel and here: dilE 2 (1026 per wave) 0.15 and
+// 0.18 ms, dilE 3 0.20 and 0.19; 48 timeslices (2189 per wave) 0.41 and 0.39,
+// 0.57 and 0.41, with five random vectors (21888 per wave) 3.2 and 0.9, 4.7 and 1.0.
+bool product_tc(Schedule const &s) {
+  if (!dev::prod_tc_supported(s.eds)) return false;
+  if (dev::prod_tc_pad(s.eds) == s.eds) return true;
+  int64_t n = 0;
+  for (auto const &w : s.waves) n += static_cast<int64_t>(w.prods.size());
+  return n * s.eds >= 16384 * static_cast<int64_t>(s.waves.size());
+}
+}  // namespace
+
 // Tensor-core plan of the factor products (product_tc.cu), per wave and
 // dependency level: the groups of plan_products, their tiles of 80 columns
 // and the scratch they need.
@@ -993,7 +1010,7 @@ void Engine::prepare_product_tc(DeviceSchedule &ds) {
       DeviceSchedule::PLevel pl{static_cast<int64_t>(groups.size()), 0,
                                 static_cast<int64_t>(r_slots.size()), 0,
                                 static_cast<int64_t>(tiles.size()), 0};
-      ProductPlan const pp = plan_products(w.prods.data() + b, e - b, eds);
+      ProductPlan const pp = plan_products(w.prods.data() + b, e - b, dev::prod_tc_pad(eds));
       int32_t const n_r = static_cast<int32_t>(pp.r_slots.size());
       r_slots.insert(r_slots.end(), pp.r_slots.begin(), pp.r_slots.end());
       int32_t const u_base = static_cast<int32_t>(u_list.size());
@@ -1028,7 +1045,8 @@ void Engine::prepare_product_tc(DeviceSchedule &ds) {
       wb.p_levels.push_back(pl);
       size_t const r_off = static_cast<size_t>((pl.n_g * a_bytes + 1023) / 1024 * 1024);
       need = std::max(need, r_off + static_cast<size_t>(n_r) * r_bytes);
-      max_expo = std::max(max_expo, 64 * pl.n_g + static_cast<int64_t>(n_r) * eds);
+      max_expo = std::max(max_expo,
+                          64 * pl.n_g + static_cast<int64_t>(n_r) * dev::prod_tc_pad(eds));
     }
     if (u_list.size() > 0x7fffffffULL) throw UnsupportedError("product GEMM lists above 2^31");
     upload(wb.p_groups, groups, stream_);
@@ -1058,8 +1076,7 @@ void Engine::prepare_product_tc(DeviceSchedule &ds) {
 void Engine::prepare_factor_tc(DeviceSchedule &ds) {
   if (ds.f_ready) return;
   Schedule const &s = ds.s;
-  std::vector<uint8_t> const need =
-      factor_layouts(s, dev::prod_tc_supported(s.eds));
+  std::vector<uint8_t> const need = factor_layouts(s, product_tc(s));
   int32_t const eds = s.eds, nev = dims_.nev, dilE = dims_.dilE, nb = geo_.nb;
   int32_t const Lt = dims_.Lt;
   int64_t const prow = 4LL * nev * Lt;            // perambulator rows
@@ -1696,7 +1713,7 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
     // ---- waves: products, traces, terms, accumulation
     values_.reserve(sizeof(double2) * std::max<int64_t>(1, s.max_values));
     term_val_.reserve(sizeof(double2) * std::max<int64_t>(1, s.max_terms));
-    bool const p_tc = mixed && dev::prod_tc_supported(eds);
+    bool const p_tc = mixed && product_tc(s);
     if (mixed) {
       prepare_trace_tc(ds);
       if (p_tc) prepare_product_tc(ds);

@@ -899,19 +899,23 @@ ProductPlan plan_products(ProdInst const *prods, int64_t n, int32_t eds) {
   int32_t const per_group = eds > 0 && eds <= 64 ? std::max(1, 64 / eds) : 1;
   // left matrices (by first appearance) with their (right index, slot)
   // lists; right matrices numbered by first appearance
-  std::map<int32_t, int32_t> lidx, ridx;
+  int32_t top = -1;
+  for (int64_t k = 0; k < n; ++k) top = std::max({top, prods[k].a, prods[k].b});
+  std::vector<int32_t> lidx(top + 1, -1), ridx(top + 1, -1);  // by slot
   std::vector<int32_t> l_slot;
   std::vector<std::vector<std::pair<int32_t, int32_t>>> lr;
   for (int64_t k = 0; k < n; ++k) {
     ProdInst const &pi = prods[k];
-    auto li = lidx.emplace(pi.a, static_cast<int32_t>(l_slot.size()));
-    if (li.second) {
+    if (lidx[pi.a] < 0) {
+      lidx[pi.a] = static_cast<int32_t>(l_slot.size());
       l_slot.push_back(pi.a);
       lr.emplace_back();
     }
-    auto ri = ridx.emplace(pi.b, static_cast<int32_t>(pp.r_slots.size()));
-    if (ri.second) pp.r_slots.push_back(pi.b);
-    lr[li.first->second].push_back({ri.first->second, pi.c});
+    if (ridx[pi.b] < 0) {
+      ridx[pi.b] = static_cast<int32_t>(pp.r_slots.size());
+      pp.r_slots.push_back(pi.b);
+    }
+    lr[lidx[pi.a]].push_back({ridx[pi.b], pi.c});
   }
   int32_t const n_l = static_cast<int32_t>(l_slot.size());
   std::vector<std::vector<int32_t>> inv(pp.r_slots.size());

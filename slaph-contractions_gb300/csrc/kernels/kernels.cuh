@@ -221,9 +221,10 @@ cudaError_t factors_df(float4 *sn, float4 *st, float4 *q0m_buf, float4 *q1r_buf,
 // slots[c] = slots[a] * slots[b] in double-float, both layouts written.
 cudaError_t products_df(float4 *slots_n, float4 *slots_t, ProdInst const *p, int64_t n,
                         int32_t eds, cudaStream_t stream);
-// The same products on the tensor cores (product_tc.cu), for eds = 16, 32 or
-// 64.  The products of one dependency level come in groups of up to 64 / eds
-// left matrices (slots l[0..n_l)) with the union of their right matrices:
+// The same products on the tensor cores (product_tc.cu), for eds = 8 .. 32 and 64.
+// Matrices are padded to P = prod_tc_pad(eds) rows and columns in the operands
+// (not in the slots).  The products of one dependency level come in groups of up
+// to 64 / P left matrices (slots l[0..n_l)) with the union of their right matrices:
 // column block u of group g is right matrix u_list[g.u_off + u] (an index into
 // the level's r_slots) and out_tab[4 (g.u_off + u) + l] is the slot of product
 // l x u, or -1 when the level does not ask for it.  Tiles: (group, n tile of
@@ -239,19 +240,26 @@ struct ProdGroup {
   int32_t u_off;  // first column block in u_list / out_tab
   int32_t ea;     // exponent index of the group's row 0 (64 g)
 };
-// One unit of GEMM work.  eds = 64: the 80-column tile nt of the group.  eds = 16,
-// 32: the n (at most kProdSteps) right matrices u_list[u .. u + n) of the group,
-// one GEMM step each; n_l and ea repeat the group's.
+// One unit of GEMM work.  eds = 64: the 80-column tile nt of the group.  eds <= 32:
+// the n (at most kProdSteps) right matrices u_list[u .. u + n) of the group, one
+// GEMM step each; n_l and ea repeat the group's.
 constexpr int32_t kProdSteps = 32;
 struct ProdTile {
   int32_t group, nt;
   int32_t u, n, n_l, ea;
 };
-inline bool prod_tc_steps(int32_t eds) { return eds == 16 || eds == 32; }
-__host__ __device__ inline int64_t prod_tc_r_bytes(int32_t eds) {
-  return 24LL * eds * eds;  // (eds / 16) k-tiles x 6 slices x eds columns x 32 bytes
+// (4 x 4 matrices fill 1/16 of a padded product and stay with the double-float
+// kernel, as those between 32 and 64 do, whose left operand leaves no room for
+// the right ones.)
+inline bool prod_tc_steps(int32_t eds) { return eds >= 8 && eds <= 32; }
+inline bool prod_tc_supported(int32_t eds) { return prod_tc_steps(eds) || eds == 64; }
+__host__ __device__ inline int32_t prod_tc_pad(int32_t eds) {
+  return eds <= 16 ? 16 : eds <= 32 ? 32 : 64;
 }
-bool prod_tc_supported(int32_t eds);
+__host__ __device__ inline int64_t prod_tc_r_bytes(int32_t eds) {
+  // (P / 16) k-tiles x 6 slices x P columns x 64 bytes
+  return 24LL * prod_tc_pad(eds) * prod_tc_pad(eds);
+}
 int64_t prod_tc_a_bytes(int32_t eds);
 cudaError_t products_tc(float4 *slots_n, float4 *slots_t, uint8_t *scratch, int64_t r_off,
                         int32_t *expo, int64_t r_expo, ProdGroup const *groups, int64_t n_groups,

@@ -19,9 +19,11 @@
 // sliced once into a stream of its own, [k-tile][slice][8-column group][512
 // bytes] with one exponent per column.
 //
-// product_step_kernel (eds = 16, 32) takes one right matrix per step against the
-// group's A operand, which stays in shared memory: a step is K = eds, one or
-// two k-tiles, so promotion and epilogue, not the MMAs, bound it.  With the
+// product_step_kernel (eds <= 32) takes one right matrix per step against the
+// group's A operand, which stays in shared memory.  Sizes below 16 or 32 are padded
+// with zeros in the operands (18^3x48, eds = 24: products 3.8 ms in the double-float
+// kernel, 1.5 ms here).  A step is one or two k-tiles, so promotion and epilogue,
+// not the MMAs, bound it.  With the
 // general tile (tc_common.cuh: 80 columns, eight promotion warps that hold 40
 // columns of running sums and hand them to an unrolled epilogue) a tile's MMAs
 // took 2.7 us of 14: the code did not fit the instruction cache and nothing
@@ -99,21 +101,27 @@ __global__ void __launch_bounds__(kPSliceThreads)
                         float4 const *slots_t, int32_t eds, int64_t a_bytes) {
   ProdGroup const gr = groups[blockIdx.x];
   int64_t const ms = static_cast<int64_t>(eds) * eds;
-  int const k_tiles = eds / (kTK / 2);
+  int const pad = prod_tc_pad(eds), k_tiles = pad / (kTK / 2);
   int const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   int const r = lane / 4, kc = lane % 4;
   uint8_t *region = scratch + static_cast<int64_t>(blockIdx.x) * a_bytes;
   for (int quad = warp; quad < (kTM / 2) / 4; quad += kPSliceThreads / 32) {
     int const cr = 4 * quad + r / 2;  // complex row of the M tile
-    int const l = cr / eds, i = cr % eds;
+    int const l = cr / pad, i = cr % pad;
     if (l >= gr.n_l) continue;  // warp-uniform: a quad lies inside one matrix
     float4 const *src =
         slots_t + static_cast<int64_t>(groups[blockIdx.x].l[l]) * ms + static_cast<int64_t>(i) * eds;
+    // the four entries of a k-tile that this lane converts (zero in the padding)
+    auto load = [&](int kt, float4 (&v)[4]) {
+      int const k0 = kt * (kTK / 2) + 4 * kc;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        v[q] = i < eds && k0 < eds ? src[k0 + q] : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
     unsigned int mx = 0;
     for (int kt = 0; kt < k_tiles; ++kt) {
       float4 v[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = src[kt * (kTK / 2) + 4 * kc + q];
+      load(kt, v);
       mx = row_max(v, mx, 1 | 2 | 4);
     }
     // |hi + lo| < 2^e whenever |hi| < 2^e (|lo| <= ulp(hi) / 2).
@@ -123,8 +131,7 @@ __global__ void __launch_bounds__(kPSliceThreads)
     uint8_t *base = region + ((arow >> 3) * 4 + kc) * 128 + (arow & 7) * 16;
     for (int kt = 0; kt < k_tiles; ++kt) {
       float4 v[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = src[kt * (kTK / 2) + 4 * kc + q];
+      load(kt, v);
       slice_row_segment<true>(v, e, r, base + static_cast<int64_t>(kt) * kStageA, kABlk);
     }
   }
@@ -137,7 +144,7 @@ __global__ void __launch_bounds__(kPSliceThreads)
     prod_slice_r_kernel(uint8_t *streams, int32_t *expo, int32_t const *r_slots,
                         float4 const *slots_n, int32_t eds) {
   int64_t const ms = static_cast<int64_t>(eds) * eds;
-  int const k_tiles = eds / (kTK / 2), n_cg = eds / 8;
+  int const pad = prod_tc_pad(eds), k_tiles = pad / (kTK / 2), n_cg = pad / 8;
   int const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   int const r = lane / 4, kc = lane % 4;
   uint8_t *stream = streams + static_cast<int64_t>(blockIdx.x) * prod_tc_r_bytes(eds);
@@ -145,19 +152,23 @@ __global__ void __launch_bounds__(kPSliceThreads)
   for (int cg = warp; cg < n_cg; cg += kPSliceThreads / 32) {
     int const j = 8 * cg + r;
     float4 const *src = mat + static_cast<int64_t>(j) * eds;
+    auto load = [&](int kt, float4 (&v)[4]) {
+      int const k0 = kt * (kTK / 2) + 4 * kc;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        v[q] = j < eds && k0 < eds ? src[k0 + q] : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
     unsigned int mx = 0;
     for (int kt = 0; kt < k_tiles; ++kt) {
       float4 v[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = src[kt * (kTK / 2) + 4 * kc + q];
+      load(kt, v);
       mx = row_max(v, mx, 1 | 2);
     }
     int const e = wide_expo(mx);  // K' = 2 eds <= 128
-    if (kc == 0) expo[static_cast<int64_t>(blockIdx.x) * eds + j] = e;
+    if (kc == 0) expo[static_cast<int64_t>(blockIdx.x) * pad + j] = e;
     for (int kt = 0; kt < k_tiles; ++kt) {
       float4 v[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = src[kt * (kTK / 2) + 4 * kc + q];
+      load(kt, v);
       // [k-tile][slice][8-column group][512 B]: a slice step is n_cg groups
       uint8_t *dst = stream + ((static_cast<int64_t>(kt) * kSlices * n_cg + cg) * 4 + kc) * 128 +
                      r * 16;
@@ -320,11 +331,11 @@ __global__ void __launch_bounds__(kThreads, 1)
 constexpr int kStepWarps = 16;  // promotion warps: quadrant w % 4, column block w / 4
 constexpr int kStepThreads = 32 * (kStepWarps + 2);
 constexpr int kStepStages = 4;  // right matrices in flight
-constexpr uint32_t kStepTmem = 256;  // columns per accumulator set (6 eds used)
+constexpr uint32_t kStepTmem = 256;  // columns per accumulator set (6 kPad used)
 
-__host__ __device__ inline uint32_t step_a_bytes(int eds) { return eds / 16 * kStageA; }
-__host__ __device__ inline uint32_t step_smem(int eds) {
-  return step_a_bytes(eds) + kStepStages * 24u * eds * eds;
+__host__ __device__ inline uint32_t step_a_bytes(int pad) { return pad / 16 * kStageA; }
+__host__ __device__ inline uint32_t step_smem(int pad) {
+  return step_a_bytes(pad) + kStepStages * 24u * pad * pad;
 }
 
 struct StepArgs {
@@ -339,19 +350,19 @@ struct StepArgs {
   float4 *slots_n, *slots_t;
   unsigned int *slot_bits;
   int *err;
+  int32_t eds;
 };
 
-template <int kEds>
+template <int kPad>
 __global__ void __launch_bounds__(kStepThreads, 1) product_step_kernel(StepArgs const g) {
-  constexpr int kKT = kEds / 16;                      // k-tiles
-  constexpr uint32_t kRB = 24u * kEds * kEds;         // bytes of a right matrix
-  constexpr int kColBlocks = kEds / 8;
+  constexpr int kKT = kPad / 16;                      // k-tiles
+  constexpr uint32_t kRB = 24u * kPad * kPad;         // bytes of a right matrix
   extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) uint64_t a_full, a_empty, b_full[kStepStages], b_empty[kStepStages];
   __shared__ __align__(8) uint64_t acc_full[2], acc_empty[2], done_bar;
   __shared__ uint32_t tmem_slot;
   int const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  uint8_t *const b_smem = smem + step_a_bytes(kEds);
+  uint8_t *const b_smem = smem + step_a_bytes(kPad);
   if (threadIdx.x == 0) {
     mbar_init(&a_full, 1);
     mbar_init(&a_empty, 1);
@@ -387,8 +398,8 @@ __global__ void __launch_bounds__(kStepThreads, 1) product_step_kernel(StepArgs 
       if (lane == 0) {
         if (n_a > 0) ok = mbar_wait(&a_empty, (n_a - 1) & 1, g.err, 1);
         if (ok) {
-          mbar_expect_tx(&a_full, step_a_bytes(kEds));
-          bulk_g2s(smem, g.scratch + t.group * g.a_bytes, step_a_bytes(kEds), &a_full);
+          mbar_expect_tx(&a_full, step_a_bytes(kPad));
+          bulk_g2s(smem, g.scratch + t.group * g.a_bytes, step_a_bytes(kPad), &a_full);
         }
       }
       ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -443,10 +454,10 @@ __global__ void __launch_bounds__(kStepThreads, 1) product_step_kernel(StepArgs 
                 uint64_t const ad =
                     smem_desc(a_base + (ks / 2) * kStageA + p * kABlk + (ks % 2) * 256, 128, 512);
                 uint64_t const bd = smem_desc(
-                    b_base + (ks / 2) * (kSlices * kEds * 64) + q0 * (kEds * 64) + (ks % 2) * 256,
+                    b_base + (ks / 2) * (kSlices * kPad * 64) + q0 * (kPad * 64) + (ks % 2) * 256,
                     128, 512);
-                mma_bf16(d + static_cast<uint32_t>((p + q0) * kEds), ad, bd,
-                         ks == 0 && p == 0 ? 0u : 1u, idesc_n(nb * kEds));
+                mma_bf16(d + static_cast<uint32_t>((p + q0) * kPad), ad, bd,
+                         ks == 0 && p == 0 ? 0u : 1u, idesc_n(nb * kPad));
               }
             }
           }
@@ -459,15 +470,16 @@ __global__ void __launch_bounds__(kStepThreads, 1) product_step_kernel(StepArgs 
       mbar_wait(&done_bar, 0, g.err, 4);
     }
   } else {
-    // Promotion: A' row 2 cr + (re | im), cr = l kEds + i; columns 8 blk .. of the
+    // Promotion: A' row 2 cr + (re | im), cr = l kPad + i; columns 8 blk .. of the
     // step's right matrix.  A warp's rows lie in one left matrix, its columns in
     // one right matrix: one product slot per warp and step.
     int const quad = warp % 4, blk = warp / 4;
-    int const row = 32 * quad + lane, cr = row / 2, l = cr / kEds, ri = cr % kEds;
-    bool const blk_on = blk < kColBlocks;
+    int const row = 32 * quad + lane, cr = row / 2, l = cr / kPad, ri = cr % kPad;
+    int const eds = g.eds;
+    bool const blk_on = 8 * blk < eds, row_on = ri < eds;
     uint32_t const lane_addr =
         tmem + (static_cast<uint32_t>(32 * quad) << 16) + static_cast<uint32_t>(8 * blk);
-    int64_t const ms = kEds * kEds;
+    int64_t const ms = static_cast<int64_t>(eds) * eds;
     uint32_t n_s = 0;
     bool ok = true;
     for (int i = blockIdx.x; i < g.n_units && ok; i += gridDim.x) {
@@ -480,7 +492,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) product_step_kernel(StepArgs 
       auto column_expo = [&](int s) {  // lane c: exponent of column 8 blk + c of step s
         int const r = __shfl_sync(0xffffffffu, idx, s);
         return blk_on && lane < 8
-                   ? g.expo[g.r_expo + static_cast<int64_t>(r) * kEds + 8 * blk + lane]
+                   ? g.expo[g.r_expo + static_cast<int64_t>(r) * kPad + 8 * blk + lane]
                    : 0;
       };
       int ec_next = column_expo(0);
@@ -498,10 +510,10 @@ __global__ void __launch_bounds__(kStepThreads, 1) product_step_kernel(StepArgs 
         if (slot >= 0) {  // warp-uniform
           uint32_t const ca = lane_addr + set * kStepTmem;
 #pragma unroll
-          for (int v = 0; v < 3; ++v) tmem_ld8_issue(ca + static_cast<uint32_t>(v * kEds), r0[v]);
+          for (int v = 0; v < 3; ++v) tmem_ld8_issue(ca + static_cast<uint32_t>(v * kPad), r0[v]);
 #pragma unroll
           for (int v = 0; v < 3; ++v)
-            tmem_ld8_issue(ca + static_cast<uint32_t>((3 + v) * kEds), r1[v]);
+            tmem_ld8_issue(ca + static_cast<uint32_t>((3 + v) * kPad), r1[v]);
           tmem_ld_wait(r0);
           tmem_ld_wait(r1);
         }
@@ -510,7 +522,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) product_step_kernel(StepArgs 
         if (lane == 0) mbar_arrive(&acc_empty[set]);
         if (slot < 0) continue;
         unsigned int mx = 0;
-        float4 *const dst = (row & 1) ? g.slots_t + slot * ms + static_cast<int64_t>(kEds) * ri
+        float4 *const dst = (row & 1) ? g.slots_t + slot * ms + static_cast<int64_t>(eds) * ri
                                       : g.slots_n + slot * ms + ri;
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
@@ -529,12 +541,14 @@ __global__ void __launch_bounds__(kStepThreads, 1) product_step_kernel(StepArgs 
           float const h = scale2(hi, sh), lw = scale2(lo, sh);
           float const oh = __shfl_xor_sync(0xffffffffu, h, 1);
           float const ol = __shfl_xor_sync(0xffffffffu, lw, 1);
-          mx = max(mx, __float_as_uint(h) & 0x7FFFFFFFu);
           int const j = 8 * blk + u;
-          // the even lane of a row pair (Re) stores the natural layout, the odd
-          // one (Im) the transposed
-          dst[(row & 1) ? j : kEds * j] = (row & 1) ? make_float4(oh, ol, h, lw)
-                                                    : make_float4(h, lw, oh, ol);
+          if (row_on && j < eds) {
+            mx = max(mx, __float_as_uint(h) & 0x7FFFFFFFu);
+            // the even lane of a row pair (Re) stores the natural layout, the odd
+            // one (Im) the transposed
+            dst[(row & 1) ? j : eds * j] = (row & 1) ? make_float4(oh, ol, h, lw)
+                                                     : make_float4(h, lw, oh, ol);
+          }
         }
         mx = __reduce_max_sync(0xffffffffu, mx);
         if (lane == 0) atomicMax(g.slot_bits + slot, mx);
@@ -551,22 +565,21 @@ __global__ void __launch_bounds__(kStepThreads, 1) product_step_kernel(StepArgs 
   }
 }
 
-template <int kEds>
+template <int kPad>
 cudaError_t launch_steps(StepArgs const &args, cudaStream_t stream) {
-  cudaError_t const e = cudaFuncSetAttribute(product_step_kernel<kEds>,
+  cudaError_t const e = cudaFuncSetAttribute(product_step_kernel<kPad>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(step_smem(kEds)));
+                                             static_cast<int>(step_smem(kPad)));
   if (e != cudaSuccess) return e;
-  product_step_kernel<kEds><<<static_cast<unsigned>(persistent_grid(args.n_units)), kStepThreads,
-                              step_smem(kEds), stream>>>(args);
+  product_step_kernel<kPad><<<static_cast<unsigned>(persistent_grid(args.n_units)), kStepThreads,
+                              step_smem(kPad), stream>>>(args);
   return cudaGetLastError();
 }
 
 }  // namespace
 
-bool prod_tc_supported(int32_t eds) { return eds == 16 || eds == 32 || eds == 64; }
 int64_t prod_tc_a_bytes(int32_t eds) {
-  return static_cast<int64_t>(eds / (kTK / 2)) * kStageA;
+  return static_cast<int64_t>(prod_tc_pad(eds) / (kTK / 2)) * kStageA;
 }
 
 cudaError_t products_tc(float4 *slots_n, float4 *slots_t, uint8_t *scratch, int64_t r_off,
@@ -588,8 +601,9 @@ cudaError_t products_tc(float4 *slots_n, float4 *slots_t, uint8_t *scratch, int6
     cudaError_t const se = cudaGetLastError();
     if (se != cudaSuccess) return se;
     StepArgs const args{scratch, a_bytes, r_off, tiles, static_cast<int32_t>(n_tiles), u_list,
-                        expo, r_expo, out_tab, slots_n, slots_t, slot_bits, err};
-    return eds == 32 ? launch_steps<32>(args, stream) : launch_steps<16>(args, stream);
+                        expo, r_expo, out_tab, slots_n, slots_t, slot_bits, err, eds};
+    return prod_tc_pad(eds) == 32 ? launch_steps<32>(args, stream)
+                                  : launch_steps<16>(args, stream);
   }
   cudaError_t e = cudaFuncSetAttribute(product_gemm_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,

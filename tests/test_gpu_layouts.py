@@ -1,7 +1,7 @@
 """Every diagram of the reference's integration test with the tensor-core
-products (4 dilE = 16, 32, 64) and without them: factors are written only in
-the layouts in which a trace or product reads them, so each trace kind has to
-find its operands."""
+products (4 dilE = 8 .. 32, padded to 16 or 32, and 64) and without them: factors
+are written only in the layouts in which a trace or product reads them, so each
+trace kind has to find its operands."""
 from __future__ import annotations
 
 import numpy as np
@@ -11,7 +11,7 @@ from conftest import GOLDEN, corr_rel_err
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dilE", [3, 4, 8, 16])
+@pytest.mark.parametrize("dilE", [1, 2, 3, 4, 5, 6, 7, 8, 9, 16])
 def test_all_diagrams_match_the_fp64_path(engine_lib, tmp_path, dilE):
     from slaph_gb300 import GlobalData
     from slaph_gb300.engine import Engine
