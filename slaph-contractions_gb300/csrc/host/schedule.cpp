@@ -896,7 +896,8 @@ TraceGroupPlan plan_trace_group(TraceShape const &shape, int32_t n_a, int32_t n_
 
 ProductPlan plan_products(ProdInst const *prods, int64_t n, int32_t eds) {
   ProductPlan pp;
-  int32_t const per_group = eds > 0 && eds <= 64 ? std::max(1, 64 / eds) : 1;
+  // at most the four left matrices that a group holds
+  int32_t const per_group = eds > 0 && eds <= 64 ? std::min(4, std::max(1, 64 / eds)) : 1;
   // left matrices (by first appearance) with their (right index, slot)
   // lists; right matrices numbered by first appearance
   int32_t top = -1;
