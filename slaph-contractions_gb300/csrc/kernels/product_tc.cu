@@ -50,26 +50,22 @@ using namespace tc;
 constexpr int kPSliceThreads = 256;
 
 // Row group (A: four complex rows = eight A' rows; B: eight columns) of one
-// k-tile: lane (r, kc) = (lane / 4, lane % 4) converts the four complex
-// entries 4 kc .. 4 kc + 3 of its row into one 16-byte row segment per slice.
-// v: the entries, e: the row's exponent; A rows are conjugated.
+// k-tile: lane (r, kc) = (lane / 4, lane % 4) stores the four complex entries
+// 4 kc .. 4 kc + 3 of its row as one 16-byte row segment per slice.  v: the
+// entries (A: the two that this lane of a row pair cuts, a_row_words), e: the
+// row's exponent; A rows are conjugated.
 template <bool kIsA>
-__device__ __forceinline__ void slice_row_segment(float4 const (&v)[4], int e, int r,
+__device__ __forceinline__ void slice_row_segment(float4 const (&v)[kIsA ? 2 : 4], int e, int r,
                                                   uint8_t *dst, uint32_t blk) {
   uint32_t w[kSlices][4];
+  if constexpr (kIsA) {
+    a_row_words(v, e, r & 1, w);
+  } else {
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    long long const fr = fixed55f(v[q].x, e) + fixed55f(v[q].y, e);
-    long long const fi = fixed55f(v[q].z, e) + fixed55f(v[q].w, e);
-    float dre[kSlices], dim[kSlices];
-    digits6(fr, dre);
-    if (kIsA) {
-      digits6(-fi, dim);
-#pragma unroll
-      for (int s = 0; s < kSlices; ++s)
-        w[s][q] = (r & 1) ? bf16x2(-dim[s], dre[s]) : bf16x2(dre[s], dim[s]);
-    } else {
-      digits6(fi, dim);
+    for (int q = 0; q < 4; ++q) {
+      float dre[kSlices], dim[kSlices];
+      digits6(fixed55f(v[q].x, e) + fixed55f(v[q].y, e), dre);
+      digits6(fixed55f(v[q].z, e) + fixed55f(v[q].w, e), dim);
 #pragma unroll
       for (int s = 0; s < kSlices; ++s) w[s][q] = bf16x2(dre[s], dim[s]);
     }
@@ -81,10 +77,11 @@ __device__ __forceinline__ void slice_row_segment(float4 const (&v)[4], int e, i
 
 // Largest |re|, |im| (high words) of the lanes' entries, over the lanes whose
 // bits `mask` differ (the lanes of one row).
-__device__ __forceinline__ unsigned int row_max(float4 const (&v)[4], unsigned int mx,
+template <int N>
+__device__ __forceinline__ unsigned int row_max(float4 const (&v)[N], unsigned int mx,
                                                 int mask) {
 #pragma unroll
-  for (int q = 0; q < 4; ++q)
+  for (int q = 0; q < N; ++q)
     mx = max(mx, max(__float_as_uint(v[q].x) & 0x7FFFFFFFu, __float_as_uint(v[q].z) & 0x7FFFFFFFu));
 #pragma unroll
   for (int o = 1; o <= 4; o <<= 1)
@@ -111,16 +108,16 @@ __global__ void __launch_bounds__(kPSliceThreads)
     if (l >= gr.n_l) continue;  // warp-uniform: a quad lies inside one matrix
     float4 const *src =
         slots_t + static_cast<int64_t>(groups[blockIdx.x].l[l]) * ms + static_cast<int64_t>(i) * eds;
-    // the four entries of a k-tile that this lane converts (zero in the padding)
-    auto load = [&](int kt, float4 (&v)[4]) {
-      int const k0 = kt * (kTK / 2) + 4 * kc;
+    // the two entries of a k-tile that this lane cuts (zero in the padding)
+    auto load = [&](int kt, float4 (&v)[2]) {
+      int const k0 = kt * (kTK / 2) + 4 * kc + 2 * (r & 1);
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
+      for (int q = 0; q < 2; ++q)
         v[q] = i < eds && k0 < eds ? src[k0 + q] : make_float4(0.f, 0.f, 0.f, 0.f);
     };
     unsigned int mx = 0;
     for (int kt = 0; kt < k_tiles; ++kt) {
-      float4 v[4];
+      float4 v[2];
       load(kt, v);
       mx = row_max(v, mx, 1 | 2 | 4);
     }
@@ -130,7 +127,7 @@ __global__ void __launch_bounds__(kPSliceThreads)
     int const arow = 2 * cr + (r & 1);
     uint8_t *base = region + ((arow >> 3) * 4 + kc) * 128 + (arow & 7) * 16;
     for (int kt = 0; kt < k_tiles; ++kt) {
-      float4 v[4];
+      float4 v[2];
       load(kt, v);
       slice_row_segment<true>(v, e, r, base + static_cast<int64_t>(kt) * kStageA, kABlk);
     }

@@ -287,6 +287,32 @@ __device__ __forceinline__ int expo_of_absbits64(unsigned long long b) {
   return ex == 0 ? -1021 : ex - 1022;
 }
 
+// Packed words of four consecutive entries of an A row pair: rows (Re x, Im x) (odd =
+// 0) and (-Im x, Re x) (odd = 1) of x = conj(v), v double-float of exponent e.
+// The two lanes of a pair, lane and lane ^ 4, cut two entries each (v: entries 2 odd
+// and 2 odd + 1) and exchange the words: cutting is what the slicing kernels' ALUs
+// do, and the second row is the first with halves swapped and one sign flipped.
+__device__ __forceinline__ void a_row_words(float4 const (&v)[2], int e, int odd,
+                                            uint32_t (&w)[kSlices][4]) {
+  uint32_t own[kSlices][2];
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    float dre[kSlices], dim[kSlices];
+    digits6(fixed55f(v[q].x, e) + fixed55f(v[q].y, e), dre);
+    digits6(-(fixed55f(v[q].z, e) + fixed55f(v[q].w, e)), dim);
+#pragma unroll
+    for (int s = 0; s < kSlices; ++s) own[s][q] = bf16x2(dre[s], dim[s]);
+  }
+#pragma unroll
+  for (int s = 0; s < kSlices; ++s)
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      uint32_t const y = __shfl_xor_sync(0xffffffffu, own[s][q], 4);
+      w[s][q] = odd ? __byte_perm(y, 0, 0x1032) ^ 0x8000u : own[s][q];
+      w[s][2 + q] = odd ? __byte_perm(own[s][q], 0, 0x1032) ^ 0x8000u : y;
+    }
+}
+
 // The tiles of one launch, each a 128 x 80 output tile of D = A' B^T over
 // k_tiles k-tiles, computed by a persistent CTA: CTA b takes tiles b, b + G,
 // b + 2G, ... (G = gridDim.x, at most one CTA per SM).  The operands:

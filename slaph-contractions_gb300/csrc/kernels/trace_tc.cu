@@ -69,7 +69,9 @@ __device__ __forceinline__ int group_expo(unsigned int bits) {
 // complex entries 4 kc .. 4 kc + 3 of core-matrix row r (B: matrix r; A:
 // matrix r / 2, A' row parity r % 2) into one 16-byte row segment per slice,
 // so that each slice store of a warp writes 512 contiguous bytes.  Integer
-// and FP32 operations only: the fixed-point value of a double-float entry is
+// and FP32 operations only (they, not HBM, bound the A slices: with each lane of a
+// row pair cutting all four entries 4.4 ms at 24^3x48 Nev 120, with two entries
+// cut and exchanged 3.7): the fixed-point value of a double-float entry is
 // the sum of those of its two words.  Rows past the group's n are not written
 // (the GEMM tiles mask them).
 template <bool kIsA>
@@ -105,21 +107,17 @@ __global__ void __launch_bounds__(kSliceThreads)
   }
   for (int kt = warp; kt < k_tiles; kt += kSliceThreads / 32) {
     uint32_t w[kSlices][4];
+    float4 const *in = src + kt * (kTK / 2);
+    if (kIsA) {
+      float4 const v[2] = {in[2 * (r & 1)], in[2 * (r & 1) + 1]};
+      a_row_words(v, e, r & 1, w);
+    } else {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float4 const v = src[kt * (kTK / 2) + q];
-      long long const fr = fixed55f(v.x, e) + fixed55f(v.y, e);
-      long long const fi = fixed55f(v.z, e) + fixed55f(v.w, e);
-      float dre[kSlices], dim[kSlices];
-      digits6(fr, dre);
-      if (kIsA) {
-        // conj: A' rows (Re x, Im x) and (-Im x, Re x) of x = conj(v)
-        digits6(-fi, dim);
-#pragma unroll
-        for (int s = 0; s < kSlices; ++s)
-          w[s][q] = (r & 1) ? bf16x2(-dim[s], dre[s]) : bf16x2(dre[s], dim[s]);
-      } else {
-        digits6(fi, dim);
+      for (int q = 0; q < 4; ++q) {
+        float4 const v = in[q];
+        float dre[kSlices], dim[kSlices];
+        digits6(fixed55f(v.x, e) + fixed55f(v.y, e), dre);
+        digits6(fixed55f(v.z, e) + fixed55f(v.w, e), dim);
 #pragma unroll
         for (int s = 0; s < kSlices; ++s) w[s][q] = bf16x2(dre[s], dim[s]);
       }
