@@ -440,7 +440,11 @@ __global__ void __launch_bounds__(256) trace_kernel(double2 *values, TraceList c
 // ---------------------------------------------------------------- terms
 // resolve_request1/2/3 (src/Diagram.cpp:9-94) with inner_product
 // (src/DilutedTrace.cpp:5-82): one thread per (request, slice pair), the
-// reference's loop order and accumulator.
+// reference's loop order and accumulator.  The FP64 units bound it.  The inner
+// sum of a product of two traces depends on the outer entry's random-vector mask
+// only, which ordered index tuples share (two orders of a pair, six of three), so
+// the sums of the first kTermMemo outer entries are kept and taken again.
+constexpr int kTermMemo = 32;
 __global__ void term_kernel(double2 *term_val, Term const *terms, int64_t n,
                             TraceList const *lists, double2 const *values,
                             uint16_t const *shape_mask, int64_t const *shape_off,
@@ -470,14 +474,33 @@ __global__ void term_kernel(double2 *term_val, Term const *terms, int64_t n,
     int64_t num = 0;
     Acc result(kahan);
     if (t.n == 2) {
+      double2 memo[kTermMemo];
+      int32_t memo_n[kTermMemo];
       for (int64_t l = 0; l < n0; ++l) {
-        Acc rs(kahan);
-        for (int64_t r = 0; r < n1; ++r) {
-          if ((m0[l] & m1[r]) != 0u) continue;
-          rs.add(x1[r * s1]);
-          ++num;
+        uint16_t const m = m0[l];
+        int f = 0;  // the first entry with this mask
+        while (f < l && f < kTermMemo && m0[f] != m) ++f;
+        bool const again = f < l && f < kTermMemo;
+        double2 inner = make_double2(0, 0);
+        int32_t cnt = 0;
+        if (again) {
+          inner = memo[f];
+          cnt = memo_n[f];
+        } else {
+          Acc rs(kahan);
+          for (int64_t r = 0; r < n1; ++r) {
+            if ((m & m1[r]) != 0u) continue;
+            rs.add(x1[r * s1]);
+            ++cnt;
+          }
+          inner = rs.value();
+          if (l < kTermMemo) {
+            memo[l] = inner;
+            memo_n[l] = cnt;
+          }
         }
-        result.add(cmul(x0[l * s0], rs.value()));
+        num += cnt;
+        result.add(cmul(x0[l * s0], inner));
       }
     } else {
       TraceList const L2 = lists[t.list[2]];

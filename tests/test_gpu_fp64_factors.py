@@ -1,7 +1,8 @@
 """FP64 factors, traces and terms at matrix sizes below and between those of the
 other tests (4 dilE = 4, 12, 16, 20, 24, 64): several trace entries per warp, row
 tiles across Dirac blocks, shared Q1 products; against the oracle, with both
-accumulators."""
+accumulators.  Seven random vectors make traces of 42 entries, more than the
+terms keep inner sums for."""
 from __future__ import annotations
 
 import numpy as np
@@ -11,15 +12,16 @@ from conftest import corr_rel_err, og, workload_inputs
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("dilE,nev", [(1, 7), (3, 13), (4, 17), (5, 16), (6, 33), (16, 35)])
-def test_pion_rho_set_matches_oracle(engine_lib, oracle_lib, tmp_path, dilE, nev):
+@pytest.mark.parametrize("dilE,nev,n_rnd", [(1, 7, 4), (3, 13, 4), (4, 17, 4), (5, 16, 4),
+                                            (6, 33, 4), (16, 35, 4), (1, 7, 7)])
+def test_pion_rho_set_matches_oracle(engine_lib, oracle_lib, tmp_path, dilE, nev, n_rnd):
     from slaph_gb300 import GlobalData, synthetic
     from slaph_gb300.engine import Engine
     ops = [o.replace("p0,1,2,3,4", "p0") for o in synthetic.PION_RHO_OPERATORS]
     corr = (["C2c:Q0:Op9:Q0:Op9:P0"]
             + [f"C3c:Q0:Op9:Q0:Op{k}:Q0:Op9:P0" for k in range(9)]
             + ["C4cD:Q0:Op9:Q0:Op9:Q0:Op9:Q0:Op9:P0", "C20:Q0:Op1:Q0:Op1:P0"])
-    w = synthetic.Workload("fp64_factors", Lt=4, L=4, nev=nev, n_rnd=4, dilT=2, dilE=dilE,
+    w = synthetic.Workload("fp64_factors", Lt=4, L=4, nev=nev, n_rnd=n_rnd, dilT=2, dilE=dilE,
                            operators=ops, correlators=corr, seed=70 + dilE)
     gd = GlobalData.from_infile(w.write_infile(str(tmp_path)))
     V, peram, noise = workload_inputs(w)
