@@ -998,12 +998,15 @@ void Engine::prepare_product_tc(DeviceSchedule &ds) {
   SLAPH_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
   size_t need = 0;
   int64_t max_expo = 0;
+  if (s.n_factor_slots + s.max_prod_slots >= 1LL << 29)
+    throw UnsupportedError("more than 2^29 matrix slots");
   for (size_t wi = 0; wi < s.waves.size(); ++wi) {
     Wave const &w = s.waves[wi];
     auto &wb = *ds.waves[wi];
     std::vector<dev::ProdGroup> groups;
     std::vector<int32_t> r_slots, u_list, out_tab;
     std::vector<dev::ProdTile> tiles;
+    std::vector<uint8_t> const need_w = product_layouts(s, w);
     wb.p_levels.clear();
     for (size_t lv = 0; lv + 1 < w.prod_level_off.size(); ++lv) {
       int64_t const b = w.prod_level_off[lv], e = w.prod_level_off[lv + 1];
@@ -1015,7 +1018,8 @@ void Engine::prepare_product_tc(DeviceSchedule &ds) {
       r_slots.insert(r_slots.end(), pp.r_slots.begin(), pp.r_slots.end());
       int32_t const u_base = static_cast<int32_t>(u_list.size());
       u_list.insert(u_list.end(), pp.u_list.begin(), pp.u_list.end());
-      out_tab.insert(out_tab.end(), pp.out_tab.begin(), pp.out_tab.end());
+      for (int32_t slot : pp.out_tab)
+        out_tab.push_back(slot < 0 ? -1 : slot << 2 | need_w[slot - s.n_factor_slots]);
       // Right matrices per unit of work: six units per SM, so that the last ones
       // end together; at least four, for which the A operand is copied once.
       int64_t steps = 0;

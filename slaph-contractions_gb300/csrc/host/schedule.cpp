@@ -815,6 +815,33 @@ std::vector<uint8_t> factor_layouts(Schedule const &s, bool tc_products) {
   return need;
 }
 
+std::vector<uint8_t> product_layouts(Schedule const &s, Wave const &w) {
+  int64_t const n = s.n_factor_slots;
+  std::vector<uint8_t> need(w.n_prod_slots, 0);
+  for (auto const &p : w.prods) {
+    if (p.a >= n) need[p.a - n] |= kNeedTransposed;
+    if (p.b >= n) need[p.b - n] |= kNeedStored;
+  }
+  // operand matrices of a shape's two sides
+  std::vector<std::pair<int32_t, int32_t>> sides(s.shapes.size(), {0, 0});
+  for (size_t k = 0; k < s.shapes.size(); ++k) {
+    for (int32_t i : s.shapes[k].i) sides[k].first = std::max(sides[k].first, i + 1);
+    for (int32_t j : s.shapes[k].j) sides[k].second = std::max(sides[k].second, j + 1);
+  }
+  // operands per first slot: the longest list that starts there
+  std::vector<int32_t> a(w.n_prod_slots, 0), b(w.n_prod_slots, 0);
+  for (int32_t k : w.unique_lists) {
+    auto const &l = w.lists[k];
+    if (l.a_base >= n) a[l.a_base - n] = std::max(a[l.a_base - n], sides[l.shape].first);
+    if (l.b_base >= n) b[l.b_base - n] = std::max(b[l.b_base - n], sides[l.shape].second);
+  }
+  for (int64_t q = 0; q < w.n_prod_slots; ++q) {
+    for (int32_t x = 0; x < a[q]; ++x) need.at(q + x) |= kNeedStored;
+    for (int32_t x = 0; x < b[q]; ++x) need.at(q + x) |= kNeedTransposed;
+  }
+  return need;
+}
+
 TraceGroupPlan plan_trace_group(TraceShape const &shape, int32_t n_a, int32_t n_b,
                                 int32_t tile_rows, int32_t tile_cols) {
   size_t const n_e = shape.i.size();

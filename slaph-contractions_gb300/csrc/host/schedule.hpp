@@ -198,12 +198,16 @@ struct ProductPlan {
 };
 ProductPlan plan_products(ProdInst const *prods, int64_t n, int32_t eds);
 
-// Layouts in which the factor slots are read, over all waves: as stored (kNeedStored) by the A side of
-// the traces and the right side of the products, transposed (kNeedTransposed)
+// Layouts in which the factor slots are read, over all waves: as stored
+// (kNeedStored) by the A side of the traces and the right side of the products,
+// transposed (kNeedTransposed)
 // by the B side of the traces and the left side of the tensor-core products
 // (both sides of other products read the stored one).
 constexpr uint8_t kNeedStored = 1, kNeedTransposed = 2;
 std::vector<uint8_t> factor_layouts(Schedule const &s, bool tc_products);
+// The same for the product slots of a wave (from n_factor_slots on) whose products
+// run on the tensor cores.
+std::vector<uint8_t> product_layouts(Schedule const &s, Wave const &w);
 
 // Builds the schedule; throws EmptyError with the reference's messages when a
 // random-vector combination is empty.  single_block_pair >= 0 restricts the

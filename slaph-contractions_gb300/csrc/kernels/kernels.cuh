@@ -226,8 +226,10 @@ cudaError_t products_df(float4 *slots_n, float4 *slots_t, ProdInst const *p, int
 // (not in the slots).  The products of one dependency level come in groups of up
 // to 64 / P left matrices (slots l[0..n_l)) with the union of their right matrices:
 // column block u of group g is right matrix u_list[g.u_off + u] (an index into
-// the level's r_slots) and out_tab[4 (g.u_off + u) + l] is the slot of product
-// l x u, or -1 when the level does not ask for it.  Tiles: (group, n tile of
+// the level's r_slots) and out_tab[4 (g.u_off + u) + l] is four times the slot of
+// product l x u plus the layouts in which it is read (1 natural, 2 transposed; for
+// eds = 64 both are written all the same), or -1 when the level does not ask for
+// it.  Tiles: (group, n tile of
 // 80 columns).  Scratch: the groups' A regions (prod_tc_a_bytes each) from 0,
 // the right-matrix streams (prod_tc_r_bytes each) from r_off; exponents: 64
 // per group from 0, eds per right matrix from r_expo.  slot_bits (as

@@ -10,7 +10,7 @@
 //   D(group row (l, i), column (u, j)) = sum_k L_l(i, k) R_u(k, j)
 // gives every product of the group; the epilogue keeps the entries of the
 // pairs the level asks for and writes them as double-float matrices into the
-// product slots, in the natural and the transposed layout, together with the
+// product slots, in the natural or the transposed layout or both, together with the
 // largest entry of every slot (for the slicing of the trace operands).
 //
 // Operands, in the split-BF16 scheme of tc_common.cuh: A rows are the rows of
@@ -31,7 +31,9 @@
 // straight pass (there is one chunk, so no running sums), two accumulator sets
 // let the next step's MMAs run meanwhile, a right matrix is one bulk copy, and
 // pairs that the level does not ask for are skipped.  24^3x48 Nev 120: 9.8 ->
-// 3.8 ms.  eds = 64 does not fit (A alone is 192 KB) and keeps the general
+// 3.8 ms.  Then the stores bound it: a product is written in the layouts in which
+// it is read only, its transposed rows in whole sectors: 3.3 ms (one block pair of
+// 64 timeslices 3.8 -> 2.8).  eds = 64 does not fit (A alone is 192 KB) and keeps the general
 // tile, whose producer gathers the B stage with one copy per (slice, matrix).
 #include <cuda_runtime.h>
 
@@ -267,7 +269,7 @@ struct ProdEpilogue {
     auto meta = [&](int c, int &slot, int &ec) {
       if (c >= ncols) return;
       int const u = c / eds;
-      slot = out_tab[4 * (gr.u_off + u) + l];
+      slot = out_tab[4 * (gr.u_off + u) + l] >> 2;  // both layouts are written
       ec = expo[r_expo + static_cast<int64_t>(tl.u_list[gr.u_off + u]) * eds + c % eds];
     };
     meta(p.cbase + lane, p.slot0, p.ec0);
@@ -333,6 +335,14 @@ constexpr uint32_t kStepTmem = 256;  // columns per accumulator set (6 kPad used
 __host__ __device__ inline uint32_t step_a_bytes(int pad) { return pad / 16 * kStageA; }
 __host__ __device__ inline uint32_t step_smem(int pad) {
   return step_a_bytes(pad) + kStepStages * 24u * pad * pad;
+}
+
+// Two float4 at a 32-byte boundary in one store (a full sector).
+__device__ __forceinline__ void store_pair(float4 *p, float4 const (&v)[2]) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0].x),
+               "f"(v[0].y), "f"(v[0].z), "f"(v[0].w), "f"(v[1].x), "f"(v[1].y), "f"(v[1].z),
+               "f"(v[1].w)
+               : "memory");
 }
 
 struct StepArgs {
@@ -495,7 +505,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) product_step_kernel(StepArgs 
       int ec_next = column_expo(0);
       for (int s = 0; s < t.n; ++s, ++n_s) {
         uint32_t const set = n_s % 2;
-        int const slot = __shfl_sync(0xffffffffu, slots, s);
+        int const entry = __shfl_sync(0xffffffffu, slots, s), slot = entry >> 2;
         int const ec_lane = ec_next;
         if (s + 1 < t.n) ec_next = column_expo(s + 1);
         if (!__all_sync(0xffffffffu, mbar_wait(&acc_full[set], (n_s / 2) & 1, g.err, 5))) {
@@ -521,30 +531,40 @@ __global__ void __launch_bounds__(kStepThreads, 1) product_step_kernel(StepArgs 
         unsigned int mx = 0;
         float4 *const dst = (row & 1) ? g.slots_t + slot * ms + static_cast<int64_t>(eds) * ri
                                       : g.slots_n + slot * ms + ri;
+        bool const store = row_on && (entry & ((row & 1) ? 2 : 1)) != 0;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          // the chunk's value in (hi, lo), as in tc_common.cuh
-          float s1, x1, s2, x2, s3, x3;
-          two_sum(__uint_as_float(r0[0][u]), __uint_as_float(r0[1][u]) * 0x1p-8f, s1, x1);
-          two_sum(s1, __uint_as_float(r0[2][u]) * 0x1p-16f, s2, x2);
-          float const low = fmaf(__uint_as_float(r1[2][u]), 0x1p-16f,
-                                 fmaf(__uint_as_float(r1[1][u]), 0x1p-8f,
-                                      __uint_as_float(r1[0][u]))) *
-                            0x1p-24f;
-          two_sum(s2, low, s3, x3);
-          float const e = (x1 + x2) + x3;
-          float const hi = s3 + e, lo = e - (hi - s3);
-          int const sh = max(er + __shfl_sync(0xffffffffu, ec_lane, u) - 14, -252);
-          float const h = scale2(hi, sh), lw = scale2(lo, sh);
-          float const oh = __shfl_xor_sync(0xffffffffu, h, 1);
-          float const ol = __shfl_xor_sync(0xffffffffu, lw, 1);
+        for (int u = 0; u < 8; u += 2) {
+          float4 out[2];
+#pragma unroll
+          for (int y = 0; y < 2; ++y) {
+            // the chunk's value in (hi, lo), as in tc_common.cuh
+            float s1, x1, s2, x2, s3, x3;
+            scaled_sum(__uint_as_float(r0[0][u + y]), __uint_as_float(r0[1][u + y]), 0x1p-8f, s1,
+                       x1);
+            scaled_sum(s1, __uint_as_float(r0[2][u + y]), 0x1p-16f, s2, x2);
+            float const low = fmaf(__uint_as_float(r1[2][u + y]), 0x1p-16f,
+                                   fmaf(__uint_as_float(r1[1][u + y]), 0x1p-8f,
+                                        __uint_as_float(r1[0][u + y])));
+            scaled_sum(s2, low, 0x1p-24f, s3, x3);
+            float const e = (x1 + x2) + x3;
+            float const hi = s3 + e, lo = e - (hi - s3);
+            int const sh = max(er + __shfl_sync(0xffffffffu, ec_lane, u + y) - 14, -252);
+            float const h = scale2(hi, sh), lw = scale2(lo, sh);
+            float const oh = __shfl_xor_sync(0xffffffffu, h, 1);
+            float const ol = __shfl_xor_sync(0xffffffffu, lw, 1);
+            if (row_on && 8 * blk + u < eds) mx = max(mx, __float_as_uint(h) & 0x7FFFFFFFu);
+            out[y] = (row & 1) ? make_float4(oh, ol, h, lw) : make_float4(h, lw, oh, ol);
+          }
+          // the even lane of a row pair (Re) stores the natural layout, the odd one
+          // (Im) the transposed, two entries of its row at once
           int const j = 8 * blk + u;
-          if (row_on && j < eds) {
-            mx = max(mx, __float_as_uint(h) & 0x7FFFFFFFu);
-            // the even lane of a row pair (Re) stores the natural layout, the odd
-            // one (Im) the transposed
-            dst[(row & 1) ? j : eds * j] = (row & 1) ? make_float4(oh, ol, h, lw)
-                                                     : make_float4(h, lw, oh, ol);
+          if (store && j < eds) {
+            if (row & 1) {
+              store_pair(dst + j, out);
+            } else {
+              dst[eds * j] = out[0];
+              dst[eds * (j + 1)] = out[1];
+            }
           }
         }
         mx = __reduce_max_sync(0xffffffffu, mx);
