@@ -116,9 +116,11 @@ __global__ void __launch_bounds__(32)
 // by warp shuffles (the second row is the first with its halves swapped and one
 // sign flipped), so that every slice store of a warp, A or B, fills whole
 // 128-byte core matrices (512 contiguous bytes).  Bound by HBM: 16 bytes read,
-// 48 (A) and 24 per family (B) written per entry.
+// 48 (A) and 24 per family (B) written per entry.  With A, four CTAs per SM (64
+// registers instead of 80) run at 5.9 TB/s, three at 5.6 (32^3x64 Nev 220: 31.6 ms
+// and 33.2).
 template <bool kA, bool kB>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, kA ? 4 : 1)
     slice_kernel(uint8_t *a_out, uint8_t *b_out, size_t slot_bytes, double2 const *V,
                  longlong2 const *phase_fx, int32_t n_fam, uint8_t const *expos, int32_t n_planes,
                  int32_t per, int64_t col0, Geometry g) {
