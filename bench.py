@@ -40,14 +40,36 @@ METRIC = "s/gauge-config, VdaggerV+pipi contractions 32³×64: FP64 vs split-pre
 UNIT = "s/gauge-config"
 
 # DRAM bytes (read + write) of the tensor-core GEMMs per unit of work, from
-# one-pass ncu captures (dram__bytes_read.sum + dram__bytes_write.sum) of the
-# full-size 32^3x64 launches; the captures and the derivation are in the
+# one-pass ncu captures (dram__bytes_read.sum + dram__bytes_write.sum) of
+# launches with the 32^3x64 shapes; the captures and the derivation are in the
 # profile summary named here.  Other workloads have no capture: their
 # roofline's traffic is null.
-NCU_TRACE_GEMM_DRAM_BYTES_PER_ENTRY = {"cfg3_32x64_pipi": 470.0}  # per dense-group entry
+NCU_TRACE_GEMM_DRAM_BYTES_PER_ENTRY = {"cfg3_32x64_pipi": 256.0}  # per dense-group entry
 NCU_TRACE_GEMM_TRAFFIC_SOURCE = "profiles/gemm_dram_traffic_cfg3_32x64_pipi.md"
-NCU_VDV_GEMM_DRAM_BYTES_PER_UNIT = {"cfg3_32x64_pipi": 0.867e9}  # per (operator, timeslice)
+NCU_VDV_GEMM_DRAM_BYTES_PER_TIMESLICE = {"cfg3_32x64_pipi": 5.78e9}
 NCU_VDV_GEMM_TRAFFIC_SOURCE = "profiles/gemm_dram_traffic_cfg3_32x64_pipi.md"
+
+
+def vdaggerv_gemm_flops(gd, w):
+    """FP64-equivalent flops of the plane sums that the split-precision VdaggerV
+    GEMM computes: 8 nev^2 3L^3 per family and timeslice.  A family is up to eight
+    momenta that share +-(py, pz) (half the entries for (0, 0), whose sums are
+    Hermitian), or one displaced operator; the operators are Fourier sums over the
+    planes, which the GEMM does not pay for."""
+    classes, displaced = {}, 0
+    for i in range(gd.plan.n_vdv_ops):
+        op = gd.plan.vdv_ops[i]
+        if i == gd.plan.index_of_unity:
+            continue
+        if op.n_disp > 0:
+            displaced += 1
+            continue
+        p = (op.momentum[1], op.momentum[2])
+        p = max(p, (-p[0], -p[1]))
+        classes[p] = classes.get(p, 0) + 1
+    units = displaced + sum(-(-n // 8) * (0.5 if p == (0, 0) else 1.0)
+                            for p, n in classes.items())
+    return w.flops_vdaggerv(units)
 
 
 def per_correlator_rel_err(out, ref):
@@ -441,9 +463,9 @@ def run_engine(args):
                   ktim[6] / K,
                   "ozaki_gemm_kernel (VdaggerV GEMM)": ktim[11] / K,
                   "vdaggerv stage (slicing + ozaki_gemm_kernel)" if precision == 1
-                  else "vdaggerv stage (vdv_fp64_kernel)": stage_ms[0],
+                  else "vdaggerv stage (vdv_family_kernel)": stage_ms[0],
                   "factor stage (q*_kernels, factor GEMMs)": stage_ms[1],
-                  "factor products (slicing + product_gemm_kernel)" if precision == 1
+                  "factor products (slicing + product_step_kernel)" if precision == 1
                   else "factor products (product_kernel)": ktim[14] / K}
     # Roofline candidates, one kernel each: (time per step in ms, roofline).
     cands = []
@@ -464,7 +486,7 @@ def run_engine(args):
             "fp64_equivalent_tflops": 8.0 * eds * eds * stats[7] / (ktim[8] / K / 1e3) / 1e12,
             "work": "21 split-BF16 products x 8 (4dilE)^2 flops per dense-group trace entry"}))
     if precision == 1 and ktim[11] > 0:
-        flops = 21 * vdv_flops  # 21 slice pairs of the real form of every (op, t) product
+        flops = 21 * vdaggerv_gemm_flops(gd, w)  # 21 slice pairs of every plane sum
         n_l = ktim[12] / K
         cands.append((ktim[11] / K, {
             "kernel": "ozaki_gemm_kernel", "bound": "tensor",
@@ -472,11 +494,12 @@ def run_engine(args):
             "unit": "TFLOP/s", "peak_source": f"{peak_src} ({note})",
             "launches_per_step": n_l, "launch_ms_avg": ktim[11] / K / n_l,
             "algorithmic_per_launch": flops / n_l,
-            "traffic": (NCU_VDV_GEMM_DRAM_BYTES_PER_UNIT.get(args.workload, 0)
-                        * n_ops * w.Lt / n_l) or None,
+            "traffic": (NCU_VDV_GEMM_DRAM_BYTES_PER_TIMESLICE.get(args.workload, 0)
+                        * w.Lt / n_l) or None,
             "traffic_source": NCU_VDV_GEMM_TRAFFIC_SOURCE,
             "fp64_equivalent_tflops": vdv_flops / (ktim[11] / K / 1e3) / 1e12,
-            "work": "21 split-BF16 products x 8 nev^2 3L^3 flops per (operator, timeslice)"}))
+            "work": ("21 split-BF16 products x 8 nev^2 3L^3 flops per (momentum family, "
+                     "timeslice), half for the Hermitian family")}))
     ms_dom, roofline = max(cands, key=lambda c: c[0]) if cands else (0.0, {})
     if roofline:
         roofline["frac"] = roofline["achieved"] / roofline["peak"]
