@@ -265,7 +265,10 @@ void Engine::set_operators(slaph_vdv_op const *ops, int32_t n, int32_t index_of_
   launch(dev::phase_fixed(phase_fx_.as<longlong2>(), phase.as<double2>(), n_ph, stream_),
          "phase_fixed");
   launch(dev::unit_roots(roots_.as<double2>(), pl.n_planes, stream_), "unit_roots");
-  std::vector<int2> const mn = dev::vdaggerv_tc_tiles(fam, dims_.nev);
+  int sms = 0;
+  SLAPH_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
+  std::vector<int2> const mn = dev::vdaggerv_tc_tiles(fam, pl.n_mom, dims_.nev, pl.n_planes,
+                                                      std::max(sms, 1), pl.cols);
   upload(mn_dev_, mn, stream_);
   pl.n_mn = static_cast<int32_t>(mn.size());
   pl.fam = fam_dev_.as<dev::VdvFamily>();

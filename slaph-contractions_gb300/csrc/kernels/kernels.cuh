@@ -116,8 +116,45 @@ cudaError_t vdaggerv_fp64(double2 *vdv, double2 const *V, VdvFamily const *fam, 
 // constant x, or the whole lattice where those are too small) of the momentum
 // operators, then one family per displaced operator; all pointers are device
 // memory kept by the caller.
+// Columns of B.  The rows of an M tile are 64 eigenvectors; where the last tile
+// would hold few, its rows i >= full of the phase families come from edge columns
+// instead: sum_x V_i conj(phase) conj(V_j) is conj(G(i, j)), with V_i as a column and
+// the rows j < full.  Order: (f, j < full) family by family, (f, j >= full), then the
+// edge columns (f, i) of the families n_lead <= f < n_mom (those before are
+// Hermitian).  full = nev: no edge columns, the plain order f nev + j.
+struct VdvColumns {
+  int32_t nev, n_fam, n_mom, n_lead, full;
+  __host__ __device__ int64_t n_cols() const { return static_cast<int64_t>(n_fam) * nev; }
+  __host__ __device__ int64_t n_all() const {
+    return n_cols() + static_cast<int64_t>(n_mom - n_lead) * (nev - full);
+  }
+  __host__ __device__ int64_t pos(int32_t f, int32_t j) const {
+    return j < full ? static_cast<int64_t>(f) * full + j
+                    : static_cast<int64_t>(n_fam) * full +
+                          static_cast<int64_t>(f) * (nev - full) + (j - full);
+  }
+  __host__ __device__ int64_t edge(int32_t f, int32_t i) const {
+    return n_cols() + static_cast<int64_t>(f - n_lead) * (nev - full) + (i - full);
+  }
+  __host__ __device__ bool phase(int32_t f) const { return f >= n_lead && f < n_mom; }
+  // Column c < n_all(): family and eigenvector; true for an edge column.
+  __host__ __device__ bool decode(int64_t c, int32_t &f, int32_t &j) const {
+    int64_t const inner = static_cast<int64_t>(n_fam) * full;
+    if (c < inner) {
+      f = static_cast<int32_t>(c / full);
+      j = static_cast<int32_t>(c % full);
+      return false;
+    }
+    bool const e = c >= n_cols();
+    int64_t const q = c - (e ? n_cols() : inner);
+    f = static_cast<int32_t>(q / (nev - full)) + (e ? n_lead : 0);
+    j = static_cast<int32_t>(q % (nev - full)) + full;
+    return e;
+  }
+};
 struct VdvTcPlan {
   int32_t n_fam, n_mom;           // families; those of momentum operators come first
+  VdvColumns cols;
   int32_t n_planes, per;          // planes, lattice entries (3 x sites) of each
   VdvFamily const *fam;           // [n_fam]
   longlong2 const *phase_fx;      // [n_fam][per / 3]: the families' phases x 2^62
@@ -125,9 +162,12 @@ struct VdvTcPlan {
   int2 const *mn;                 // GEMM tiles (m, n) of one plane
   int32_t n_mn;
 };
-// The (m, n) tiles of one plane: all but those of Hermitian families below the
-// diagonal.
-std::vector<int2> vdaggerv_tc_tiles(std::vector<VdvFamily> const &fam, int32_t nev);
+// The columns and (m, n) tiles of one plane, without the tiles of which no entry is
+// wanted (below the diagonal of Hermitian families; the last M tile where edge
+// columns stand in for it).  Edge columns are taken where they cost less.
+std::vector<int2> vdaggerv_tc_tiles(std::vector<VdvFamily> const &fam, int32_t n_mom,
+                                    int32_t nev, int32_t n_planes, int32_t sm_count,
+                                    VdvColumns &cols);
 // Scratch for `batch` timeslices per GEMM launch.
 size_t vdaggerv_tc_scratch_bytes(Geometry g, VdvTcPlan const &pl, int32_t batch);
 // phase_fx[k] = round(phase[k] 2^62) per component, the fixed-point phases the

@@ -102,8 +102,10 @@ __global__ void __launch_bounds__(32)
 }
 
 // Slices of timeslice blockIdx.y (slots at slot_bytes).  kA: the A slices of V, [m_tile][K tile][slice][kTM x
-// kTK]; kB: the B slices of phase_f V for n_fam families at B columns
-// col0 + f nev + j, [n_tile][K tile][slice][kTN x kTK].
+// kTK]; kB: the B slices of phase_f V for the families f0 .. f0 + n_fam - 1 at their
+// columns (VdvColumns), [n_tile][K tile][slice][kTN x kTK]; kEdge: their edge columns,
+// of the eigenvectors from cols.full on with the conjugate phase (a launch of its own:
+// as a second pass of the loop over families it slowed every launch by a tenth).
 //
 // A warp covers eight eigenvectors in one K tile: lane (r, kg) = (lane % 8,
 // lane / 8) takes eigenvector 8 rg + r and the 4 complex K entries 4 kg .. 4 kg
@@ -119,11 +121,11 @@ __global__ void __launch_bounds__(32)
 // 48 (A) and 24 per family (B) written per entry.  With A, four CTAs per SM (64
 // registers instead of 80) run at 5.9 TB/s, three at 5.6 (32^3x64 Nev 220: 31.6 ms
 // and 33.2).
-template <bool kA, bool kB>
+template <bool kA, bool kB, bool kEdge>
 __global__ void __launch_bounds__(256, kA ? 4 : 1)
     slice_kernel(uint8_t *a_out, uint8_t *b_out, size_t slot_bytes, double2 const *V,
                  longlong2 const *phase_fx, int32_t n_fam, uint8_t const *expos, int32_t n_planes,
-                 int32_t per, int64_t col0, Geometry g) {
+                 int32_t per, VdvColumns cols, int32_t f0, Geometry g) {
   a_out += blockIdx.y * slot_bytes;
   b_out += blockIdx.y * slot_bytes;
   int32_t const *expo = reinterpret_cast<int32_t const *>(expos + blockIdx.y * slot_bytes);
@@ -132,10 +134,11 @@ __global__ void __launch_bounds__(256, kA ? 4 : 1)
   int const lane = threadIdx.x % 32;
   int32_t const ktp = plane_k_tiles(per);
   int64_t const k_tiles = static_cast<int64_t>(ktp) * n_planes;
-  int64_t const groups = (g.nev + 7) / 8;
+  int const first = kEdge ? cols.full / 8 : 0;  // group of eight eigenvectors
+  int64_t const groups = (g.nev + 7) / 8 - first;
   if (wid >= groups * k_tiles) return;
   int64_t const kt = wid / groups;
-  int const rg = static_cast<int>(wid % groups);
+  int const rg = first + static_cast<int>(wid % groups);
   int const r = lane % 8, kg = lane / 8;
   int const j = rg * 8 + r;
   bool const row_ok = j < g.nev;
@@ -192,12 +195,16 @@ __global__ void __launch_bounds__(256, kA ? 4 : 1)
       vi[q] *= 4;
     }
     int32_t const sites = per / 3;
-    for (int f = 0; f < n_fam; ++f) {
+    // columns of eigenvector j, family after family (below 2^31)
+    uint32_t gc = static_cast<uint32_t>(kEdge ? cols.edge(f0, j) : cols.pos(f0, j));
+    uint32_t const gstep = kEdge || j >= cols.full ? g.nev - cols.full : cols.full;
+    for (int f = 0; f < n_fam; ++f, gc += gstep) {
       longlong2 const *ph = phase_fx + static_cast<int64_t>(f) * sites;
       uint32_t w[kSlices][4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        longlong2 const p = ph[site[q]];
+        longlong2 p = ph[site[q]];
+        if (kEdge) p.y = -p.y;
         long long const wr = __mul64hi(vr[q], p.x) - __mul64hi(vi[q], p.y);
         long long const wi = __mul64hi(vr[q], p.y) + __mul64hi(vi[q], p.x);
         float dre[kSlices], dim[kSlices];
@@ -206,7 +213,6 @@ __global__ void __launch_bounds__(256, kA ? 4 : 1)
 #pragma unroll
         for (int s = 0; s < kSlices; ++s) w[s][q] = bf16x2(dre[s], dim[s]);
       }
-      int64_t const gc = col0 + static_cast<int64_t>(f) * g.nev + j;
       int64_t const nt = gc / kTN;
       int const rr = static_cast<int>(gc % kTN);
       uint8_t *dst =
@@ -269,15 +275,16 @@ struct VdvTiles {
 };
 
 // Epilogue of one tile: D = (hi + lo) 2^(e_i + f_c - 14), rows (2i, 2i+1) =
-// (Re, Im) of the plane sum G(i, j) of family f for the tile's B columns c = f
-// nev + j, written to sums[(plane n_cols + c) nev + i] of the slot; e: exponents
-// of the eigenvectors (A rows), f: those of the B columns (the eigenvectors'
-// for momentum families, |phase| = 1; those of D(V) for the displaced ones, f >=
-// n_mom, at (1 + f) nev).  A warp stores 16 consecutive i of a column: 256 bytes.
+// (Re, Im) of the plane sum G(i, j) of family f for the tile's B columns c = (f, j),
+// written to sums[((plane n_fam + f) nev + j) nev + i] of the slot, of an edge column
+// (f, k) conjugated to entry (k, i); e: exponents of the eigenvectors (A rows), f:
+// those of the B columns (the eigenvectors' for momentum families, |phase| = 1; those
+// of D(V) for the displaced ones, f >= n_mom, at (1 + f) nev).  A warp stores 16
+// consecutive i of a column: 256 bytes.
 struct VdvEpilogue {
   VdvTiles tl;
   size_t s_off;
-  int nev, n_mom, n_cols;
+  VdvColumns cols;
   struct Pre {};
   __device__ __forceinline__ Pre prepare(int, int, int) const { return Pre{}; }
   __device__ __forceinline__ void operator()(Pre const &, int it, int row, int col0,
@@ -285,27 +292,42 @@ struct VdvEpilogue {
                                              float const (&lo)[kColsW]) const {
     int mt, nt, plane, slot;
     tl.decode(it, mt, nt, plane, slot);
+    int const nev = cols.nev, lane = threadIdx.x % 32;
     int const i = mt * (kTM / 2) + row / 2;
-    if (i >= nev) return;
     uint8_t const *sbase = tl.scratch + slot * tl.slot_bytes;
     int32_t const *expo = reinterpret_cast<int32_t const *>(sbase + tl.e_off);
     double *sums = reinterpret_cast<double *>(const_cast<uint8_t *>(sbase) + s_off) +
-                   2 * static_cast<int64_t>(plane) * n_cols * nev + 2 * i + (row & 1);
-    int const ei = expo[i];
-    int const c0 = nt * kTN + col0;
-    int f = c0 / nev, j = c0 - f * nev - 1;
+                   2 * static_cast<int64_t>(plane) * cols.n_cols() * nev + (row & 1);
+    int const ei = i < nev ? expo[i] : 0;
+    // Lane k looks up the warp's columns k and 32 + k; the column loop takes them by
+    // warp shuffles.  at: offset of the entry for i = 0; kind: 1 wanted, 2 edge, 4 only
+    // for i < full (what edge columns, or the columns they stand in for, hold beyond
+    // belongs to other columns).
+    int64_t at[2];
+    int ex[2], kind[2];
 #pragma unroll
-    for (int jj = 0; jj < kColsW; ++jj) {
-      int const c = c0 + jj;
-      if (++j == nev) {
-        j = 0;
-        ++f;
-      }
-      if (c < n_cols) {
-        int const ec = f < n_mom ? expo[j] : expo[(1 + f) * nev + j];
-        sums[2 * static_cast<int64_t>(c) * nev] =
-            df_scaled(hi[jj], lo[jj], ei + ec - 14);
-      }
+    for (int h = 0; h < 2; ++h) {
+      int64_t const c = static_cast<int64_t>(nt) * kTN + col0 + 32 * h + lane;
+      at[h] = 0;
+      ex[h] = kind[h] = 0;
+      if (32 * h + lane >= kColsW || c >= cols.n_all()) continue;
+      int32_t f, j;
+      bool const edge = cols.decode(c, f, j);
+      at[h] = (static_cast<int64_t>(f) * nev + (edge ? 0 : j)) * nev + (edge ? j : 0);
+      ex[h] = f < cols.n_mom ? expo[j] : expo[(1 + f) * nev + j];
+      kind[h] = 1 | (edge ? 2 : 0) | (edge || (j < cols.full && cols.phase(f)) ? 4 : 0);
+    }
+#pragma unroll
+    for (int c = 0; c < kColsW; ++c) {
+      int const ec = __shfl_sync(0xffffffffu, ex[c / 32], c % 32);
+      int const kd = __shfl_sync(0xffffffffu, kind[c / 32], c % 32);
+      int64_t const a = __shfl_sync(0xffffffffu, at[c / 32], c % 32);
+      if (!(kd & 1) || i >= ((kd & 4) ? cols.full : nev)) continue;
+      double const v = df_scaled(hi[c], lo[c], ei + ec - 14);
+      if (kd & 2)
+        sums[2 * (a + static_cast<int64_t>(i) * nev)] = (row & 1) ? -v : v;
+      else
+        sums[2 * (a + i)] = v;
     }
   }
 };
@@ -313,10 +335,9 @@ struct VdvEpilogue {
 // The GEMM: n_mn x n_planes x batch tiles over persistent CTAs, kThreads
 // threads each.
 __global__ void __launch_bounds__(kThreads, 1)
-    ozaki_gemm_kernel(VdvTiles tl, int32_t n_tiles, size_t s_off, int32_t n_cols, int32_t n_mom,
-                      Geometry g, int *err) {
+    ozaki_gemm_kernel(VdvTiles tl, int32_t n_tiles, size_t s_off, VdvColumns cols, int *err) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  VdvEpilogue epi{tl, s_off, g.nev, n_mom, n_cols};
+  VdvEpilogue epi{tl, s_off, cols};
   ozaki_tiles(smem, n_tiles, tl.k_tiles, tl, err, epi);
 }
 
@@ -427,8 +448,8 @@ TcLayout tc_layout(Geometry const &g, VdvTcPlan const &pl) {
   L.ktp = plane_k_tiles(pl.per);
   L.k_tiles = static_cast<int64_t>(L.ktp) * pl.n_planes;
   int64_t const m_tiles = (2LL * g.nev + kTM - 1) / kTM;
-  L.n_cols = static_cast<int64_t>(pl.n_fam) * g.nev;
-  int64_t const n_tiles = (L.n_cols + kTN - 1) / kTN;
+  L.n_cols = pl.cols.n_cols();
+  int64_t const n_tiles = (pl.cols.n_all() + kTN - 1) / kTN;
   L.a_bytes = static_cast<size_t>(m_tiles * L.k_tiles) * kStageA;
   L.s_off = L.a_bytes + static_cast<size_t>(n_tiles * L.k_tiles) * kStageB;
   L.e_off = L.s_off + static_cast<size_t>(pl.n_planes * L.n_cols * g.nev) * sizeof(double2);
@@ -441,18 +462,50 @@ TcLayout tc_layout(Geometry const &g, VdvTcPlan const &pl) {
 
 }  // namespace
 
-std::vector<int2> vdaggerv_tc_tiles(std::vector<VdvFamily> const &fam, int32_t nev) {
-  std::vector<int2> out;
-  int64_t const n_cols = static_cast<int64_t>(fam.size()) * nev;
-  for (int64_t nt = 0; nt * kTN < n_cols; ++nt)
-    for (int32_t mt = 0; mt * (kTM / 2) < nev; ++mt) {
-      // wanted: a column (f, j) of the tile with a full family or j >= the
-      // tile's first row
-      bool want = false;
-      for (int64_t c = nt * kTN; c < std::min<int64_t>(n_cols, (nt + 1) * kTN) && !want; ++c)
-        want = !fam[c / nev].herm || c % nev >= mt * (kTM / 2);
-      if (want) out.push_back(make_int2(mt, static_cast<int32_t>(nt)));
+std::vector<int2> vdaggerv_tc_tiles(std::vector<VdvFamily> const &fam, int32_t n_mom,
+                                    int32_t nev, int32_t n_planes, int32_t sm_count,
+                                    VdvColumns &cols) {
+  int32_t const rows = kTM / 2;
+  VdvColumns base{nev, static_cast<int32_t>(fam.size()), n_mom, 0, nev};
+  while (base.n_lead < n_mom && fam[base.n_lead].herm) ++base.n_lead;
+  auto tiles = [&](VdvColumns const &v) {
+    std::vector<int2> out;
+    for (int64_t nt = 0; nt * kTN < v.n_all(); ++nt)
+      for (int32_t mt = 0; mt * rows < nev; ++mt) {
+        // wanted: a column (f, j) of the tile with a full family or j >= the tile's
+        // first row, and for the rows i >= full none that an edge column stands in for
+        bool want = false, last = mt * rows >= v.full;
+        for (int64_t c = nt * kTN; c < std::min(v.n_all(), (nt + 1) * kTN) && !want; ++c) {
+          int32_t f, j;
+          if (v.decode(c, f, j))
+            want = !last;
+          else
+            want = fam[f].herm ? j >= mt * rows : !(last && j < v.full && v.phase(f));
+        }
+        if (want) out.push_back(make_int2(mt, static_cast<int32_t>(nt)));
+      }
+    return out;
+  };
+  cols = base;
+  std::vector<int2> out = tiles(base);
+  VdvColumns edge = base;
+  edge.full = nev / rows * rows;
+  if (edge.full > 0 && edge.full < nev && edge.n_all() > edge.n_cols()) {
+    // A k-tile of a round of tiles takes 1.3 us, that of one more column's slices
+    // 0.1 ns.  Rounds of one timeslice per launch, as streamed eigenvectors have them.
+    // 32^3x64 Nev 220, three families (56 columns more, 7 rounds -> 6): GEMM 98.9 ->
+    // 86.3 ms, slices 31.5 -> 34.3, pass 171.8 -> 162.2.  24^3x48 Nev 120 (112 more, 2 rounds
+    // either way): GEMM 10.0 -> 9.2 but slices 1.4 ms longer, so the plain columns stay.
+    std::vector<int2> const e = tiles(edge);
+    auto rounds = [&](std::vector<int2> const &t) {
+      return (static_cast<int64_t>(t.size()) * n_planes + sm_count - 1) / sm_count;
+    };
+    int64_t const more = (edge.n_all() - edge.n_cols()) * n_planes;
+    if (13000 * (rounds(out) - rounds(e)) > more) {
+      cols = edge;
+      out = e;
     }
+  }
   return out;
 }
 
@@ -505,7 +558,7 @@ cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, VdvTcPlan const &pl, int
       (n_disp > 0 && (!disp->n_steps || !disp->steps || !disp->U || !disp->W)))
     return cudaErrorInvalidValue;
   TcLayout const L = tc_layout(g, pl);
-  if (L.k_tiles > 0x7fffffffLL / kTK || L.n_cols > 0x7fffffffLL) return cudaErrorInvalidValue;
+  if (L.k_tiles > 0x7fffffffLL / kTK || pl.cols.n_all() > 0x7fffffffLL) return cudaErrorInvalidValue;
   int64_t batch = static_cast<int64_t>(scratch_bytes / L.slot_bytes);
   if (batch < 1) return cudaErrorInvalidValue;
   int64_t const per_t = static_cast<int64_t>(pl.n_mn) * pl.n_planes;
@@ -517,6 +570,8 @@ cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, VdvTcPlan const &pl, int
   if (e != cudaSuccess) return e;
   // one warp per (K tile, group of 8 eigenvectors)
   unsigned const sb = static_cast<unsigned>((L.k_tiles * ((g.nev + 7) / 8) * 32 + 255) / 256);
+  unsigned const eb = static_cast<unsigned>(
+      (L.k_tiles * ((g.nev + 7) / 8 - pl.cols.full / 8) * 32 + 255) / 256);
   unsigned const nc = static_cast<unsigned>((g.dim_row + kNormChunk - 1) / kNormChunk);
   size_t const links = static_cast<size_t>(g.dim_row / 3) * 27;  // of one timeslice
   int32_t const sites = pl.per / 3;
@@ -542,13 +597,18 @@ cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, VdvTcPlan const &pl, int
     expo_kernel<<<dim3(static_cast<unsigned>(g.nev), unb), 32, 0, stream>>>(
         base + L.n_off, base + L.e_off, L.slot_bytes, Vb, g);
     if (pl.n_mom > 0)
-      slice_kernel<true, true><<<dim3(sb, unb), 256, 0, stream>>>(
+      slice_kernel<true, true, false><<<dim3(sb, unb), 256, 0, stream>>>(
           base, base + L.a_bytes, L.slot_bytes, Vb, pl.phase_fx, pl.n_mom, base + L.e_off,
-          pl.n_planes, pl.per, 0, g);
+          pl.n_planes, pl.per, pl.cols, 0, g);
     else
-      slice_kernel<true, false><<<dim3(sb, unb), 256, 0, stream>>>(
+      slice_kernel<true, false, false><<<dim3(sb, unb), 256, 0, stream>>>(
           base, base + L.a_bytes, L.slot_bytes, Vb, nullptr, 0, base + L.e_off, pl.n_planes,
-          pl.per, 0, g);
+          pl.per, pl.cols, 0, g);
+    if (pl.cols.n_all() > pl.cols.n_cols())
+      slice_kernel<false, true, true><<<dim3(eb, unb), 256, 0, stream>>>(
+          nullptr, base + L.a_bytes, L.slot_bytes, Vb,
+          pl.phase_fx + static_cast<int64_t>(pl.cols.n_lead) * sites, pl.n_mom - pl.cols.n_lead,
+          base + L.e_off, pl.n_planes, pl.per, pl.cols, pl.cols.n_lead, g);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     // Displaced operators: B = D(V_t) with phase 1 and its own column exponents.
@@ -568,9 +628,9 @@ cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, VdvTcPlan const &pl, int
         uint8_t *expo_w = slot + L.e_off + static_cast<size_t>(1 + f) * g.nev * sizeof(int32_t);
         expo_kernel<<<dim3(static_cast<unsigned>(g.nev), 1), 32, 0, stream>>>(slot + L.n_off, expo_w,
                                                                           0, Wt, g);
-        slice_kernel<false, true><<<dim3(sb, 1), 256, 0, stream>>>(
+        slice_kernel<false, true, false><<<dim3(sb, 1), 256, 0, stream>>>(
             nullptr, slot + L.a_bytes, 0, Wt, pl.phase_fx + static_cast<int64_t>(f) * sites, 1,
-            expo_w, pl.n_planes, pl.per, static_cast<int64_t>(f) * g.nev, g);
+            expo_w, pl.n_planes, pl.per, pl.cols, f, g);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
       }
@@ -584,7 +644,7 @@ cudaError_t vdaggerv_tc(double2 *vdv, double2 const *V, VdvTcPlan const &pl, int
     int64_t const n_tiles = per_t * nb;
     ozaki_gemm_kernel<<<static_cast<unsigned>(persistent_grid(n_tiles)), kThreads, kSmemBytes,
                         stream>>>(tl, static_cast<int32_t>(n_tiles), L.s_off,
-                                  static_cast<int32_t>(L.n_cols), pl.n_mom, g, err);
+                                  pl.cols, err);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (timed) {

@@ -108,7 +108,9 @@ def test_families_reproduce_their_momenta(planner, L, p2, sheared, max_ops):
 @pytest.mark.parametrize("L,nev,p2", [
     ((4, 4, 4), 1, 4), ((4, 4, 4), 33, 9), ((3, 3, 3), 16, 2), ((5, 5, 5), 31, 5),
     ((7, 7, 7), 65, 3), ((6, 6, 6), 80, 4), ((9, 9, 9), 2, 1), ((4, 6, 5), 34, 3),
-    ((2, 8, 3), 20, 2), ((8, 2, 2), 11, 1), ((1, 9, 7), 17, 3), ((11, 11, 11), 97, 3)])
+    ((2, 8, 3), 20, 2), ((8, 2, 2), 11, 1), ((1, 9, 7), 17, 3), ((11, 11, 11), 97, 3),
+    # a last tile of few rows and enough tiles that edge columns save a round
+    ((40, 4, 4), 71, 4), ((60, 4, 5), 150, 3), ((48, 4, 4), 97, 1), ((33, 5, 4), 65, 9)])
 def test_build_matches_the_matrix_product(engine_lib, L, nev, p2, precision):
     from slaph_gb300 import _lib
     from slaph_gb300.engine import Engine
@@ -171,3 +173,41 @@ def test_split_precision_build_scales_exactly(engine_lib, shift):
         ref = V.conj() @ (np.exp(-2j * np.pi * (np.array(p) @ x) / L) * V).T
         # 47 bits of each row's scale per term, 192 terms
         assert np.max(np.abs(blocks[0][i] - ref)) < 2 * 192 * 2.0 ** -46
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nev", [64, 67, 195, 200])
+def test_displaced_and_momentum_operators_share_tiles(engine_lib, nev):
+    """Displaced operators need every row of the last tile, momentum operators
+    take edge columns for it: both in one build, against the FP64 build."""
+    from slaph_gb300 import _lib
+    from slaph_gb300.engine import Engine
+    L, Lt = 12, 2
+    moms = momenta(2)
+    disp = [b">x", b"<y>z"]
+    ops = (_lib.VdvOp * (len(moms) + len(disp)))()
+    for i, p in enumerate(moms):
+        ops[i].id, ops[i].momentum = i, (C.c_int32 * 3)(*p)
+    for d, s in enumerate(disp):
+        ops[len(moms) + d].id, ops[len(moms) + d].n_disp = len(moms) + d, len(s) // 2
+        ops[len(moms) + d].disp = s
+    eng = Engine(_lib.Dims(Lt, L, L, L, nev, 1, 2, 2))
+    _lib.check(_lib.lib().slaph_engine_set_operators(eng._h, ops, len(ops), -1))
+    rng = np.random.default_rng(nev)
+    V = rng.standard_normal((Lt, nev, 3 * L ** 3, 2)).view(np.complex128)[..., 0]
+    V /= np.linalg.norm(V, axis=2, keepdims=True)
+    for t in range(Lt):
+        eng.set_eigenvectors(t, V[t])
+        u, _ = np.linalg.qr(rng.standard_normal((L ** 3, 3, 3, 3, 2)).view(np.complex128)[..., 0])
+        eng.set_gauge(t, np.ascontiguousarray(u).reshape(L ** 3, 3, 9))
+    blocks = []
+    for precision in (0, 1):
+        eng.vdaggerv_build(precision)
+        blocks.append([eng.vdaggerv_fetch(i, t) for i in range(len(ops)) for t in range(Lt)])
+    # as above: 3 L^3 terms, the split 2^-46 of each row's scale per term; a
+    # displaced vector of two steps has entries up to the norm of the
+    # eigenvector times its longest run of links
+    tol = 4 * np.sqrt(3 * L ** 3) * 2.0 ** -44
+    for a, b in zip(*blocks):
+        assert np.max(np.abs(a - b)) < tol * max(1.0, np.max(np.abs(a)))
+    eng.close()
