@@ -357,9 +357,7 @@ void Engine::set_time_dilution(int32_t dilT) {
   SLAPH_CK(cudaStreamSynchronize(stream_));
   std::fill(pend_p_.begin(), pend_p_.end(), 0);
   sched_.reset();
-  sched_plan_ = nullptr;
   bp_scheds_.clear();
-  bp_plan_ = nullptr;
 }
 
 void Engine::set_gauge(int32_t t, double const *U) {
@@ -681,10 +679,10 @@ void Engine::vdaggerv_fetch(int32_t op, int32_t t, double *out) {
 }
 
 void Engine::prepare_schedule(slaph_plan const *plan, int bp) {
-  if (sched_ && sched_plan_ == plan && sched_bp_ == bp) return;
+  if (sched_ && sched_bp_ == bp && same_plan(sched_plan_, *plan)) return;
   sched_.reset();
   sched_ = make_schedule(plan, bp);
-  sched_plan_ = plan;
+  sched_plan_ = plan_words(*plan);
   sched_bp_ = bp;
 }
 
@@ -1521,9 +1519,9 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
   // over the block pairs in the same order either way.
   std::vector<DeviceSchedule *> scheds;
   if (factor_lifetime_ == SLAPH_FACTORS_BLOCK_PAIR) {
-    if (bp_plan_ != plan) {
+    if (!same_plan(bp_plan_, *plan)) {
       bp_scheds_.clear();
-      bp_plan_ = plan;
+      bp_plan_ = plan_words(*plan);
     }
     int const nb = dims_.Lt / dims_.dilT;
     for (int b = 0; b < nb * (nb + 1) / 2; ++b) {

@@ -201,12 +201,12 @@ class Engine {
       f_out_, f_work_;
 
   std::unique_ptr<DeviceSchedule> sched_;
-  slaph_plan const *sched_plan_ = nullptr;
+  std::vector<int32_t> sched_plan_;  // plan_words of its plan
   int sched_bp_ = -2;
   // Factors per block pair: one schedule per block pair of bp_plan_.
   int factor_lifetime_ = SLAPH_FACTORS_CONFIGURATION;
   std::map<int, std::unique_ptr<DeviceSchedule>> bp_scheds_;
-  slaph_plan const *bp_plan_ = nullptr;
+  std::vector<int32_t> bp_plan_;
 
   int64_t peram_elems() const;
   void prepare_schedule(slaph_plan const *plan, int single_block_pair);

@@ -18,6 +18,8 @@ namespace slaph {
 
 namespace {
 
+constexpr int kTraceArity[SLAPH_TR_KINDS] = {1, 2, 2, 3, 3, 4, 4, 6};
+
 // A DilutedFactor without data: random-vector pair and used-index mask.
 struct SymE {
   int32_t r1, r2;
@@ -729,11 +731,10 @@ class Builder {
   }
 
   int32_t trace_list(slaph_trace_request const &r, int src, int snk, Memo64<int32_t> &memo) {
-    static int const arity[SLAPH_TR_KINDS] = {1, 2, 2, 3, 3, 4, 4, 6};
     if (r.kind < 0 || r.kind >= SLAPH_TR_KINDS) throw ArgError("unknown trace kind");
     if (r.tr_id < 0 || r.tr_id >= plan_.n_trace_ids[r.kind] || r.tr_id >= (1 << 24))
       throw ArgError("trace id out of range");
-    if (r.n_loc != arity[r.kind]) throw ArgError("trace request location count mismatch");
+    if (r.n_loc != kTraceArity[r.kind]) throw ArgError("trace request location count mismatch");
     // The reference memoises by the tuple of times (include/DilutedTraceFactory.hpp:
     // 44-57); a pattern of source/sink locations gives that tuple from (src, snk).
     int pattern = 0;
@@ -747,7 +748,7 @@ class Builder {
     if (int32_t const *hit = memo.find(key)) return *hit;
     int k[6];
     for (int l = 0; l < r.n_loc; ++l) k[l] = r.loc[l] == 0 ? src : snk;
-    int const *c = plan_.trace_ql_ids[r.kind] + static_cast<int64_t>(r.tr_id) * arity[r.kind];
+    int const *c = plan_.trace_ql_ids[r.kind] + static_cast<int64_t>(r.tr_id) * kTraceArity[r.kind];
     int32_t const id = build_trace(r.kind, k, c);
     memo.emplace(key, id);
     return id;
@@ -782,6 +783,68 @@ class Builder {
 };
 
 }  // namespace
+
+namespace {
+
+// Calls word(int32) for everything that build_schedule reads of a plan, until one
+// call returns false.  Counts come before what they count, so that plans with equal
+// words are equal; tables that are not given (null) count as absent.
+template <typename F>
+bool visit_plan(slaph_plan const &p, F &&word) {
+  if (!word(p.n_vdv_ops)) return false;
+  for (int type = 0; type < 3; ++type) {
+    int32_t const n = p.factors[type] ? p.n_factors[type] : 0;
+    if (!word(p.n_factors[type]) || !word(n)) return false;
+    for (int32_t k = 0; k < n; ++k) {
+      slaph_factor_index const &f = p.factors[type][k];
+      int32_t const pairs = f.rnd_pairs ? f.n_rnd_pairs : 0;
+      if (!word(f.id_vdaggerv) || !word(f.need_vdaggerv_daggering) || !word(f.gamma) ||
+          !word(f.n_rnd_pairs) || !word(pairs))
+        return false;
+      for (int32_t q = 0; q < 2 * pairs; ++q)
+        if (!word(f.rnd_pairs[q])) return false;
+    }
+  }
+  for (int kind = 0; kind < SLAPH_TR_KINDS; ++kind) {
+    int32_t const n = p.trace_ql_ids[kind] ? p.n_trace_ids[kind] : 0;
+    if (!word(p.n_trace_ids[kind]) || !word(n)) return false;
+    for (int64_t k = 0; k < static_cast<int64_t>(n) * kTraceArity[kind]; ++k)
+      if (!word(p.trace_ql_ids[kind][k])) return false;
+  }
+  if (!word(p.n_diagrams)) return false;
+  for (int32_t d = 0; d < p.n_diagrams; ++d) {
+    slaph_diagram const &dg = p.diagrams[d];
+    if (!word(dg.n_requests)) return false;
+    for (int32_t i = 0; i < dg.n_requests; ++i) {
+      slaph_correlator_request const &req = dg.requests[i];
+      if (!word(req.n_traces)) return false;
+      for (int32_t k = 0; k < std::min(req.n_traces, 3); ++k) {
+        slaph_trace_request const &r = req.traces[k];
+        if (!word(r.kind) || !word(r.tr_id) || !word(r.n_loc)) return false;
+        for (int32_t l = 0; l < std::min(r.n_loc, 6); ++l)
+          if (!word(r.loc[l])) return false;
+      }
+    }
+  }
+  return true;
+}
+
+}  // namespace
+
+std::vector<int32_t> plan_words(slaph_plan const &plan) {
+  std::vector<int32_t> words;
+  visit_plan(plan, [&](int32_t w) {
+    words.push_back(w);
+    return true;
+  });
+  return words;
+}
+
+bool same_plan(std::vector<int32_t> const &words, slaph_plan const &plan) {
+  size_t at = 0;
+  return visit_plan(plan, [&](int32_t w) { return at < words.size() && words[at++] == w; }) &&
+         at == words.size();
+}
 
 Schedule build_schedule(slaph_dims const &dims, slaph_plan const &plan, int single_block_pair) {
   if (dims.Lt < 1 || dims.dilT < 1 || dims.Lt % dims.dilT != 0 || dims.dilE < 1 || dims.nev < 1)

@@ -209,6 +209,12 @@ std::vector<uint8_t> factor_layouts(Schedule const &s, bool tc_products);
 // run on the tensor cores.
 std::vector<uint8_t> product_layouts(Schedule const &s, Wave const &w);
 
+// What build_schedule reads of a plan, word by word.  A schedule belongs to the
+// contents of its plan: the address may hold another plan by the next call (a front
+// end freed and one made in its place, or tables changed by the caller).
+std::vector<int32_t> plan_words(slaph_plan const &plan);
+bool same_plan(std::vector<int32_t> const &words, slaph_plan const &plan);
+
 // Builds the schedule; throws EmptyError with the reference's messages when a
 // random-vector combination is empty.  single_block_pair >= 0 restricts the
 // work to that block pair.
