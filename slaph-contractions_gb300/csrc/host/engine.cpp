@@ -1076,8 +1076,9 @@ void Engine::prepare_product_tc(DeviceSchedule &ds) {
 //          rows (m, a), columns (gamma, r2, b2, c), K = (bd, v):
 //          A = conj(s(bd, a) Q2M_m(a, bd nev + v)),
 //          B = Gval[gamma][bd] P_r2((4t+Grow[gamma][bd]) nev + v, b2 eds + c)
-// Dense double-float outputs go to f_out_; gathers write the factor slots, in the
-// layouts in which they are read.
+// Dense double-float outputs go to f_out_ (Q2M without its exponents, dev::kTabRelative:
+// it may leave the range of FP32 where Q2 does not); gathers write the factor slots, in
+// the layouts in which they are read.
 void Engine::prepare_factor_tc(DeviceSchedule &ds) {
   if (ds.f_ready) return;
   Schedule const &s = ds.s;
@@ -1133,7 +1134,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
     vec.push_back(v);
   };
   auto add_tiles = [&](int64_t a_reg, int64_t b_reg, size_t a_tile, size_t b_tile, int32_t rows,
-                       int32_t cols, int64_t out, int32_t ea, int32_t eb) {
+                       int32_t cols, int64_t out, int32_t ea, int32_t eb, int64_t tab = -1) {
     int32_t const mts = (rows + dev::kTrTileRows - 1) / dev::kTrTileRows;
     int32_t const nts = (cols + dev::kTrTileCols - 1) / dev::kTrTileCols;
     for (int32_t mt = 0; mt < mts; ++mt)
@@ -1148,7 +1149,7 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
         t.rows = std::min(dev::kTrTileRows, rows - mt * dev::kTrTileRows);
         t.cols = std::min(dev::kTrTileCols, cols - nt * dev::kTrTileCols);
         t.ld = rows;
-        t.tab = -1;
+        t.tab = tab;
         tiles.push_back(t);
       }
   };
@@ -1333,7 +1334,8 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
                   eA_x1[k], eB_x1[k]);
       if (o.q2m_rows > 0)
         add_tiles(regA_q2m[k], regB_q2m[k], a_tile1, b_tile1, o.q2m_rows,
-                  static_cast<int32_t>(o.codes.size()) * nev, o.q2m, eA_q2m[k], eB_q2m[k]);
+                  static_cast<int32_t>(o.codes.size()) * nev, o.q2m, eA_q2m[k], eB_q2m[k],
+                  dev::kTabRelative);
     }
     b.t1[1] = static_cast<int64_t>(tiles.size()) - b.t1[0];
     need_scr = std::max(need_scr, off1);
@@ -1362,10 +1364,12 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
             v.expo = expo++;
             v.n_seg = 4;
             v.seg_len = nev;
+            v.e_col = eB_q2m[k] + ci * nev;
             for (int32_t bd = 0; bd < 4; ++bd) {
               bool const flip = (bd + r == 3) || (bd - r > 1) || (r - bd > 1);
               v.seg[bd].src = o.q2m + ((p * eds + a) * 4 + bd) + ld * (static_cast<int64_t>(ci) * nev);
               v.seg[bd].factor = flip ? 2 : 0;
+              v.seg[bd].e_row = eA_q2m[k] + (p * eds + a) * 4 + bd;
             }
             vec.push_back(v);
           }
@@ -1687,8 +1691,8 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
         cuda_check(dev::tc_gemm_df(fo, scr, ex, ft + b.t1[0], b.t1[1], kt1, err_.as<int>(), stream_),
                    "factor GEMM (X1, Q2M)");
         count(b.t1[1]);
-        cuda_check(dev::gvec_slice_df(scr, ex, fv + b.a_q2[0], b.a_q2[1], fi, true, true, fo, kt2,
-                                      stream_),
+        cuda_check(dev::gvec_slice_relative(scr, ex, fv + b.a_q2[0], b.a_q2[1], fi, fo, kt2,
+                                            stream_),
                    "slice Q2 A");
         cuda_check(dev::gvec_slice_f64(scr, ex, fv + b.b_q2[0], b.b_q2[1], fi, false, false,
                                        peram_.as<double2>(), kt2, stream_),

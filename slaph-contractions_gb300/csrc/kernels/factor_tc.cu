@@ -68,7 +68,11 @@ __device__ __forceinline__ void to_fixed(float4 v, int e, long long &fr, long lo
 // (as in the VdaggerV slicing), so that every slice store of a warp fills 512
 // contiguous bytes.  One row per CTA with 4-byte stores took 8.1 ms at 24^3x48
 // Nev 120, eight rows 4.6.
-template <bool kIsA, typename T>
+//
+// kRel: a relative source (Q2M).  The product of a perambulator and VdaggerV may
+// leave the range of FP32 where Q2, with the second perambulator, does not; its
+// entries keep their exponents apart, which the row's exponent takes in.
+template <bool kIsA, typename T, bool kRel = false>
 __global__ void __launch_bounds__(kGThreads)
     gvec_slice_kernel(uint8_t *scratch, int32_t *expo, GVecGroup const *groups, GVec const *items,
                       T const *src, int32_t k_tiles, int32_t conj) {
@@ -80,6 +84,12 @@ __global__ void __launch_bounds__(kGThreads)
     reinterpret_cast<uint32_t *>(it)[w] =
         reinterpret_cast<uint32_t const *>(items + gr.first)[w];
   __syncthreads();
+  if (kRel) {  // the exponents of the segments' rows in the place of their indices
+    static_assert(8 * kGMaxSeg <= kGThreads, "one thread per segment");
+    int const i = threadIdx.x / kGMaxSeg, s = threadIdx.x % kGMaxSeg;
+    if (i < gr.n && s < it[i].n_seg) it[i].seg[s].e_row = expo[it[i].seg[s].e_row];
+    __syncthreads();
+  }
   int const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   int const r = lane % 8, kg = lane / 8;
   bool const on = r < gr.n;
@@ -89,6 +99,9 @@ __global__ void __launch_bounds__(kGThreads)
     s = (k >= len) + (k >= 2 * len) + (k >= 3 * len);
     return src[v.seg[s].src + static_cast<int64_t>(k - s * len) * v.stride];
   };
+  // exponent of entry k (segment s) of a relative source
+  auto entry_expo = [&](int k, int s) { return v.seg[s].e_row + expo[v.e_col + k - s * len] - 14; };
+  constexpr int kRelBias = 1 << 20;  // of the exponents in mx, 0 for a zero row
   unsigned long long mx = 0;
   for (int kt = warp; kt < k_tiles; kt += kWarps)
 #pragma unroll
@@ -96,7 +109,9 @@ __global__ void __launch_bounds__(kGThreads)
       int const k = kt * (kTK / 2) + 4 * kg + q;
       int s;
       if (on && k < K) {
-        unsigned long long const b = absbits(load(k, s));
+        unsigned long long b = absbits(load(k, s));
+        if (kRel && b != 0)
+          b = static_cast<unsigned long long>(kRelBias + expo_of(b, src) + entry_expo(k, s));
         mx = b > mx ? b : mx;
       }
     }
@@ -109,7 +124,7 @@ __global__ void __launch_bounds__(kGThreads)
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < kWarps; ++w) mx = red[w][r] > mx ? red[w][r] : mx;
-  int const e = expo_of(mx, src);
+  int const e = !kRel ? expo_of(mx, src) : mx != 0 ? static_cast<int>(mx) - kRelBias : 0;
   if (warp == 0 && kg == 0 && on) expo[v.expo] = e;
   uint8_t *region = scratch + it[0].dst;
   int const row0 = it[0].row;  // a multiple of 8
@@ -121,7 +136,8 @@ __global__ void __launch_bounds__(kGThreads)
       long long fr = 0, fi = 0;
       if (on && k < K) {
         int s;
-        to_fixed(load(k, s), e, fr, fi);
+        T const x = load(k, s);
+        to_fixed(x, kRel ? e - entry_expo(k, s) : e, fr, fi);
         long long const re = fr, im = fi;
         switch (v.seg[s].factor & 3) {
           case 1: fr = -im; fi = re; break;   // x i
@@ -277,6 +293,15 @@ cudaError_t gvec_slice_df(uint8_t *scratch, int32_t *expo, GVecGroup const *grou
   else
     gvec_slice_kernel<false, float4><<<static_cast<unsigned>(n), kGThreads, 0, stream>>>(
         scratch, expo, groups, items, src, k_tiles, conj ? 1 : 0);
+  return cudaGetLastError();
+}
+
+cudaError_t gvec_slice_relative(uint8_t *scratch, int32_t *expo, GVecGroup const *groups,
+                                int64_t n, GVec const *items, float4 const *src, int32_t k_tiles,
+                                cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  gvec_slice_kernel<true, float4, true><<<static_cast<unsigned>(n), kGThreads, 0, stream>>>(
+      scratch, expo, groups, items, src, k_tiles, 1);
   return cudaGetLastError();
 }
 

@@ -337,7 +337,8 @@ struct TrSliceGroup {
   int32_t pad;
 };
 // One output tile of 64 rows x 80 columns of one GEMM.  tab < 0: value (r, c) at
-// out + c ld + r.  Otherwise the rows are stacked blocks of n_a operand groups
+// out + c ld + r (kTabRelative, tc_gemm_df only: without its factor 2^(e_r + e_c - 14),
+// e_r and e_c the exponents of its row and column).  Otherwise the rows are stacked blocks of n_a operand groups
 // and the columns of n_b: row r of the tile is group ia of block u, (row0 + r) =
 // u n_a + ia, column c group ib of block v, (col0 + c) = v n_b + ib, and the
 // value belongs to entry e = entries[tab + u tab_ld + v] (none when negative),
@@ -352,6 +353,7 @@ struct TrTile {
   int32_t n_a, n_b, row0, col0, tab_ld;
 };
 constexpr int32_t kTrTileRows = 64, kTrTileCols = 80;
+constexpr int64_t kTabRelative = -2;
 int64_t trace_tc_k_tiles(int32_t eds);
 size_t trace_tc_a_bytes(int32_t rows, int32_t eds);  // A region of `rows` matrices
 size_t trace_tc_b_bytes(int32_t cols, int32_t eds);  // B region of `cols` matrices
@@ -389,11 +391,13 @@ cudaError_t tc_gemm_df(float4 *out, uint8_t const *scratch, int32_t const *expo,
 
 // One GEMM operand row (A) or column (B) gathered from up to four strided
 // segments of a source array, each with an exact factor (0: +1, 1: +i, 2: -1,
-// 3: -i).  K = n_seg * seg_len, zero-padded to the region's k-tiles.
+// 3: -i).  K = n_seg * seg_len, zero-padded to the region's k-tiles.  A relative
+// source (kTabRelative) holds entry j of a segment without its factor 2^(x + y - 14), x
+// and y the exponents at e_row and GVec::e_col + j.
 struct GSeg {
   int64_t src;
   int32_t factor;
-  int32_t pad;
+  int32_t e_row;
 };
 constexpr int kGMaxSeg = 4;
 struct GVec {
@@ -402,6 +406,7 @@ struct GVec {
   int32_t row;     // row (A) or column (B) within the region
   int32_t expo;    // index of its exponent
   int32_t n_seg, seg_len;
+  int32_t e_col, pad;
   GSeg seg[kGMaxSeg];
 };
 // Up to eight consecutive operand vectors of one region, items[first .. first +
@@ -411,13 +416,16 @@ struct GVecGroup {
   int32_t n, pad;
 };
 // Slices the operand vectors of n groups (A rows with put conj(v) when conj, or B
-// columns) from an FP64 or a double-float source.
+// columns) from an FP64, a double-float or a relative double-float source.
 cudaError_t gvec_slice_f64(uint8_t *scratch, int32_t *expo, GVecGroup const *groups, int64_t n,
                            GVec const *items, bool is_a, bool conj, double2 const *src, int32_t k_tiles,
                            cudaStream_t stream);
 cudaError_t gvec_slice_df(uint8_t *scratch, int32_t *expo, GVecGroup const *groups, int64_t n,
                           GVec const *items, bool is_a, bool conj, float4 const *src, int32_t k_tiles,
                           cudaStream_t stream);
+cudaError_t gvec_slice_relative(uint8_t *scratch, int32_t *expo, GVecGroup const *groups,
+                                int64_t n, GVec const *items, float4 const *src, int32_t k_tiles,
+                                cudaStream_t stream);  // A rows, conjugated
 // Q1 factor slots from the dense product X1 (factor_tc.cu); Q2 slots from the
 // dense Q2 GEMM output; both double-float, as tc_gemm_df writes them.  need: the
 // layouts to write (1 stored, 2 transposed); slot_bits: largest |re|, |im| of
