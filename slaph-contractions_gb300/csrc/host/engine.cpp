@@ -813,6 +813,7 @@ std::unique_ptr<DeviceSchedule> Engine::make_schedule(slaph_plan const *plan, in
 // cut into 64 x 80 tiles.  Groups are packed into batches of at most the scratch
 // capacity (a group larger than that raises it).
 void Engine::prepare_trace_tc(DeviceSchedule &ds) {
+  static_assert(kTraceGroupBits == dev::kTrGroupBits, "columns are packed as planned");
   if (ds.tc_ready) return;
   Schedule const &s = ds.s;
   int32_t const eds = s.eds;

@@ -939,8 +939,9 @@ TraceGroupPlan plan_trace_group(TraceShape const &shape, int32_t n_a, int32_t n_
   };
   TraceGroupPlan best;
   bool have = false;
+  bool const packs = n_b <= 1 << kTraceGroupBits && nj < 1 << (31 - kTraceGroupBits);
   for (int option = 0; option < 4; ++option) {
-    if ((option & 2) && n_b >= 1 << 15) continue;  // the tile epilogue holds groups in 16 bits
+    if (option != 0 && !packs) continue;
     TraceGroupPlan p;
     p.a = blocks(has_i, 0, (option & 1) != 0);
     p.b = blocks(has_j, ni, (option & 2) != 0);

@@ -164,6 +164,10 @@ constexpr int32_t kMinSplitA = 32, kMinSplitB = 32;
 // tile_cols that a small group leaves mostly empty, but also computes pairs of a
 // component that are not entries.  Of the four combinations the one with the
 // fewest tiles is taken (tiles without an entry are left out).
+// The epilogue of stacked tiles packs the block and the group of a column into one
+// int, the group in the low kTraceGroupBits: larger groups and longer operand lists are
+// not stacked.
+constexpr int32_t kTraceGroupBits = 16;
 struct TraceGroupPlan {
   std::vector<std::vector<int32_t>> a, b;  // operand indices of every block
   struct Tile {

@@ -354,6 +354,7 @@ struct TrTile {
 };
 constexpr int32_t kTrTileRows = 64, kTrTileCols = 80;
 constexpr int64_t kTabRelative = -2;
+constexpr int32_t kTrGroupBits = 16;  // v << kTrGroupBits | ib in the epilogue: n_b <= 2^16
 int64_t trace_tc_k_tiles(int32_t eds);
 size_t trace_tc_a_bytes(int32_t rows, int32_t eds);  // A region of `rows` matrices
 size_t trace_tc_b_bytes(int32_t cols, int32_t eds);  // B region of `cols` matrices

@@ -144,7 +144,7 @@ struct TraceEpilogue {
   struct Pre {
     TrTile t;
     int e0, e1, er;
-    int v0, v1;  // block v << 16 | group ib
+    int v0, v1;  // block v << kTrGroupBits | group ib
   };
   __device__ __forceinline__ Pre prepare(int i, int row, int col0) const {
     Pre p;
@@ -156,8 +156,8 @@ struct TraceEpilogue {
     p.v0 = p.v1 = 0;
     if (p.t.tab >= 0) {
       int const c0 = p.t.col0 + col0 + lane, c1 = c0 + 32;
-      p.v0 = (c0 / p.t.n_b) << 16 | (c0 % p.t.n_b);
-      p.v1 = (c1 / p.t.n_b) << 16 | (c1 % p.t.n_b);
+      p.v0 = (c0 / p.t.n_b) << kTrGroupBits | (c0 % p.t.n_b);
+      p.v1 = (c1 / p.t.n_b) << kTrGroupBits | (c1 % p.t.n_b);
     }
     return p;
   }
@@ -201,12 +201,12 @@ struct TraceEpilogue {
       int const ec = __shfl_sync(0xffffffffu, c < 32 ? p.e0 : p.e1, c % 32);
       int const vb = __shfl_sync(0xffffffffu, c < 32 ? p.v0 : p.v1, c % 32);
       if (!row_ok || col0 + c >= t.cols) continue;
-      if (vb >> 16 != v_at) {
-        v_at = vb >> 16;
+      if (vb >> kTrGroupBits != v_at) {
+        v_at = vb >> kTrGroupBits;
         e_at = tab[v_at];
       }
       if (e_at >= 0)
-        dst[2 * (e_at * plane + static_cast<int64_t>(vb & 0xFFFF) * t.n_a)] =
+        dst[2 * (e_at * plane + static_cast<int64_t>(vb & ((1 << kTrGroupBits) - 1)) * t.n_a)] =
             df_scaled(hi[c], lo[c], p.er + ec - 14);
     }
   }
