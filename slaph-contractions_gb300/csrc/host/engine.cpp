@@ -703,7 +703,6 @@ constexpr int64_t kX1Batch = 4096;
 
 void plan_shared_q1(DeviceSchedule &ds, Schedule const &s, cudaStream_t stream) {
   if (ds.x1_ready) return;
-  ds.x1_ready = true;
   auto key = [&](int32_t k) {
     auto const &q = s.q1[k];
     return std::make_tuple(q.t, q.b, q.r, q.r2);
@@ -715,27 +714,35 @@ void plan_shared_q1(DeviceSchedule &ds, Schedule const &s, cudaStream_t stream) 
   for (size_t k = 0; k < ord.size(); ++k)
     if (k == 0 || key(ord[k]) != key(ord[k - 1])) ++distinct;
   if (distinct == 0 ||
-      static_cast<double>(ord.size()) < kQ1Share * static_cast<double>(distinct))
+      static_cast<double>(ord.size()) < kQ1Share * static_cast<double>(distinct)) {
+    ds.x1_ready = true;
     return;
+  }
   std::vector<dev::X1Inst> xs;
   std::vector<dev::Q1Pick> picks;
+  std::vector<DeviceSchedule::X1Batch> batches;
+  int64_t most = 0;
   for (size_t k = 0; k < ord.size(); ++k) {
     auto const &q = s.q1[ord[k]];
     if (k == 0 || key(ord[k]) != key(ord[k - 1])) {
       if (xs.size() % kX1Batch == 0)
-        ds.x1_batches.push_back({static_cast<int64_t>(xs.size()), 0,
-                                 static_cast<int64_t>(picks.size()), 0});
+        batches.push_back({static_cast<int64_t>(xs.size()), 0,
+                           static_cast<int64_t>(picks.size()), 0});
       xs.push_back({q.t, q.b, q.r, q.r2});
-      ++ds.x1_batches.back().n_x;
-      ds.x1_max = std::max(ds.x1_max, ds.x1_batches.back().n_x);
+      ++batches.back().n_x;
+      most = std::max(most, batches.back().n_x);
     }
-    auto &b = ds.x1_batches.back();
+    auto &b = batches.back();
     picks.push_back({static_cast<int32_t>(b.n_x - 1), q.gamma, q.slot});
     ++b.n_p;
   }
   upload(ds.x1, xs, stream);
   upload(ds.q1_picks, picks, stream);
   SLAPH_CK(cudaStreamSynchronize(stream));
+  // in place only now: a failed allocation above leaves no batches behind
+  ds.x1_batches = std::move(batches);
+  ds.x1_max = most;
+  ds.x1_ready = true;
 }
 
 }  // namespace
