@@ -218,6 +218,9 @@ void Engine::set_operators(slaph_vdv_op const *ops, int32_t n, int32_t index_of_
       throw UnsupportedError("displaced operators need a cubic spatial lattice");
   }
   if (index_of_unity >= n) throw ArgError("index_of_unity out of range");
+  // until the end: a failure below leaves no table whose device buffers are gone
+  ops_set_ = false;
+  vdv_built_ = false;
   ops_.assign(ops, ops + n);
   index_of_unity_ = index_of_unity;
   // Momentum operators by family and displaced operators (V^H D(V), momentum
@@ -279,7 +282,6 @@ void Engine::set_operators(slaph_vdv_op const *ops, int32_t n, int32_t index_of_
   vdv_.reserve(sizeof(double2) * 2LL * std::max(n, 1) * dims_.Lt * dims_.nev * dims_.nev);
   SLAPH_CK(cudaStreamSynchronize(stream_));
   ops_set_ = true;
-  vdv_built_ = false;
 }
 
 void Engine::set_eigenvector_slots(int32_t n) {

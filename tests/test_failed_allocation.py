@@ -102,10 +102,31 @@ static int shared_q1(int fail) {
   return 0;
 }
 
+// A table of operators, then a larger one that fails: neither is in place.
+static int operators(int fail) {
+  Engine e(slaph_dims{2, 4, 4, 4, 5, 1, 2, 2});
+  std::vector<slaph_vdv_op> ops(5);
+  for (int k = 0; k < 5; ++k) ops[k] = slaph_vdv_op{k, {k, 1, 0}, 0, {}};
+  e.set_operators(ops.data(), 1, -1);
+  calls_left = fail;
+  bool const failed = throws([&] { e.set_operators(ops.data(), 5, -1); });
+  calls_left = -1;
+  if (!failed) return 2;  // fewer calls than that
+  bool state = false;
+  try {
+    e.vdaggerv_build(SLAPH_MIXED);
+  } catch (StateError const &) {
+    state = true;
+  }
+  EXPECT(state);
+  e.set_operators(ops.data(), 5, -1);
+  return 0;
+}
+
 int main(int, char **argv) {
   fail_copies = std::atoi(argv[2]) != 0;
   int const fail = std::atoi(argv[3]);
-  return shared_q1(fail);
+  return argv[1][0] == 'q' ? shared_q1(fail) : operators(fail);
 }
 """
 
@@ -132,3 +153,15 @@ def program(tmp_path_factory):
 def test_shared_q1_plan(program, copies, fail):
     r = program("q1", copies, fail)
     assert r.returncode == 0, r.stdout
+
+
+@pytest.mark.parametrize("copies", [0, 1], ids=["malloc", "memcpy"])
+def test_operator_table(program, copies):
+    tried = 0
+    for fail in range(20):
+        r = program("operators", copies, fail)
+        if r.returncode == 2:
+            break
+        assert r.returncode == 0, (fail, r.returncode, r.stdout)
+        tried += 1
+    assert tried >= 3
