@@ -152,7 +152,12 @@ struct Schedule {
 // and 80 B groups); smaller bipartite sets stay residual.
 constexpr int32_t kMinGroupA = 16, kMinGroupB = 16;
 // The same for the groups found after the lists with both operands at one
-// timeslice are set aside (group_lists).
+// timeslice are set aside (group_lists).  The sets of 28 x 28 that time blocks of
+// four leave (tests/test_schedule.py counts them among the residual lists) stay with
+// the double-float kernel, which keeps every product of the operands' digits: as
+// groups they gain 0-3 %.  48 timeslices, dilE 4, four vectors: residual traces 6.9 ->
+// 6.0 ms, slices and GEMM 5.6 -> 5.9, pass 24.7 -> 24.1; dilE 8, five vectors: pass
+// 107.1 -> 106.3; 8 timeslices: 1.70 either way.
 constexpr int32_t kMinSplitA = 32, kMinSplitB = 32;
 
 // GEMM plan of a dense trace group of n_a x n_b operand groups.  The entries
