@@ -1086,7 +1086,7 @@ void Engine::prepare_product_tc(DeviceSchedule &ds) {
 //          rows (m, a), columns (gamma, r2, b2, c), K = (bd, v):
 //          A = conj(s(bd, a) Q2M_m(a, bd nev + v)),
 //          B = Gval[gamma][bd] P_r2((4t+Grow[gamma][bd]) nev + v, b2 eds + c)
-// Dense double-float outputs go to f_out_ (Q2M without its exponents, dev::kTabRelative:
+// Dense double-float outputs go to f_out_ (Q2M without its rows' exponents, dev::kTabRelative:
 // it may leave the range of FP32 where Q2 does not); gathers write the factor slots, in
 // the layouts in which they are read.
 void Engine::prepare_factor_tc(DeviceSchedule &ds) {
@@ -1374,7 +1374,6 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
             v.expo = expo++;
             v.n_seg = 4;
             v.seg_len = nev;
-            v.e_col = eB_q2m[k] + ci * nev;
             for (int32_t bd = 0; bd < 4; ++bd) {
               bool const flip = (bd + r == 3) || (bd - r > 1) || (r - bd > 1);
               v.seg[bd].src = o.q2m + ((p * eds + a) * 4 + bd) + ld * (static_cast<int64_t>(ci) * nev);

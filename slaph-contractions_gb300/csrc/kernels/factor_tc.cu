@@ -71,7 +71,8 @@ __device__ __forceinline__ void to_fixed(float4 v, int e, long long &fr, long lo
 //
 // kRel: a relative source (Q2M).  The product of a perambulator and VdaggerV may
 // leave the range of FP32 where Q2, with the second perambulator, does not; its
-// entries keep their exponents apart, which the row's exponent takes in.
+// segments keep the exponents of their perambulator rows apart, which the row's
+// exponent takes in.
 template <bool kIsA, typename T, bool kRel = false>
 __global__ void __launch_bounds__(kGThreads)
     gvec_slice_kernel(uint8_t *scratch, int32_t *expo, GVecGroup const *groups, GVec const *items,
@@ -84,10 +85,15 @@ __global__ void __launch_bounds__(kGThreads)
     reinterpret_cast<uint32_t *>(it)[w] =
         reinterpret_cast<uint32_t const *>(items + gr.first)[w];
   __syncthreads();
-  if (kRel) {  // the exponents of the segments' rows in the place of their indices
+  // kRel: the exponents of the segments' rows, biased, in the place of their indices.
+  // The bits of a value's magnitude plus 2^23 times that order the values of all
+  // segments and hold the (biased) exponent from bit 23 on.
+  constexpr int kRelBias = 4096;
+  if (kRel) {
     static_assert(8 * kGMaxSeg <= kGThreads, "one thread per segment");
     int const i = threadIdx.x / kGMaxSeg, s = threadIdx.x % kGMaxSeg;
-    if (i < gr.n && s < it[i].n_seg) it[i].seg[s].e_row = expo[it[i].seg[s].e_row];
+    if (i < gr.n && s < it[i].n_seg)
+      it[i].seg[s].e_row = expo[it[i].seg[s].e_row] + kRelBias;
     __syncthreads();
   }
   int const warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -99,9 +105,6 @@ __global__ void __launch_bounds__(kGThreads)
     s = (k >= len) + (k >= 2 * len) + (k >= 3 * len);
     return src[v.seg[s].src + static_cast<int64_t>(k - s * len) * v.stride];
   };
-  // exponent of entry k (segment s) of a relative source
-  auto entry_expo = [&](int k, int s) { return v.seg[s].e_row + expo[v.e_col + k - s * len] - 14; };
-  constexpr int kRelBias = 1 << 20;  // of the exponents in mx, 0 for a zero row
   unsigned long long mx = 0;
   for (int kt = warp; kt < k_tiles; kt += kWarps)
 #pragma unroll
@@ -111,7 +114,7 @@ __global__ void __launch_bounds__(kGThreads)
       if (on && k < K) {
         unsigned long long b = absbits(load(k, s));
         if (kRel && b != 0)
-          b = static_cast<unsigned long long>(kRelBias + expo_of(b, src) + entry_expo(k, s));
+          b += static_cast<unsigned long long>(v.seg[s].e_row) << 23;
         mx = b > mx ? b : mx;
       }
     }
@@ -124,7 +127,9 @@ __global__ void __launch_bounds__(kGThreads)
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < kWarps; ++w) mx = red[w][r] > mx ? red[w][r] : mx;
-  int const e = !kRel ? expo_of(mx, src) : mx != 0 ? static_cast<int>(mx) - kRelBias : 0;
+  int const e = !kRel    ? expo_of(mx, src)
+                : mx != 0 ? static_cast<int>(mx >> 23) - 126 - kRelBias
+                          : 0;
   if (warp == 0 && kg == 0 && on) expo[v.expo] = e;
   uint8_t *region = scratch + it[0].dst;
   int const row0 = it[0].row;  // a multiple of 8
@@ -137,7 +142,7 @@ __global__ void __launch_bounds__(kGThreads)
       if (on && k < K) {
         int s;
         T const x = load(k, s);
-        to_fixed(x, kRel ? e - entry_expo(k, s) : e, fr, fi);
+        to_fixed(x, kRel ? e + kRelBias - v.seg[s].e_row : e, fr, fi);
         long long const re = fr, im = fi;
         switch (v.seg[s].factor & 3) {
           case 1: fr = -im; fi = re; break;   // x i

@@ -337,8 +337,8 @@ struct TrSliceGroup {
   int32_t pad;
 };
 // One output tile of 64 rows x 80 columns of one GEMM.  tab < 0: value (r, c) at
-// out + c ld + r (kTabRelative, tc_gemm_df only: without its factor 2^(e_r + e_c - 14),
-// e_r and e_c the exponents of its row and column).  Otherwise the rows are stacked blocks of n_a operand groups
+// out + c ld + r (kTabRelative, tc_gemm_df only: without the factor 2^e of its row's
+// exponent e).  Otherwise the rows are stacked blocks of n_a operand groups
 // and the columns of n_b: row r of the tile is group ia of block u, (row0 + r) =
 // u n_a + ia, column c group ib of block v, (col0 + c) = v n_b + ib, and the
 // value belongs to entry e = entries[tab + u tab_ld + v] (none when negative),
@@ -392,9 +392,8 @@ cudaError_t tc_gemm_df(float4 *out, uint8_t const *scratch, int32_t const *expo,
 
 // One GEMM operand row (A) or column (B) gathered from up to four strided
 // segments of a source array, each with an exact factor (0: +1, 1: +i, 2: -1,
-// 3: -i).  K = n_seg * seg_len, zero-padded to the region's k-tiles.  A relative
-// source (kTabRelative) holds entry j of a segment without its factor 2^(x + y - 14), x
-// and y the exponents at e_row and GVec::e_col + j.
+// 3: -i).  K = n_seg * seg_len, zero-padded to the region's k-tiles.  In a relative
+// source (kTabRelative) a segment is without the factor 2^e of the exponent at e_row.
 struct GSeg {
   int64_t src;
   int32_t factor;
@@ -407,7 +406,7 @@ struct GVec {
   int32_t row;     // row (A) or column (B) within the region
   int32_t expo;    // index of its exponent
   int32_t n_seg, seg_len;
-  int32_t e_col, pad;
+  int32_t pad[2];  // to 26 words: eight in shared memory, the same word of each, meet no bank twice
   GSeg seg[kGMaxSeg];
 };
 // Up to eight consecutive operand vectors of one region, items[first .. first +

@@ -172,8 +172,8 @@ struct TraceEpilogue {
 #pragma unroll
       for (int c = 0; c < kColsW; ++c) {
         int const ec = __shfl_sync(0xffffffffu, c < 32 ? p.e0 : p.e1, c % 32);
-        int const sh =
-            t.tab == kTabRelative ? 0 : min(max(p.er + ec - 14, -252), 254);  // above: infinity
+        int const er = t.tab == kTabRelative ? 0 : p.er;
+        int const sh = min(max(er + ec - 14, -252), 254);  // above: infinity
         if (row_ok && col0 + c < t.cols)
           dst[2 * static_cast<int64_t>(col0 + c) * t.ld] =
               make_float2(scale2(hi[c], sh), scale2(lo[c], sh));
