@@ -208,15 +208,17 @@ __device__ M3 proj_su3(M3 const &m) {
   double const np = cnorm(p), nq = cnorm(q), nr = cnorm(r);
   double const c1 = a[0] + a[1] + a[2];
   double const c2 = (fma(a[0], a[1], -np) + fma(a[0], a[2], -nq)) + fma(a[1], a[2], -nr);
-  if (!(c2 > 0.1 * c1 * c1 && c1 > 1e-20 && c1 < 1e20)) return polar_su3(m);
+  // c2 / c1^2 in FP32, the scale by the exponent of c1 (2^-64 .. 2^64): no FP64 operation
+  double const is = rsqrt(c1), is2 = is * is;
+  float const t2 = static_cast<float>(4 * c2 * is2 * is2);
+  unsigned int const scale = static_cast<unsigned int>(__double2hiint(c1)) - ((1023u - 64u) << 20);
+  if (!(t2 > 0.4f) || scale >= 128u << 20) return polar_su3(m);
   double2 const det = det3(m);
   double const d2 = cnorm(det);
   double const iw = rsqrt(d2);
   double const w = d2 * iw;
   // in units of sqrt(tr A) while in FP32
-  double const is = rsqrt(c1), is2 = is * is;
-  float const t2 = static_cast<float>(4 * c2 * is2 * is2),
-              tw = static_cast<float>(8 * w * is2 * is);
+  float const tw = static_cast<float>(8 * w * is2 * is);
   float x0 = 1.7320508f;
 #pragma unroll
   for (int k = 0; k < 6; ++k) {
