@@ -44,11 +44,11 @@ extern "C" {
 /* ---- enums ------------------------------------------------------------- */
 enum slaph_precision {
   SLAPH_FP64 = 0,  /* every product in FP64                                   */
-  SLAPH_MIXED = 1  /* VdaggerV and the traces of dense trace groups as
-                      split-BF16 tensor-core products with exact FP32 partial
-                      sums; diluted factors, factor products and the other
-                      traces in compensated double-float (2 x FP32)
-                      arithmetic; terms and correlator sums in FP64.
+  SLAPH_MIXED = 1  /* VdaggerV, the factors Q1 and Q2, most factor products
+                      and the traces of dense trace groups as split-BF16
+                      tensor-core products with FP32 partial sums; the other
+                      factors, products and traces in compensated double-float
+                      (2 x FP32) arithmetic; terms and correlator sums in FP64.
                       Correlators agree with SLAPH_FP64 to about 1e-12
                       relative (tested at 1e-10)                                */
 };
@@ -317,8 +317,9 @@ int slaph_engine_set_time_dilution(slaph_engine *eng, int32_t dilT);
  * (src/OperatorFactory.cpp:253-260): GaugeField::smearing_hyp
  * (src/GaugeField.cpp:322-427) with (alpha1, alpha2, iterations) applied on
  * the device to the stored links of every timeslice, in place, in FP64.  The
- * SU(3) back-projection proj_to_su3_imp (:203-210) takes (M^H M)^(-1/2) from a
- * Jacobi eigen-decomposition, equal to the reference's Eigen matrix square
+ * SU(3) back-projection proj_to_su3_imp (:203-210) takes the unitary polar
+ * factor of M in closed form or, for matrices of bad condition or scale, by
+ * Newton's iteration: M (M^H M)^(-1/2) of the reference's Eigen matrix square
  * root to rounding.  Needs slaph_engine_set_gauge for every timeslice first;
  * iterations = 0 leaves the links unchanged (the reference's default). */
 int slaph_engine_smear_gauge_hyp(slaph_engine *eng, double alpha1, double alpha2,
@@ -389,7 +390,9 @@ int slaph_vdaggerv_file_name(const char *path_vdaggerv, int32_t config, const sl
  * (request order), Lt complex values C[t] = sum / Lt exactly as Diagram::write
  * stores them (src/Diagram.cpp:132-147): [total_requests][Lt][2] doubles.
  * single_block_pair >= 0 restricts the work to that block pair, as the
- * reference's --single_time_slice_combination (src/Correlators.cpp:88-90). */
+ * reference's --single_time_slice_combination (src/Correlators.cpp:88-90).
+ * The work lists of the last plan are kept for the next call and belong to the
+ * plan's contents, not to its address. */
 int slaph_contract(slaph_engine *eng, const slaph_plan *plan, int precision, int accumulator,
                    int single_block_pair, double *corr_out);
 /* Number of doubles slaph_contract writes for this plan. */
