@@ -200,16 +200,27 @@ class Engine {
   DevBuf slots_, df_slots_, df_slots_t_, values_, term_val_, running_, tr_expo_,
       f_out_, f_work_;
 
+  // The plan that schedules were made for: its contents (plan_words), and where it was.
+  struct KeptPlan {
+    std::vector<int32_t> words;
+    slaph_plan const *at = nullptr;
+    int32_t n_vdv = 0;
+    int64_t n_outputs = 0;
+    void keep(slaph_plan const &plan);
+    // Whether `plan` is this one.  At the same address, with the same sizes of its
+    // inputs and outputs, the comparison is put off (later = true): see contract.
+    bool is(slaph_plan const &plan, bool &later) const;
+  };
   std::unique_ptr<DeviceSchedule> sched_;
-  std::vector<int32_t> sched_plan_;  // plan_words of its plan
+  KeptPlan sched_plan_;
   int sched_bp_ = -2;
   // Factors per block pair: one schedule per block pair of bp_plan_.
   int factor_lifetime_ = SLAPH_FACTORS_CONFIGURATION;
   std::map<int, std::unique_ptr<DeviceSchedule>> bp_scheds_;
-  std::vector<int32_t> bp_plan_;
+  KeptPlan bp_plan_;
 
   int64_t peram_elems() const;
-  void prepare_schedule(slaph_plan const *plan, int single_block_pair);
+  void prepare_schedule(slaph_plan const *plan, int single_block_pair, bool &later);
   std::unique_ptr<DeviceSchedule> make_schedule(slaph_plan const *plan, int single_block_pair);
   void prepare_trace_tc(DeviceSchedule &ds);
   void prepare_factor_tc(DeviceSchedule &ds);

@@ -104,8 +104,8 @@ def test_tables_that_are_not_given_are_not_read(words):
 @pytest.mark.parametrize("precision", [0, 1])
 def test_contract_follows_the_plan_at_one_address(engine_lib, tmp_path, precision,
                                                   per_block_pair):
-    """The plan of one diagram, then that of two (more correlators), over one
-    operator table."""
+    """The plan of one diagram, then that of two (more correlators), then as many
+    correlators in another order, over one operator table."""
     from slaph_gb300 import GlobalData, _lib, synthetic
     from slaph_gb300.engine import Engine
     w = synthetic.Workload("one_address", Lt=4, L=4, nev=8, n_rnd=4, dilT=2, dilE=2,
@@ -134,9 +134,15 @@ def test_contract_follows_the_plan_at_one_address(engine_lib, tmp_path, precisio
     want = fresh.contract(gd.plan_ptr, precision)
     fresh.close()
     eng = engine()
-    for k, box in enumerate(at_one_address(C.byref(first), gd.plan_ptr)):
+    last = _lib.Plan()
+    C.memmove(C.byref(last), gd.plan_ptr, C.sizeof(_lib.Plan))
+    turned = (_lib.Diagram * 2)(gd.plan.diagrams[1], gd.plan.diagrams[0])
+    last.diagrams = turned
+    n0 = gd.plan.diagrams[0].n_requests
+    assert gd.plan.n_diagrams == 2 and not np.array_equal(want, np.roll(want, -n0, 0))
+    for k, box in enumerate(at_one_address(C.byref(first), gd.plan_ptr, gd.plan_ptr,
+                                           C.byref(last), gd.plan_ptr)):
         out = eng.contract(C.pointer(box), precision)
-        n = len(out)
-        assert n < len(want) if k == 0 else n == len(want)
-        assert np.array_equal(out, want[:n])
+        ref = np.roll(want, -n0, 0) if k == 3 else want[:n0] if k == 0 else want
+        assert np.array_equal(out, ref)
     eng.close()
