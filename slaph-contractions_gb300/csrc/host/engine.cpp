@@ -1532,8 +1532,32 @@ void Engine::prepare_factor_tc(DeviceSchedule &ds) {
   ds.f_ready = true;
 }
 
+// A plan at the address of the last one is taken to be that one and compared while
+// the device works (6781 correlators: 50 us, a tenth of a small block pair); where it
+// is another after all, or the attempt failed and it is another, the contraction is done
+// again with a schedule of its own.  The work in vain stays within the engine's buffers:
+// it has the sizes of the new plan.
 void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
                       int single_block_pair, double *corr_out) {
+  bool later = false;
+  int64_t const launches_before = launches_;
+  try {
+    if (contract_once(plan, precision, accumulator, single_block_pair, corr_out, later)) return;
+  } catch (std::exception const &) {
+    if (!later || same_plan(kept_plan().words, *plan)) throw;
+  }
+  SLAPH_CK(cudaStreamSynchronize(stream_));
+  sched_.reset();
+  bp_scheds_.clear();
+  launches_ = launches_before;
+  later = false;
+  contract_once(plan, precision, accumulator, single_block_pair, corr_out, later);
+}
+
+// False, and corr_out as it was, when `later` became true and the plan is not the kept
+// one.
+bool Engine::contract_once(slaph_plan const *plan, int precision, int accumulator,
+                           int single_block_pair, double *corr_out, bool &later) {
   if (!plan || !corr_out) throw ArgError("null plan or output");
   if (!vdv_built_) throw StateError("slaph_vdaggerv_build must be called before contract");
   if (precision != SLAPH_FP64 && precision != SLAPH_MIXED)
@@ -1553,15 +1577,9 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
   // that block pair and dropped after it, as the reference clears its factor
   // caches per block pair, src/Correlators.cpp:116); the correlator sums run
   // over the block pairs in the same order either way.
-  // A plan at the address of the last one is taken to be that one and compared while
-  // the device works (6781 correlators: 50 us, a tenth of a small block pair); where it
-  // is another after all, the work is done again with a schedule of its own.  The work
-  // in vain stays within the engine's buffers: it has the sizes of the new plan.
-  bool later = false;
-  int64_t const launches_before = launches_;
   std::vector<DeviceSchedule *> scheds;
   if (factor_lifetime_ == SLAPH_FACTORS_BLOCK_PAIR) {
-    if (!bp_plan_.is(*plan, later)) {
+    if (bp_scheds_.empty() || !bp_plan_.is(*plan, later)) {
       bp_scheds_.clear();
       bp_plan_.keep(*plan);
     }
@@ -1890,19 +1908,8 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
   }
   if (mixed)
     SLAPH_CK(cudaMemcpyAsync(flag, err_.as<void>(), sizeof(int), cudaMemcpyDeviceToHost, stream_));
-  bool const other =
-      later && !same_plan(factor_lifetime_ == SLAPH_FACTORS_BLOCK_PAIR ? bp_plan_.words
-                                                                       : sched_plan_.words,
-                          *plan);
+  if (later && !same_plan(kept_plan().words, *plan)) return false;
   SLAPH_CK(cudaStreamSynchronize(stream_));
-  if (other) {
-    sched_.reset();
-    bp_scheds_.clear();
-    bp_plan_ = KeptPlan();
-    launches_ = launches_before;
-    contract(plan, precision, accumulator, single_block_pair, corr_out);
-    return;
-  }
   for (auto const &sp : spans) *sp.sum += elapsed_ms(sp.from, sp.to);
   timings[1] = t_f;
   timings[2] = t_pt;
@@ -1921,6 +1928,7 @@ void Engine::contract(slaph_plan const *plan, int precision, int accumulator,
                        std::to_string(*flag) + ")");
   if (n_host > 0) std::memcpy(corr_out, host, n_host * sizeof(double2));
   for (int k = 0; k < 8; ++k) stats[k] = st[k];
+  return true;
 }
 
 }  // namespace slaph

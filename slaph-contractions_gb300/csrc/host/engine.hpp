@@ -220,6 +220,11 @@ class Engine {
   KeptPlan bp_plan_;
 
   int64_t peram_elems() const;
+  KeptPlan const &kept_plan() const {
+    return factor_lifetime_ == SLAPH_FACTORS_BLOCK_PAIR ? bp_plan_ : sched_plan_;
+  }
+  bool contract_once(slaph_plan const *plan, int precision, int accumulator,
+                     int single_block_pair, double *corr_out, bool &later);
   void prepare_schedule(slaph_plan const *plan, int single_block_pair, bool &later);
   std::unique_ptr<DeviceSchedule> make_schedule(slaph_plan const *plan, int single_block_pair);
   void prepare_trace_tc(DeviceSchedule &ds);
